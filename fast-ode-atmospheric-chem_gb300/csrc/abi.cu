@@ -34,6 +34,7 @@ struct fo_plan {
   void* blob = nullptr;  // device copy of every table
   int device = -1;
   fo::GenModule* gen = nullptr;  // the generated variant's module (fo_plan_generate)
+  fo::ScratchLayout gen_layout{};  // the generated variant's scratch layout
   fo::GenOptions gen_options;    // its register tile and solve block (fo_plan_set_generation)
   fo_gen_info gen_info{};
   std::mutex gen_mutex;
@@ -198,6 +199,7 @@ int fo_plan_create(const fo_mechanism_desc* mech, int32_t ordering, fo_plan** ou
     return fail(FO_E_ALLOC, "host allocation failed");
   }
   const fo::HostTables& t = plan->host;
+  plan->gen_layout = fo::gen_layout_of(t).s;
   std::vector<char> buf;
   size_t o_perm = append(buf, t.perm), o_mass = append(buf, t.mass), o_react = append(buf, t.react),
          o_sptr = append(buf, t.s_ptr), o_srxn = append(buf, t.s_rxn), o_sval = append(buf, t.s_val),
@@ -375,6 +377,7 @@ int fill_params(const fo_plan* plan, const fo_options* opt, int32_t ngroups, con
   if (smem > (size_t)smem_max)
     return fail(FO_E_UNSUPPORTED, "species x group size exceed shared memory: use smaller groups");
   fo::SolveParams p = base_params(plan);
+  if (variant == FO_VARIANT_GENERATED) p.sl = plan->gen_layout;
   p.o.tab = kTableaus[opt->tableau];
   p.o.controller = opt->controller;
   p.o.b = opt->b;
@@ -729,6 +732,7 @@ int fo_adjoint_interval(const fo_plan* plan, const fo_options* opt, int32_t ngro
   } else if (a.p.o.variant == FO_VARIANT_COMPACT || a.p.o.variant == FO_VARIANT_GENERATED) {
     // the table-driven transposed solves need the whole vector on chip
     a.p.o.variant = plan->dev.elp ? FO_VARIANT_PIPELINED : FO_VARIANT_PLAIN;
+    a.p.sl = layout_of(plan->host);
     smem = smem_bytes(plan->host, a.p.lanes, a.p.o.variant);
   }
   a.p.slot_doubles = a.al.items * a.p.lanes;

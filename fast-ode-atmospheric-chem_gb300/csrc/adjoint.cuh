@@ -339,6 +339,7 @@ __device__ void adjoint_group(const AdjParams& a, double* w) {
   double* ys = scr + a.al.ys * L;
   double* U = scr + a.al.u * L;
   double* ybar = scr + a.al.ybar * L;
+  load_rate_constants(p, ln, scr);
   for (int i = 0; i < n; ++i) SCR(Y, i) = a.Ycp[ln.cell * a.ycs + (int64_t)__ldg(p.t.perm + i) * a.yss];
   // replay the projection's updates (constrained systems), keeping the state
   // before each

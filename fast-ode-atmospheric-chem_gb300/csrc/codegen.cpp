@@ -88,12 +88,31 @@ class Ptx {
     line("add.rn.f64 %%d%d, %%d%d, %%d%d;", r, a, b);
     return r;
   }
-  int constant(double v) {
+  int sub(int a, int b) {
     const int r = reg();
+    line("sub.rn.f64 %%d%d, %%d%d, %%d%d;", r, a, b);
+    return r;
+  }
+  // a * v and a * v + c with an immediate v
+  int mul_imm(int a, double v) {
+    const int r = reg();
+    line("mul.rn.f64 %%d%d, %%d%d, 0d%016llX;", r, a, bits_of(v));
+    return r;
+  }
+  int fma_imm(int a, double v, int c) {
+    const int r = reg();
+    line("fma.rn.f64 %%d%d, %%d%d, 0d%016llX, %%d%d;", r, a, bits_of(v), c);
+    return r;
+  }
+  static unsigned long long bits_of(double v) {
     unsigned long long bits;
     static_assert(sizeof(bits) == sizeof(v), "");
     std::memcpy(&bits, &v, sizeof(v));
-    line("mov.f64 %%d%d, 0d%016llX;", r, bits);
+    return bits;
+  }
+  int constant(double v) {
+    const int r = reg();
+    line("mov.f64 %%d%d, 0d%016llX;", r, bits_of(v));
     return r;
   }
   int recip(int x) {
@@ -369,6 +388,96 @@ void emit_solve_t(Ptx& x, const HostTables& t, const ScratchLayout& sl, const Pa
   }
 }
 
+// Rates and forcing at the evaluation point (item yr): r_j = k_j * prod x,
+// then F_i = sum of S[i, j] r_j in ascending j, into item ft; the operations
+// of the table-driven loops in their order (a leading 0 or 1 and products
+// with +-1 are folded, which changes no value). Reactions and rows are
+// emitted in batches, a batch's loads before its arithmetic and stores, so
+// that one latency covers the batch. The table-driven loops were bound by one
+// dependent chain of loads per row and entry (TS1's attempts spent about 90%
+// of their time there): eight intervals of TS1 on 64 cells took 297 ms with
+// them and take 142 ms; one interval of 65,536 cells of the 210/500 mechanism
+// 140.6 ms and 128.3 ms.
+void emit_rhs(Ptx& x, const HostTables& t, const ScratchLayout& sl) {
+  constexpr int kBatch = 8;
+  for (int j0 = 0; j0 < t.R; j0 += kBatch) {
+    const int j1 = std::min(t.R, j0 + kBatch);
+    std::vector<std::vector<int>> v(j1 - j0);
+    for (int j = j0; j < j1; ++j) {
+      v[j - j0].push_back(x.load(sl.kc + j));
+      for (int q = 0; q < t.P; ++q)
+        if (t.react[(size_t)j * t.P + q] != t.n) v[j - j0].push_back(x.load(sl.yr + t.react[(size_t)j * t.P + q]));
+    }
+    for (int j = j0; j < j1; ++j) {
+      const std::vector<int>& f = v[j - j0];
+      int r = f[0];
+      if (f.size() > 1) {
+        int prod = f[1];
+        for (size_t q = 2; q < f.size(); ++q) prod = x.mul(prod, f[q]);
+        r = x.mul(f[0], prod);
+      }
+      x.store(sl.r + j, r);
+    }
+  }
+  for (int i = 0; i < t.n; ++i) {
+    int acc = -1;
+    for (int q = t.s_ptr[i]; q < t.s_ptr[i + 1]; ++q) {
+      const int r = x.load(sl.r + t.s_rxn[q]);
+      const double c = t.s_val[q];
+      if (acc < 0) acc = c == 1.0 ? r : c == -1.0 ? x.neg(r) : x.mul_imm(r, c);
+      else acc = c == 1.0 ? x.add(acc, r) : c == -1.0 ? x.sub(acc, r) : x.fma_imm(r, c, acc);
+    }
+    x.store(sl.ft + i, acc < 0 ? x.constant(0.0) : acc);
+  }
+}
+
+// The negated Jacobian values at the evaluation point, in assembly order:
+// d[j, p] = k_j * prod of the other reactants, then the sums of -S[i, j] d
+// over each entry's terms.
+void emit_jac(Ptx& x, const HostTables& t, const GenLayout& gl) {
+  constexpr int kBatch = 8;
+  const ScratchLayout& sl = gl.s;
+  for (int j0 = 0; j0 < t.R; j0 += kBatch) {
+    const int j1 = std::min(t.R, j0 + kBatch);
+    struct One { int item, k; std::vector<int> x; };
+    std::vector<One> ones;
+    for (int j = j0; j < j1; ++j) {
+      int k = -1;
+      std::vector<int> f(t.P, -1);
+      for (int a = 0; a < t.P; ++a) {
+        const int item = gl.d_item[(size_t)j * t.P + a];
+        if (item < 0) continue;
+        One o{item, -1, {}};
+        if (k < 0) k = x.load(sl.kc + j);
+        o.k = k;
+        for (int q = 0; q < t.P; ++q) {
+          const int s = t.react[(size_t)j * t.P + q];
+          if (q == a || s == t.n) continue;
+          if (f[q] < 0) f[q] = x.load(sl.yr + s);
+          o.x.push_back(f[q]);
+        }
+        ones.push_back(std::move(o));
+      }
+    }
+    for (const One& o : ones) {
+      int d = o.k;
+      for (int f : o.x) d = x.mul(d, f);
+      x.store(o.item, d);
+    }
+  }
+  for (size_t e = 0; e + 1 < t.jt_ptr.size(); ++e) {
+    int acc = -1;
+    for (int q = t.jt_ptr[e]; q < t.jt_ptr[e + 1]; ++q) {
+      const int jp = t.jt_idx[q];
+      const int d = x.load(gl.d_item[jp] >= 0 ? gl.d_item[jp] : sl.kc + jp / t.P);
+      const double c = t.jt_val[q];
+      if (acc < 0) acc = c == 1.0 ? d : c == -1.0 ? x.neg(d) : x.mul_imm(d, c);
+      else acc = c == 1.0 ? x.add(acc, d) : c == -1.0 ? x.sub(acc, d) : x.add(acc, x.mul_imm(d, c));
+    }
+    x.store(sl.negj + (int64_t)e, acc < 0 ? x.constant(0.0) : acc);
+  }
+}
+
 // One function whose body dispatches on the mechanism index parameter %m
 // to the mechanism's code (`bodies[i]`, all numbered in one register space).
 std::string function(const char* name, const char* params, const Ptx& x, const std::vector<std::string>& bodies,
@@ -441,15 +550,16 @@ std::string generate_ptx(const std::vector<const HostTables*>& ts, const std::ve
     if (o.tile < 1 || o.tile > 16 || o.solve_block < 1 || o.solve_block > 64 || o.solve_keep < 0 ||
         o.piece_lines < 1)
       throw std::invalid_argument("generation options out of range");
-  Ptx s, st;
-  std::vector<std::string> sb, tb;
+  Ptx s, st, f, jv;
+  std::vector<std::string> sb, tb, fb, jb;
   // the factorization of mechanism m: pieces[m][k] = the k-th function
   std::vector<std::vector<Ptx>> pieces(ts.size());
   int64_t total = 0;
   for (size_t m = 0; m < ts.size(); ++m) {
     const HostTables* t = ts[m];
     const GenOptions& o = os[m];
-    const ScratchLayout sl = layout_of(*t);
+    const GenLayout gl = gen_layout_of(*t);
+    const ScratchLayout& sl = gl.s;
     const Pattern P = pattern_of(*t);
     // consecutive row blocks up to about o.piece_lines instructions each
     const int nb = (t->n + o.tile - 1) / o.tile;
@@ -477,6 +587,12 @@ std::string generate_ptx(const std::vector<const HostTables*>& ts, const std::ve
     emit_solve_t(st, *t, sl, P, o.solve_block);
     tb.push_back(std::move(st.body));
     st.body.clear();
+    emit_rhs(f, *t, sl);
+    fb.push_back(std::move(f.body));
+    f.body.clear();
+    emit_jac(jv, *t, gl);
+    jb.push_back(std::move(jv.body));
+    jv.body.clear();
   }
   if (fma_count) *fma_count = total;
   std::string out = ".version 9.0\n.target sm_103a\n.address_size 64\n\n";
@@ -488,6 +604,14 @@ std::string generate_ptx(const std::vector<const HostTables*>& ts, const std::ve
   out += "\n";
   out += function("fo_gen_solve_t", ".param .b64 fo_gen_solve_t_base, .param .b32 fo_gen_solve_t_mech", st, tb,
                   "\tld.param.b64 %p, [fo_gen_solve_t_base];\n\tld.param.b32 %m, [fo_gen_solve_t_mech];\n"
+                  "\tcvta.to.global.u64 %b, %p;\n");
+  out += "\n";
+  out += function("fo_gen_rhs", ".param .b64 fo_gen_rhs_base, .param .b32 fo_gen_rhs_mech", f, fb,
+                  "\tld.param.b64 %p, [fo_gen_rhs_base];\n\tld.param.b32 %m, [fo_gen_rhs_mech];\n"
+                  "\tcvta.to.global.u64 %b, %p;\n");
+  out += "\n";
+  out += function("fo_gen_jac", ".param .b64 fo_gen_jac_base, .param .b32 fo_gen_jac_mech", jv, jb,
+                  "\tld.param.b64 %p, [fo_gen_jac_base];\n\tld.param.b32 %m, [fo_gen_jac_mech];\n"
                   "\tcvta.to.global.u64 %b, %p;\n");
   return out;
 }

@@ -81,6 +81,7 @@ struct DevOptions {
 struct ScratchLayout {
   int64_t lu, negj, d, r, y, ynew, f0, ft, yr, k;  // offsets
   int64_t xs;                                      // the generated solves' vector (n items)
+  int64_t kc;                                      // the generated evaluations' rate constants (R items)
   int64_t items;                                   // total items per lane
 };
 

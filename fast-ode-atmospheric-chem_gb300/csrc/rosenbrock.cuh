@@ -21,6 +21,10 @@
 // `mech` the mechanism's index in the module (several mechanisms share one).
 extern "C" __device__ void fo_gen_factor(double* base, double alpha, int mech);
 extern "C" __device__ void fo_gen_solve(double* base, int mech);
+// forcing and negated Jacobian values at the point in item yr (rates and
+// constants in kc), the forcing into item ft
+extern "C" __device__ void fo_gen_rhs(double* base, int mech);
+extern "C" __device__ void fo_gen_jac(double* base, int mech);
 extern "C" __device__ void fo_gen_solve_t(double* base, int mech);   // the adjoint's transposed solve
 #endif
 
@@ -101,9 +105,56 @@ __device__ void eval_forcing(const SolveParams& p, const Lane& ln, const double*
   }
 }
 
+// v = u for a per-lane vector of n items, kBatch loads in flight.
+__device__ __forceinline__ void copy_items(const Lane& ln, int n, const double* u, double* v) {
+  constexpr int kBatch = 8;
+  const int L = ln.L, lane = ln.lane;
+  for (int i = 0; i < n; i += kBatch) {
+    double b[kBatch];
+#pragma unroll
+    for (int q = 0; q < kBatch; ++q)
+      if (i + q < n) b[q] = SCR(u, i + q);
+#pragma unroll
+    for (int q = 0; q < kBatch; ++q)
+      if (i + q < n) SCR(v, i + q) = b[q];
+  }
+}
+
+// What the generated evaluations keep for a group's interval: its rate
+// constants in the slot (item kc).
+__device__ __forceinline__ void load_rate_constants(const SolveParams& p, const Lane& ln, double* scr) {
+#ifdef FO_LINK_GENERATED
+  constexpr int kBatch = 8;
+  const int L = ln.L, lane = ln.lane;
+  const double* __restrict__ kc = p.k + ln.cell * p.kcs;
+  double* out = scr + p.sl.kc * L;
+  for (int j = 0; j < p.t.R; j += kBatch) {
+    double b[kBatch];
+#pragma unroll
+    for (int q = 0; q < kBatch; ++q)
+      if (j + q < p.t.R) b[q] = __ldg(kc + (int64_t)(j + q) * p.krs);
+#pragma unroll
+    for (int q = 0; q < kBatch; ++q)
+      if (j + q < p.t.R) SCR(out, j + q) = b[q];
+  }
+#endif
+}
+
+// F(x) into f. The generated form evaluates at the slot's point yr (x is
+// copied there) and leaves the point for eval_negjac, which follows at the
+// same x wherever it is called.
 __device__ __noinline__ void eval_rhs(const SolveParams& p, const Lane& ln, const double* x, double* r, double* f) {
+#ifdef FO_LINK_GENERATED
+  double* base = r - p.sl.r * ln.L;
+  double* yr = base + p.sl.yr * ln.L;
+  double* ft = base + p.sl.ft * ln.L;
+  if (x != yr) copy_items(ln, p.t.n, x, yr);
+  fo_gen_rhs(base + ln.lane, p.o.gen_index);
+  if (f != ft) copy_items(ln, p.t.n, ft, f);
+#else
   eval_rates(p, ln, x, r);
   eval_forcing(p, ln, r, f);
+#endif
 }
 
 // Negated Jacobian values in assembly order: d[j,p] = k_j prod_{q != p} x_q,
@@ -111,6 +162,9 @@ __device__ __noinline__ void eval_rhs(const SolveParams& p, const Lane& ln, cons
 // (fastode/chem.py:92-102).
 __device__ __noinline__ void eval_negjac(const SolveParams& p, const Lane& ln, const double* __restrict__ x,
                                          double* __restrict__ d, double* __restrict__ negj) {
+#ifdef FO_LINK_GENERATED
+  fo_gen_jac(negj - p.sl.negj * ln.L + ln.lane, p.o.gen_index);
+#else
   constexpr int kBatch = 8;
   const int L = ln.L, lane = ln.lane;
   const int n = p.t.n, R = p.t.R, P = p.t.P;
@@ -142,6 +196,7 @@ __device__ __noinline__ void eval_negjac(const SolveParams& p, const Lane& ln, c
     for (; t < t1; ++t) acc = __dadd_rn(acc, __dmul_rn(__ldg(p.t.jt_val + t), SCR(d, __ldg(p.t.jt_idx + t))));
     SCR(negj, e) = acc;
   }
+#endif
 }
 
 // Row r of the stage matrix alpha*M - J scattered into the dense work row w
@@ -936,6 +991,7 @@ __device__ __noinline__ void solve_group_restarting(const SolveParams& p, int g,
   double* dd = scr + p.sl.d * L;
   double* rr = scr + p.sl.r * L;
   double* lu = scr + p.sl.lu * L;
+  load_rate_constants(p, ln, scr);
   for (int i = 0; i < n; ++i) SCR(Y, i) = p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss];
   const double rounding = 2.220446049250313e-16;
   const double h_min = __dmul_rn(1.0e-15, dt);
@@ -1060,6 +1116,7 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
   double* rr = scr + p.sl.r * L;
   double* lu = scr + p.sl.lu * L;
   const bool in_place = solves_in_place(p);   // Newton update solved in place in F
+  load_rate_constants(p, ln, scr);
   for (int i = 0; i < n; ++i) {
     const double v = p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss];
     SCR(Yn, i) = v;
@@ -1275,6 +1332,7 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
   double* rr = scr + p.sl.r * L;
   double* lu = scr + p.sl.lu * L;
 
+  load_rate_constants(p, ln, scr);
   for (int i = 0; i < n; ++i) SCR(Y, i) = p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss];
 
   double* mem = p.memory + (int64_t)g * 3;
