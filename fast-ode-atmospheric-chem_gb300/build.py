@@ -20,7 +20,7 @@ CSRC = PKG / "csrc"
 LIBDIR = PKG / "_lib"
 LIBNAME = "libfastode_gb300.so"
 SOURCES = ["integrator.cu", "adjoint.cu", "abi.cu", "utility.cu", "scoring.cu", "static_scratch.cu", "symbolic.cpp",
-           "codegen.cpp", "jit.cpp", "embed.cpp"]
+           "layout.cpp", "codegen.cpp", "jit.cpp", "embed.cpp"]
 # the integrator of the generated variant, compiled as relocatable device code
 # and embedded in the library (embed.cpp), where each plan links it with its
 # mechanism's generated code

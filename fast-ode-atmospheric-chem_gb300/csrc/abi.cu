@@ -199,7 +199,13 @@ int fo_plan_create(const fo_mechanism_desc* mech, int32_t ordering, fo_plan** ou
     return fail(FO_E_ALLOC, "host allocation failed");
   }
   const fo::HostTables& t = plan->host;
-  plan->gen_layout = fo::gen_layout_of(t).s;
+  try {
+    plan->gen_layout = fo::gen_layout_of(t).s;
+  } catch (const std::exception& e) {
+    const std::string what = e.what();
+    delete plan;
+    return fail(FO_E_ALLOC, what);
+  }
   std::vector<char> buf;
   size_t o_perm = append(buf, t.perm), o_mass = append(buf, t.mass), o_react = append(buf, t.react),
          o_sptr = append(buf, t.s_ptr), o_srxn = append(buf, t.s_rxn), o_sval = append(buf, t.s_val),
@@ -364,10 +370,9 @@ int fill_params(const fo_plan* plan, const fo_options* opt, int32_t ngroups, con
   if (!(dt > 0.0)) return fail(FO_E_INVALID, "dt must be positive");
   if (opt->max_steps < 0) return fail(FO_E_INVALID, "max_steps must be non-negative");
   const int lanes = lanes_for(max_group_cells);
-  // the generated variant keeps nothing on chip but the reduction buffer,
-  // plus the projection's dense work row for a constrained mechanism
+  // the generated variant keeps nothing on chip but the reduction buffer
   const size_t smem = variant == FO_VARIANT_GENERATED
-                          ? sizeof(double) * (32 + (plan->dev.has_constraints ? (size_t)plan->host.n * lanes : 0))
+                          ? sizeof(double) * 32
                           : smem_bytes(plan->host, lanes, variant);
   int dev = 0, smem_max = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -726,9 +731,7 @@ int fo_adjoint_interval(const fo_plan* plan, const fo_options* opt, int32_t ngro
   a.al = adjoint_layout(plan->host, max_steps);
   const bool generated = a.p.o.variant == FO_VARIANT_GENERATED && plan->gen != nullptr;
   if (generated) {
-    // the generated adjoint keeps nothing else on chip but the projection's
-    // dense work row (constrained mechanisms)
-    smem = sizeof(double) * (32 + (plan->dev.has_constraints ? (size_t)plan->host.n * a.p.lanes : 0));
+    smem = sizeof(double) * 32;
   } else if (a.p.o.variant == FO_VARIANT_COMPACT || a.p.o.variant == FO_VARIANT_GENERATED) {
     // the table-driven transposed solves need the whole vector on chip
     a.p.o.variant = plan->dev.elp ? FO_VARIANT_PIPELINED : FO_VARIANT_PLAIN;

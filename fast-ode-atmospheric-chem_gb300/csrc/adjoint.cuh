@@ -197,7 +197,7 @@ __device__ __noinline__ void reverse_step(const AdjParams& a, const Lane& ln, do
     // the generated transposed solve works on the slot's solve vector
     double* muv = scr + p.sl.xs * L;
     for (int i = 0; i < n; ++i) SCR(muv, i) = SCR(Kbar + (int64_t)r * n * L, i);
-    fo_gen_solve_t(scr + lane, p.o.gen_index);                           // mu_r
+    fo_gen_solve_t(scr + lane, TEAM_W, TEAM_N, p.o.gen_index);           // mu_r
 #else
     double* muv = w;
     for (int i = 0; i < n; ++i) WROW(i) = SCR(Kbar + (int64_t)r * n * L, i);
@@ -239,7 +239,8 @@ __device__ __noinline__ void reverse_step(const AdjParams& a, const Lane& ln, do
   hvp_jacobian(a, ln, y, jbar, dbar, ybar);
 }
 
-// x = A^-T b with the factors in lu (b and x per-lane vectors; may alias).
+// x = A^-T b with the projection's factors in lu (b and x per-lane vectors;
+// may alias).
 __device__ void solve_transposed_into(const SolveParams& p, const Lane& ln, const double* lu, double* scr, double* w,
                                       const double* b, double* x) {
   const int L = ln.L, lane = ln.lane;
@@ -247,7 +248,7 @@ __device__ void solve_transposed_into(const SolveParams& p, const Lane& ln, cons
 #ifdef FO_LINK_GENERATED
   double* v = scr + p.sl.xs * L;
   for (int i = 0; i < n; ++i) SCR(v, i) = SCR(b, i);
-  fo_gen_solve_t(scr + lane, p.o.gen_index);
+  fo_gen_solve_tp(scr + lane, TEAM_W, TEAM_N, p.o.gen_index);
   for (int i = 0; i < n; ++i) SCR(x, i) = SCR(v, i);
 #else
   for (int i = 0; i < n; ++i) WROW(i) = SCR(b, i);
@@ -269,7 +270,7 @@ __device__ void projection_delta(const AdjParams& a, const Lane& ln, const doubl
   alg_residual(p, ln, y, scr + p.sl.r * L, G);
   eval_negjac(p, ln, y, scr + p.sl.d * L, negj);
   factor_any(p, ln, 1.0, negj, lu, w, true);
-  solve_into(p, ln, lu, w, G, delta);
+  solve_into(p, ln, lu, w, G, delta, true);
 }
 
 // The reverse sweep of one projection update y' = y + s delta(y) (algebraic

@@ -1,4 +1,5 @@
-// Straight-line PTX for one mechanism's factorization and triangular solves.
+// Straight-line PTX for one mechanism's evaluations, factorization and
+// triangular solves, shared among the warps of a group's team.
 //
 // Why straight-line code. The table-driven kernels (rosenbrock.cuh) spend
 // about 40 integer, address and control instructions around every FP64
@@ -7,36 +8,45 @@
 // the instruction stream is the arithmetic itself: one DFMA per update plus
 // its share of the operand loads.
 //
-// The factorization: row blocks of `tile` rows, each cut into column tiles of
-// `tile` columns, processed left to right (L tiles, the diagonal tile, U
-// tiles). A tile's entries live in registers from assembly to store; every
-// pivot k that updates the tile contributes the outer product of its
-// multipliers l(i, k) (rows of the tile) and its U row u(k, j) (columns of
-// the tile), loaded once per tile: 2t loads for up to t^2 independent FMAs.
-// Pivots inside the tile follow in ascending order. Each entry therefore
-// receives exactly the updates of the row-by-row elimination, in ascending
-// pivot order, with the same operations (fma(-l, u, a); l = a * (1 / pivot);
-// 1 / pivot by an IEEE division), so the factors are those of every other
-// variant bit for bit. Only structurally nonzero products are emitted: the
-// fill pattern's closure (l(i,k) != 0 and u(k,j) != 0 imply (i,j) in the
-// pattern) makes each pivot's contribution to a tile a full rectangle.
+// Why teams. A group is one warp's 32 lanes wide, and one warp issues a DFMA
+// every 64 cycles on its SM sub-partition whatever the rest of the chip does,
+// so a launch of few groups leaves most of the FP64 units idle. A group is
+// therefore worked on by a team of 1 to 16 warps (a block), every warp holding
+// the same 32 cells: the generated work is cut into tasks (a row, a block of
+// rows by columns, a range of reactions), the tasks are scheduled into steps
+// of kSegments segments that depend on earlier steps only, and warp w of W
+// runs segments w, w + W, ... of a step before the team's barrier. One module
+// serves every team size, and since a task is run by one warp with one order
+// of operations, results do not depend on the team size.
 //
-// The solves: blocks of `solve_block` rows; each row sums its terms in
-// ascending column order, as the plain variant's loops do, so results match
-// that variant bit for bit. In the forward solve a solution value used by
-// several rows of a block is loaded once for the block; in the backward
-// solve the `solve_keep` values of later blocks used by most rows stay in
-// registers for the block and the rest are loaded at each use (holding all of
-// them made the register allocator spill about 47 KB per solve to local
-// memory, which missed every cache). The transposed solve of the adjoint follows
-// the same pattern with rows and columns exchanged.
+// The factorization: the leading rows are single-row tasks (their elimination
+// DAG gives the parallelism); the rows of the trailing dense square are
+// blocks of `tile` rows whose multipliers of the leading pivots are one task
+// and whose columns in the square are tiles of `tile` columns, one task each:
+// a tile's entries live in registers from assembly to store, and every pivot
+// contributes the outer product of its multipliers and its U row, loaded once
+// per tile (2t loads for up to t^2 independent FMAs). Only structurally
+// nonzero products are emitted. The dense square itself is eliminated by a
+// loop over its blocks (dense_lu in rosenbrock.cuh), a few kilobytes of code
+// for about 60% of the multiply-adds. Every entry receives the updates of the
+// row-by-row elimination in ascending pivot order with the same operations
+// (fma(-l, u, a); l = a * (1 / pivot); 1 / pivot by an IEEE division), so the
+// factors are those of every other variant bit for bit.
+//
+// The solves: leading rows are single-row tasks; rows of the square are blocks
+// of `solve_block` rows, each updated by one finished block at a time. Every
+// row sums its terms in the order in which their values finish (ascending
+// columns forward, descending columns backward), as the plain variant's loops
+// do, so results match that variant bit for bit.
 #include "codegen.h"
 
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <stdexcept>
+#include <utility>
 #include <vector>
 
 #include "layout.h"
@@ -47,7 +57,8 @@ namespace {
 class Ptx {
  public:
   std::string body;
-  int next = 1;  // %d0 is alpha
+  int next = 1;      // %d0 is alpha
+  int64_t fmas = 0;  // updates of a factorization emitted
 
   int reg() { return next++; }
 
@@ -122,286 +133,441 @@ class Ptx {
   }
 };
 
-// Dense map of the LU storage: position of (i, j), or -1.
-struct Pattern {
-  int n;
-  std::vector<int32_t> pos;
-  int32_t at(int i, int j) const { return pos[(size_t)i * n + j]; }
+using Emit = std::function<void(Ptx&)>;
+// One phase: steps[s][g] is what segment g of step s does.
+using Phase = std::vector<std::vector<std::vector<Emit>>>;
+
+// One unit of generated work: `after` lists the tasks it reads from.
+struct Task {
+  std::vector<int> after;
+  Emit emit;
 };
 
-Pattern pattern_of(const HostTables& t) {
-  Pattern P;
-  P.n = t.n;
-  P.pos.assign((size_t)t.n * t.n, -1);
-  for (int i = 0; i < t.n; ++i)
-    for (int q = t.lu_row_ptr[i]; q < t.lu_row_ptr[i + 1]; ++q) P.pos[(size_t)i * t.n + t.lu_col[q]] = q;
-  return P;
+// Cost of a task in units of one multiply-add: operand loads and stores take
+// about a quarter of a DFMA's issue time, a division nine.
+int64_t cost_of(const Task& t) {
+  Ptx x;
+  t.emit(x);
+  int64_t c = 0;
+  for (size_t at = 0; at < x.body.size(); at = x.body.find('\n', at) + 1) {
+    const char* l = x.body.c_str() + at + 1;
+    c += !std::strncmp(l, "ld", 2) || !std::strncmp(l, "st", 2) ? 1 : !std::strncmp(l, "div", 3) ? 36
+         : !std::strncmp(l, "neg", 3) || !std::strncmp(l, "mov", 3) ? 0 : 4;
+  }
+  return c / 4 + 1;
 }
 
-// Row blocks [ib_begin, ib_end) of the factorization. A row block reads the
-// entries earlier blocks stored and keeps nothing in registers past its end,
-// so consecutive ranges can be separate functions called one after another.
-void emit_factor(Ptx& x, const HostTables& t, const ScratchLayout& sl, const Pattern& P, int b, int ib_begin,
-                 int ib_end, int64_t* nfma) {
-  const int n = t.n;
-  // Jacobian entry (assembly order) stored at each LU position, or -1
-  std::vector<int32_t> jac_at(t.lu_col.size(), -1);
-  for (size_t e = 0; e < t.j_lu_pos.size(); ++e) jac_at[t.j_lu_pos[e]] = (int32_t)e;
-  const int nb = (n + b - 1) / b;
-  std::vector<int> a((size_t)b * b);
-  auto A = [&](int i, int j, int i0, int j0) -> int& { return a[(size_t)(i - i0) * b + (j - j0)]; };
-  for (int ib = std::max(0, ib_begin); ib < std::min(nb, ib_end); ++ib) {
-    const int i0 = ib * b, i1 = std::min(n, i0 + b);
-    for (int jb = 0; jb < nb; ++jb) {
-      const int j0 = jb * b, j1 = std::min(n, j0 + b);
-      bool any = false;
-      for (int i = i0; i < i1 && !any; ++i)
-        for (int j = j0; j < j1; ++j)
-          if (P.at(i, j) >= 0) { any = true; break; }
-      if (!any) continue;
-      // assembly: -J (or 0 on fill) plus alpha * mass on the diagonal
-      for (int i = i0; i < i1; ++i)
-        for (int j = j0; j < j1; ++j) {
-          const int q = P.at(i, j);
-          if (q < 0) continue;
-          int v = jac_at[q] >= 0 ? x.load(sl.negj + jac_at[q]) : x.constant(0.0);
-          if (i == j) {
-            const double m = t.mass[i];
-            // alpha * 1 is alpha exactly; any other mass takes the product
-            v = x.add(v, m == 1.0 ? 0 : x.mul(0, x.constant(m)));
+// Tasks into steps of kSegments segments. A step takes every task whose
+// inputs are ready, longest first onto the least loaded segment; a task whose
+// last inputs are made in one segment of the step follows them there when
+// that does not lengthen the step (a short step is lengthened: a barrier and
+// the first loads of a step cost about kStepCost), or when it is the only
+// task left to run.
+Phase schedule(const std::vector<Task>& tasks) {
+  constexpr int64_t kStepCost = 48;
+  const int n = (int)tasks.size();
+  std::vector<int64_t> cost(n);
+  std::vector<int> waits(n, 0), step(n, -1), segment(n, -1);
+  std::vector<std::vector<int>> before(n);
+  for (int i = 0; i < n; ++i) {
+    cost[i] = cost_of(tasks[i]);
+    waits[i] = (int)tasks[i].after.size();
+    for (int a : tasks[i].after) before[a].push_back(i);
+  }
+  std::vector<int> ready;
+  for (int i = 0; i < n; ++i)
+    if (!waits[i]) ready.push_back(i);
+  Phase out;
+  for (int s = 0, done = 0; done < n; ++s) {
+    if (ready.empty()) throw std::logic_error("cyclic tasks");
+    std::stable_sort(ready.begin(), ready.end(), [&](int a, int b) { return cost[a] > cost[b]; });
+    std::vector<std::vector<int>> seg(kSegments);
+    std::vector<int64_t> load(kSegments, 0);
+    std::vector<int> placed, next;
+    auto place = [&](int i, int g) {
+      seg[g].push_back(i);
+      load[g] += cost[i];
+      step[i] = s;
+      segment[i] = g;
+      placed.push_back(i);
+      ++done;
+    };
+    for (int i : ready) place(i, (int)(std::min_element(load.begin(), load.end()) - load.begin()));
+    const bool serial = placed.size() < 3;
+    const int64_t limit = std::max(*std::max_element(load.begin(), load.end()), kStepCost);
+    for (size_t q = 0; q < placed.size(); ++q) {
+      std::vector<int> made;
+      for (int i : before[placed[q]])
+        if (!--waits[i]) made.push_back(i);
+      for (int i : made) {
+        // in this step if its inputs of this step share a segment
+        int g = -1;
+        bool one = true;
+        for (int a : tasks[i].after)
+          if (step[a] == s) {
+            if (g >= 0 && segment[a] != g) one = false;
+            g = segment[a];
           }
-          A(i, j, i0, j0) = v;
-        }
-      // pivots left of the tile (and above it): outer products
-      const int kmax = std::min(i0, j0);
-      std::vector<int> rows, cols, nl(b), u(b);
-      for (int k = 0; k < kmax; ++k) {
-        rows.clear();
-        cols.clear();
-        for (int i = i0; i < i1; ++i)
-          if (P.at(i, k) >= 0) rows.push_back(i);
-        if (rows.empty()) continue;
-        for (int j = j0; j < j1; ++j)
-          if (P.at(k, j) >= 0) cols.push_back(j);
-        if (cols.empty()) continue;
-        for (int i : rows) nl[i - i0] = x.neg(x.load(sl.lu + P.at(i, k)));
-        for (int j : cols) u[j - j0] = x.load(sl.lu + P.at(k, j));
-        for (int i : rows)
-          for (int j : cols) {
-            if (P.at(i, j) < 0) throw std::logic_error("fill pattern not closed");
-            int& r = A(i, j, i0, j0);
-            r = x.fma(nl[i - i0], u[j - j0], r);
-            ++*nfma;
-          }
-      }
-      if (jb < ib) {
-        // an L tile: the multipliers of pivots j0..j1-1, then their updates
-        // inside the tile
-        for (int k = j0; k < j1; ++k) {
-          rows.clear();
-          for (int i = i0; i < i1; ++i)
-            if (P.at(i, k) >= 0) rows.push_back(i);
-          if (rows.empty()) continue;
-          const int rk = x.load(sl.lu + P.at(k, k));
-          for (int i : rows) {
-            int& l = A(i, k, i0, j0);
-            l = x.mul(l, rk);
-            x.store(sl.lu + P.at(i, k), l);
-            nl[i - i0] = x.neg(l);
-          }
-          for (int j = k + 1; j < j1; ++j) {
-            if (P.at(k, j) < 0) continue;
-            const int uu = x.load(sl.lu + P.at(k, j));
-            for (int i : rows) {
-              int& r = A(i, j, i0, j0);
-              r = x.fma(nl[i - i0], uu, r);
-              ++*nfma;
-            }
-          }
-        }
-      } else if (jb == ib) {
-        // the diagonal tile: dense elimination inside it
-        for (int k = i0; k < i1; ++k) {
-          const int rk = x.recip(A(k, k, i0, j0));
-          x.store(sl.lu + P.at(k, k), rk);
-          for (int j = k + 1; j < i1; ++j)
-            if (P.at(k, j) >= 0) x.store(sl.lu + P.at(k, j), A(k, j, i0, j0));
-          for (int i = k + 1; i < i1; ++i) {
-            if (P.at(i, k) < 0) continue;
-            int& l = A(i, k, i0, j0);
-            l = x.mul(l, rk);
-            x.store(sl.lu + P.at(i, k), l);
-            const int nli = x.neg(l);
-            for (int j = k + 1; j < i1; ++j) {
-              if (P.at(k, j) < 0) continue;
-              int& r = A(i, j, i0, j0);
-              r = x.fma(nli, A(k, j, i0, j0), r);
-              ++*nfma;
-            }
-          }
-        }
-      } else {
-        // a U tile: rows of the block finish in order and update the rows
-        // below them (multipliers from the diagonal tile)
-        for (int k = i0; k < i1; ++k) {
-          cols.clear();
-          for (int j = j0; j < j1; ++j)
-            if (P.at(k, j) >= 0) {
-              cols.push_back(j);
-              x.store(sl.lu + P.at(k, j), A(k, j, i0, j0));
-            }
-          if (cols.empty()) continue;
-          for (int i = k + 1; i < i1; ++i) {
-            if (P.at(i, k) < 0) continue;
-            const int nli = x.neg(x.load(sl.lu + P.at(i, k)));
-            for (int j : cols) {
-              int& r = A(i, j, i0, j0);
-              r = x.fma(nli, A(k, j, i0, j0), r);
-              ++*nfma;
-            }
-          }
-        }
+        const bool alone = serial && made.size() == 1 && next.empty() && q + 1 == placed.size();
+        if (one && (alone || load[g] + cost[i] <= limit)) place(i, g);
+        else next.push_back(i);
       }
     }
+    ready = std::move(next);
+    out.emplace_back(kSegments);
+    for (int g = 0; g < kSegments; ++g)
+      for (int i : seg[g]) out.back()[g].push_back(tasks[i].emit);
+    while (!out.back().empty() && out.back().back().empty()) out.back().pop_back();
+  }
+  return out;
+}
+
+// A matrix to factor: its filled pattern, where its entries live, and what
+// they start from.
+struct Matrix {
+  int n = 0, d0 = 0;              // rows from d0 on form the dense square
+  std::vector<int64_t> item;      // n*n: item of (i, j), or -1
+  std::vector<int64_t> start;     // n*n: item of -J(i, j), or -1 (zero)
+  std::vector<double> mass;       // the diagonal gains alpha * mass
+  std::vector<char> unit;         // rows that are those of the identity
+  int64_t at(int i, int j) const { return item[(size_t)i * n + j]; }
+};
+
+Matrix full_matrix(const HostTables& t, const GenLayout& gl) {
+  Matrix A;
+  A.n = t.n;
+  A.d0 = gl.d0;
+  A.item.assign((size_t)t.n * t.n, -1);
+  A.start.assign((size_t)t.n * t.n, -1);
+  A.unit.assign(t.n, 0);
+  A.mass = t.mass;
+  for (int i = 0; i < t.n; ++i)
+    for (int q = t.lu_row_ptr[i]; q < t.lu_row_ptr[i + 1]; ++q) A.item[(size_t)i * t.n + t.lu_col[q]] = gl.lu_item[q];
+  for (int i = 0; i < t.n; ++i)
+    for (int e = t.j_row_ptr[i]; e < t.j_row_ptr[i + 1]; ++e) A.start[(size_t)i * t.n + t.j_col[e]] = gl.s.negj + e;
+  return A;
+}
+
+// The projection's matrix diag(M) - J with the differential rows of J
+// dropped (alpha = 1): only the algebraic rows have entries off the diagonal,
+// so its factors are a small part of the full pattern's, in the same storage.
+Matrix projection_matrix(const HostTables& t, const GenLayout& gl) {
+  Matrix A;
+  A.n = A.d0 = t.n;
+  A.item.assign((size_t)t.n * t.n, -1);
+  A.start.assign((size_t)t.n * t.n, -1);
+  A.unit.assign(t.n, 0);
+  A.mass = t.mass;
+  std::vector<char> in((size_t)t.n * t.n, 0);
+  for (int i = 0; i < t.n; ++i) {
+    in[(size_t)i * t.n + i] = 1;
+    A.unit[i] = t.mass[i] == 1.0;
+    if (t.mass[i] != 0.0) continue;
+    for (int e = t.j_row_ptr[i]; e < t.j_row_ptr[i + 1]; ++e) {
+      in[(size_t)i * t.n + t.j_col[e]] = 1;
+      A.start[(size_t)i * t.n + t.j_col[e]] = gl.s.negj + e;
+    }
+  }
+  for (int k = 0; k < t.n; ++k)
+    for (int i = k + 1; i < t.n; ++i)
+      if (in[(size_t)i * t.n + k])
+        for (int j = k + 1; j < t.n; ++j)
+          if (in[(size_t)k * t.n + j]) in[(size_t)i * t.n + j] = 1;
+  int64_t o = gl.s.lu;
+  for (size_t q = 0; q < in.size(); ++q)
+    if (in[q]) A.item[q] = o++;
+  return A;
+}
+
+// The columns below `limit` of rows that do not eliminate one another (one
+// row, or rows whose columns below `limit` all lie left of them): assembly,
+// every pivot's updates in ascending order, the multipliers (in place, and of
+// one row the reciprocal pivot and its U entries), `width` columns at a time.
+void emit_rows(Ptx& x, const Matrix& A, const std::vector<int>& rows, int limit, int width) {
+  std::vector<int> cols;
+  for (int j = 0; j < limit; ++j)
+    for (int i : rows)
+      if (A.at(i, j) >= 0) {
+        cols.push_back(j);
+        break;
+      }
+  const int m = (int)rows.size();
+  for (size_t c0 = 0; c0 < cols.size(); c0 += width) {
+    const size_t c1 = std::min(cols.size(), c0 + width);
+    const int first = cols[c0], last = cols[c1 - 1];
+    std::vector<int> acc((size_t)m * (c1 - c0), -1), nl(m, -1);
+    auto at = [&](int r, size_t c) -> int& { return acc[(size_t)r * (c1 - c0) + (c - c0)]; };
+    for (int r = 0; r < m; ++r)
+      for (size_t c = c0; c < c1; ++c) {
+        const int i = rows[r], j = cols[c];
+        if (A.at(i, j) < 0) continue;
+        const int64_t from = A.start[(size_t)i * A.n + j];
+        int v = from >= 0 ? x.load(from) : x.constant(0.0);
+        // alpha * 1 is alpha exactly; any other mass takes the product
+        if (i == j) v = x.add(v, A.mass[i] == 1.0 ? 0 : x.mul_imm(0, A.mass[i]));
+        at(r, c) = v;
+      }
+    for (size_t ck = 0; ck < cols.size(); ++ck) {
+      const int k = cols[ck];
+      if (k >= rows[0] || k > last) break;
+      const bool here = k >= first;
+      std::vector<size_t> to;
+      for (size_t c = c0; c < c1; ++c)
+        if (cols[c] > k && A.at(k, cols[c]) >= 0) to.push_back(c);
+      if (!here && to.empty()) continue;
+      const int rk = here && !A.unit[k] ? x.load(A.at(k, k)) : -1;
+      for (int r = 0; r < m; ++r) {
+        nl[r] = -1;
+        if (A.at(rows[r], k) < 0) continue;
+        if (here) {
+          int& l = at(r, ck);
+          if (rk >= 0) l = x.mul(l, rk);   // else the pivot is 1
+          x.store(A.at(rows[r], k), l);
+          nl[r] = x.neg(l);
+        } else {
+          nl[r] = x.neg(x.load(A.at(rows[r], k)));
+        }
+      }
+      for (size_t c : to) {
+        const int u = x.load(A.at(k, cols[c]));
+        for (int r = 0; r < m; ++r)
+          if (nl[r] >= 0) {
+            if (at(r, c) < 0) throw std::logic_error("fill pattern not closed");
+            at(r, c) = x.fma(nl[r], u, at(r, c));
+            ++x.fmas;
+          }
+      }
+    }
+    for (int r = 0; r < m; ++r)
+      for (size_t c = c0; c < c1; ++c) {
+        if (at(r, c) < 0 || cols[c] < rows[r]) continue;
+        x.store(A.at(rows[r], cols[c]), cols[c] == rows[r] ? x.recip(at(r, c)) : at(r, c));
+      }
   }
 }
 
-void emit_solve(Ptx& x, const HostTables& t, const ScratchLayout& sl, const Pattern& P, int b, int keep) {
-  const int n = t.n;
-  const int nb = (n + b - 1) / b;
-  std::vector<int> xv(n, -1);   // registers of solution values finished in this block
-  // forward: x_r -= sum over k < r of L(r, k) x_k, ascending k
-  for (int ib = 0; ib < nb; ++ib) {
-    const int i0 = ib * b, i1 = std::min(n, i0 + b);
-    std::vector<int> acc(b);
-    for (int i = i0; i < i1; ++i) acc[i - i0] = x.load(sl.xs + i);
-    for (int k = 0; k < i0; ++k) {
+// A tile of the dense square before its own elimination: assembly (structural
+// zeros too) and the updates of the pivots before the square.
+void emit_tile(Ptx& x, const Matrix& A, const GenLayout& gl, int i0, int i1, int j0, int j1) {
+  const int b = j1 - j0;
+  std::vector<int> acc((size_t)(i1 - i0) * b), nl(i1 - i0);
+  for (int i = i0; i < i1; ++i)
+    for (int j = j0; j < j1; ++j) {
+      const int64_t from = A.start[(size_t)i * A.n + j];
+      int v = from >= 0 ? x.load(from) : x.constant(0.0);
+      if (i == j) v = x.add(v, A.mass[i] == 1.0 ? 0 : x.mul_imm(0, A.mass[i]));
+      acc[(size_t)(i - i0) * b + j - j0] = v;
+    }
+  for (int k = 0; k < A.d0; ++k) {
+    std::vector<int> rows, cols;
+    for (int i = i0; i < i1; ++i)
+      if (A.at(i, k) >= 0) rows.push_back(i);
+    for (int j = j0; j < j1; ++j)
+      if (A.at(k, j) >= 0) cols.push_back(j);
+    if (rows.empty() || cols.empty()) continue;
+    for (int i : rows) nl[i - i0] = x.neg(x.load(A.at(i, k)));
+    for (int j : cols) {
+      const int u = x.load(A.at(k, j));
+      for (int i : rows) {
+        if (A.at(i, j) < 0) throw std::logic_error("fill pattern not closed");
+        int& r = acc[(size_t)(i - i0) * b + j - j0];
+        r = x.fma(nl[i - i0], u, r);
+        ++x.fmas;
+      }
+    }
+  }
+  for (int i = i0; i < i1; ++i)
+    for (int j = j0; j < j1; ++j) x.store(gl.dense_item(i, j), acc[(size_t)(i - i0) * b + j - j0]);
+}
+
+// The factorization up to the dense square's own elimination.
+std::vector<Task> factor_tasks(const Matrix& A, const GenLayout& gl, int tile) {
+  constexpr int kRowWidth = 24;   // columns of a single row at a time
+  std::vector<Task> tasks;
+  std::vector<int> row_task(A.n, -1);
+  auto pivots = [&](const std::vector<int>& rows) {
+    std::vector<int> after;
+    for (int k = 0; k < std::min(A.d0, rows[0]); ++k)
+      for (int i : rows)
+        if (A.at(i, k) >= 0) {
+          if (row_task[k] >= 0) after.push_back(row_task[k]);
+          break;
+        }
+    return after;
+  };
+  for (int i = 0; i < A.d0; ++i) {
+    if (A.unit[i]) continue;
+    const std::vector<int> rows{i};
+    row_task[i] = (int)tasks.size();
+    tasks.push_back({pivots(rows), [&A, rows](Ptx& x) { emit_rows(x, A, rows, A.n, kRowWidth); }});
+  }
+  for (int i0 = A.d0; i0 < A.n; i0 += tile) {
+    const int i1 = std::min(A.n, i0 + tile);
+    std::vector<int> rows;
+    for (int i = i0; i < i1; ++i) rows.push_back(i);
+    std::vector<int> after = pivots(rows);
+    if (!after.empty()) {
+      const int mine = (int)tasks.size();
+      tasks.push_back({after, [&A, rows, tile](Ptx& x) { emit_rows(x, A, rows, A.d0, tile); }});
+      after = {mine};
+    }
+    for (int j0 = A.d0; j0 < A.n; j0 += tile) {
+      const int j1 = std::min(A.n, j0 + tile);
+      tasks.push_back({after, [&A, &gl, i0, i1, j0, j1](Ptx& x) { emit_tile(x, A, gl, i0, i1, j0, j1); }});
+    }
+  }
+  return tasks;
+}
+
+// One triangular solve in place on the solve vector (item xs): row r's value
+// is x_r minus the sum of entry(r, k) x_k over the rows k finished before it,
+// in that order, times the item scale(r) where that is not -1. Rows finish
+// in ascending order (`up`) or descending order.
+std::vector<Task> triangle_tasks(const Matrix& A, const ScratchLayout& sl, int block, bool up,
+                                 std::function<int64_t(int, int)> entry, std::function<int64_t(int)> scale) {
+  const int n = A.n, d0 = A.d0;
+  std::vector<Task> tasks;
+  std::vector<int> maker(n, -1);       // the task that finishes each row (none: it is never changed)
+  // rows [i0, i1) of the vector minus their terms in columns [k0, k1), then,
+  // when `finish`, the rows themselves in order
+  auto emit = [&sl, up, entry, scale](Ptx& x, int i0, int i1, int k0, int k1, bool finish) {
+    std::vector<int> acc(i1 - i0, -1);
+    auto sum = [&](int i, int64_t q, int xk) {
+      if (acc[i - i0] < 0) acc[i - i0] = x.load(sl.xs + i);
+      acc[i - i0] = x.fma(x.neg(x.load(q)), xk, acc[i - i0]);
+    };
+    for (int m = 0; m < k1 - k0; ++m) {
+      const int k = up ? k0 + m : k1 - 1 - m;
       int xk = -1;
       for (int i = i0; i < i1; ++i) {
-        const int q = P.at(i, k);
+        const int64_t q = entry(i, k);
         if (q < 0) continue;
         if (xk < 0) xk = x.load(sl.xs + k);
-        acc[i - i0] = x.fma(x.neg(x.load(sl.lu + q)), xk, acc[i - i0]);
+        sum(i, q, xk);
       }
     }
-    for (int i = i0; i < i1; ++i) {
-      for (int k = i0; k < i; ++k) {
-        const int q = P.at(i, k);
-        if (q >= 0) acc[i - i0] = x.fma(x.neg(x.load(sl.lu + q)), acc[k - i0], acc[i - i0]);
+    if (finish)
+      for (int m = 0; m < i1 - i0; ++m) {
+        const int k = up ? i0 + m : i1 - 1 - m;
+        if (acc[k - i0] < 0) acc[k - i0] = x.load(sl.xs + k);
+        if (scale(k) >= 0) acc[k - i0] = x.mul(acc[k - i0], x.load(scale(k)));
+        for (int i = up ? k + 1 : i0; i < (up ? i1 : k); ++i)
+          if (entry(i, k) >= 0) sum(i, entry(i, k), acc[k - i0]);
       }
-      x.store(sl.xs + i, acc[i - i0]);
-    }
-  }
-  // backward: x_r = (x_r - sum over j > r of U(r, j) x_j) / pivot, ascending j.
-  // A row's in-block terms come before its terms in later blocks, so the
-  // later blocks' values x_j cannot be summed ahead for the whole block; the
-  // `keep` values used by most rows of the block stay in registers from their
-  // first load to the end of the block, the others are loaded at each use
-  // (keeping every one would hold up to n values live and spill them).
-  for (int ib = nb - 1; ib >= 0; --ib) {
-    const int i0 = ib * b, i1 = std::min(n, i0 + b);
-    std::vector<int> uses(n, 0);
-    for (int r = i0; r < i1; ++r)
-      for (int q = t.lu_diag[r] + 1; q < t.lu_row_ptr[r + 1]; ++q)
-        if (t.lu_col[q] >= i1) ++uses[t.lu_col[q]];
-    std::vector<int> order;
-    for (int j = i1; j < n; ++j)
-      if (uses[j] > 1) order.push_back(j);
-    std::stable_sort(order.begin(), order.end(), [&](int u, int v) { return uses[u] > uses[v]; });
-    std::vector<char> kept(n, 0);
-    for (size_t m = 0; m < order.size() && (int)m < keep; ++m) kept[order[m]] = 1;
-    std::vector<int> ext(n, -1);
-    for (int r = i1 - 1; r >= i0; --r) {
-      int acc = x.load(sl.xs + r);
-      for (int q = t.lu_diag[r] + 1; q < t.lu_row_ptr[r + 1]; ++q) {
-        const int j = t.lu_col[q];
-        int xj;
-        if (j < i1) {
-          xj = xv[j];
-        } else if (kept[j]) {
-          if (ext[j] < 0) ext[j] = x.load(sl.xs + j);
-          xj = ext[j];
-        } else {
-          xj = x.load(sl.xs + j);
+    for (int i = i0; i < i1; ++i)
+      if (acc[i - i0] >= 0) x.store(sl.xs + i, acc[i - i0]);
+  };
+  auto terms = [&](int i0, int i1, int k0, int k1) {
+    std::vector<int> after;
+    bool any = false;
+    for (int k = k0; k < k1; ++k)
+      for (int i = i0; i < i1; ++i)
+        if (entry(i, k) >= 0) {
+          any = true;
+          if (maker[k] >= 0) after.push_back(maker[k]);
+          break;
         }
-        acc = x.fma(x.neg(x.load(sl.lu + q)), xj, acc);
-      }
-      xv[r] = x.mul(acc, x.load(sl.lu + t.lu_diag[r]));
-      x.store(sl.xs + r, xv[r]);
+    std::sort(after.begin(), after.end());
+    after.erase(std::unique(after.begin(), after.end()), after.end());
+    return std::make_pair(any, after);
+  };
+  auto leading = [&]() {
+    for (int m = 0; m < d0; ++m) {
+      const int i = up ? m : d0 - 1 - m;
+      const int k0 = up ? 0 : i + 1, k1 = up ? i : n;
+      auto [any, after] = terms(i, i + 1, k0, k1);
+      if (!any && scale(i) < 0) continue;
+      maker[i] = (int)tasks.size();
+      tasks.push_back({after, [=](Ptx& x) { emit(x, i, i + 1, k0, k1, true); }});
     }
-  }
+  };
+  auto square = [&]() {
+    const int nb = (n - d0 + block - 1) / block;
+    auto lo = [=](int b) { return d0 + b * block; };
+    auto hi = [=](int b) { return std::min(n, d0 + (b + 1) * block); };
+    std::vector<int> last(nb, -1);       // the latest task on each block's rows
+    for (int b = 0; b < nb && up; ++b) {  // the columns before the square
+      auto [any, after] = terms(lo(b), hi(b), 0, d0);
+      if (!any) continue;
+      last[b] = (int)tasks.size();
+      const int i0 = lo(b), i1 = hi(b);
+      tasks.push_back({after, [=](Ptx& x) { emit(x, i0, i1, 0, d0, false); }});
+    }
+    for (int m = 0; m < nb; ++m) {
+      const int b = up ? m : nb - 1 - m;
+      const int i0 = lo(b), i1 = hi(b);
+      std::vector<int> after;
+      if (last[b] >= 0) after.push_back(last[b]);
+      const int mine = (int)tasks.size();
+      tasks.push_back({after, [=](Ptx& x) { emit(x, i0, i1, i0, i0, true); }});
+      for (int i = i0; i < i1; ++i) maker[i] = mine;
+      for (int c = up ? b + 1 : 0; c < (up ? nb : b); ++c) {
+        auto [any, from] = terms(lo(c), hi(c), i0, i1);
+        if (!any) continue;
+        if (last[c] >= 0) from.push_back(last[c]);
+        last[c] = (int)tasks.size();
+        const int r0 = lo(c), r1 = hi(c);
+        tasks.push_back({from, [=](Ptx& x) { emit(x, r0, r1, i0, i1, false); }});
+      }
+    }
+  };
+  if (up) leading();
+  square();
+  if (!up) leading();
+  return tasks;
 }
 
-// The transposed solve A^T x = b in place on the solve vector, the gather
-// form of the adjoint's scatter loops (U^T z = b by rows ascending, then
-// L^T x = z by rows descending): entry c receives fma(-U(r, c), z_r, .) for
-// r ascending, then z_c = . * (1 / pivot_c); later fma(-L(r, c), x_r, .) for r
-// descending; the operations of the table-driven kernel in its order.
-void emit_solve_t(Ptx& x, const HostTables& t, const ScratchLayout& sl, const Pattern& P, int b) {
-  const int n = t.n;
-  const int nb = (n + b - 1) / b;
-  std::vector<int> xv(n, -1);
-  // U^T z = b, columns of U ascending
-  for (int ib = 0; ib < nb; ++ib) {
-    const int c0 = ib * b, c1 = std::min(n, c0 + b);
-    std::vector<int> acc(b);
-    for (int c = c0; c < c1; ++c) acc[c - c0] = x.load(sl.xs + c);
-    for (int r = 0; r < c0; ++r) {
-      int zr = -1;
-      for (int c = c0; c < c1; ++c) {
-        const int q = P.at(r, c);
-        if (q < 0) continue;
-        if (zr < 0) zr = x.load(sl.xs + r);
-        acc[c - c0] = x.fma(x.neg(x.load(sl.lu + q)), zr, acc[c - c0]);
-      }
-    }
-    for (int c = c0; c < c1; ++c) {
-      for (int r = c0; r < c; ++r) {
-        const int q = P.at(r, c);
-        if (q >= 0) acc[c - c0] = x.fma(x.neg(x.load(sl.lu + q)), xv[r], acc[c - c0]);
-      }
-      xv[c] = x.mul(acc[c - c0], x.load(sl.lu + P.at(c, c)));
-      x.store(sl.xs + c, xv[c]);
-    }
+// (LU)^-1: L by ascending rows, then U by descending rows and 1 / pivot.
+Phase solve_phase(const Matrix& A, const ScratchLayout& sl, int block) {
+  auto below = [&A](int i, int k) { return k < i ? A.at(i, k) : (int64_t)-1; };
+  auto above = [&A](int i, int k) { return k > i ? A.at(i, k) : (int64_t)-1; };
+  auto none = [](int) { return (int64_t)-1; };
+  auto pivot = [&A](int i) { return A.unit[i] ? (int64_t)-1 : A.at(i, i); };
+  Phase p = schedule(triangle_tasks(A, sl, block, true, below, none));
+  Phase q = schedule(triangle_tasks(A, sl, block, false, above, pivot));
+  p.insert(p.end(), q.begin(), q.end());
+  return p;
+}
+
+// (LU)^-T: U^T by ascending rows and 1 / pivot, then L^T by descending rows.
+Phase solve_t_phase(const Matrix& A, const ScratchLayout& sl, int block) {
+  auto below = [&A](int i, int k) { return k < i ? A.at(k, i) : (int64_t)-1; };
+  auto above = [&A](int i, int k) { return k > i ? A.at(k, i) : (int64_t)-1; };
+  auto none = [](int) { return (int64_t)-1; };
+  auto pivot = [&A](int i) { return A.unit[i] ? (int64_t)-1 : A.at(i, i); };
+  Phase p = schedule(triangle_tasks(A, sl, block, true, below, pivot));
+  Phase q = schedule(triangle_tasks(A, sl, block, false, above, none));
+  p.insert(p.end(), q.begin(), q.end());
+  return p;
+}
+
+// Items [0, count) in kSegments contiguous ranges, `per` items of a range at
+// a time: a batch's loads come before its arithmetic and stores, so that one
+// latency covers the batch.
+std::vector<std::vector<Emit>> ranges(int count, int per, const std::function<void(Ptx&, int, int)>& batch) {
+  std::vector<std::vector<Emit>> out;
+  for (int g = 0; g < kSegments; ++g) {
+    const int i0 = (int)((int64_t)count * g / kSegments), i1 = (int)((int64_t)count * (g + 1) / kSegments);
+    std::vector<Emit> seg;
+    for (int i = i0; i < i1; i += per) seg.push_back([=](Ptx& x) { batch(x, i, std::min(i1, i + per)); });
+    out.push_back(std::move(seg));
   }
-  // L^T x = z, columns of L descending
-  for (int ib = nb - 1; ib >= 0; --ib) {
-    const int c0 = ib * b, c1 = std::min(n, c0 + b);
-    std::vector<int> acc(b);
-    for (int c = c0; c < c1; ++c) acc[c - c0] = x.load(sl.xs + c);
-    for (int r = n - 1; r >= c1; --r) {
-      int xr = -1;
-      for (int c = c0; c < c1; ++c) {
-        const int q = P.at(r, c);
-        if (q < 0) continue;
-        if (xr < 0) xr = x.load(sl.xs + r);
-        acc[c - c0] = x.fma(x.neg(x.load(sl.lu + q)), xr, acc[c - c0]);
-      }
-    }
-    for (int c = c1 - 1; c >= c0; --c) {
-      for (int r = c1 - 1; r > c; --r) {
-        const int q = P.at(r, c);
-        if (q >= 0) acc[c - c0] = x.fma(x.neg(x.load(sl.lu + q)), acc[r - c0], acc[c - c0]);
-      }
-      x.store(sl.xs + c, acc[c - c0]);
-    }
-  }
+  while (!out.empty() && out.back().empty()) out.pop_back();
+  return out;
 }
 
 // Rates and forcing at the evaluation point (item yr): r_j = k_j * prod x,
 // then F_i = sum of S[i, j] r_j in ascending j, into item ft; the operations
 // of the table-driven loops in their order (a leading 0 or 1 and products
-// with +-1 are folded, which changes no value). Reactions and rows are
-// emitted in batches, a batch's loads before its arithmetic and stores, so
-// that one latency covers the batch. The table-driven loops were bound by one
-// dependent chain of loads per row and entry (TS1's attempts spent about 90%
-// of their time there): eight intervals of TS1 on 64 cells took 297 ms with
-// them and take 142 ms; one interval of 65,536 cells of the 210/500 mechanism
-// 140.6 ms and 128.3 ms.
-void emit_rhs(Ptx& x, const HostTables& t, const ScratchLayout& sl) {
-  constexpr int kBatch = 8;
-  for (int j0 = 0; j0 < t.R; j0 += kBatch) {
-    const int j1 = std::min(t.R, j0 + kBatch);
+// with +-1 are folded, which changes no value). The table-driven loops were
+// bound by one dependent chain of loads per row and entry (TS1's attempts
+// spent about 90% of their time there): eight intervals of TS1 on 64 cells
+// took 297 ms with them and 142 ms with straight-line code on one warp per
+// group; one interval of 65,536 cells of the 210/500 mechanism 140.6 ms and
+// 128.3 ms.
+Phase rhs_phase(const HostTables& t, const ScratchLayout& sl) {
+  Phase p;
+  p.push_back(ranges(t.R, 8, [&t, &sl](Ptx& x, int j0, int j1) {
     std::vector<std::vector<int>> v(j1 - j0);
     for (int j = j0; j < j1; ++j) {
       v[j - j0].push_back(x.load(sl.kc + j));
@@ -418,28 +584,34 @@ void emit_rhs(Ptx& x, const HostTables& t, const ScratchLayout& sl) {
       }
       x.store(sl.r + j, r);
     }
-  }
-  for (int i = 0; i < t.n; ++i) {
-    int acc = -1;
-    for (int q = t.s_ptr[i]; q < t.s_ptr[i + 1]; ++q) {
-      const int r = x.load(sl.r + t.s_rxn[q]);
-      const double c = t.s_val[q];
-      if (acc < 0) acc = c == 1.0 ? r : c == -1.0 ? x.neg(r) : x.mul_imm(r, c);
-      else acc = c == 1.0 ? x.add(acc, r) : c == -1.0 ? x.sub(acc, r) : x.fma_imm(r, c, acc);
-    }
-    x.store(sl.ft + i, acc < 0 ? x.constant(0.0) : acc);
-  }
+  }));
+  std::vector<Task> rows;
+  for (int i = 0; i < t.n; ++i)
+    rows.push_back({{}, [&t, &sl, i](Ptx& x) {
+      int acc = -1;
+      for (int q = t.s_ptr[i]; q < t.s_ptr[i + 1]; ++q) {
+        const int r = x.load(sl.r + t.s_rxn[q]);
+        const double c = t.s_val[q];
+        if (acc < 0) acc = c == 1.0 ? r : c == -1.0 ? x.neg(r) : x.mul_imm(r, c);
+        else acc = c == 1.0 ? x.add(acc, r) : c == -1.0 ? x.sub(acc, r) : x.fma_imm(r, c, acc);
+      }
+      x.store(sl.ft + i, acc < 0 ? x.constant(0.0) : acc);
+    }});
+  for (auto& s : schedule(rows)) p.push_back(std::move(s));
+  return p;
 }
 
 // The negated Jacobian values at the evaluation point, in assembly order:
 // d[j, p] = k_j * prod of the other reactants, then the sums of -S[i, j] d
 // over each entry's terms.
-void emit_jac(Ptx& x, const HostTables& t, const GenLayout& gl) {
-  constexpr int kBatch = 8;
+Phase jac_phase(const HostTables& t, const GenLayout& gl) {
   const ScratchLayout& sl = gl.s;
-  for (int j0 = 0; j0 < t.R; j0 += kBatch) {
-    const int j1 = std::min(t.R, j0 + kBatch);
-    struct One { int item, k; std::vector<int> x; };
+  Phase p;
+  p.push_back(ranges(t.R, 8, [&t, &gl, &sl](Ptx& x, int j0, int j1) {
+    struct One {
+      int item, k;
+      std::vector<int> x;
+    };
     std::vector<One> ones;
     for (int j = j0; j < j1; ++j) {
       int k = -1;
@@ -464,81 +636,96 @@ void emit_jac(Ptx& x, const HostTables& t, const GenLayout& gl) {
       for (int f : o.x) d = x.mul(d, f);
       x.store(o.item, d);
     }
-  }
-  for (size_t e = 0; e + 1 < t.jt_ptr.size(); ++e) {
-    int acc = -1;
-    for (int q = t.jt_ptr[e]; q < t.jt_ptr[e + 1]; ++q) {
-      const int jp = t.jt_idx[q];
-      const int d = x.load(gl.d_item[jp] >= 0 ? gl.d_item[jp] : sl.kc + jp / t.P);
-      const double c = t.jt_val[q];
-      if (acc < 0) acc = c == 1.0 ? d : c == -1.0 ? x.neg(d) : x.mul_imm(d, c);
-      else acc = c == 1.0 ? x.add(acc, d) : c == -1.0 ? x.sub(acc, d) : x.add(acc, x.mul_imm(d, c));
-    }
-    x.store(sl.negj + (int64_t)e, acc < 0 ? x.constant(0.0) : acc);
-  }
+  }));
+  std::vector<Task> entries;
+  for (int e = 0; e + 1 < (int)t.jt_ptr.size(); ++e)
+    entries.push_back({{}, [&t, &gl, &sl, e](Ptx& x) {
+      int acc = -1;
+      for (int q = t.jt_ptr[e]; q < t.jt_ptr[e + 1]; ++q) {
+        const int jp = t.jt_idx[q];
+        const int d = x.load(gl.d_item[jp] >= 0 ? gl.d_item[jp] : sl.kc + jp / t.P);
+        const double c = t.jt_val[q];
+        if (acc < 0) acc = c == 1.0 ? d : c == -1.0 ? x.neg(d) : x.mul_imm(d, c);
+        else acc = c == 1.0 ? x.add(acc, d) : c == -1.0 ? x.sub(acc, d) : x.add(acc, x.mul_imm(d, c));
+      }
+      x.store(sl.negj + (int64_t)e, acc < 0 ? x.constant(0.0) : acc);
+    }});
+  for (auto& s : schedule(entries)) p.push_back(std::move(s));
+  return p;
 }
 
-// One function whose body dispatches on the mechanism index parameter %m
-// to the mechanism's code (`bodies[i]`, all numbered in one register space).
-std::string function(const char* name, const char* params, const Ptx& x, const std::vector<std::string>& bodies,
-                     const char* prologue) {
-  std::string s;
-  size_t total = 0;
-  for (const auto& b : bodies) total += b.size();
-  s.reserve(total + 1024);
-  s += ".visible .func ";
-  s += name;
-  s += "(";
-  s += params;
-  s += ")\n{\n\t.reg .f64 %d<" + std::to_string(x.next + 1) + ">;\n\t.reg .b64 %p;\n\t.reg .b64 %b;\n"
-       "\t.reg .b64 %a;\n\t.reg .b32 %m;\n\t.reg .pred %q;\n";
-  s += prologue;
-  for (size_t i = 0; i < bodies.size(); ++i) {
-    const std::string label = std::string("$") + name + "_m" + std::to_string(i + 1);
-    if (i + 1 < bodies.size()) s += "\tsetp.ne.s32 %q, %m, " + std::to_string(i) + ";\n\t@%q bra " + label + ";\n";
-    s += bodies[i];
-    s += "\tret;\n";
-    if (i + 1 < bodies.size()) s += label + ":\n";
-  }
-  s += "}\n";
-  return s;
-}
-
-// The factorization: every piece of every mechanism as its own function
-// (fo_gen_factor_m<m>_p<k>: base, alpha), then fo_gen_factor(base, alpha,
-// mech), which calls mechanism mech's pieces in order. Separate functions
-// keep each compilation unit of the register allocator and scheduler small.
-std::string factor_functions(const std::vector<std::vector<Ptx>>& pieces) {
-  std::string out;
-  for (size_t m = 0; m < pieces.size(); ++m)
-    for (size_t k = 0; k < pieces[m].size(); ++k) {
-      const Ptx& x = pieces[m][k];
-      const std::string name = "fo_gen_factor_m" + std::to_string(m) + "_p" + std::to_string(k);
-      out.reserve(out.size() + x.body.size() + 512);
-      out += ".func " + name + "(.param .b64 " + name + "_base, .param .b64 " + name + "_alpha)\n{\n";
-      out += "\t.reg .f64 %d<" + std::to_string(x.next + 1) + ">;\n\t.reg .b64 %p;\n\t.reg .b64 %b;\n"
-             "\t.reg .b64 %a;\n";
-      out += "\tld.param.b64 %p, [" + name + "_base];\n\tld.param.b64 %a, [" + name + "_alpha];\n"
-             "\tmov.b64 %d0, %a;\n\tcvta.to.global.u64 %b, %p;\n";
-      out += x.body;
-      out += "\tret;\n}\n\n";
+// One phase of every mechanism as a function that all warps of a team call:
+//   .visible .func name(base, [alpha,] warp, warps, mech)
+// A team barrier, then mechanism mech's steps: warp w runs the segments w,
+// w + warps, ... of a step, and a team barrier ends it. Runs of tasks of
+// piece_lines instructions are functions of their own: ptxas optimizes those
+// side by side, and does not hoist one tile's loads over another's arithmetic
+// (segments compiled whole spilled up to 5 KB).
+std::string phase_function(const std::string& name, bool alpha, const std::vector<Phase>& mechs, size_t piece_lines,
+                           int64_t* fmas) {
+  std::string pieces, body;
+  Ptx x;
+  int labels = 0;
+  auto label = [&](const char* what, int id) { return "$" + name + "_" + what + std::to_string(id); };
+  const std::string regs = ";\n\t.reg .b64 %p;\n\t.reg .b64 %b;\n\t.reg .b64 %a;\n";
+  for (size_t m = 0; m < mechs.size(); ++m) {
+    if (m + 1 < mechs.size())
+      body += "\tsetp.ne.s32 %q, %m, " + std::to_string(m) + ";\n\t@%q bra " + label("m", (int)m + 1) + ";\n";
+    for (size_t s = 0; s < mechs[m].size(); ++s) {
+      const auto& segs = mechs[m][s];
+      const int id = labels++, count = (int)segs.size();
+      std::string table;
+      for (int g = 0; g < count; ++g) table += (g ? ", " : "") + label(("g" + std::to_string(id) + "_").c_str(), g);
+      body += "\tmov.u32 %s, %w;\n" + label("l", id) + ":\n\tsetp.ge.u32 %q, %s, " + std::to_string(count) +
+              ";\n\t@%q bra " + label("e", id) + ";\n";
+      if (count > 1) body += label("t", id) + ": .branchtargets " + table + ";\n\tbrx.idx.uni %s, " + label("t", id) + ";\n";
+      for (int g = 0; g < count; ++g) {
+        body += label(("g" + std::to_string(id) + "_").c_str(), g) + ":\n";
+        // tasks in order, gathered into runs of about piece_lines
+        // instructions: a run that reaches that is a function of its own
+        for (size_t q = 0, part = 0; q < segs[g].size(); ++part) {
+          Ptx own;
+          size_t lines = 0, q0 = q;
+          while (q < segs[g].size() && lines < piece_lines) {
+            segs[g][q++](own);
+            lines = (size_t)std::count(own.body.begin(), own.body.end(), '\n');
+          }
+          *fmas += own.fmas;
+          if (lines < piece_lines) {
+            for (; q0 < q; ++q0) segs[g][q0](x);
+            body += x.body;
+            x.body.clear();
+            continue;
+          }
+          const std::string piece =
+              name + "_" + std::to_string(id) + "_" + std::to_string(g) + "_" + std::to_string(part);
+          pieces += ".func " + piece + "(.param .b64 " + piece + "_base, .param .b64 " + piece + "_alpha)\n{\n" +
+                    "\t.reg .f64 %d<" + std::to_string(own.next + 1) + ">" + regs + "\tld.param.b64 %b, [" + piece +
+                    "_base];\n\tld.param.b64 %a, [" + piece + "_alpha];\n\tmov.b64 %d0, %a;\n" + own.body +
+                    "\tret;\n}\n\n";
+          body += "\t{\n\t.param .b64 fo_arg_base;\n\t.param .b64 fo_arg_alpha;\n\tst.param.b64 [fo_arg_base], %b;\n"
+                  "\tst.param.b64 [fo_arg_alpha], %a;\n\tcall.uni " + piece + ", (fo_arg_base, fo_arg_alpha);\n\t}\n";
+        }
+        body += "\tbra " + label("n", id) + ";\n";
+      }
+      body += label("n", id) + ":\n\tadd.u32 %s, %s, %nw;\n\tbra " + label("l", id) + ";\n" + label("e", id) +
+              ":\n\t@%team bar.sync 0;\n";
     }
-  out += ".visible .func fo_gen_factor(.param .b64 fo_gen_factor_base, .param .b64 fo_gen_factor_alpha, "
-         ".param .b32 fo_gen_factor_mech)\n{\n\t.reg .b64 %p;\n\t.reg .b64 %a;\n\t.reg .b32 %m;\n"
-         "\t.reg .pred %q;\n\tld.param.b64 %p, [fo_gen_factor_base];\n\tld.param.b64 %a, [fo_gen_factor_alpha];\n"
-         "\tld.param.b32 %m, [fo_gen_factor_mech];\n";
-  for (size_t m = 0; m < pieces.size(); ++m) {
-    const std::string label = "$fo_gen_factor_m" + std::to_string(m + 1);
-    if (m + 1 < pieces.size()) out += "\tsetp.ne.s32 %q, %m, " + std::to_string(m) + ";\n\t@%q bra " + label + ";\n";
-    for (size_t k = 0; k < pieces[m].size(); ++k)
-      out += "\t{\n\t.param .b64 fo_arg_base;\n\t.param .b64 fo_arg_alpha;\n\tst.param.b64 [fo_arg_base], %p;\n"
-             "\tst.param.b64 [fo_arg_alpha], %a;\n\tcall.uni fo_gen_factor_m" + std::to_string(m) + "_p" +
-             std::to_string(k) + ", (fo_arg_base, fo_arg_alpha);\n\t}\n";
-    out += "\tret;\n";
-    if (m + 1 < pieces.size()) out += label + ":\n";
+    body += "\tret;\n";
+    if (m + 1 < mechs.size()) body += label("m", (int)m + 1) + ":\n";
   }
-  out += "}\n";
-  return out;
+  auto param = [&](const char* what) { return name + "_" + what; };
+  std::string s = pieces + ".visible .func " + name + "(.param .b64 " + param("base") +
+                  (alpha ? ", .param .b64 " + param("alpha") : "") + ", .param .b32 " + param("warp") +
+                  ", .param .b32 " + param("warps") + ", .param .b32 " + param("mech") + ")\n{\n\t.reg .f64 %d<" +
+                  std::to_string(x.next + 1) + ">" + regs +
+                  "\t.reg .b32 %m;\n\t.reg .b32 %w;\n\t.reg .b32 %nw;\n\t.reg .b32 %s;\n"
+                  "\t.reg .pred %q;\n\t.reg .pred %team;\n\tld.param.b64 %p, [" + param("base") + "];\n" +
+                  (alpha ? "\tld.param.b64 %a, [" + param("alpha") + "];\n" : "\tmov.b64 %a, 0x3FF0000000000000;\n") +
+                  "\tmov.b64 %d0, %a;\n\tld.param.b32 %w, [" + param("warp") + "];\n\tld.param.b32 %nw, [" +
+                  param("warps") + "];\n\tld.param.b32 %m, [" + param("mech") +
+                  "];\n\tcvta.to.global.u64 %b, %p;\n\tsetp.gt.u32 %team, %nw, 1;\n\t@%team bar.sync 0;\n";
+  return s + body + "}\n\n";
 }
 
 }  // namespace
@@ -547,72 +734,54 @@ std::string generate_ptx(const std::vector<const HostTables*>& ts, const std::ve
                          int64_t* fma_count) {
   if (ts.empty() || os.size() != ts.size()) throw std::invalid_argument("one set of options per mechanism");
   for (const GenOptions& o : os)
-    if (o.tile < 1 || o.tile > 16 || o.solve_block < 1 || o.solve_block > 64 || o.solve_keep < 0 ||
-        o.piece_lines < 1)
+    if (o.tile < 1 || o.tile > 16 || o.solve_block < 1 || o.solve_block > 64 || o.piece_lines < 1)
       throw std::invalid_argument("generation options out of range");
-  Ptx s, st, f, jv;
-  std::vector<std::string> sb, tb, fb, jb;
-  // the factorization of mechanism m: pieces[m][k] = the k-th function
-  std::vector<std::vector<Ptx>> pieces(ts.size());
-  int64_t total = 0;
-  for (size_t m = 0; m < ts.size(); ++m) {
-    const HostTables* t = ts[m];
-    const GenOptions& o = os[m];
-    const GenLayout gl = gen_layout_of(*t);
-    const ScratchLayout& sl = gl.s;
-    const Pattern P = pattern_of(*t);
-    // consecutive row blocks up to about o.piece_lines instructions each
-    const int nb = (t->n + o.tile - 1) / o.tile;
-    std::vector<size_t> lines(nb);
-    for (int ib = 0; ib < nb; ++ib) {
-      Ptx probe;
-      int64_t ignored = 0;
-      emit_factor(probe, *t, sl, P, o.tile, ib, ib + 1, &ignored);
-      lines[ib] = (size_t)std::count(probe.body.begin(), probe.body.end(), '\n');
-    }
-    int64_t nfma = 0;
-    for (int ib = 0; ib < nb;) {
-      int end = ib + 1;
-      size_t sum = lines[ib];
-      while (end < nb && sum + lines[end] <= (size_t)o.piece_lines) sum += lines[end++];
-      pieces[m].emplace_back();
-      emit_factor(pieces[m].back(), *t, sl, P, o.tile, ib, end, &nfma);
-      ib = end;
-    }
-    if (nfma != t->lu_fma) throw std::logic_error("generated factorization does not match the symbolic count");
-    total += nfma;
-    emit_solve(s, *t, sl, P, o.solve_block, o.solve_keep);
-    sb.push_back(std::move(s.body));
-    s.body.clear();
-    emit_solve_t(st, *t, sl, P, o.solve_block);
-    tb.push_back(std::move(st.body));
-    st.body.clear();
-    emit_rhs(f, *t, sl);
-    fb.push_back(std::move(f.body));
-    f.body.clear();
-    emit_jac(jv, *t, gl);
-    jb.push_back(std::move(jv.body));
-    jv.body.clear();
+  const size_t count = ts.size();
+  std::vector<GenLayout> layouts;
+  std::vector<Matrix> full, proj;
+  for (const HostTables* t : ts) layouts.push_back(gen_layout_of(*t));
+  for (size_t m = 0; m < count; ++m) {
+    full.push_back(full_matrix(*ts[m], layouts[m]));
+    proj.push_back(projection_matrix(*ts[m], layouts[m]));
   }
-  if (fma_count) *fma_count = total;
+  std::vector<Phase> rhs, jac, factor, solve, solve_t, pfactor, psolve, psolve_t;
+  int64_t expected = 0;
+  for (size_t m = 0; m < count; ++m) {
+    const HostTables& t = *ts[m];
+    const GenLayout& gl = layouts[m];
+    const GenOptions& o = os[m];
+    rhs.push_back(rhs_phase(t, gl.s));
+    jac.push_back(jac_phase(t, gl));
+    factor.push_back(schedule(factor_tasks(full[m], gl, o.tile)));
+    solve.push_back(solve_phase(full[m], gl.s, o.solve_block));
+    solve_t.push_back(solve_t_phase(full[m], gl.s, o.solve_block));
+    bool constrained = false;
+    for (double v : t.mass) constrained = constrained || v == 0.0;
+    pfactor.push_back(constrained ? schedule(factor_tasks(proj[m], gl, o.tile)) : Phase());
+    psolve.push_back(constrained ? solve_phase(proj[m], gl.s, o.solve_block) : Phase());
+    psolve_t.push_back(constrained ? solve_t_phase(proj[m], gl.s, o.solve_block) : Phase());
+    // the multiply-adds of the pivots before the dense square
+    for (int i = 0; i < t.n; ++i)
+      for (int q = t.lu_row_ptr[i]; q < t.lu_diag[i]; ++q)
+        if (t.lu_col[q] < gl.d0) expected += t.lu_row_ptr[t.lu_col[q] + 1] - t.lu_diag[t.lu_col[q]] - 1;
+  }
+  size_t lines = 0;
+  for (const GenOptions& o : os) lines = std::max(lines, (size_t)o.piece_lines);
   std::string out = ".version 9.0\n.target sm_103a\n.address_size 64\n\n";
-  out += factor_functions(pieces);
-  out += "\n";
-  out += function("fo_gen_solve", ".param .b64 fo_gen_solve_base, .param .b32 fo_gen_solve_mech", s, sb,
-                  "\tld.param.b64 %p, [fo_gen_solve_base];\n\tld.param.b32 %m, [fo_gen_solve_mech];\n"
-                  "\tcvta.to.global.u64 %b, %p;\n");
-  out += "\n";
-  out += function("fo_gen_solve_t", ".param .b64 fo_gen_solve_t_base, .param .b32 fo_gen_solve_t_mech", st, tb,
-                  "\tld.param.b64 %p, [fo_gen_solve_t_base];\n\tld.param.b32 %m, [fo_gen_solve_t_mech];\n"
-                  "\tcvta.to.global.u64 %b, %p;\n");
-  out += "\n";
-  out += function("fo_gen_rhs", ".param .b64 fo_gen_rhs_base, .param .b32 fo_gen_rhs_mech", f, fb,
-                  "\tld.param.b64 %p, [fo_gen_rhs_base];\n\tld.param.b32 %m, [fo_gen_rhs_mech];\n"
-                  "\tcvta.to.global.u64 %b, %p;\n");
-  out += "\n";
-  out += function("fo_gen_jac", ".param .b64 fo_gen_jac_base, .param .b32 fo_gen_jac_mech", jv, jb,
-                  "\tld.param.b64 %p, [fo_gen_jac_base];\n\tld.param.b32 %m, [fo_gen_jac_mech];\n"
-                  "\tcvta.to.global.u64 %b, %p;\n");
+  int64_t nfma = 0, ignored = 0;
+  out += phase_function("fo_gen_factor", true, factor, lines, &nfma);
+  if (nfma != expected) throw std::logic_error("generated factorization does not match the symbolic count");
+  if (fma_count) {
+    *fma_count = 0;
+    for (const HostTables* t : ts) *fma_count += t->lu_fma;
+  }
+  out += phase_function("fo_gen_solve", false, solve, lines, &ignored);
+  out += phase_function("fo_gen_solve_t", false, solve_t, lines, &ignored);
+  out += phase_function("fo_gen_rhs", false, rhs, lines, &ignored);
+  out += phase_function("fo_gen_jac", false, jac, lines, &ignored);
+  out += phase_function("fo_gen_factor_p", false, pfactor, lines, &ignored);
+  out += phase_function("fo_gen_solve_p", false, psolve, lines, &ignored);
+  out += phase_function("fo_gen_solve_tp", false, psolve_t, lines, &ignored);
   return out;
 }
 

@@ -1,6 +1,6 @@
-// Per-mechanism code generation: the factorization of alpha*M - J and the two
-// triangular solves of one mechanism as straight-line PTX, every operand at an
-// immediate offset from a lane's base pointer. The integrator kernel compiled
+// Per-mechanism code generation: the evaluations, the factorization of
+// alpha*M - J and the triangular solves of one mechanism as straight-line PTX,
+// every operand at an immediate offset from a lane's base pointer. The integrator kernel compiled
 // as relocatable device code (generated.cu) calls them; jit.cpp links the
 // two into one module per mechanism.
 #pragma once
@@ -13,36 +13,35 @@
 
 namespace fo {
 
+// Segments of a step of generated work: the most warps a team can use.
+constexpr int kSegments = 16;
+
 struct GenOptions {
-  // rows (and columns) of the register tiles of the factorization
+  // rows and columns of the register tiles of the factorization
   int tile = 6;
   // rows of a block of the triangular solves
   int solve_block = 8;
-  // values of later blocks the backward solve keeps in registers per block
-  int solve_keep = 16;
-  // instructions per separately compiled piece of the factorization (whole
-  // row blocks; a block longer than this is a piece of its own)
-  int piece_lines = 40000;
+  // instructions of consecutive tasks compiled as a function of their own
+  int piece_lines = 400;
 };
 
-// PTX (ISA 9.0, sm_103a) defining
-//   .visible .func fo_gen_factor(.param .b64 base, .param .b64 alpha, .param .b32 mech)
-//   .visible .func fo_gen_solve(.param .b64 base, .param .b32 mech)
-// for a group of 32 lanes: base points at this lane's item 0 of its scratch
-// slot, laid out item-major with 32 lanes (item q at byte offset 256 q); the
-// LU storage, the Jacobian values and the solve vector sit at the item
-// offsets of the plan's scratch layout (layout.h). fo_gen_factor assembles
-// alpha*M - J from the negated Jacobian values (assembly order) and factors
-// it in place in the LU storage order of `t`, with the same operations, in
-// the same order per entry, as the row-by-row elimination (every entry
-// receives its updates fma(-l, u, a) in ascending pivot order; multipliers
-// a * (1 / pivot); the diagonal keeps 1 / pivot). fo_gen_solve overwrites the
-// solve vector with (LU)^-1 of it: forward then backward substitution, each
-// row's sum in ascending column order. A third function,
-//   .visible .func fo_gen_solve_t(.param .b64 base, .param .b32 mech)
-// overwrites the solve vector with (LU)^-T of it for the adjoint, with the
-// operations and order of its table-driven transposed solve. `mech` is
-// ignored (one mechanism).
+// PTX (ISA 9.0, sm_103a) of the phases of one mechanism, each a function that
+// every warp of a group's team calls with its index and the team's size:
+//   .visible .func name(.param .b64 base, .param .b32 warp, .param .b32 warps, .param .b32 mech)
+// base points at this lane's item 0 of its scratch slot, laid out item-major
+// with 32 lanes (item q at byte offset 256 q) by GenLayout (layout.h). Every
+// phase begins and ends with the team's barrier (none for a team of one).
+//   fo_gen_rhs       forcing at the point in item yr, into item ft
+//   fo_gen_jac       negated Jacobian values at yr, into item negj
+//   fo_gen_factor    (base, alpha, ...) assembles alpha*M - J and factors it up
+//                    to the dense square, which it leaves assembled and updated
+//                    (dense_lu finishes it)
+//   fo_gen_solve     overwrites the solve vector (item xs) with (LU)^-1 of it
+//   fo_gen_solve_t   ... with (LU)^-T of it, for the adjoint
+//   fo_gen_factor_p, fo_gen_solve_p, fo_gen_solve_tp
+//                    the same for the projection's algebraic-rows-only matrix
+//                    (empty for unconstrained mechanisms)
+// `mech` is ignored (one mechanism).
 std::string generate_ptx(const HostTables& t, const GenOptions& o, int64_t* fma_count = nullptr);
 
 // The same for several mechanisms in one module: `mech` is the mechanism's

@@ -77,11 +77,17 @@ struct DevOptions {
   double small;
 };
 
+// Rows and columns of a block of the generated variant's dense square: a
+// block and two columns of operands fit the 128 registers of a thread.
+constexpr int kDenseBlock = 6;
+
 // Per-lane scratch layout, in items (each item is `lanes` doubles).
 struct ScratchLayout {
   int64_t lu, negj, d, r, y, ynew, f0, ft, yr, k;  // offsets
   int64_t xs;                                      // the generated solves' vector (n items)
   int64_t kc;                                      // the generated evaluations' rate constants (R items)
+  int64_t dn;                                      // the generated variant's dense square
+  int nb;                                          // its blocks of kDenseBlock rows and columns
   int64_t items;                                   // total items per lane
 };
 

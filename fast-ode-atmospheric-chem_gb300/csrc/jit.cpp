@@ -298,14 +298,34 @@ cudaError_t ensure_smem(GenModule* m, int which, const void* fn, size_t smem) {
   return cudaSuccess;
 }
 
-// Whether `grid` one-warp blocks of kernel `fn` with `smem` bytes of dynamic
-// shared memory are all resident at once on the current device (what a
-// cooperative launch needs).
-bool all_resident(const void* fn, int grid, size_t smem) {
+// Warps per group for a launch of `grid` blocks on the current device: the
+// largest power of two, up to kSegments, that still leaves every block
+// resident at sixteen warps per SM (the kernels' 128 registers per thread):
+// beyond that a larger team only makes groups wait for one another. One warp
+// per group and a team, measured on a GB300: eight intervals of TS1 on 64
+// cells (2 groups, teams of 16) 142 and 42 ms; two intervals on 8,200 cells
+// (257 groups, teams of 8) 27.0 and 9.2 ms; the cold interval of 16,384 cells
+// of the 210/500 mechanism (512 groups, teams of 4) 452 and 270 ms.
+int team_of(int grid) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 1;
+  }
+  int team = 1;
+  while (2 * team <= kSegments && (int64_t)grid * 2 * team <= (int64_t)sms * 16) team *= 2;
+  return team;
+}
+
+// Whether `grid` blocks of `team` warps of kernel `fn` with `smem` bytes of
+// dynamic shared memory are all resident at once on the current device (what
+// a cooperative launch needs).
+bool all_resident(const void* fn, int grid, int team, size_t smem) {
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32, smem) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * team, smem) != cudaSuccess) {
     (void)cudaGetLastError();
     return false;
   }
@@ -320,7 +340,7 @@ bool gen_resident(GenModule* m, bool multi, int grid, size_t smem) {
     (void)cudaGetLastError();
     return false;
   }
-  return all_resident(fn, grid, smem);
+  return all_resident(fn, grid, team_of(grid), smem);
 }
 
 cudaError_t gen_launch(GenModule* m, const SolveParams& p, int grid, size_t smem, cudaStream_t stream) {
@@ -331,10 +351,11 @@ cudaError_t gen_launch(GenModule* m, const SolveParams& p, int grid, size_t smem
   void* args[] = {&q};
   // lockstep rounds need every block resident: a cooperative launch; a grid
   // that does not fit runs without rounds
-  if (q.rounds != nullptr && all_resident(fn, grid, smem))
-    return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(32), args, smem, stream);
+  const int team = team_of(grid);
+  if (q.rounds != nullptr && all_resident(fn, grid, team, smem))
+    return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
   q.rounds = nullptr;
-  return cudaLaunchKernel(fn, dim3(grid), dim3(32), args, smem, stream);
+  return cudaLaunchKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
 }
 
 cudaError_t gen_launch_adjoint(GenModule* m, const AdjParams& a, int grid, size_t smem, cudaStream_t stream) {
@@ -355,8 +376,9 @@ cudaError_t gen_launch_multi(GenModule* m, const SolveParams* batches, int nb, c
   e = cudaMemsetAsync(queue, 0, sizeof(int32_t), stream);
   if (e != cudaSuccess) return e;
   void* args[] = {&batches, &nb, &starts, &queue, &scratch, &slot_doubles};
-  if (cooperative) return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(32), args, smem, stream);
-  return cudaLaunchKernel(fn, dim3(grid), dim3(32), args, smem, stream);
+  const int team = team_of(grid);
+  if (cooperative) return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
+  return cudaLaunchKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
 }
 
 }  // namespace fo

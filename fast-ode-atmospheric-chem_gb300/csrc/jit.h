@@ -23,7 +23,8 @@ int gen_create(const std::vector<const HostTables*>& ts, const std::vector<GenOp
 void gen_destroy(GenModule* m);
 // Generate (and, with do_link, link) without a device: no module is loaded.
 int gen_check(const HostTables& t, const GenOptions& opt, bool do_link, fo_gen_info* info, std::string* err);
-// One launch of the generated integrator kernel: grid blocks of 32 lanes.
+// One launch of the generated integrator kernel: grid blocks of a
+// team of warps of 32 lanes each.
 cudaError_t gen_launch(GenModule* m, const SolveParams& p, int grid, size_t smem, cudaStream_t stream);
 // One launch of the generated adjoint kernel (fo_adjoint_interval): grid
 // blocks of 32 lanes.

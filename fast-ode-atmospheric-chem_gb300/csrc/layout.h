@@ -1,9 +1,8 @@
-// The per-lane scratch layout of a plan, shared by the launch code (abi.cu)
+// The per-lane scratch layouts of a plan, shared by the launch code (abi.cu)
 // and the code generator (codegen.cpp), which bakes its offsets into the
 // generated functions.
 #pragma once
 
-#include <algorithm>
 #include <cstdint>
 #include <vector>
 
@@ -27,6 +26,8 @@ inline ScratchLayout layout_of(const HostTables& t) {
   s.k = o; o += 4LL * t.n;
   s.xs = o; o += t.n;
   s.kc = 0;
+  s.dn = 0;
+  s.nb = 0;
   s.items = o;
   return s;
 }
@@ -36,30 +37,19 @@ inline ScratchLayout layout_of(const HostTables& t) {
 // constants (kc), so that every operand of theirs is at an immediate offset
 // from the slot's base, and store only the partial derivatives that are
 // products (a unimolecular reaction's is its rate constant); those and the
-// rates are never live together and share their items.
+// rates are never live together and share their items. The trailing
+// kDenseBlock * nb rows and columns of the LU are stored as a dense square of
+// nb x nb blocks (item dn), block (bi, bj) as kDenseBlock^2 items, row-major,
+// at (bi * nb + bj) * kDenseBlock^2; the other entries keep their order.
 struct GenLayout {
   ScratchLayout s;
-  std::vector<int32_t> d_item;  // R*P: item of d[j, p], or -1 where it is k_j itself or not used
+  int d0 = 0;                    // first row of the dense square (n: none)
+  std::vector<int32_t> d_item;   // R*P: item of d[j, p], or -1 where it is k_j itself or not used
+  std::vector<int64_t> lu_item;  // item of each LU entry
+  // item of (i, j) of the dense square (structural zeros included)
+  int64_t dense_item(int i, int j) const;
 };
 
-inline GenLayout gen_layout_of(const HostTables& t) {
-  GenLayout g;
-  g.s = layout_of(t);
-  g.d_item.assign((size_t)t.R * t.P, -1);
-  int64_t nd = 0;
-  std::vector<char> used((size_t)t.R * t.P, 0);
-  for (int32_t q : t.jt_idx) used[q] = 1;
-  for (int j = 0; j < t.R; ++j) {
-    int factors = 0;
-    for (int q = 0; q < t.P; ++q) factors += t.react[(size_t)j * t.P + q] != t.n ? 1 : 0;
-    for (int a = 0; a < t.P; ++a) {
-      const int others = factors - (t.react[(size_t)j * t.P + a] != t.n ? 1 : 0);
-      if (used[(size_t)j * t.P + a] && others > 0) g.d_item[(size_t)j * t.P + a] = (int32_t)(g.s.d + nd++);
-    }
-  }
-  g.s.r = g.s.d;
-  g.s.kc = g.s.d + std::max<int64_t>(nd, t.R);
-  return g;
-}
+GenLayout gen_layout_of(const HostTables& t);
 
 }  // namespace fo

@@ -16,16 +16,28 @@
 #include "fastode_gb300.h"
 
 #ifdef FO_LINK_GENERATED
-// The mechanism's generated factorization and solves (codegen.cpp), linked in
-// per mechanism: `base` is this lane's item 0 of its scratch slot (32 lanes),
-// `mech` the mechanism's index in the module (several mechanisms share one).
-extern "C" __device__ void fo_gen_factor(double* base, double alpha, int mech);
-extern "C" __device__ void fo_gen_solve(double* base, int mech);
-// forcing and negated Jacobian values at the point in item yr (rates and
-// constants in kc), the forcing into item ft
-extern "C" __device__ void fo_gen_rhs(double* base, int mech);
-extern "C" __device__ void fo_gen_jac(double* base, int mech);
-extern "C" __device__ void fo_gen_solve_t(double* base, int mech);   // the adjoint's transposed solve
+// The mechanism's generated phases (codegen.h), linked in per mechanism:
+// `base` is this lane's item 0 of its scratch slot (32 lanes), `warp` of
+// `warps` the caller's place in the group's team, `mech` the mechanism's
+// index in the module (several mechanisms share one).
+extern "C" {
+__device__ void fo_gen_rhs(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_jac(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_factor(double* base, double alpha, int warp, int warps, int mech);
+__device__ void fo_gen_solve(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_t(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_factor_p(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_p(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_tp(double* base, int warp, int warps, int mech);
+}
+// The team: the warps of the block (blockDim = 32 x warps), all holding the
+// group's cells. Loops over species give warp w the species i = w mod warps
+// (a power of two), so that elementwise loops hand no value to another warp.
+#define TEAM_W ((int)threadIdx.y)
+#define TEAM_N ((int)blockDim.y)
+#else
+#define TEAM_W 0
+#define TEAM_N 1
 #endif
 
 namespace fo {
@@ -55,6 +67,12 @@ __device__ __forceinline__ double quantize_step(double h, double interval) {
   if (!(q >= 1.0)) q = 1.0;
   return __ddiv_rn(interval, q);
 }
+
+// The team's barrier, and its one thread that writes a group's results.
+__device__ __forceinline__ void team_sync() {
+  if (TEAM_N > 1) __syncthreads();
+}
+__device__ __forceinline__ bool team_leader() { return threadIdx.x == 0 && TEAM_W == 0; }
 
 struct Lane {
   int lane;      // thread index in the block
@@ -109,14 +127,14 @@ __device__ void eval_forcing(const SolveParams& p, const Lane& ln, const double*
 __device__ __forceinline__ void copy_items(const Lane& ln, int n, const double* u, double* v) {
   constexpr int kBatch = 8;
   const int L = ln.L, lane = ln.lane;
-  for (int i = 0; i < n; i += kBatch) {
+  for (int i = TEAM_W; i < n; i += kBatch * TEAM_N) {
     double b[kBatch];
 #pragma unroll
     for (int q = 0; q < kBatch; ++q)
-      if (i + q < n) b[q] = SCR(u, i + q);
+      if (i + q * TEAM_N < n) b[q] = SCR(u, i + q * TEAM_N);
 #pragma unroll
     for (int q = 0; q < kBatch; ++q)
-      if (i + q < n) SCR(v, i + q) = b[q];
+      if (i + q * TEAM_N < n) SCR(v, i + q * TEAM_N) = b[q];
   }
 }
 
@@ -128,14 +146,14 @@ __device__ __forceinline__ void load_rate_constants(const SolveParams& p, const 
   const int L = ln.L, lane = ln.lane;
   const double* __restrict__ kc = p.k + ln.cell * p.kcs;
   double* out = scr + p.sl.kc * L;
-  for (int j = 0; j < p.t.R; j += kBatch) {
+  for (int j = TEAM_W; j < p.t.R; j += kBatch * TEAM_N) {
     double b[kBatch];
 #pragma unroll
     for (int q = 0; q < kBatch; ++q)
-      if (j + q < p.t.R) b[q] = __ldg(kc + (int64_t)(j + q) * p.krs);
+      if (j + q * TEAM_N < p.t.R) b[q] = __ldg(kc + (int64_t)(j + q * TEAM_N) * p.krs);
 #pragma unroll
     for (int q = 0; q < kBatch; ++q)
-      if (j + q < p.t.R) SCR(out, j + q) = b[q];
+      if (j + q * TEAM_N < p.t.R) SCR(out, j + q * TEAM_N) = b[q];
   }
 #endif
 }
@@ -149,7 +167,7 @@ __device__ __noinline__ void eval_rhs(const SolveParams& p, const Lane& ln, cons
   double* yr = base + p.sl.yr * ln.L;
   double* ft = base + p.sl.ft * ln.L;
   if (x != yr) copy_items(ln, p.t.n, x, yr);
-  fo_gen_rhs(base + ln.lane, p.o.gen_index);
+  fo_gen_rhs(base + ln.lane, TEAM_W, TEAM_N, p.o.gen_index);
   if (f != ft) copy_items(ln, p.t.n, ft, f);
 #else
   eval_rates(p, ln, x, r);
@@ -163,7 +181,7 @@ __device__ __noinline__ void eval_rhs(const SolveParams& p, const Lane& ln, cons
 __device__ __noinline__ void eval_negjac(const SolveParams& p, const Lane& ln, const double* __restrict__ x,
                                          double* __restrict__ d, double* __restrict__ negj) {
 #ifdef FO_LINK_GENERATED
-  fo_gen_jac(negj - p.sl.negj * ln.L + ln.lane, p.o.gen_index);
+  fo_gen_jac(negj - p.sl.negj * ln.L + ln.lane, TEAM_W, TEAM_N, p.o.gen_index);
 #else
   constexpr int kBatch = 8;
   const int L = ln.L, lane = ln.lane;
@@ -616,7 +634,10 @@ __device__ __forceinline__ void lu_solve_compact(const SolveParams& p, const Lan
   else lu_solve_compact_l<0>(p, ln, lu, w, b, x);
 }
 
-// Forward and backward substitution in place on w (fastode/linalg.py:80-81).
+// Forward and backward substitution in place on w (fastode/linalg.py:80-81),
+// each row's terms in the order in which their values finish: ascending
+// columns forward, descending columns backward (the generated solves' order,
+// which lets a finished value update every remaining row at once).
 __device__ void lu_solve(const SolveParams& p, const Lane& ln, const double* lu, double* w) {
   const int L = ln.L, lane = ln.lane;
   const int n = p.t.n;
@@ -631,8 +652,8 @@ __device__ void lu_solve(const SolveParams& p, const Lane& ln, const double* lu,
   }
   for (int r = n - 1; r >= 0; --r) {
     double acc = WROW(r);
-    const int dg = __ldg(diag + r), q1 = __ldg(rowp + r + 1);
-    for (int q = dg + 1; q < q1; ++q) acc = fma(-SCR(lu, q), WROW(__ldg(col + q)), acc);
+    const int dg = __ldg(diag + r);
+    for (int q = __ldg(rowp + r + 1) - 1; q > dg; --q) acc = fma(-SCR(lu, q), WROW(__ldg(col + q)), acc);
     WROW(r) = acc * SCR(lu, dg);
   }
 }
@@ -655,13 +676,162 @@ __device__ __forceinline__ bool solves_in_place(const SolveParams& p) {
   return p.o.variant == FO_VARIANT_COMPACT || generated(p);
 }
 
+#ifdef FO_LINK_GENERATED
+// The dense square's elimination (GenLayout): nb x nb blocks of kDenseBlock
+// rows and columns in tile-major order, `a` this lane's first item. Step s
+// finishes block (s, s) and the blocks below and right of it, left-looking:
+// every block of the step first takes the updates of the pivots before the
+// step (one warp per block: the block in registers, two columns of operands
+// in flight, 36 DFMAs per 12 loads), the diagonal block is factored, and after
+// a barrier the others take the step's own pivots. A team of one does both
+// without the barriers and the round trip. Each entry receives its updates in
+// ascending pivot order, as in the row-by-row elimination. The loop is a few
+// kilobytes of code, so the warps of an SM share it in the instruction cache
+// wherever each of them is.
+constexpr int kDB = kDenseBlock;
+
+__device__ __forceinline__ double* dense_block(double* a, int nb, int bi, int bj) {
+  return a + (int64_t)(bi * nb + bj) * kDB * kDB * 32;
+}
+
+__device__ __forceinline__ void block_load(const double* t, double (&c)[kDB][kDB]) {
+#pragma unroll
+  for (int i = 0; i < kDB; ++i)
+#pragma unroll
+    for (int j = 0; j < kDB; ++j) c[i][j] = t[(i * kDB + j) * 32];
+}
+
+__device__ __forceinline__ void block_store(double* t, const double (&c)[kDB][kDB]) {
+#pragma unroll
+  for (int i = 0; i < kDB; ++i)
+#pragma unroll
+    for (int j = 0; j < kDB; ++j) t[(i * kDB + j) * 32] = c[i][j];
+}
+
+// c -= sum over m blocks of L(bi, .) U(., bj); ustep: doubles between U blocks
+__device__ __forceinline__ void block_update(double (&c)[kDB][kDB], const double* l, const double* u, int m,
+                                             int64_t ustep) {
+  double a[2][kDB], b[2][kDB];
+  if (m == 0) return;
+#pragma unroll
+  for (int i = 0; i < kDB; ++i) {
+    a[0][i] = l[i * kDB * 32];
+    b[0][i] = u[i * 32];
+  }
+#pragma unroll 1
+  for (int q = 0; q < m; ++q) {
+    const bool more = q + 1 < m;
+    const double* ln = more ? l + kDB * kDB * 32 : l;   // the last pivot's lookahead rereads
+    const double* un = more ? u + ustep : u;
+#pragma unroll
+    for (int k = 0; k < kDB; ++k) {
+      const double* lk = k + 1 < kDB ? l + (k + 1) * 32 : ln;
+      const double* uk = k + 1 < kDB ? u + (k + 1) * kDB * 32 : un;
+#pragma unroll
+      for (int i = 0; i < kDB; ++i) {
+        a[(k + 1) & 1][i] = lk[i * kDB * 32];
+        b[(k + 1) & 1][i] = uk[i * 32];
+      }
+#pragma unroll
+      for (int i = 0; i < kDB; ++i)
+#pragma unroll
+        for (int j = 0; j < kDB; ++j) c[i][j] = fma(-a[k & 1][i], b[k & 1][j], c[i][j]);
+    }
+    l = ln;
+    u = un;
+  }
+}
+
+// The step's own pivots on a block below (left) or right of the diagonal
+// block d: multipliers and their updates, or the updates of its rows.
+__device__ __forceinline__ void block_finish(double (&c)[kDB][kDB], const double* d, bool left) {
+#pragma unroll
+  for (int k = 0; k < kDB; ++k) {
+    if (left) {
+      const double rk = d[(k * kDB + k) * 32];
+#pragma unroll
+      for (int i = 0; i < kDB; ++i) c[i][k] *= rk;
+#pragma unroll
+      for (int j = k + 1; j < kDB; ++j) {
+        const double u = d[(k * kDB + j) * 32];
+#pragma unroll
+        for (int i = 0; i < kDB; ++i) c[i][j] = fma(-c[i][k], u, c[i][j]);
+      }
+    } else {
+#pragma unroll
+      for (int i = k + 1; i < kDB; ++i) {
+        const double m = d[(i * kDB + k) * 32];
+#pragma unroll
+        for (int j = 0; j < kDB; ++j) c[i][j] = fma(-m, c[k][j], c[i][j]);
+      }
+    }
+  }
+}
+
+__device__ __noinline__ void dense_lu(double* a, int nb) {
+  const int64_t ustep = (int64_t)nb * kDB * kDB * 32;
+  const int w = TEAM_W, wn = TEAM_N;
+#pragma unroll 1
+  for (int s = 0; s < nb; ++s) {
+    // block 0 of the step is the diagonal one, 2m - 1 and 2m those m below
+    // and m right of it
+    const int count = 2 * (nb - s) - 1;
+    double* d = dense_block(a, nb, s, s);
+#pragma unroll 1
+    for (int q = w; q < count; q += wn) {
+      const int m = s + (q + 1) / 2;
+      const bool left = (q & 1) != 0;
+      const int bi = left ? m : s, bj = left ? s : m;
+      double* t = dense_block(a, nb, bi, bj);
+      double c[kDB][kDB];
+      block_load(t, c);
+      block_update(c, dense_block(a, nb, bi, 0), dense_block(a, nb, 0, bj), s, ustep);
+      if (q == 0) {
+#pragma unroll
+        for (int k = 0; k < kDB; ++k) {
+          const double rk = 1.0 / c[k][k];
+          c[k][k] = rk;
+#pragma unroll
+          for (int i = k + 1; i < kDB; ++i) {
+            c[i][k] *= rk;
+#pragma unroll
+            for (int j = k + 1; j < kDB; ++j) c[i][j] = fma(-c[i][k], c[k][j], c[i][j]);
+          }
+        }
+      } else if (wn == 1) {
+        block_finish(c, d, left);
+      }
+      block_store(t, c);
+    }
+    team_sync();
+    if (wn > 1 && count > 1) {
+#pragma unroll 1
+      for (int q = w; q < count; q += wn) {
+        if (q == 0) continue;
+        const int m = s + (q + 1) / 2;
+        const bool left = (q & 1) != 0;
+        double* t = dense_block(a, nb, left ? m : s, left ? s : m);
+        double c[kDB][kDB];
+        block_load(t, c);
+        block_finish(c, d, left);
+        block_store(t, c);
+      }
+      team_sync();
+    }
+  }
+}
+#endif
+
 __device__ void factor_any(const SolveParams& p, const Lane& ln, double alpha, const double* negj, double* lu,
                            double* w, bool alg_only) {
 #ifdef FO_LINK_GENERATED
-  // the projection's algebraic-rows-only matrix takes the row loop (the same
-  // factors, in the same storage, bit for bit)
-  if (alg_only) factor(p, ln, alpha, negj, lu, w, alg_only);
-  else fo_gen_factor(lu - p.sl.lu * ln.L + ln.lane, alpha, p.o.gen_index);
+  double* base = lu - p.sl.lu * ln.L + ln.lane;
+  if (alg_only) {
+    fo_gen_factor_p(base, TEAM_W, TEAM_N, p.o.gen_index);
+  } else {
+    fo_gen_factor(base, alpha, TEAM_W, TEAM_N, p.o.gen_index);
+    if (p.sl.nb > 0) dense_lu(base + p.sl.dn * ln.L, p.sl.nb);
+  }
 #else
   if (p.o.variant == FO_VARIANT_PLAIN) factor(p, ln, alpha, negj, lu, w, alg_only);
   else if (p.o.variant == FO_VARIANT_COMPACT) {
@@ -680,18 +850,19 @@ __device__ __forceinline__ void solve_in_w(const SolveParams& p, const Lane& ln,
   else lu_solve_pipelined<0>(p, ln, lu, w);
 }
 
-// x = A^-1 b with the factors in lu (b and x per-lane vectors, may alias).
+// x = A^-1 b with the factors in lu (b and x per-lane vectors, may alias);
+// alg_only: the factors are the projection's.
 __device__ void solve_into(const SolveParams& p, const Lane& ln, const double* lu, double* w, const double* b,
-                           double* x) {
+                           double* x, bool alg_only = false) {
 #ifdef FO_LINK_GENERATED
   // the generated solves work on the slot's solve vector (item xs), whose
   // offset they know, so every access is an immediate offset from one base
-  const int L = ln.L, lane = ln.lane;
-  double* base = const_cast<double*>(lu) - p.sl.lu * L;
-  double* xs = base + p.sl.xs * L;
-  for (int i = 0; i < p.t.n; ++i) SCR(xs, i) = SCR(b, i);
-  fo_gen_solve(base + lane, p.o.gen_index);
-  for (int i = 0; i < p.t.n; ++i) SCR(x, i) = SCR(xs, i);
+  double* base = const_cast<double*>(lu) - p.sl.lu * ln.L;
+  double* xs = base + p.sl.xs * ln.L;
+  if (b != xs) copy_items(ln, p.t.n, b, xs);
+  if (alg_only) fo_gen_solve_p(base + ln.lane, TEAM_W, TEAM_N, p.o.gen_index);
+  else fo_gen_solve(base + ln.lane, TEAM_W, TEAM_N, p.o.gen_index);
+  if (x != xs) copy_items(ln, p.t.n, xs, x);
 #else
   if (p.o.variant == FO_VARIANT_COMPACT) {
     lu_solve_compact(p, ln, lu, w, b, x);
@@ -734,70 +905,133 @@ __device__ __noinline__ double attempt(const SolveParams& p, const Lane& ln, dou
   double* lu = scr + p.sl.lu * L;
   double* rr = scr + p.sl.r * L;
   const double* forcing = F0;
+  constexpr int kBatch = 4;   // species of a warp whose loads are in flight together
   for (int r = 0; r < tb.S; ++r) {
     if (r > 0 && tb.new_forcing[r]) {
-      for (int i = 0; i < n; ++i) {
-        double v = SCR(Y, i);
+      for (int i0 = TEAM_W; i0 < n; i0 += kBatch * TEAM_N) {
+        double v[kBatch];
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b)
+          if (i0 + b * TEAM_N < n) v[b] = SCR(Y, i0 + b * TEAM_N);
         for (int s = 0; s < r; ++s)
-          if (tb.a[r][s] != 0.0) v = __dadd_rn(v, __dmul_rn(tb.a[r][s], SCR(K + (int64_t)s * n * L, i)));
-        SCR(Yr, i) = v;
-        if (U != nullptr) SCR(U + (int64_t)r * n * L, i) = v;   // stage point kept for the adjoint
+          if (tb.a[r][s] != 0.0) {
+            double ks[kBatch];
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b)
+              if (i0 + b * TEAM_N < n) ks[b] = SCR(K + (int64_t)s * n * L, i0 + b * TEAM_N);
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b)
+              if (i0 + b * TEAM_N < n) v[b] = __dadd_rn(v[b], __dmul_rn(tb.a[r][s], ks[b]));
+          }
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+          const int i = i0 + b * TEAM_N;
+          if (i >= n) continue;
+          SCR(Yr, i) = v[b];
+          if (U != nullptr) SCR(U + (int64_t)r * n * L, i) = v[b];   // stage point kept for the adjoint
+        }
       }
       eval_rhs(p, ln, Yr, rr, Ft);
       ++c_rhs;
       forcing = Ft;
     }
     double* Kr = K + (int64_t)r * n * L;
-    const bool in_place = solves_in_place(p);   // right-hand side in Kr, solved in place
+    // the generated and compact solves take their right-hand side from a
+    // per-lane vector (the generated ones from theirs), the others from w
+    const bool in_place = solves_in_place(p);
+    double* rhs = generated(p) ? scr + p.sl.xs * L : Kr;
     // the stage's c(r, s) / H once per stage rather than once per species
     // (the same quotients, so the same sums bit for bit)
     double coefs[4];
     for (int s = 0; s < r; ++s) coefs[s] = __ddiv_rn(tb.c[r][s], H);
-    for (int i = 0; i < n; ++i) {
-      double v = SCR(forcing, i);
+    for (int i0 = TEAM_W; i0 < n; i0 += kBatch * TEAM_N) {
+      double v[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b)
+        if (i0 + b * TEAM_N < n) v[b] = SCR(forcing, i0 + b * TEAM_N);
       for (int s = 0; s < r; ++s) {
         const double coef = coefs[s];
-        if (coef != 0.0) {
-          double ks = SCR(K + (int64_t)s * n * L, i);
-          if (dae) ks = __dmul_rn(ks, __ldg(p.t.mass + i));
-          v = __dadd_rn(v, __dmul_rn(coef, ks));
+        if (coef == 0.0) continue;
+        double ks[kBatch];
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+          const int i = i0 + b * TEAM_N;
+          if (i >= n) continue;
+          ks[b] = SCR(K + (int64_t)s * n * L, i);
+          if (dae) ks[b] = __dmul_rn(ks[b], __ldg(p.t.mass + i));
         }
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b)
+          if (i0 + b * TEAM_N < n) v[b] = __dadd_rn(v[b], __dmul_rn(coef, ks[b]));
       }
-      if (in_place) SCR(Kr, i) = v;
-      else WROW(i) = v;
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int i = i0 + b * TEAM_N;
+        if (i >= n) continue;
+        if (in_place) SCR(rhs, i) = v[b];
+        else WROW(i) = v[b];
+      }
     }
     if (in_place) {
-      solve_into(p, ln, lu, w, Kr, Kr);
+      solve_into(p, ln, lu, w, rhs, Kr);
     } else {
       solve_in_w(p, ln, lu, w);
       for (int i = 0; i < n; ++i) SCR(Kr, i) = WROW(i);
     }
     ++c_solves;
   }
-  // Y_new, E and the weighted sum of squares
-  double acc = 0.0;
-  for (int i = 0; i < n; ++i) {
-    const double y = SCR(Y, i);
-    double yn = y, e = 0.0;
-    for (int r = 0; r < tb.S; ++r) {
-      const double kv = SCR(K + (int64_t)r * n * L, i);
-      if (tb.m[r] != 0.0) yn = __dadd_rn(yn, __dmul_rn(tb.m[r], kv));
-      if (tb.e[r] != 0.0) e = __dadd_rn(e, __dmul_rn(tb.e[r], kv));
+  // Y_new, E and the weighted sum of squares: min(n, 16) interleaved partial
+  // sums (species s, s + 16, ...), added in order, whatever the team's size
+  constexpr int kPartials = 16;
+  const int np = n < kPartials ? n : kPartials;
+  for (int s0 = TEAM_W; s0 < np; s0 += TEAM_N) {
+    double acc = 0.0;
+    for (int i0 = s0; i0 < n; i0 += kBatch * np) {
+      double yv[kBatch], yn[kBatch], e[kBatch], tol[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int i = i0 + b * np;
+        if (i >= n) continue;
+        yv[b] = yn[b] = SCR(Y, i);
+        e[b] = 0.0;
+        tol[b] = __ldg(p.atol + __ldg(p.t.perm + i));
+      }
+      for (int r = 0; r < tb.S; ++r) {
+        double ks[kBatch];
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b)
+          if (i0 + b * np < n) ks[b] = SCR(K + (int64_t)r * n * L, i0 + b * np);
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+          if (i0 + b * np >= n) continue;
+          if (tb.m[r] != 0.0) yn[b] = __dadd_rn(yn[b], __dmul_rn(tb.m[r], ks[b]));
+          if (tb.e[r] != 0.0) e[b] = __dadd_rn(e[b], __dmul_rn(tb.e[r], ks[b]));
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int i = i0 + b * np;
+        if (i >= n) continue;
+        SCR(Ynew, i) = yn[b];
+        // the restarting loop replaces the algebraic rows of the estimate by
+        // the step change (fastode/solvers.py:238-239)
+        if (p.o.loop == FO_LOOP_RESTARTING && p.o.step_change_rows && dae && __ldg(p.t.mass + i) == 0.0)
+          e[b] = __dsub_rn(yn[b], yv[b]);
+        const double ymax = npmax(fabs(yv[b]), fabs(yn[b]));
+        const double q = __ddiv_rn(e[b], __dadd_rn(tol[b], __dmul_rn(p.rtol, ymax)));
+        acc = __dadd_rn(acc, __dmul_rn(q, q));
+      }
     }
-    SCR(Ynew, i) = yn;
-    // the restarting loop replaces the algebraic rows of the estimate by the
-    // step change (fastode/solvers.py:238-239)
-    if (p.o.loop == FO_LOOP_RESTARTING && p.o.step_change_rows && dae && __ldg(p.t.mass + i) == 0.0)
-      e = __dsub_rn(yn, y);
-    const double ymax = npmax(fabs(y), fabs(yn));
-    const double s = __ddiv_rn(e, __dadd_rn(__ldg(p.atol + __ldg(p.t.perm + i)), __dmul_rn(p.rtol, ymax)));
-    acc = __dadd_rn(acc, __dmul_rn(s, s));
+    SCR(Ft, s0) = acc;
   }
-  return ln.active ? acc : 0.0;
+  team_sync();
+  double total = 0.0;
+  for (int s0 = 0; s0 < np; ++s0) total = __dadd_rn(total, SCR(Ft, s0));
+  return ln.active ? total : 0.0;
 }
 
 __device__ void trace_record(const SolveParams& p, int g, int& nrec, double t, double H, double err, double outcome) {
-  if (p.trace == nullptr || threadIdx.x != 0) {
+  if (p.trace == nullptr || !team_leader()) {
     ++nrec;
     return;
   }
@@ -814,10 +1048,10 @@ __device__ void trace_record(const SolveParams& p, int g, int& nrec, double t, d
 // Block-wide max with NaN propagation (numpy max) and block-wide AND.
 __device__ double block_max(double v, double* red) {
   for (int off = 16; off > 0; off >>= 1) v = npmax(v, __shfl_xor_sync(0xffffffffu, v, off));
-  const int nw = blockDim.x >> 5;
+  const int nw = (blockDim.x >> 5) * TEAM_N;
   if (nw == 1) return v;
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  if ((threadIdx.x & 31) == 0) red[(threadIdx.x >> 5) + TEAM_W] = v;
   __syncthreads();
   double s = red[0];
   for (int i = 1; i < nw; ++i) s = npmax(s, red[i]);
@@ -837,7 +1071,7 @@ __device__ bool alg_finite(const SolveParams& p, const Lane& ln, const double* A
   const int L = ln.L, lane = ln.lane;
   bool ok = true;
   if (ln.active)
-    for (int i = 0; i < p.t.n; ++i)
+    for (int i = TEAM_W; i < p.t.n; i += TEAM_N)
       if (__ldg(p.t.mass + i) == 0.0 && !isfinite(SCR(A, i))) ok = false;
   return block_all(ok);
 }
@@ -847,7 +1081,7 @@ __device__ double alg_absmax(const SolveParams& p, const Lane& ln, const double*
   const int L = ln.L, lane = ln.lane;
   double m = 0.0;
   if (ln.active)
-    for (int i = 0; i < p.t.n; ++i)
+    for (int i = TEAM_W; i < p.t.n; i += TEAM_N)
       if (__ldg(p.t.mass + i) == 0.0) m = npmax(m, fabs(SCR(A, i)));
   return block_max(m, red);
 }
@@ -859,7 +1093,7 @@ __device__ double weighted(const SolveParams& p, const Lane& ln, const double* Z
   const int L = ln.L, lane = ln.lane;
   double m = 0.0;
   if (ln.active)
-    for (int i = 0; i < p.t.n; ++i) {
+    for (int i = TEAM_W; i < p.t.n; i += TEAM_N) {
       if (__ldg(p.t.mass + i) != 0.0) continue;
       const double z = SCR(Z, i), d = SCR(D, i);
       const double scale =
@@ -877,14 +1111,10 @@ __device__ double weighted(const SolveParams& p, const Lane& ln, const double* Z
 __device__ void alg_residual(const SolveParams& p, const Lane& ln, const double* Z, double* rr, double* G) {
   const int L = ln.L, lane = ln.lane;
   eval_rhs(p, ln, Z, rr, G);
-  for (int i = 0; i < p.t.n; ++i)
+  for (int i = TEAM_W; i < p.t.n; i += TEAM_N)
     if (__ldg(p.t.mass + i) != 0.0) SCR(G, i) = 0.0;
 }
 
-__device__ void factor_any(const SolveParams& p, const Lane& ln, double alpha, const double* negj, double* lu,
-                           double* w, bool alg_only);
-__device__ void solve_into(const SolveParams& p, const Lane& ln, const double* lu, double* w, const double* b,
-                           double* x);
 
 // Consistent initialization of the algebraic species, fastode/solvers.py:100-178:
 // damped Newton with the algebraic-rows-only matrix (alpha = 1), accepted on
@@ -919,20 +1149,20 @@ __device__ __noinline__ bool project(const SolveParams& p, const Lane& ln, doubl
     ++pc.jac;
     factor_any(p, ln, 1.0, negj, lu, w, true);
     ++pc.lu;
-    solve_into(p, ln, lu, w, G, delta);
+    solve_into(p, ln, lu, w, G, delta, true);
     ++pc.solves;
     if (!alg_finite(p, ln, delta)) break;
     const double q = weighted(p, ln, Y, delta, red);
     if (q <= tol) return true;
     if (update == max_updates) break;
     if (!have_orig) {
-      for (int i = 0; i < n; ++i) SCR(orig, i) = SCR(Y, i);
+      for (int i = TEAM_W; i < n; i += TEAM_N) SCR(orig, i) = SCR(Y, i);
       have_orig = true;
     }
     double step = 1.0, step_used = 0.0;
     bool accepted = false;
     for (int bt = 0; bt <= max_backtracks; ++bt) {
-      for (int i = 0; i < n; ++i) {
+      for (int i = TEAM_W; i < n; i += TEAM_N) {
         double v = SCR(Y, i);
         if (__ldg(p.t.mass + i) == 0.0) v = __dadd_rn(v, __dmul_rn(step, SCR(delta, i)));
         SCR(cand, i) = v;
@@ -948,7 +1178,7 @@ __device__ __noinline__ bool project(const SolveParams& p, const Lane& ln, doubl
         accepted = true;
         break;
       }
-      solve_into(p, ln, lu, w, Gc, trial);
+      solve_into(p, ln, lu, w, Gc, trial, true);
       ++pc.solves;
       if (!alg_finite(p, ln, trial)) continue;
       const double qt = weighted(p, ln, cand, trial, red);
@@ -959,10 +1189,10 @@ __device__ __noinline__ bool project(const SolveParams& p, const Lane& ln, doubl
     }
     if (!accepted) break;
     trace_record(p, g, nrec, 0.0, step_used, q, 2.0);
-    for (int i = 0; i < n; ++i) SCR(Y, i) = SCR(cand, i);
+    for (int i = TEAM_W; i < n; i += TEAM_N) SCR(Y, i) = SCR(cand, i);
   }
   if (have_orig)
-    for (int i = 0; i < n; ++i) SCR(Y, i) = SCR(orig, i);
+    for (int i = TEAM_W; i < n; i += TEAM_N) SCR(Y, i) = SCR(orig, i);
   return false;
 }
 
@@ -992,7 +1222,7 @@ __device__ __noinline__ void solve_group_restarting(const SolveParams& p, int g,
   double* rr = scr + p.sl.r * L;
   double* lu = scr + p.sl.lu * L;
   load_rate_constants(p, ln, scr);
-  for (int i = 0; i < n; ++i) SCR(Y, i) = p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss];
+  for (int i = TEAM_W; i < n; i += TEAM_N) SCR(Y, i) = p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss];
   const double rounding = 2.220446049250313e-16;
   const double h_min = __dmul_rn(1.0e-15, dt);
   const double h_max = dt;
@@ -1064,12 +1294,12 @@ __device__ __noinline__ void solve_group_restarting(const SolveParams& p, int g,
   if (status < 0) status = FO_STATUS_CONVERGED;
   const bool clamp = status != FO_STATUS_PROJECTION_FAILED;
   if (ln.active)
-    for (int i = 0; i < n; ++i) {
+    for (int i = TEAM_W; i < n; i += TEAM_N) {
       double y = SCR(Y, i);
       if (clamp && (!p.t.has_constraints || __ldg(p.t.mass + i) == 1.0)) y = clamp0(y);
       p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss] = y;
     }
-  if (threadIdx.x == 0) {
+  if (team_leader()) {
     long long* cn = p.counts + (int64_t)g * FO_NUM_COUNTS;
     cn[0] += c_steps;
     cn[1] += c_acc;
@@ -1117,7 +1347,7 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
   double* lu = scr + p.sl.lu * L;
   const bool in_place = solves_in_place(p);   // Newton update solved in place in F
   load_rate_constants(p, ln, scr);
-  for (int i = 0; i < n; ++i) {
+  for (int i = TEAM_W; i < n; i += TEAM_N) {
     const double v = p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss];
     SCR(Yn, i) = v;
     SCR(Yn1, i) = v;
@@ -1140,7 +1370,7 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
       ++c_jac;
       factor_any(p, ln, 1.0 / H, negj, lu, w, false);
       ++c_lu;
-      for (int i = 0; i < n; ++i) {
+      for (int i = TEAM_W; i < n; i += TEAM_N) {
         const double v = __dsub_rn(SCR(F, i), __ddiv_rn(__dsub_rn(SCR(Yn1, i), SCR(Yn, i)), H));
         if (in_place) SCR(F, i) = v;
         else WROW(i) = v;
@@ -1150,7 +1380,7 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
       ++c_solves;
       ++iterations;
       bool conv = true;
-      for (int i = 0; i < n; ++i) {
+      for (int i = TEAM_W; i < n; i += TEAM_N) {
         const double d = in_place ? SCR(F, i) : WROW(i);
         const double y = clamp0(__dadd_rn(SCR(Yn1, i), d));
         SCR(Yn1, i) = y;
@@ -1172,17 +1402,17 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
         ++c_unconv;
         status = FO_STATUS_ACCEPTED_UNCONVERGED;
         bool finite = true;
-        for (int i = 0; i < n; ++i) finite = finite && isfinite(SCR(Yn1, i));
+        for (int i = TEAM_W; i < n; i += TEAM_N) finite = finite && isfinite(SCR(Yn1, i));
         if (!block_all(!ln.active || finite)) status = FO_STATUS_NAN_OR_INF;
         break;
       }
-      for (int i = 0; i < n; ++i) SCR(Yn1, i) = SCR(Yn, i);
+      for (int i = TEAM_W; i < n; i += TEAM_N) SCR(Yn1, i) = SCR(Yn, i);
       H = __dmul_rn(H, o.reductions[n_fail]);
       ++n_fail;
     } else {
       ++c_acc;
       t = __dadd_rn(t, H);
-      for (int i = 0; i < n; ++i) SCR(Yn, i) = SCR(Yn1, i);
+      for (int i = TEAM_W; i < n; i += TEAM_N) SCR(Yn, i) = SCR(Yn1, i);
       ++n_success;
       if (n_success >= 2) {
         n_success = 0;
@@ -1192,12 +1422,12 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
     H = pymin(H, __dsub_rn(dt, t));
   }
   if (ln.active)
-    for (int i = 0; i < n; ++i) {
+    for (int i = TEAM_W; i < n; i += TEAM_N) {
       double y = SCR(Yn1, i);
       if (!p.t.has_constraints || __ldg(p.t.mass + i) == 1.0) y = clamp0(y);
       p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss] = y;
     }
-  if (threadIdx.x == 0) {
+  if (team_leader()) {
     long long* cn = p.counts + (int64_t)g * FO_NUM_COUNTS;
     cn[0] += c_steps;
     cn[1] += c_acc;
@@ -1239,7 +1469,7 @@ constexpr long long kRoundSpinLimit = 7500000;
 __device__ int round_barrier(unsigned int* w, int active) {
   __shared__ int result;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (team_leader()) {
     volatile unsigned int* vw = w;
     if (vw[4] != 0u) {
       result = -1;
@@ -1287,7 +1517,7 @@ __device__ __forceinline__ void load_batch_params(const SolveParams* __restrict_
   __syncthreads();
   const long long* src = reinterpret_cast<const long long*>(batches + b);
   long long* dst = reinterpret_cast<long long*>(&shared);
-  for (int i = threadIdx.x; i < (int)(sizeof(SolveParams) / sizeof(long long)); i += blockDim.x) dst[i] = src[i];
+  for (int i = threadIdx.x; TEAM_W == 0 && i < (int)(sizeof(SolveParams) / sizeof(long long)); i += blockDim.x) dst[i] = src[i];
   __syncthreads();
   current = b;
 }
@@ -1333,7 +1563,7 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
   double* lu = scr + p.sl.lu * L;
 
   load_rate_constants(p, ln, scr);
-  for (int i = 0; i < n; ++i) SCR(Y, i) = p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss];
+  for (int i = TEAM_W; i < n; i += TEAM_N) SCR(Y, i) = p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss];
 
   double* mem = p.memory + (int64_t)g * 3;
   double h_next = mem[0], err_prev = mem[1], h_prev = mem[2];
@@ -1457,13 +1687,13 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
   // returns the restored state unclamped (fastode/solvers.py:323-325)
   const bool clamp = status != FO_STATUS_PROJECTION_FAILED;
   if (ln.active) {
-    for (int i = 0; i < n; ++i) {
+    for (int i = TEAM_W; i < n; i += TEAM_N) {
       double y = SCR(Y, i);
       if (clamp && (!p.t.has_constraints || __ldg(p.t.mass + i) == 1.0)) y = clamp0(y);
       p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss] = y;
     }
   }
-  if (threadIdx.x == 0) {
+  if (team_leader()) {
     mem[0] = proposed;
     mem[1] = err_prev;
     mem[2] = h_prev;

@@ -74,8 +74,7 @@ class Part:
         lanes = ((self.max_cells + 31) // 32) * 32
         kernel = getattr(self.alg, "kernel", "pipelined")
         if kernel == "generated" and self.max_cells <= 32:
-            # the reduction buffer, and the projection's work row of a constrained mechanism
-            return 8 * (32 + (self.n * lanes if self.plan.has_constraints else 0))
+            return 8 * 32                     # the reduction buffer
         return 8 * (32 + self.plan.smem_items("compact" if kernel == "generated" else kernel) * lanes)
 
     def generated(self) -> bool:
