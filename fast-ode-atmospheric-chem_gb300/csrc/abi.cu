@@ -61,6 +61,7 @@ int fo::set_last_error(int code, const char* what) { return fail(code, what); }
 
 namespace {
 
+using fo::adjoint_layout;
 using fo::layout_of;
 
 const fo::DevTableau kTableaus[2] = {
@@ -667,30 +668,6 @@ int fo_multi_destroy(fo_multi* m) {
 }
 
 }  // extern "C"
-
-namespace {
-
-fo::AdjLayout adjoint_layout(const fo::HostTables& t, int max_steps) {
-  fo::AdjLayout a;
-  int64_t o = layout_of(t).items;
-  a.ys = o; o += (int64_t)max_steps * t.n;
-  a.u = o; o += 4LL * t.n;
-  a.kbar = o; o += 4LL * t.n;
-  a.fbar = o; o += 4LL * t.n;
-  a.ybar = o; o += t.n;
-  a.g = o; o += t.n;
-  a.jbar = o; o += (int64_t)t.j_col.size();
-  a.dbar = o; o += (int64_t)t.R * t.P;
-  bool constrained = false;
-  for (double m : t.mass) constrained = constrained || m == 0.0;
-  a.yp = o; o += constrained ? (int64_t)fo::kMaxProjectionUpdates * t.n : 0;
-  a.pdelta = o; o += constrained ? t.n : 0;
-  a.pmu = o; o += constrained ? t.n : 0;
-  a.items = o;
-  return a;
-}
-
-}  // namespace
 
 extern "C" {
 

@@ -82,11 +82,78 @@ __device__ __noinline__ void lu_solve_transposed(const SolveParams& p, const Lan
   }
 }
 
+#ifdef FO_LINK_GENERATED
+// logk_bar_j += w_j rate_j (w_j alone without rates), each warp its reactions.
+__device__ __forceinline__ void add_log_k(const AdjParams& a, const Lane& ln, const double* w, const double* rate) {
+  constexpr int kBatch = 8;
+  const int L = ln.L, lane = ln.lane, R = a.p.t.R;
+  double* th = a.thbar + ln.cell * a.tcs;
+  for (int j0 = TEAM_W; j0 < R; j0 += kBatch * TEAM_N) {
+    double t[kBatch], u[kBatch], r[kBatch];
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      const int j = j0 + b * TEAM_N;
+      if (j >= R) continue;
+      t[b] = th[(int64_t)j * a.trs];
+      u[b] = SCR(w, j);
+      r[b] = rate ? SCR(rate, j) : 1.0;
+    }
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      const int j = j0 + b * TEAM_N;
+      if (j < R && ln.active) th[(int64_t)j * a.trs] = fma(u[b], r[b], t[b]);
+    }
+  }
+}
+#endif
+
+// jbar_e = sum over the rows' stages s = S-1 .. 0 of mu_s[i] K_s[col(e)] (the
+// stages' outer products on the Jacobian's pattern); `only_algebraic`: zero on
+// the differential rows.
+__device__ __forceinline__ void outer_products(const SolveParams& p, const Lane& ln, int S, const double* mu,
+                                               const double* K, double* jbar, bool only_algebraic) {
+  constexpr int kBatch = 8;
+  const int L = ln.L, lane = ln.lane, n = p.t.n;
+  for (int i = TEAM_W; i < n; i += TEAM_N) {
+    const bool zero = only_algebraic && __ldg(p.t.mass + i) != 0.0;
+    double m[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) m[s] = s < S ? SCR(mu + (int64_t)s * n * L, i) : 0.0;
+    const int e1 = __ldg(p.t.j_row_ptr + i + 1);
+    for (int e0 = __ldg(p.t.j_row_ptr + i); e0 < e1; e0 += kBatch) {
+      double acc[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) acc[b] = 0.0;
+#pragma unroll
+      for (int s = 3; s >= 0; --s) {
+        if (s >= S || zero) continue;
+        double v[kBatch];
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b)
+          if (e0 + b < e1) v[b] = SCR(K + (int64_t)s * n * L, __ldg(p.t.j_col + e0 + b));
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b)
+          if (e0 + b < e1) acc[b] = fma(m[s], v[b], acc[b]);
+      }
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b)
+        if (e0 + b < e1) SCR(jbar, e0 + b) = acc[b];
+    }
+  }
+}
+
 // g = J(x)^T v for the mass-action forcing at x, and logk_bar += r(x) * (S^T v).
 __device__ __noinline__ void vjp_forcing(const AdjParams& a, const Lane& ln, const double* x, const double* v,
                                          double* g) {
   const SolveParams& p = a.p;
   const int L = ln.L, lane = ln.lane;
+#ifdef FO_LINK_GENERATED
+  double* base = g - a.al.g * L;
+  copy_items(ln, p.t.n, x, base + p.sl.yr * L);
+  copy_items(ln, p.t.n, v, base + a.al.v * L);
+  fo_gen_vjp(base + lane, TEAM_W, TEAM_N, p.o.gen_index);
+  add_log_k(a, ln, base + a.al.w * L, base + a.al.rate * L);
+#else
   const int n = p.t.n, R = p.t.R, P = p.t.P;
   const double* kc = p.k + ln.cell * p.kcs;
   double* th = a.thbar + ln.cell * a.tcs;
@@ -114,6 +181,7 @@ __device__ __noinline__ void vjp_forcing(const AdjParams& a, const Lane& ln, con
       SCR(g, s) = fma(wj, d, SCR(g, s));
     }
   }
+#endif
 }
 
 // ybar += grad_y sum_e Jbar_e J_e(y) and logk_bar += its log k derivative:
@@ -122,6 +190,12 @@ __device__ __noinline__ void hvp_jacobian(const AdjParams& a, const Lane& ln, co
                                           double* dbar, double* ybar) {
   const SolveParams& p = a.p;
   const int L = ln.L, lane = ln.lane;
+#ifdef FO_LINK_GENERATED
+  double* base = ybar - a.al.ybar * L;
+  copy_items(ln, p.t.n, y, base + p.sl.yr * L);
+  fo_gen_hvp(base + lane, TEAM_W, TEAM_N, p.o.gen_index);
+  add_log_k(a, ln, base + a.al.w * L, nullptr);
+#else
   const int n = p.t.n, R = p.t.R, P = p.t.P;
   const double* kc = p.k + ln.cell * p.kcs;
   double* th = a.thbar + ln.cell * a.tcs;
@@ -162,6 +236,7 @@ __device__ __noinline__ void hvp_jacobian(const AdjParams& a, const Lane& ln, co
     }
     if (ln.active) th[(int64_t)j * a.trs] += th_j;
   }
+#endif
 }
 
 // The reverse sweep of one step whose forward pass left K_r and the stage
@@ -176,7 +251,9 @@ __device__ __noinline__ void reverse_step(const AdjParams& a, const Lane& ln, do
   const bool dae = p.t.has_constraints != 0;
   const double* K = scr + p.sl.k * L;
   const double* U = scr + a.al.u * L;
+#ifndef FO_LINK_GENERATED
   const double* lu = scr + p.sl.lu * L;
+#endif
   double* Kbar = scr + a.al.kbar * L;
   double* Fbar = scr + a.al.fbar * L;
   double* ybar = scr + a.al.ybar * L;
@@ -185,32 +262,28 @@ __device__ __noinline__ void reverse_step(const AdjParams& a, const Lane& ln, do
   double* dbar = scr + a.al.dbar * L;
   const int S = tb.S;
   for (int r = 0; r < S; ++r)
-    for (int i = 0; i < n; ++i) {
+    for (int i = TEAM_W; i < n; i += TEAM_N) {
       SCR(Kbar + (int64_t)r * n * L, i) = tb.m[r] * SCR(ybar, i);
       SCR(Fbar + (int64_t)r * n * L, i) = 0.0;
     }
-  for (int e = 0; e < p.t.nnzj; ++e) SCR(jbar, e) = 0.0;
   for (int r = S - 1; r >= 0; --r) {
     int f = r;
     while (f > 0 && !tb.new_forcing[f]) --f;
 #ifdef FO_LINK_GENERATED
     // the generated transposed solve works on the slot's solve vector
     double* muv = scr + p.sl.xs * L;
-    for (int i = 0; i < n; ++i) SCR(muv, i) = SCR(Kbar + (int64_t)r * n * L, i);
+    for (int i = TEAM_W; i < n; i += TEAM_N) SCR(muv, i) = SCR(Kbar + (int64_t)r * n * L, i);
     fo_gen_solve_t(scr + lane, TEAM_W, TEAM_N, p.o.gen_index);           // mu_r
 #else
     double* muv = w;
-    for (int i = 0; i < n; ++i) WROW(i) = SCR(Kbar + (int64_t)r * n * L, i);
+    for (int i = TEAM_W; i < n; i += TEAM_N) WROW(i) = SCR(Kbar + (int64_t)r * n * L, i);
     lu_solve_transposed(p, ln, lu, w);                                   // w = mu_r
 #endif
-    const double* Kr = K + (int64_t)r * n * L;
     double coefs[4];                                                     // c(r, s) / h once per stage
     for (int s = 0; s < r; ++s) coefs[s] = tb.c[r][s] / h;
-    for (int i = 0; i < n; ++i) {
+    for (int i = TEAM_W; i < n; i += TEAM_N) {
       const double mu = SCR(muv, i);
-      const int e1 = __ldg(p.t.j_row_ptr + i + 1);
-      for (int e = __ldg(p.t.j_row_ptr + i); e < e1; ++e)
-        SCR(jbar, e) = fma(mu, SCR(Kr, __ldg(p.t.j_col + e)), SCR(jbar, e));
+      SCR(Kbar + (int64_t)r * n * L, i) = mu;   // kept for the outer products
       double* Ff = Fbar + (int64_t)f * n * L;
       SCR(Ff, i) += mu;
       for (int s = 0; s < r; ++s) {
@@ -225,7 +298,7 @@ __device__ __noinline__ void reverse_step(const AdjParams& a, const Lane& ln, do
     if (r == f) {
       const double* x = r == 0 ? y : U + (int64_t)r * n * L;
       vjp_forcing(a, ln, x, Fbar + (int64_t)f * n * L, g);
-      for (int i = 0; i < n; ++i) {
+      for (int i = TEAM_W; i < n; i += TEAM_N) {
         const double gi = SCR(g, i);
         SCR(ybar, i) += gi;
         for (int s = 0; s < r; ++s)
@@ -236,6 +309,7 @@ __device__ __noinline__ void reverse_step(const AdjParams& a, const Lane& ln, do
       }
     }
   }
+  outer_products(p, ln, S, Kbar, K, jbar, false);
   hvp_jacobian(a, ln, y, jbar, dbar, ybar);
 }
 
@@ -247,13 +321,13 @@ __device__ void solve_transposed_into(const SolveParams& p, const Lane& ln, cons
   const int n = p.t.n;
 #ifdef FO_LINK_GENERATED
   double* v = scr + p.sl.xs * L;
-  for (int i = 0; i < n; ++i) SCR(v, i) = SCR(b, i);
+  for (int i = TEAM_W; i < n; i += TEAM_N) SCR(v, i) = SCR(b, i);
   fo_gen_solve_tp(scr + lane, TEAM_W, TEAM_N, p.o.gen_index);
-  for (int i = 0; i < n; ++i) SCR(x, i) = SCR(v, i);
+  for (int i = TEAM_W; i < n; i += TEAM_N) SCR(x, i) = SCR(v, i);
 #else
-  for (int i = 0; i < n; ++i) WROW(i) = SCR(b, i);
+  for (int i = TEAM_W; i < n; i += TEAM_N) WROW(i) = SCR(b, i);
   lu_solve_transposed(p, ln, lu, w);
-  for (int i = 0; i < n; ++i) SCR(x, i) = WROW(i);
+  for (int i = TEAM_W; i < n; i += TEAM_N) SCR(x, i) = WROW(i);
 #endif
 }
 
@@ -290,18 +364,13 @@ __device__ void reverse_projection_update(const AdjParams& a, const Lane& ln, do
   double* jbar = scr + a.al.jbar * L;
   double* dbar = scr + a.al.dbar * L;
   projection_delta(a, ln, y, scr, w, delta);                       // lu: the factors of A(y)
-  for (int i = 0; i < n; ++i) SCR(mu, i) = s * SCR(ybar, i);
+  for (int i = TEAM_W; i < n; i += TEAM_N) SCR(mu, i) = s * SCR(ybar, i);
   solve_transposed_into(p, ln, scr + p.sl.lu * L, scr, w, mu, mu);
-  for (int i = 0; i < n; ++i) {
-    const bool alg = __ldg(p.t.mass + i) == 0.0;
-    const double m = SCR(mu, i);
-    const int e1 = __ldg(p.t.j_row_ptr + i + 1);
-    for (int e = __ldg(p.t.j_row_ptr + i); e < e1; ++e)
-      SCR(jbar, e) = alg ? m * SCR(delta, __ldg(p.t.j_col + e)) : 0.0;
-    if (!alg) SCR(mu, i) = 0.0;                                     // G has no differential rows
-  }
+  outer_products(p, ln, 1, mu, delta, jbar, true);
+  for (int i = TEAM_W; i < n; i += TEAM_N)
+    if (__ldg(p.t.mass + i) != 0.0) SCR(mu, i) = 0.0;               // G has no differential rows
   vjp_forcing(a, ln, y, mu, g);
-  for (int i = 0; i < n; ++i) SCR(ybar, i) += SCR(g, i);
+  for (int i = TEAM_W; i < n; i += TEAM_N) SCR(ybar, i) += SCR(g, i);
   hvp_jacobian(a, ln, y, jbar, dbar, ybar);
 }
 
@@ -332,7 +401,7 @@ __device__ void adjoint_group(const AdjParams& a, double* w) {
   double* scr = p.scratch + (int64_t)g * p.slot_doubles;
   const int s0 = a.step_ptr[g], m = a.step_ptr[g + 1] - s0;
   if (m > a.max_steps) {
-    if (threadIdx.x == 0) a.status[g] = FO_STATUS_TOO_MANY_STEPS;
+    if (team_leader()) a.status[g] = FO_STATUS_TOO_MANY_STEPS;
     return;
   }
   double* Y = scr + p.sl.y * L;
@@ -341,27 +410,27 @@ __device__ void adjoint_group(const AdjParams& a, double* w) {
   double* U = scr + a.al.u * L;
   double* ybar = scr + a.al.ybar * L;
   load_rate_constants(p, ln, scr);
-  for (int i = 0; i < n; ++i) SCR(Y, i) = a.Ycp[ln.cell * a.ycs + (int64_t)__ldg(p.t.perm + i) * a.yss];
+  for (int i = TEAM_W; i < n; i += TEAM_N) SCR(Y, i) = a.Ycp[ln.cell * a.ycs + (int64_t)__ldg(p.t.perm + i) * a.yss];
   // replay the projection's updates (constrained systems), keeping the state
   // before each
   const int q0 = a.proj_ptr ? a.proj_ptr[g] : 0, nq = a.proj_ptr ? a.proj_ptr[g + 1] - q0 : 0;
   if (nq > kMaxProjectionUpdates) {
-    if (threadIdx.x == 0) a.status[g] = FO_STATUS_PROJECTION_FAILED;
+    if (team_leader()) a.status[g] = FO_STATUS_PROJECTION_FAILED;
     return;
   }
   double* yp = scr + a.al.yp * L;
   for (int u = 0; u < nq; ++u) {
     double* yu = yp + (int64_t)u * n * L;
     double* delta = scr + a.al.pdelta * L;
-    for (int i = 0; i < n; ++i) SCR(yu, i) = SCR(Y, i);
+    for (int i = TEAM_W; i < n; i += TEAM_N) SCR(yu, i) = SCR(Y, i);
     projection_delta(a, ln, Y, scr, w, delta);
     const double st = a.proj_steps[q0 + u];
-    for (int i = 0; i < n; ++i)
+    for (int i = TEAM_W; i < n; i += TEAM_N)
       if (__ldg(p.t.mass + i) == 0.0) SCR(Y, i) = __dadd_rn(SCR(Y, i), __dmul_rn(st, SCR(delta, i)));
   }
   // replay the accepted steps, keeping the state at the start of each
   for (int s = 0; s < m; ++s) {
-    for (int i = 0; i < n; ++i) SCR(ys + (int64_t)s * n * L, i) = SCR(Y, i);
+    for (int i = TEAM_W; i < n; i += TEAM_N) SCR(ys + (int64_t)s * n * L, i) = SCR(Y, i);
     fixed_step(a, ln, a.steps[s0 + s], Y, Ynew, scr, w, U);
     double* t = Y;
     Y = Ynew;
@@ -370,16 +439,16 @@ __device__ void adjoint_group(const AdjParams& a, double* w) {
   const bool constrained = p.t.has_constraints != 0;
   if (a.mode == 0) {
     if (ln.active)
-      for (int i = 0; i < n; ++i) {
+      for (int i = TEAM_W; i < n; i += TEAM_N) {
         double y = SCR(Y, i);
         if (!constrained || __ldg(p.t.mass + i) == 1.0) y = clamp0(y);
         a.Yout[ln.cell * a.ocs + (int64_t)__ldg(p.t.perm + i) * a.oss] = y;
       }
-    if (threadIdx.x == 0) a.status[g] = FO_STATUS_CONVERGED;
+    if (team_leader()) a.status[g] = FO_STATUS_CONVERGED;
     return;
   }
   // dL/dY at the end of the interval through the clamp
-  for (int i = 0; i < n; ++i) {
+  for (int i = TEAM_W; i < n; i += TEAM_N) {
     double lam = a.lam[ln.cell * a.lcs + (int64_t)__ldg(p.t.perm + i) * a.lss];
     if ((!constrained || __ldg(p.t.mass + i) == 1.0) && !(SCR(Y, i) > 0.0)) lam = 0.0;
     SCR(ybar, i) = lam;
@@ -393,13 +462,13 @@ __device__ void adjoint_group(const AdjParams& a, double* w) {
   for (int u = nq - 1; u >= 0; --u)
     reverse_projection_update(a, ln, a.proj_steps[q0 + u], yp + (int64_t)u * n * L, scr, w);
   bool finite = true;
-  for (int i = 0; i < n; ++i) {
+  for (int i = TEAM_W; i < n; i += TEAM_N) {
     const double v = SCR(ybar, i);
     if (!isfinite(v)) finite = false;
     if (ln.active) a.lam[ln.cell * a.lcs + (int64_t)__ldg(p.t.perm + i) * a.lss] = v;
   }
   finite = __syncthreads_and(finite ? 1 : 0) != 0;
-  if (threadIdx.x == 0) a.status[g] = finite ? FO_STATUS_CONVERGED : FO_STATUS_NAN_OR_INF;
+  if (team_leader()) a.status[g] = finite ? FO_STATUS_CONVERGED : FO_STATUS_NAN_OR_INF;
 }
 
 }  // namespace

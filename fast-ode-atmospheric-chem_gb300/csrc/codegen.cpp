@@ -45,6 +45,7 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <memory>
 #include <stdexcept>
 #include <utility>
 #include <vector>
@@ -654,6 +655,127 @@ Phase jac_phase(const HostTables& t, const GenLayout& gl) {
   return p;
 }
 
+// The adjoint's forcing product: g = J(yr)^T v (items v, g of the adjoint's
+// scratch), reaction by reaction the weights w_j = (S^T v)_j and the rates,
+// then species by species the sums of w_j d[j, q] over the reactant slots
+// that hold it, in ascending (j, q): the table-driven scatter's order. A
+// gather per species needs no order between the warps of a team: with the
+// scatter the adjoint ran one warp per group (4,096 cells of the 210/500
+// mechanism, one cold interval recorded and reversed: 1.42 s, now 0.315 s).
+Phase vjp_phase(const HostTables& t, const GenLayout& gl, const AdjLayout& al) {
+  const ScratchLayout& sl = gl.s;
+  Phase p;
+  p.push_back(ranges(t.R, 4, [&t, &gl, &sl, &al](Ptx& x, int j0, int j1) {
+    for (int j = j0; j < j1; ++j) {
+      const int k = x.load(sl.kc + j);
+      std::vector<int> f(t.P, -1);
+      for (int q = 0; q < t.P; ++q)
+        if (t.react[(size_t)j * t.P + q] != t.n) f[q] = x.load(sl.yr + t.react[(size_t)j * t.P + q]);
+      int w = -1;
+      for (int e = t.st_ptr[j]; e < t.st_ptr[j + 1]; ++e) {
+        const int v = x.load(al.v + t.st_sp[e]);
+        w = w < 0 ? x.mul_imm(v, t.st_val[e]) : x.fma_imm(v, t.st_val[e], w);
+      }
+      x.store(al.w + j, w < 0 ? x.constant(0.0) : w);
+      int rate = k;
+      for (int q = 0; q < t.P; ++q)
+        if (f[q] >= 0) rate = x.mul(rate, f[q]);
+      x.store(al.rate + j, rate);
+      for (int a = 0; a < t.P; ++a) {
+        if (gl.d_item[(size_t)j * t.P + a] < 0) continue;
+        int d = k;
+        for (int q = 0; q < t.P; ++q)
+          if (q != a && f[q] >= 0) d = x.mul(d, f[q]);
+        x.store(gl.d_item[(size_t)j * t.P + a], d);
+      }
+    }
+  }));
+  std::vector<std::vector<int>> uses(t.n);
+  for (int jq = 0; jq < t.R * t.P; ++jq)
+    if (t.react[jq] != t.n && t.st_ptr[jq / t.P] < t.st_ptr[jq / t.P + 1]) uses[t.react[jq]].push_back(jq);
+  std::vector<Task> rows;
+  for (int i = 0; i < t.n; ++i)
+    rows.push_back({{}, [&t, &gl, &sl, &al, i, u = uses[i]](Ptx& x) {
+      int acc = -1;
+      for (int jq : u) {
+        const int w = x.load(al.w + jq / t.P);
+        const int d = x.load(gl.d_item[jq] >= 0 ? gl.d_item[jq] : sl.kc + jq / t.P);
+        acc = acc < 0 ? x.mul(w, d) : x.fma(w, d, acc);
+      }
+      x.store(al.g + i, acc < 0 ? x.constant(0.0) : acc);
+    }});
+  for (auto& s : schedule(rows)) p.push_back(std::move(s));
+  return p;
+}
+
+// The second derivatives of the Jacobian at yr contracted with jbar: dbar, the
+// adjoint of every d[j, q], and the reactions' log k derivatives (item w),
+// then ybar gains dbar[j, q] dd over the slots q2 != q that hold each species,
+// in ascending (j, q, q2).
+Phase hvp_phase(const HostTables& t, const GenLayout& gl, const AdjLayout& al) {
+  const ScratchLayout& sl = gl.s;
+  // the Jacobian entries each d[j, q] enters, in ascending order
+  auto terms = std::make_shared<std::vector<std::vector<std::pair<int, double>>>>((size_t)t.R * t.P);
+  for (int e = 0; e + 1 < (int)t.jt_ptr.size(); ++e)
+    for (int q = t.jt_ptr[e]; q < t.jt_ptr[e + 1]; ++q) (*terms)[t.jt_idx[q]].push_back({e, -t.jt_val[q]});
+  Phase p;
+  std::vector<Task> reactions;
+  for (int j = 0; j < t.R; ++j)
+    reactions.push_back({{}, [&t, &sl, &al, terms, j](Ptx& x) {
+      const int k = x.load(sl.kc + j);
+      std::vector<int> f(t.P, -1);
+      for (int q = 0; q < t.P; ++q)
+        if (t.react[(size_t)j * t.P + q] != t.n) f[q] = x.load(sl.yr + t.react[(size_t)j * t.P + q]);
+      int th = -1;
+      for (int q = 0; q < t.P; ++q) {
+        if (f[q] < 0) continue;
+        int db = -1;
+        for (const auto& [e, c] : (*terms)[(size_t)j * t.P + q]) {
+          const int v = x.load(al.jbar + e);
+          db = db < 0 ? x.mul_imm(v, c) : x.fma_imm(v, c, db);
+        }
+        if (db < 0) db = x.constant(0.0);
+        x.store(al.dbar + (int64_t)j * t.P + q, db);
+        int d = k;
+        for (int q2 = 0; q2 < t.P; ++q2)
+          if (q2 != q && f[q2] >= 0) d = x.mul(d, f[q2]);
+        th = th < 0 ? x.mul(db, d) : x.fma(db, d, th);
+      }
+      x.store(al.w + j, th < 0 ? x.constant(0.0) : th);
+    }});
+  for (auto& s : schedule(reactions)) p.push_back(std::move(s));
+  struct Use {
+    int jq, q2;
+  };
+  std::vector<std::vector<Use>> uses(t.n);
+  for (int j = 0; j < t.R; ++j)
+    for (int q = 0; q < t.P; ++q) {
+      if (t.react[(size_t)j * t.P + q] == t.n || (*terms)[(size_t)j * t.P + q].empty()) continue;
+      for (int q2 = 0; q2 < t.P; ++q2)
+        if (q2 != q && t.react[(size_t)j * t.P + q2] != t.n)
+          uses[t.react[(size_t)j * t.P + q2]].push_back({j * t.P + q, q2});
+    }
+  std::vector<Task> rows;
+  for (int i = 0; i < t.n; ++i) {
+    if (uses[i].empty()) continue;
+    rows.push_back({{}, [&t, &sl, &al, i, u = uses[i]](Ptx& x) {
+      int acc = x.load(al.ybar + i);
+      for (const Use& o : u) {
+        const int j = o.jq / t.P;
+        const int db = x.load(al.dbar + o.jq);
+        int dd = x.load(sl.kc + j);
+        for (int q3 = 0; q3 < t.P; ++q3)
+          if (q3 != o.jq % t.P && q3 != o.q2 && t.react[(size_t)j * t.P + q3] != t.n)
+            dd = x.mul(dd, x.load(sl.yr + t.react[(size_t)j * t.P + q3]));
+        acc = x.fma(db, dd, acc);
+      }
+      x.store(al.ybar + i, acc);
+    }});
+  }
+  for (auto& s : schedule(rows)) p.push_back(std::move(s));
+  return p;
+}
+
 // One phase of every mechanism as a function that all warps of a team call:
 //   .visible .func name(base, [alpha,] warp, warps, mech)
 // A team barrier, then mechanism mech's steps: warp w runs the segments w,
@@ -738,13 +860,17 @@ std::string generate_ptx(const std::vector<const HostTables*>& ts, const std::ve
       throw std::invalid_argument("generation options out of range");
   const size_t count = ts.size();
   std::vector<GenLayout> layouts;
+  std::vector<AdjLayout> adjoints;
   std::vector<Matrix> full, proj;
-  for (const HostTables* t : ts) layouts.push_back(gen_layout_of(*t));
+  for (const HostTables* t : ts) {
+    layouts.push_back(gen_layout_of(*t));
+    adjoints.push_back(adjoint_layout(*t, 0));
+  }
   for (size_t m = 0; m < count; ++m) {
     full.push_back(full_matrix(*ts[m], layouts[m]));
     proj.push_back(projection_matrix(*ts[m], layouts[m]));
   }
-  std::vector<Phase> rhs, jac, factor, solve, solve_t, pfactor, psolve, psolve_t;
+  std::vector<Phase> rhs, jac, factor, solve, solve_t, pfactor, psolve, psolve_t, vjp, hvp;
   int64_t expected = 0;
   for (size_t m = 0; m < count; ++m) {
     const HostTables& t = *ts[m];
@@ -752,6 +878,8 @@ std::string generate_ptx(const std::vector<const HostTables*>& ts, const std::ve
     const GenOptions& o = os[m];
     rhs.push_back(rhs_phase(t, gl.s));
     jac.push_back(jac_phase(t, gl));
+    vjp.push_back(vjp_phase(t, gl, adjoints[m]));
+    hvp.push_back(hvp_phase(t, gl, adjoints[m]));
     factor.push_back(schedule(factor_tasks(full[m], gl, o.tile)));
     solve.push_back(solve_phase(full[m], gl.s, o.solve_block));
     solve_t.push_back(solve_t_phase(full[m], gl.s, o.solve_block));
@@ -779,6 +907,8 @@ std::string generate_ptx(const std::vector<const HostTables*>& ts, const std::ve
   out += phase_function("fo_gen_solve_t", false, solve_t, lines, &ignored);
   out += phase_function("fo_gen_rhs", false, rhs, lines, &ignored);
   out += phase_function("fo_gen_jac", false, jac, lines, &ignored);
+  out += phase_function("fo_gen_vjp", false, vjp, lines, &ignored);
+  out += phase_function("fo_gen_hvp", false, hvp, lines, &ignored);
   out += phase_function("fo_gen_factor_p", false, pfactor, lines, &ignored);
   out += phase_function("fo_gen_solve_p", false, psolve, lines, &ignored);
   out += phase_function("fo_gen_solve_tp", false, psolve_t, lines, &ignored);

@@ -38,6 +38,8 @@ struct GenOptions {
 //                    (dense_lu finishes it)
 //   fo_gen_solve     overwrites the solve vector (item xs) with (LU)^-1 of it
 //   fo_gen_solve_t   ... with (LU)^-T of it, for the adjoint
+//   fo_gen_vjp       the adjoint's J(yr)^T v, weights and rates
+//   fo_gen_hvp       the adjoint's second derivatives of the Jacobian at yr
 //   fo_gen_factor_p, fo_gen_solve_p, fo_gen_solve_tp
 //                    the same for the projection's algebraic-rows-only matrix
 //                    (empty for unconstrained mechanisms)

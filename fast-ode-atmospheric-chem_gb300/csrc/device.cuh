@@ -117,19 +117,24 @@ struct SolveParams {
   int round_attempts;            // attempts per round
 };
 
-// Extra per-lane scratch of the adjoint (items after the forward layout).
+// Extra per-lane scratch of the adjoint (items after the forward layout). The
+// parts whose size depends on the call (ys, yp) come last, so that the offsets
+// of the others are the mechanism's alone (the generated phases know them).
 struct AdjLayout {
-  int64_t ys;     // max_steps * n: state at the start of every step
   int64_t u;      // 4n: stage points of the stages that evaluate F anew
   int64_t kbar;   // 4n
   int64_t fbar;   // 4n
   int64_t ybar;   // n
   int64_t g;      // n: a forcing vector-Jacobian product
+  int64_t v;      // n: its vector (generated)
   int64_t jbar;   // nnzj
   int64_t dbar;   // R*P
-  int64_t yp;     // constrained systems: kMaxProjectionUpdates * n, the state before each projection update
-  int64_t pdelta; // n: a projection update's Newton correction
+  int64_t w;      // R: a reaction's weight S^T v, or its log k derivative (generated)
+  int64_t rate;   // R: its rate (generated)
+  int64_t pdelta; // constrained systems, n: a projection update's Newton correction
   int64_t pmu;    // n: its adjoint
+  int64_t yp;     // kMaxProjectionUpdates * n, the state before each projection update
+  int64_t ys;     // max_steps * n: state at the start of every step
   int64_t items;  // total items per lane, forward layout included
 };
 

@@ -364,7 +364,7 @@ cudaError_t gen_launch_adjoint(GenModule* m, const AdjParams& a, int grid, size_
   if (e != cudaSuccess) return e;
   AdjParams q = a;
   void* args[] = {&q};
-  return cudaLaunchKernel(fn, dim3(grid), dim3(32), args, smem, stream);
+  return cudaLaunchKernel(fn, dim3(grid), dim3(32, team_of(grid)), args, smem, stream);
 }
 
 cudaError_t gen_launch_multi(GenModule* m, const SolveParams* batches, int nb, const int32_t* starts,

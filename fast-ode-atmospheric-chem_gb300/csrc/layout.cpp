@@ -65,6 +65,9 @@ GenLayout gen_layout_of(const HostTables& t) {
   // the partial derivatives that are products
   std::vector<char> used((size_t)t.R * t.P, 0);
   for (int32_t q : t.jt_idx) used[q] = 1;
+  for (int j = 0; j < t.R; ++j)
+    if (t.st_ptr[j] < t.st_ptr[j + 1])
+      for (int a = 0; a < t.P; ++a) used[(size_t)j * t.P + a] = t.react[(size_t)j * t.P + a] != t.n;
   std::vector<int64_t> product((size_t)t.R * t.P, -1);
   int64_t nd = 0;
   for (int j = 0; j < t.R; ++j) {
@@ -107,6 +110,29 @@ GenLayout gen_layout_of(const HostTables& t) {
   for (size_t q = 0; q < product.size(); ++q)
     if (product[q] >= 0) g.d_item[q] = (int32_t)(s.d + product[q]);
   return g;
+}
+
+AdjLayout adjoint_layout(const HostTables& t, int max_steps) {
+  AdjLayout a;
+  bool constrained = false;
+  for (double m : t.mass) constrained = constrained || m == 0.0;
+  int64_t o = layout_of(t).items;
+  a.u = o; o += 4LL * t.n;
+  a.kbar = o; o += 4LL * t.n;
+  a.fbar = o; o += 4LL * t.n;
+  a.ybar = o; o += t.n;
+  a.g = o; o += t.n;
+  a.v = o; o += t.n;
+  a.jbar = o; o += (int64_t)t.j_col.size();
+  a.dbar = o; o += (int64_t)t.R * t.P;
+  a.w = o; o += t.R;
+  a.rate = o; o += t.R;
+  a.pdelta = o; o += constrained ? t.n : 0;
+  a.pmu = o; o += constrained ? t.n : 0;
+  a.yp = o; o += constrained ? (int64_t)kMaxProjectionUpdates * t.n : 0;
+  a.ys = o; o += (int64_t)max_steps * t.n;
+  a.items = o;
+  return a;
 }
 
 }  // namespace fo

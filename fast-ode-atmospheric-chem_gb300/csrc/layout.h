@@ -52,4 +52,6 @@ struct GenLayout {
 
 GenLayout gen_layout_of(const HostTables& t);
 
+AdjLayout adjoint_layout(const HostTables& t, int max_steps);
+
 }  // namespace fo

@@ -29,6 +29,8 @@ __device__ void fo_gen_solve_t(double* base, int warp, int warps, int mech);
 __device__ void fo_gen_factor_p(double* base, int warp, int warps, int mech);
 __device__ void fo_gen_solve_p(double* base, int warp, int warps, int mech);
 __device__ void fo_gen_solve_tp(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_vjp(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_hvp(double* base, int warp, int warps, int mech);
 }
 // The team: the warps of the block (blockDim = 32 x warps), all holding the
 // group's cells. Loops over species give warp w the species i = w mod warps

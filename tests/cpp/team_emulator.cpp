@@ -292,6 +292,54 @@ int main(int argc, char** argv) {
     }
     J[e] = acc;
   }
+  // the adjoint's products, as its table-driven loops scatter them
+  const fo::AdjLayout al = fo::adjoint_layout(t, 3);
+  std::vector<double> v(n), jbar(J.size()), ybar(n), gref(n, 0.0), wref(R), dbar((size_t)R * P, 0.0), thref(R, 0.0);
+  for (double& q : v) q = U(rng) - 0.5;
+  for (double& q : jbar) q = U(rng) - 0.5;
+  for (double& q : ybar) q = U(rng) - 0.5;
+  std::vector<double> yref = ybar;
+  for (size_t e = 0; e < J.size(); ++e)
+    for (int q = t.jt_ptr[e]; q < t.jt_ptr[e + 1]; ++q)
+      dbar[t.jt_idx[q]] = std::fma(-t.jt_val[q], jbar[e], dbar[t.jt_idx[q]]);
+  for (int j = 0; j < R; ++j) {
+    double w = 0.0;
+    for (int e = t.st_ptr[j]; e < t.st_ptr[j + 1]; ++e) w = std::fma(t.st_val[e], v[t.st_sp[e]], w);
+    wref[j] = w;
+    for (int q = 0; q < P; ++q) {
+      const int s = t.react[j * P + q];
+      if (s == n) continue;
+      gref[s] = std::fma(w, d[j * P + q], gref[s]);
+      thref[j] = std::fma(dbar[j * P + q], d[j * P + q], thref[j]);
+      for (int q2 = 0; q2 < P; ++q2) {
+        if (q2 == q || t.react[j * P + q2] == n) continue;
+        double dd = k[j];
+        for (int q3 = 0; q3 < P; ++q3)
+          if (q3 != q && q3 != q2 && t.react[j * P + q3] != n) dd *= X(t.react[j * P + q3]);
+        yref[t.react[j * P + q2]] = std::fma(dbar[j * P + q], dd, yref[t.react[j * P + q2]]);
+      }
+    }
+  }
+  for (int warps : {1, 8, 16}) {
+    Machine M(fs, al.items);
+    for (int j = 0; j < R; ++j) M.mem[gl.s.kc + j] = k[j];
+    for (int i = 0; i < n; ++i) {
+      M.mem[gl.s.yr + i] = x[i];
+      M.mem[al.v + i] = v[i];
+      M.mem[al.ybar + i] = ybar[i];
+    }
+    for (size_t e = 0; e < J.size(); ++e) M.mem[al.jbar + e] = jbar[e];
+    M.call("fo_gen_vjp", warps);
+    for (int i = 0; i < n; ++i)
+      if (!same(M.mem[al.g + i], gref[i])) return printf("vjp %d\n", i), 20;
+    for (int j = 0; j < R; ++j)
+      if (!same(M.mem[al.w + j], wref[j])) return printf("weight %d\n", j), 21;
+    M.call("fo_gen_hvp", warps);
+    for (int i = 0; i < n; ++i)
+      if (!same(M.mem[al.ybar + i], yref[i])) return printf("hvp %d\n", i), 22;
+    for (int j = 0; j < R; ++j)
+      if (!same(M.mem[al.w + j], thref[j])) return printf("log k %d\n", j), 23;
+  }
   std::vector<double> b(n);
   for (double& v : b) v = U(rng);
   for (int proj = 0; proj < (algebraic ? 2 : 1); ++proj) {
