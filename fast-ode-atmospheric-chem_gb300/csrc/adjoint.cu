@@ -10,7 +10,7 @@ namespace fo {
 
 __global__ void __maxnreg__(255) adjoint_kernel(AdjParams a) {
   extern __shared__ double smem[];
-  adjoint_group(a, smem + 32);
+  adjoint_group(a, smem);
 }
 
 cudaError_t launch_adjoint(const AdjParams& a, int grid, int lanes, size_t smem, cudaStream_t stream) {

@@ -377,17 +377,21 @@ __device__ void reverse_projection_update(const AdjParams& a, const Lane& ln, do
 // One fixed step of size h from y (F, J, factorization, stages), the forward
 // kernel's arithmetic exactly; y_new in ynew, stage points in U.
 __device__ __forceinline__ void fixed_step(const AdjParams& a, const Lane& ln, double h, const double* y,
-                                           double* ynew, double* scr, double* w, double* U) {
+                                           double* ynew, double* scr, double* w, double* red, double* U) {
   const SolveParams& p = a.p;
   const int L = ln.L;
   long long cr = 0, cs = 0;
   eval_rhs(p, ln, y, scr + p.sl.r * L, scr + p.sl.f0 * L);
   eval_negjac(p, ln, y, scr + p.sl.d * L, scr + p.sl.negj * L);
-  factor_any(p, ln, 1.0 / __dmul_rn(h, p.o.tab.gamma), scr + p.sl.negj * L, scr + p.sl.lu * L, w, false);
-  attempt(p, ln, h, y, ynew, scr, w, cr, cs, U);
+  const double alpha = team_once(red + kSlotAlpha, [&] { return 1.0 / __dmul_rn(h, p.o.tab.gamma); });
+  factor_any(p, ln, alpha, scr + p.sl.negj * L, scr + p.sl.lu * L, w, false);
+  attempt(p, ln, h, y, ynew, scr, w, red, cr, cs, U);
 }
 
-__device__ void adjoint_group(const AdjParams& a, double* w) {
+// smem: the reduction buffer (32 doubles), then the work row
+__device__ void adjoint_group(const AdjParams& a, double* smem) {
+  double* const red = smem;
+  double* const w = smem + 32;
   const SolveParams& p = a.p;
   const int L = blockDim.x, lane = threadIdx.x;
   const int g = blockIdx.x;
@@ -431,7 +435,7 @@ __device__ void adjoint_group(const AdjParams& a, double* w) {
   // replay the accepted steps, keeping the state at the start of each
   for (int s = 0; s < m; ++s) {
     for (int i = TEAM_W; i < n; i += TEAM_N) SCR(ys + (int64_t)s * n * L, i) = SCR(Y, i);
-    fixed_step(a, ln, a.steps[s0 + s], Y, Ynew, scr, w, U);
+    fixed_step(a, ln, a.steps[s0 + s], Y, Ynew, scr, w, red, U);
     double* t = Y;
     Y = Ynew;
     Ynew = t;
@@ -456,7 +460,7 @@ __device__ void adjoint_group(const AdjParams& a, double* w) {
   for (int s = m - 1; s >= 0; --s) {
     const double h = a.steps[s0 + s];
     const double* y = ys + (int64_t)s * n * L;
-    fixed_step(a, ln, h, y, Ynew, scr, w, U);
+    fixed_step(a, ln, h, y, Ynew, scr, w, red, U);
     reverse_step(a, ln, h, y, scr, w);
   }
   for (int u = nq - 1; u >= 0; --u)

@@ -75,5 +75,5 @@ extern "C" __global__ void __launch_bounds__(32 * 16, 1)
 // generated factorization, solves and transposed solves.
 extern "C" __global__ void __launch_bounds__(32 * 16, 1) fo_generated_adjoint_kernel(fo::AdjParams a) {
   extern __shared__ double smem[];
-  fo::adjoint_group(a, smem + 32);
+  fo::adjoint_group(a, smem);
 }

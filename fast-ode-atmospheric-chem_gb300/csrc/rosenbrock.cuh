@@ -891,10 +891,48 @@ __device__ double block_sum(double v, double* red) {
   return s;
 }
 
+// A scalar that one warp of the team computes for all: f() by warp 0, handed
+// on in shared memory (`slot`, one per use). Every warp takes the same
+// decisions from it, and the FP64 units do its work once: with the
+// controller's powers and divisions evaluated by all sixteen warps, an attempt
+// of a 20-species mechanism took 142 us, with them done once 103 us.
+template <class F>
+__device__ __forceinline__ double team_once(double* slot, F f) {
+  if (TEAM_N == 1) return f();
+  if (TEAM_W == 0) {
+    const double v = f();
+    if (threadIdx.x == 0) *slot = v;
+  }
+  __syncthreads();
+  return *slot;
+}
+// Slots of the reduction buffer (32 doubles, the first sixteen block_max's).
+enum { kSlotError = 16, kSlotStep, kSlotAlpha, kSlotStart, kSlotPower, kSlotCoef = kSlotPower + 3 };
+
+// The controller's powers err^(1/k), (err err_prev)^(-1/(b k)) and
+// (H / h_prev)^(-1/b) (fastode/solvers.py:297-303), each by its own warp; the
+// last two only when `filter`, the first only when not.
+__device__ __forceinline__ void team_powers(const DevOptions& o, double* red, bool filter, double err, double err_prev,
+                                            double H, double h_prev, double elem_exp, double (&v)[3]) {
+  for (int q = TEAM_W; q < 3; q += TEAM_N) {
+    if (filter != (q > 0)) continue;
+    const double base = q == 0 ? err : q == 1 ? __dmul_rn(err, err_prev) : __ddiv_rn(H, h_prev);
+    const double e = q == 0 ? elem_exp : q == 1 ? -1.0 / __dmul_rn(o.b, o.k_exp) : -1.0 / o.b;
+    const double r = pow(base, e);
+    if (TEAM_N == 1) v[q] = r;
+    else if (threadIdx.x == 0) red[kSlotPower + q] = r;
+  }
+  if (TEAM_N == 1) return;
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 3; ++q) v[q] = red[kSlotPower + q];
+}
+
 // One attempt's stages (fastode/solvers.py:54-86), then Y_new, the error
 // estimate and this lane's share of the error norm (fastode/solvers.py:37-43).
+// A team returns it in warp 0.
 __device__ __noinline__ double attempt(const SolveParams& p, const Lane& ln, double H, const double* Y, double* Ynew,
-                                       double* scr, double* w, long long& c_rhs, long long& c_solves,
+                                       double* scr, double* w, double* red, long long& c_rhs, long long& c_solves,
                                        double* U = nullptr) {
   const int L = ln.L, lane = ln.lane;
   const int n = p.t.n;
@@ -907,6 +945,14 @@ __device__ __noinline__ double attempt(const SolveParams& p, const Lane& ln, dou
   double* lu = scr + p.sl.lu * L;
   double* rr = scr + p.sl.r * L;
   const double* forcing = F0;
+  // the stages' quotients c(r, s) / H, each by one warp of a team
+  if (TEAM_N > 1) {
+    for (int q = TEAM_W; q < 6; q += TEAM_N) {
+      const int r = q < 1 ? 1 : q < 3 ? 2 : 3;
+      if (r < tb.S && threadIdx.x == 0) red[kSlotCoef + q] = __ddiv_rn(tb.c[r][q - r * (r - 1) / 2], H);
+    }
+    __syncthreads();
+  }
   constexpr int kBatch = 4;   // species of a warp whose loads are in flight together
   for (int r = 0; r < tb.S; ++r) {
     if (r > 0 && tb.new_forcing[r]) {
@@ -945,7 +991,8 @@ __device__ __noinline__ double attempt(const SolveParams& p, const Lane& ln, dou
     // the stage's c(r, s) / H once per stage rather than once per species
     // (the same quotients, so the same sums bit for bit)
     double coefs[4];
-    for (int s = 0; s < r; ++s) coefs[s] = __ddiv_rn(tb.c[r][s], H);
+    for (int s = 0; s < r; ++s)
+      coefs[s] = TEAM_N > 1 ? red[kSlotCoef + r * (r - 1) / 2 + s] : __ddiv_rn(tb.c[r][s], H);
     for (int i0 = TEAM_W; i0 < n; i0 += kBatch * TEAM_N) {
       double v[kBatch];
 #pragma unroll
@@ -1027,6 +1074,7 @@ __device__ __noinline__ double attempt(const SolveParams& p, const Lane& ln, dou
     SCR(Ft, s0) = acc;
   }
   team_sync();
+  if (TEAM_W != 0) return 0.0;
   double total = 0.0;
   for (int s0 = 0; s0 < np; ++s0) total = __dadd_rn(total, SCR(Ft, s0));
   return ln.active ? total : 0.0;
@@ -1257,11 +1305,14 @@ __device__ __noinline__ void solve_group_restarting(const SolveParams& p, int g,
     ++c_jac;
     bool accepted = false;
     while (!accepted) {
-      factor_any(p, ln, 1.0 / __dmul_rn(H, o.tab.gamma), negj, lu, w, false);
+      const double alpha = team_once(red + kSlotAlpha, [&] { return 1.0 / __dmul_rn(H, o.tab.gamma); });
+      factor_any(p, ln, alpha, negj, lu, w, false);
       ++c_lu;
-      const double total = block_sum(attempt(p, ln, H, Y, Ynew, scr, w, c_rhs, c_solves), red);
-      double err = sqrt(__ddiv_rn(total, nsize));
-      if (!isnan(err)) err = pymax(err, 1.0e-10);
+      const double part = attempt(p, ln, H, Y, Ynew, scr, w, red, c_rhs, c_solves);
+      const double err = team_once(red + kSlotError, [&] {
+        const double e = sqrt(__ddiv_rn(block_sum(part, red), nsize));
+        return isnan(e) ? e : pymax(e, 1.0e-10);
+      });
       ++nsteps;
       ++c_steps;
       if (isnan(err) || isinf(err)) {
@@ -1269,8 +1320,9 @@ __device__ __noinline__ void solve_group_restarting(const SolveParams& p, int g,
         status = FO_STATUS_NAN_OR_INF;
         break;
       }
-      const double fac = pymin(6.0, pymax(0.2, __ddiv_rn(0.9, pow(err, elem_exp))));
-      double Hnew = __dmul_rn(H, fac);
+      double Hnew = team_once(red + kSlotStep, [&] {
+        return __dmul_rn(H, pymin(6.0, pymax(0.2, __ddiv_rn(0.9, pow(err, elem_exp)))));
+      });
       if (err < 1.0 || H < h_min) {
         trace_record(p, g, nrec, t, H, err, 1.0);
         ++c_acc;
@@ -1574,7 +1626,7 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
   const double h_max = dt;
   double H = (o.carry && h_next > 0.0) ? h_next : __dmul_rn(1.0e-6, dt);
   H = pymin(pymax(h_min, H), h_max);
-  if (o.quantize) H = quantize_step(H, dt);
+  H = team_once(red + kSlotStart, [&] { return o.quantize ? quantize_step(H, dt) : H; });
   double proposed = H;
   const double elem_exp = 1.0 / o.k_exp;
   const double up = 1.0 + 1.0e-8, down = 1.0 - 1.0e-8;
@@ -1621,12 +1673,14 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
         status = FO_STATUS_STEP_TOO_SMALL;
         break;
       }
-      factor_any(p, ln, 1.0 / __dmul_rn(H, o.tab.gamma), negj, lu, w, false);
+      const double alpha = team_once(red + kSlotAlpha, [&] { return 1.0 / __dmul_rn(H, o.tab.gamma); });
+      factor_any(p, ln, alpha, negj, lu, w, false);
       ++c_lu;
-      const double part = attempt(p, ln, H, Y, Ynew, scr, w, c_rhs, c_solves);
-      const double total = block_sum(part, red);
-      double err = sqrt(__ddiv_rn(total, nsize));
-      if (!isnan(err)) err = pymax(err, 1.0e-10);
+      const double part = attempt(p, ln, H, Y, Ynew, scr, w, red, c_rhs, c_solves);
+      const double err = team_once(red + kSlotError, [&] {
+        const double e = sqrt(__ddiv_rn(block_sum(part, red), nsize));
+        return isnan(e) ? e : pymax(e, 1.0e-10);
+      });
       ++nsteps;
       ++c_steps;
       if (isnan(err) || isinf(err)) {
@@ -1644,32 +1698,35 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
       } else if (err < 1.0) {
         trace_record(p, g, nrec, t, H, err, 1.0);
         // fastode/solvers.py:297-303
-        double fac = __ddiv_rn(o.safety, pow(err, elem_exp));
-        if (o.controller == FO_CONTROLLER_H211B && err_prev > 0.0 && h_prev > 0.0) {
-          fac = __dmul_rn(__dmul_rn(o.safety, pow(__dmul_rn(err, err_prev), -1.0 / __dmul_rn(o.b, o.k_exp))),
-                          pow(__ddiv_rn(H, h_prev), -1.0 / o.b));
-        }
-        fac = pymin(o.fac_max, pymax(o.fac_min, fac));
+        const bool filter = o.controller == FO_CONTROLLER_H211B && err_prev > 0.0 && h_prev > 0.0;
+        double pw[3];
+        team_powers(o, red, filter, err, err_prev, H, h_prev, elem_exp, pw);
         ++c_acc;
         t = last ? dt : __dadd_rn(t, H);
         double* tmp = Y; Y = Ynew; Ynew = tmp;
         err_prev = err;
         h_prev = H;
-        double Hnew = __dmul_rn(H, fac);
-        if (reject_last) Hnew = pymin(Hnew, H);
-        Hnew = pymax(h_min, pymin(Hnew, h_max));
-        if (o.quantize) Hnew = quantize_step(Hnew, dt);
+        const double Hnew = team_once(red + kSlotStep, [&] {
+          double fac = filter ? __dmul_rn(__dmul_rn(o.safety, pw[1]), pw[2]) : __ddiv_rn(o.safety, pw[0]);
+          fac = pymin(o.fac_max, pymax(o.fac_min, fac));
+          double h = __dmul_rn(H, fac);
+          if (reject_last) h = pymin(h, H);
+          h = pymax(h_min, pymin(h, h_max));
+          return o.quantize ? quantize_step(h, dt) : h;
+        });
         reject_last = reject_more = false;
         proposed = Hnew;
         H = Hnew;
         accepted = true;
       } else {
         trace_record(p, g, nrec, t, H, err, 0.0);
-        double Hnew = __dmul_rn(H, pymax(o.fac_min, __ddiv_rn(o.safety, pow(err, elem_exp))));
-        if (reject_more) Hnew = __dmul_rn(H, 0.1);
+        const double Hnew = team_once(red + kSlotStep, [&] {
+          double h = __dmul_rn(H, pymax(o.fac_min, __ddiv_rn(o.safety, pow(err, elem_exp))));
+          if (reject_more) h = __dmul_rn(H, 0.1);
+          return o.quantize ? quantize_step(h, dt) : h;
+        });
         reject_more = reject_last;
         reject_last = true;
-        if (o.quantize) Hnew = quantize_step(Hnew, dt);
         H = Hnew;
         last = __dsub_rn(dt, t) <= __dmul_rn(H, up);
         shortened = last && __dsub_rn(dt, t) < __dmul_rn(H, down);
