@@ -17,6 +17,7 @@
 #include "jit.h"
 #include "layout.h"
 #include "symbolic.h"
+#include "tableaus.h"
 
 namespace fo {
 cudaError_t launch_solve(const SolveParams& p, int grid, size_t smem, cudaStream_t stream);
@@ -63,28 +64,6 @@ namespace {
 
 using fo::adjoint_layout;
 using fo::layout_of;
-
-const fo::DevTableau kTableaus[2] = {
-    // ROS3 (fastode/tableaus.py:70-80)
-    {0.43586652150845899941601945119356,
-     3,
-     {{0, 0, 0, 0}, {1.0, 0, 0, 0}, {1.0, 0.0, 0, 0}, {0, 0, 0, 0}},
-     {{0, 0, 0, 0},
-      {-0.10156171083877702091975600115545e01, 0, 0, 0},
-      {0.40759956452537699824805835358067e01, 0.92076794298330791242156818474003e01, 0, 0},
-      {0, 0, 0, 0}},
-     {1.0, 0.61697947043828245592553615689730e01, -0.42772256543218573326238373806514, 0},
-     {0.5, -0.29079558716805469821718236208017e01, 0.22354069897811569627360909276199, 0},
-     {1, 1, 0, 0}},
-    // RODAS3 (fastode/tableaus.py:82-90)
-    {0.5,
-     4,
-     {{0, 0, 0, 0}, {0.0, 0, 0, 0}, {2.0, 0.0, 0, 0}, {2.0, 0.0, 1.0, 0}},
-     {{0, 0, 0, 0}, {4.0, 0, 0, 0}, {1.0, -1.0, 0, 0}, {1.0, -1.0, -8.0 / 3.0, 0}},
-     {2.0, 0.0, 1.0, 1.0},
-     {0.0, 0.0, 0.0, 1.0},
-     {1, 0, 1, 1}},
-};
 
 int lanes_for(int cells) { return ((cells + 31) / 32) * 32; }
 
@@ -384,7 +363,8 @@ int fill_params(const fo_plan* plan, const fo_options* opt, int32_t ngroups, con
     return fail(FO_E_UNSUPPORTED, "species x group size exceed shared memory: use smaller groups");
   fo::SolveParams p = base_params(plan);
   if (variant == FO_VARIANT_GENERATED) p.sl = plan->gen_layout;
-  p.o.tab = kTableaus[opt->tableau];
+  p.o.tab = fo::tableau_of(opt->tableau);
+  p.o.tableau = opt->tableau;
   p.o.controller = opt->controller;
   p.o.b = opt->b;
   p.o.safety = opt->safety;
@@ -514,7 +494,8 @@ int fo_solve(const fo_plan* plan, const fo_options* opt, int32_t ngroups, const 
   // header, zeroed for every launch
   p.rounds = nullptr;
   p.round_attempts = 1;
-  if (opt->lockstep && p.o.variant == FO_VARIANT_GENERATED && p.o.loop == FO_LOOP_ALGORITHM) {
+  if (opt->lockstep && p.o.variant == FO_VARIANT_GENERATED && p.o.loop == FO_LOOP_ALGORITHM &&
+      fo::gen_rounds_pay(grid)) {
     p.rounds = reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + kRoundsOffset);
     e = cudaMemsetAsync(p.rounds, 0, kRoundsWords * sizeof(unsigned int), s);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(rounds)");
@@ -620,7 +601,7 @@ int fo_multi_prepare(int32_t nb, const fo_batch_desc* b, void* workspace, size_t
     lockstep = lockstep && d.opt.lockstep && params[j].o.loop == FO_LOOP_ALGORITHM;
     cost_max = std::max<int64_t>(cost_max, d.plan->host.lu_fma + 3 * d.plan->host.solve_fma);
   }
-  if (lockstep) lockstep = fo::gen_resident(m->gen, true, m->grid, smem);
+  if (lockstep) lockstep = fo::gen_rounds_pay(m->grid) && fo::gen_resident(m->gen, true, m->grid, smem);
   m->d_rounds = lockstep ? reinterpret_cast<unsigned int*>(ws + kRoundsOffset) : nullptr;
   for (int j = 0; j < nb; ++j) {
     fo::SolveParams& p = params[j];

@@ -381,11 +381,10 @@ __device__ __forceinline__ void fixed_step(const AdjParams& a, const Lane& ln, d
   const SolveParams& p = a.p;
   const int L = ln.L;
   long long cr = 0, cs = 0;
-  eval_rhs(p, ln, y, scr + p.sl.r * L, scr + p.sl.f0 * L);
-  eval_negjac(p, ln, y, scr + p.sl.d * L, scr + p.sl.negj * L);
-  const double alpha = team_once(red + kSlotAlpha, [&] { return 1.0 / __dmul_rn(h, p.o.tab.gamma); });
+  begin_step(p, ln, y, scr, false);
+  const double alpha = attempt_scalars(p.o.tab, red, h);
   factor_any(p, ln, alpha, scr + p.sl.negj * L, scr + p.sl.lu * L, w, false);
-  attempt(p, ln, h, y, ynew, scr, w, red, cr, cs, U);
+  attempt(p, ln, h, y, ynew, scr, w, red, cr, cs, true, U);
 }
 
 // smem: the reduction buffer (32 doubles), then the work row

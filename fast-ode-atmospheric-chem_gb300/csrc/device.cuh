@@ -63,6 +63,7 @@ struct DevTableau {
 
 struct DevOptions {
   DevTableau tab;
+  int tableau;     // FO_TABLEAU_*
   int controller;  // 0 h211b, 1 elementary
   double b, safety, fac_min, fac_max;
   int carry, quantize, carry_memory, max_steps;

@@ -318,6 +318,15 @@ int team_of(int grid) {
   return team;
 }
 
+// Whether lockstep rounds pay for launches of such teams: they keep the
+// groups of an SM in the same part of the generated code, which pays where
+// three or more share an SM (teams of up to four), and make every group wait
+// for the slowest each attempt. With and without rounds, ms: 210/500 cold,
+// 16,384 cells (teams of 4) 268 and 300; 9,600 cells (8) 198 and 168; 4,800
+// cells (16) 115 and 95; TS1, 65,536 cells (1) 44.8 and 53.0, 2,048 cells (16)
+// 4.9 and 4.8; 20/40, 64 cells x 20 (16) 2.7 and 2.4.
+bool rounds_pay(int team) { return team <= 4; }
+
 // Whether `grid` blocks of `team` warps of kernel `fn` with `smem` bytes of
 // dynamic shared memory are all resident at once on the current device (what
 // a cooperative launch needs).
@@ -333,6 +342,8 @@ bool all_resident(const void* fn, int grid, int team, size_t smem) {
 }
 
 }  // namespace
+
+bool gen_rounds_pay(int grid) { return rounds_pay(team_of(grid)); }
 
 bool gen_resident(GenModule* m, bool multi, int grid, size_t smem) {
   const void* fn = reinterpret_cast<const void*>(multi ? m->multi_kernel : m->kernel);

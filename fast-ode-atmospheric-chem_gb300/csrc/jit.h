@@ -38,5 +38,7 @@ cudaError_t gen_launch_multi(GenModule* m, const SolveParams* batches, int nb, c
 // Whether `grid` blocks of the single-batch (multi false) or several-mechanism
 // kernel are all resident at once on the current device.
 bool gen_resident(GenModule* m, bool multi, int grid, size_t smem);
+// Whether lockstep rounds pay for a launch of `grid` blocks.
+bool gen_rounds_pay(int grid);
 
 }  // namespace fo

@@ -14,6 +14,7 @@
 
 #include "device.cuh"
 #include "fastode_gb300.h"
+#include "tableaus.h"
 
 #ifdef FO_LINK_GENERATED
 // The mechanism's generated phases (codegen.h), linked in per mechanism:
@@ -909,16 +910,25 @@ __device__ __forceinline__ double team_once(double* slot, F f) {
 // Slots of the reduction buffer (32 doubles, the first sixteen block_max's).
 enum { kSlotError = 16, kSlotStep, kSlotAlpha, kSlotStart, kSlotPower, kSlotCoef = kSlotPower + 3 };
 
-// The controller's powers err^(1/k), (err err_prev)^(-1/(b k)) and
-// (H / h_prev)^(-1/b) (fastode/solvers.py:297-303), each by its own warp; the
-// last two only when `filter`, the first only when not.
+// err^(1/k) for the embedded order's k = 3.
+__device__ __forceinline__ double error_root(double err) { return cbrt(err); }
+
+// The filter's powers (err err_prev)^(-1/(b k)) and (H / h_prev)^(-1/b)
+// (fastode/solvers.py:297-303), each by its own warp, or err^(1/k) alone. For
+// the default b = 4 they are roots: about 2,500 cycles one after another where
+// pow takes 12,000, with roundings of the same size.
 __device__ __forceinline__ void team_powers(const DevOptions& o, double* red, bool filter, double err, double err_prev,
-                                            double H, double h_prev, double elem_exp, double (&v)[3]) {
+                                            double H, double h_prev, double (&v)[3]) {
   for (int q = TEAM_W; q < 3; q += TEAM_N) {
     if (filter != (q > 0)) continue;
-    const double base = q == 0 ? err : q == 1 ? __dmul_rn(err, err_prev) : __ddiv_rn(H, h_prev);
-    const double e = q == 0 ? elem_exp : q == 1 ? -1.0 / __dmul_rn(o.b, o.k_exp) : -1.0 / o.b;
-    const double r = pow(base, e);
+    double r;
+    if (q == 0) {
+      r = error_root(err);
+    } else {
+      const double base = q == 1 ? __dmul_rn(err, err_prev) : __ddiv_rn(H, h_prev);
+      if (o.b == 4.0) r = __ddiv_rn(1.0, sqrt(sqrt(q == 1 ? cbrt(base) : base)));
+      else r = pow(base, q == 1 ? -1.0 / __dmul_rn(o.b, o.k_exp) : -1.0 / o.b);
+    }
     if (TEAM_N == 1) v[q] = r;
     else if (threadIdx.x == 0) red[kSlotPower + q] = r;
   }
@@ -928,12 +938,221 @@ __device__ __forceinline__ void team_powers(const DevOptions& o, double* red, bo
   for (int q = 0; q < 3; ++q) v[q] = red[kSlotPower + q];
 }
 
+// The scalars of an attempt of step H: returns alpha = 1 / (H gamma); a team
+// divides it and the stages' c(r, s) / H side by side, one warp each.
+__device__ __forceinline__ double attempt_scalars(const DevTableau& tb, double* red, double H) {
+  if (TEAM_N == 1) return 1.0 / __dmul_rn(H, tb.gamma);
+  for (int q = TEAM_W; q < 7; q += TEAM_N) {
+    const int r = q < 1 ? 1 : q < 3 ? 2 : 3;
+    double v = 0.0;
+    if (q == 6) v = 1.0 / __dmul_rn(H, tb.gamma);
+    else if (r < tb.S) v = __ddiv_rn(tb.c[r][q - r * (r - 1) / 2], H);
+    if (threadIdx.x == 0) red[q == 6 ? kSlotAlpha : kSlotCoef + q] = v;
+  }
+  __syncthreads();
+  return red[kSlotAlpha];
+}
+
+// F (item f0; the generated form leaves it in ft) and the negated Jacobian at
+// the step's start Y. `at_yr`: the last attempt left Y in item yr too (the
+// generated form's evaluation point).
+__device__ __forceinline__ void begin_step(const SolveParams& p, const Lane& ln, const double* Y, double* scr,
+                                           bool at_yr) {
+  const int L = ln.L;
+#ifdef FO_LINK_GENERATED
+  if (!at_yr) copy_items(ln, p.t.n, Y, scr + p.sl.yr * L);
+  fo_gen_rhs(scr + ln.lane, TEAM_W, TEAM_N, p.o.gen_index);
+  fo_gen_jac(scr + ln.lane, TEAM_W, TEAM_N, p.o.gen_index);
+#else
+  eval_rhs(p, ln, Y, scr + p.sl.r * L, scr + p.sl.f0 * L);
+  eval_negjac(p, ln, Y, scr + p.sl.d * L, scr + p.sl.negj * L);
+#endif
+}
+
+#ifdef FO_LINK_GENERATED
+// numpy.maximum(|a|, |b|): for magnitudes the integer order is the numeric
+// one, with NaN above everything, and the compare stays off the FP64 units.
+__device__ __forceinline__ double max_magnitude(double a, double b) {
+  const long long x = __double_as_longlong(fabs(a)), y = __double_as_longlong(fabs(b));
+  return __longlong_as_double(x > y ? x : y);
+}
+
+// One attempt of the generated integrator (what `attempt` below does for the
+// table-driven variants, the same operations in the same order), compiled for
+// each tableau: its coefficients are immediates, products with zero and one
+// are left out (which changes no value), and a stage's operands are loaded
+// together. A stage's solution stays in the solve vector until the next loop
+// over species reads it, which also stores it; the last one is stored only
+// for the adjoint (U). `fresh`: F of the step's start is in item ft and is
+// kept in f0 for further attempts. Y_new is left in item yr as well, the point
+// of the next evaluation. With the loops driven by the tableau in memory these
+// parts took 97,000 of an attempt's 195,000 cycles for a 20-species mechanism
+// (team of 16).
+template <int kTableau>
+__device__ __noinline__ double attempt_generated(const SolveParams& p, const Lane& ln, double H, const double* Y_,
+                                                 double* Ynew_, double* scr, double* red, double* U, bool fresh) {
+  constexpr DevTableau tb = tableau_of(kTableau);
+  constexpr int S = tb.S, kBatch = 4, kPartials = 16;
+  const int n = p.t.n, lane = ln.lane, warp = TEAM_W, warps = TEAM_N, mech = p.o.gen_index;
+  const bool dae = p.t.has_constraints != 0;
+  double* const base = scr + lane;
+  const double* const Y = Y_ + lane;
+  double* const Ynew = Ynew_ + lane;
+  double* const F0 = base + p.sl.f0 * 32;
+  double* const Ft = base + p.sl.ft * 32;
+  double* const Yr = base + p.sl.yr * 32;
+  double* const xs = base + p.sl.xs * 32;
+  double* const K = base + p.sl.k * 32;
+  const double* const mass = p.t.mass;
+  const int64_t kn = (int64_t)n * 32;
+  bool anew = false;   // F was evaluated after the step's start
+#pragma unroll
+  for (int r = 0; r < S; ++r) {
+    if (r > 0 && tb.new_forcing[r]) {
+      for (int i0 = warp; i0 < n; i0 += kBatch * warps) {
+        double y[kBatch], k[S][kBatch];
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+          const int i = i0 + b * warps;
+          if (i >= n) continue;
+          y[b] = Y[i * 32];
+          k[r - 1][b] = xs[i * 32];
+#pragma unroll
+          for (int s = 0; s + 1 < r; ++s)
+            if (tb.a[r][s] != 0.0) k[s][b] = K[s * kn + i * 32];
+        }
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+          const int i = i0 + b * warps;
+          if (i >= n) continue;
+          double v = y[b];
+#pragma unroll
+          for (int s = 0; s < r; ++s)
+            if (tb.a[r][s] != 0.0) v = __dadd_rn(v, tb.a[r][s] == 1.0 ? k[s][b] : __dmul_rn(tb.a[r][s], k[s][b]));
+          K[(r - 1) * kn + i * 32] = k[r - 1][b];
+          Yr[i * 32] = v;
+          if (U != nullptr) U[r * kn + i * 32 + lane] = v;   // stage point kept for the adjoint
+        }
+      }
+      fo_gen_rhs(base, warp, warps, mech);
+      anew = true;
+    }
+    double coef[S];
+#pragma unroll
+    for (int s = 0; s < r; ++s)
+      coef[s] = tb.c[r][s] == 0.0 ? 0.0
+                : warps > 1       ? red[kSlotCoef + r * (r - 1) / 2 + s]
+                                  : __ddiv_rn(tb.c[r][s], H);
+    const double* const f = anew || (r == 0 && fresh) ? Ft : F0;
+    const bool keep = r == 0 && fresh;                    // F of the step's start into f0
+    const bool move = r > 0 && !tb.new_forcing[r];        // the last solution into K
+    for (int i0 = warp; i0 < n; i0 += kBatch * warps) {
+      double v[kBatch], k[S][kBatch];
+      long long m[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int i = i0 + b * warps;
+        if (i >= n) continue;
+        v[b] = f[i * 32];
+#pragma unroll
+        for (int s = 0; s < r; ++s)
+          if (tb.c[r][s] != 0.0 || (move && s == r - 1))
+            k[s][b] = move && s == r - 1 ? xs[i * 32] : K[s * kn + i * 32];
+        if (r > 0 && dae) m[b] = __double_as_longlong(__ldg(mass + i));
+      }
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int i = i0 + b * warps;
+        if (i >= n) continue;
+        if (keep) F0[i * 32] = v[b];
+        if (move) K[(r - 1) * kn + i * 32] = k[r - 1][b];
+#pragma unroll
+        for (int s = 0; s < r; ++s)
+          if (tb.c[r][s] != 0.0) {
+            double ks = k[s][b];
+            if (dae && m[b] != 0x3ff0000000000000ll) ks = __dmul_rn(ks, __longlong_as_double(m[b]));
+            v[b] = __dadd_rn(v[b], __dmul_rn(coef[s], ks));
+          }
+        xs[i * 32] = v[b];
+      }
+    }
+    fo_gen_solve(base, warp, warps, mech);
+  }
+  // Y_new, E and the weighted sum of squares: min(n, 16) interleaved partial
+  // sums (species s, s + 16, ...), added in order, whatever the team's size
+  const int np = n < kPartials ? n : kPartials;
+  const bool change = p.o.loop == FO_LOOP_RESTARTING && p.o.step_change_rows && dae;
+  const double* const atol = p.atol;
+  const int32_t* const perm = p.t.perm;
+  const double rtol = p.rtol;
+  for (int s0 = warp; s0 < np; s0 += warps) {
+    double acc = 0.0;
+    for (int i0 = s0; i0 < n; i0 += kBatch * np) {
+      double y[kBatch], k[S][kBatch], tol[kBatch];
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int i = i0 + b * np;
+        if (i >= n) continue;
+        tol[b] = __ldg(atol + __ldg(perm + i));
+        y[b] = Y[i * 32];
+#pragma unroll
+        for (int r = 0; r < S; ++r)
+          if (tb.m[r] != 0.0 || tb.e[r] != 0.0 || r == S - 1) k[r][b] = r == S - 1 ? xs[i * 32] : K[r * kn + i * 32];
+      }
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int i = i0 + b * np;
+        if (i >= n) continue;
+        double yn = y[b], e = 0.0;
+        bool first = true;
+#pragma unroll
+        for (int r = 0; r < S; ++r) {
+          if (tb.m[r] != 0.0) yn = __dadd_rn(yn, tb.m[r] == 1.0 ? k[r][b] : __dmul_rn(tb.m[r], k[r][b]));
+          if (tb.e[r] != 0.0) {
+            const double term = tb.e[r] == 1.0 ? k[r][b] : __dmul_rn(tb.e[r], k[r][b]);
+            e = first ? term : __dadd_rn(e, term);
+            first = false;
+          }
+        }
+        Ynew[i * 32] = yn;
+        Yr[i * 32] = yn;
+        if (U != nullptr) K[(S - 1) * kn + i * 32] = k[S - 1][b];
+        // the restarting loop replaces the algebraic rows of the estimate by
+        // the step change (fastode/solvers.py:238-239)
+        if (change && __ldg(mass + i) == 0.0) e = __dsub_rn(yn, y[b]);
+        const double q = __ddiv_rn(e, __dadd_rn(tol[b], __dmul_rn(rtol, max_magnitude(y[b], yn))));
+        acc = __dadd_rn(acc, __dmul_rn(q, q));
+      }
+    }
+    Ft[s0 * 32] = acc;
+  }
+  team_sync();
+  if (warp != 0) return 0.0;
+  double part[kPartials], total = 0.0;
+#pragma unroll
+  for (int s0 = 0; s0 < kPartials; ++s0) part[s0] = s0 < np ? Ft[s0 * 32] : 0.0;
+#pragma unroll
+  for (int s0 = 0; s0 < kPartials; ++s0)
+    if (s0 < np) total = __dadd_rn(total, part[s0]);
+  return ln.active ? total : 0.0;
+}
+
+// A team returns the norm's sum in warp 0.
+__device__ __forceinline__ double attempt(const SolveParams& p, const Lane& ln, double H, const double* Y, double* Ynew,
+                                          double* scr, double*, double* red, long long& c_rhs, long long& c_solves,
+                                          bool fresh, double* U = nullptr) {
+  const bool ros3 = p.o.tableau == FO_TABLEAU_ROS3;
+  c_rhs += ros3 ? 1 : 2;
+  c_solves += ros3 ? 3 : 4;
+  return ros3 ? attempt_generated<FO_TABLEAU_ROS3>(p, ln, H, Y, Ynew, scr, red, U, fresh)
+              : attempt_generated<FO_TABLEAU_RODAS3>(p, ln, H, Y, Ynew, scr, red, U, fresh);
+}
+#else
 // One attempt's stages (fastode/solvers.py:54-86), then Y_new, the error
 // estimate and this lane's share of the error norm (fastode/solvers.py:37-43).
-// A team returns it in warp 0.
 __device__ __noinline__ double attempt(const SolveParams& p, const Lane& ln, double H, const double* Y, double* Ynew,
-                                       double* scr, double* w, double* red, long long& c_rhs, long long& c_solves,
-                                       double* U = nullptr) {
+                                       double* scr, double* w, double*, long long& c_rhs, long long& c_solves,
+                                       bool, double* U = nullptr) {
   const int L = ln.L, lane = ln.lane;
   const int n = p.t.n;
   const DevTableau& tb = p.o.tab;
@@ -945,35 +1164,27 @@ __device__ __noinline__ double attempt(const SolveParams& p, const Lane& ln, dou
   double* lu = scr + p.sl.lu * L;
   double* rr = scr + p.sl.r * L;
   const double* forcing = F0;
-  // the stages' quotients c(r, s) / H, each by one warp of a team
-  if (TEAM_N > 1) {
-    for (int q = TEAM_W; q < 6; q += TEAM_N) {
-      const int r = q < 1 ? 1 : q < 3 ? 2 : 3;
-      if (r < tb.S && threadIdx.x == 0) red[kSlotCoef + q] = __ddiv_rn(tb.c[r][q - r * (r - 1) / 2], H);
-    }
-    __syncthreads();
-  }
   constexpr int kBatch = 4;   // species of a warp whose loads are in flight together
   for (int r = 0; r < tb.S; ++r) {
     if (r > 0 && tb.new_forcing[r]) {
-      for (int i0 = TEAM_W; i0 < n; i0 += kBatch * TEAM_N) {
+      for (int i0 = 0; i0 < n; i0 += kBatch) {
         double v[kBatch];
 #pragma unroll
         for (int b = 0; b < kBatch; ++b)
-          if (i0 + b * TEAM_N < n) v[b] = SCR(Y, i0 + b * TEAM_N);
+          if (i0 + b < n) v[b] = SCR(Y, i0 + b);
         for (int s = 0; s < r; ++s)
           if (tb.a[r][s] != 0.0) {
             double ks[kBatch];
 #pragma unroll
             for (int b = 0; b < kBatch; ++b)
-              if (i0 + b * TEAM_N < n) ks[b] = SCR(K + (int64_t)s * n * L, i0 + b * TEAM_N);
+              if (i0 + b < n) ks[b] = SCR(K + (int64_t)s * n * L, i0 + b);
 #pragma unroll
             for (int b = 0; b < kBatch; ++b)
-              if (i0 + b * TEAM_N < n) v[b] = __dadd_rn(v[b], __dmul_rn(tb.a[r][s], ks[b]));
+              if (i0 + b < n) v[b] = __dadd_rn(v[b], __dmul_rn(tb.a[r][s], ks[b]));
           }
 #pragma unroll
         for (int b = 0; b < kBatch; ++b) {
-          const int i = i0 + b * TEAM_N;
+          const int i = i0 + b;
           if (i >= n) continue;
           SCR(Yr, i) = v[b];
           if (U != nullptr) SCR(U + (int64_t)r * n * L, i) = v[b];   // stage point kept for the adjoint
@@ -984,45 +1195,41 @@ __device__ __noinline__ double attempt(const SolveParams& p, const Lane& ln, dou
       forcing = Ft;
     }
     double* Kr = K + (int64_t)r * n * L;
-    // the generated and compact solves take their right-hand side from a
-    // per-lane vector (the generated ones from theirs), the others from w
-    const bool in_place = solves_in_place(p);
-    double* rhs = generated(p) ? scr + p.sl.xs * L : Kr;
+    const bool in_place = solves_in_place(p);   // right-hand side in Kr, solved in place
     // the stage's c(r, s) / H once per stage rather than once per species
     // (the same quotients, so the same sums bit for bit)
     double coefs[4];
-    for (int s = 0; s < r; ++s)
-      coefs[s] = TEAM_N > 1 ? red[kSlotCoef + r * (r - 1) / 2 + s] : __ddiv_rn(tb.c[r][s], H);
-    for (int i0 = TEAM_W; i0 < n; i0 += kBatch * TEAM_N) {
+    for (int s = 0; s < r; ++s) coefs[s] = __ddiv_rn(tb.c[r][s], H);
+    for (int i0 = 0; i0 < n; i0 += kBatch) {
       double v[kBatch];
 #pragma unroll
       for (int b = 0; b < kBatch; ++b)
-        if (i0 + b * TEAM_N < n) v[b] = SCR(forcing, i0 + b * TEAM_N);
+        if (i0 + b < n) v[b] = SCR(forcing, i0 + b);
       for (int s = 0; s < r; ++s) {
         const double coef = coefs[s];
         if (coef == 0.0) continue;
         double ks[kBatch];
 #pragma unroll
         for (int b = 0; b < kBatch; ++b) {
-          const int i = i0 + b * TEAM_N;
+          const int i = i0 + b;
           if (i >= n) continue;
           ks[b] = SCR(K + (int64_t)s * n * L, i);
           if (dae) ks[b] = __dmul_rn(ks[b], __ldg(p.t.mass + i));
         }
 #pragma unroll
         for (int b = 0; b < kBatch; ++b)
-          if (i0 + b * TEAM_N < n) v[b] = __dadd_rn(v[b], __dmul_rn(coef, ks[b]));
+          if (i0 + b < n) v[b] = __dadd_rn(v[b], __dmul_rn(coef, ks[b]));
       }
 #pragma unroll
       for (int b = 0; b < kBatch; ++b) {
-        const int i = i0 + b * TEAM_N;
+        const int i = i0 + b;
         if (i >= n) continue;
-        if (in_place) SCR(rhs, i) = v[b];
+        if (in_place) SCR(Kr, i) = v[b];
         else WROW(i) = v[b];
       }
     }
     if (in_place) {
-      solve_into(p, ln, lu, w, rhs, Kr);
+      solve_into(p, ln, lu, w, Kr, Kr);
     } else {
       solve_in_w(p, ln, lu, w);
       for (int i = 0; i < n; ++i) SCR(Kr, i) = WROW(i);
@@ -1030,10 +1237,11 @@ __device__ __noinline__ double attempt(const SolveParams& p, const Lane& ln, dou
     ++c_solves;
   }
   // Y_new, E and the weighted sum of squares: min(n, 16) interleaved partial
-  // sums (species s, s + 16, ...), added in order, whatever the team's size
+  // sums (species s, s + 16, ...), added in order, as the generated variant's
+  // teams sum it
   constexpr int kPartials = 16;
   const int np = n < kPartials ? n : kPartials;
-  for (int s0 = TEAM_W; s0 < np; s0 += TEAM_N) {
+  for (int s0 = 0; s0 < np; ++s0) {
     double acc = 0.0;
     for (int i0 = s0; i0 < n; i0 += kBatch * np) {
       double yv[kBatch], yn[kBatch], e[kBatch], tol[kBatch];
@@ -1073,12 +1281,11 @@ __device__ __noinline__ double attempt(const SolveParams& p, const Lane& ln, dou
     }
     SCR(Ft, s0) = acc;
   }
-  team_sync();
-  if (TEAM_W != 0) return 0.0;
   double total = 0.0;
   for (int s0 = 0; s0 < np; ++s0) total = __dadd_rn(total, SCR(Ft, s0));
   return ln.active ? total : 0.0;
 }
+#endif
 
 __device__ void trace_record(const SolveParams& p, int g, int& nrec, double t, double H, double err, double outcome) {
   if (p.trace == nullptr || !team_leader()) {
@@ -1266,10 +1473,7 @@ __device__ __noinline__ void solve_group_restarting(const SolveParams& p, int g,
   int nrec = 0;
   double* Y = scr + p.sl.y * L;
   double* Ynew = scr + p.sl.ynew * L;
-  double* F0 = scr + p.sl.f0 * L;
   double* negj = scr + p.sl.negj * L;
-  double* dd = scr + p.sl.d * L;
-  double* rr = scr + p.sl.r * L;
   double* lu = scr + p.sl.lu * L;
   load_rate_constants(p, ln, scr);
   for (int i = TEAM_W; i < n; i += TEAM_N) SCR(Y, i) = p.Y[ln.cell * p.ycs + (int64_t)__ldg(p.t.perm + i) * p.yss];
@@ -1277,7 +1481,6 @@ __device__ __noinline__ void solve_group_restarting(const SolveParams& p, int g,
   const double h_min = __dmul_rn(1.0e-15, dt);
   const double h_max = dt;
   double H = pymin(pymax(h_min, __dmul_rn(1.0e-6, dt)), h_max);
-  const double elem_exp = 1.0 / o.k_exp;
   const double nsize = (double)(C * n);
   int status = -1;
   ProjectionCounts pc;
@@ -1287,7 +1490,7 @@ __device__ __noinline__ void solve_group_restarting(const SolveParams& p, int g,
   c_lu += pc.lu;
   c_solves += pc.solves;
   double t = 0.0;
-  bool reject_last = false, reject_more = false;
+  bool reject_last = false, reject_more = false, at_yr = false;
   int nsteps = 0;
   while (status < 0 && __dadd_rn(__dsub_rn(t, dt), rounding) <= 0.0) {
     if (nsteps > o.max_steps) {
@@ -1299,16 +1502,18 @@ __device__ __noinline__ void solve_group_restarting(const SolveParams& p, int g,
       break;
     }
     H = pymin(H, fabs(__dsub_rn(dt, t)));
-    eval_rhs(p, ln, Y, rr, F0);
+    begin_step(p, ln, Y, scr, at_yr);
+    at_yr = true;
     ++c_rhs;
-    eval_negjac(p, ln, Y, dd, negj);
     ++c_jac;
+    bool fresh = true;
     bool accepted = false;
     while (!accepted) {
-      const double alpha = team_once(red + kSlotAlpha, [&] { return 1.0 / __dmul_rn(H, o.tab.gamma); });
+      const double alpha = attempt_scalars(o.tab, red, H);
       factor_any(p, ln, alpha, negj, lu, w, false);
       ++c_lu;
-      const double part = attempt(p, ln, H, Y, Ynew, scr, w, red, c_rhs, c_solves);
+      const double part = attempt(p, ln, H, Y, Ynew, scr, w, red, c_rhs, c_solves, fresh);
+      fresh = false;
       const double err = team_once(red + kSlotError, [&] {
         const double e = sqrt(__ddiv_rn(block_sum(part, red), nsize));
         return isnan(e) ? e : pymax(e, 1.0e-10);
@@ -1321,7 +1526,7 @@ __device__ __noinline__ void solve_group_restarting(const SolveParams& p, int g,
         break;
       }
       double Hnew = team_once(red + kSlotStep, [&] {
-        return __dmul_rn(H, pymin(6.0, pymax(0.2, __ddiv_rn(0.9, pow(err, elem_exp)))));
+        return __dmul_rn(H, pymin(6.0, pymax(0.2, __ddiv_rn(0.9, error_root(err)))));
       });
       if (err < 1.0 || H < h_min) {
         trace_record(p, g, nrec, t, H, err, 1.0);
@@ -1610,10 +1815,7 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
 
   double* Y = scr + p.sl.y * L;
   double* Ynew = scr + p.sl.ynew * L;
-  double* F0 = scr + p.sl.f0 * L;
   double* negj = scr + p.sl.negj * L;
-  double* dd = scr + p.sl.d * L;
-  double* rr = scr + p.sl.r * L;
   double* lu = scr + p.sl.lu * L;
 
   load_rate_constants(p, ln, scr);
@@ -1628,12 +1830,11 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
   H = pymin(pymax(h_min, H), h_max);
   H = team_once(red + kSlotStart, [&] { return o.quantize ? quantize_step(H, dt) : H; });
   double proposed = H;
-  const double elem_exp = 1.0 / o.k_exp;
   const double up = 1.0 + 1.0e-8, down = 1.0 - 1.0e-8;
   const double rounding = 2.220446049250313e-16;
 
   double t = 0.0;
-  bool reject_last = false, reject_more = false;
+  bool reject_last = false, reject_more = false, at_yr = false;
   int nsteps = 0;
   int status = -1;  // running
   const double nsize = (double)(C * n);
@@ -1659,10 +1860,11 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
     bool shortened = last && __dsub_rn(dt, t) < __dmul_rn(H, down);
     double H_ctrl = H;
     if (last) H = __dsub_rn(dt, t);
-    eval_rhs(p, ln, Y, rr, F0);
+    begin_step(p, ln, Y, scr, at_yr);
+    at_yr = true;
     ++c_rhs;
-    eval_negjac(p, ln, Y, dd, negj);
     ++c_jac;
+    bool fresh = true;
     bool accepted = false;
     while (!accepted) {
       if (nsteps >= o.max_steps) {
@@ -1673,10 +1875,11 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
         status = FO_STATUS_STEP_TOO_SMALL;
         break;
       }
-      const double alpha = team_once(red + kSlotAlpha, [&] { return 1.0 / __dmul_rn(H, o.tab.gamma); });
+      const double alpha = attempt_scalars(o.tab, red, H);
       factor_any(p, ln, alpha, negj, lu, w, false);
       ++c_lu;
-      const double part = attempt(p, ln, H, Y, Ynew, scr, w, red, c_rhs, c_solves);
+      const double part = attempt(p, ln, H, Y, Ynew, scr, w, red, c_rhs, c_solves, fresh);
+      fresh = false;
       const double err = team_once(red + kSlotError, [&] {
         const double e = sqrt(__ddiv_rn(block_sum(part, red), nsize));
         return isnan(e) ? e : pymax(e, 1.0e-10);
@@ -1700,7 +1903,7 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
         // fastode/solvers.py:297-303
         const bool filter = o.controller == FO_CONTROLLER_H211B && err_prev > 0.0 && h_prev > 0.0;
         double pw[3];
-        team_powers(o, red, filter, err, err_prev, H, h_prev, elem_exp, pw);
+        team_powers(o, red, filter, err, err_prev, H, h_prev, pw);
         ++c_acc;
         t = last ? dt : __dadd_rn(t, H);
         double* tmp = Y; Y = Ynew; Ynew = tmp;
@@ -1721,7 +1924,7 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
       } else {
         trace_record(p, g, nrec, t, H, err, 0.0);
         const double Hnew = team_once(red + kSlotStep, [&] {
-          double h = __dmul_rn(H, pymax(o.fac_min, __ddiv_rn(o.safety, pow(err, elem_exp))));
+          double h = __dmul_rn(H, pymax(o.fac_min, __ddiv_rn(o.safety, error_root(err))));
           if (reject_more) h = __dmul_rn(H, 0.1);
           return o.quantize ? quantize_step(h, dt) : h;
         });
