@@ -8,6 +8,7 @@ symbolic analysis and kept on the device.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 import weakref
 
 import numpy as np
@@ -82,6 +83,8 @@ class Plan:
         _abi.check(_abi.lib().fo_plan_permutation(handle, _ptr(perm, C.c_int32)), "fo_plan_permutation")
         self.perm = perm
         self._workspaces = {}
+        self.staging = []                    # idle buffers of drop-in calls (solvers._Staging)
+        self.staging_lock = threading.Lock()
         self.gen_info = None
 
     def generate(self, cache_dir=None) -> dict:

