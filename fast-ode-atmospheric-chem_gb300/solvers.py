@@ -48,7 +48,7 @@ def quantize(h: float, interval: float) -> float:
 
 
 def tableau_id(tab) -> int:
-    name = getattr(tab, "name", str(tab)).lower()
+    name = (tab.name if hasattr(tab, "name") else str(tab)).lower()   # str of a tableau prints its arrays
     if name == "ros3":
         return 0
     if name == "rodas3":
