@@ -11,8 +11,8 @@
 // Why teams. A group is one warp's 32 lanes wide, and one warp issues a DFMA
 // every 64 cycles on its SM sub-partition whatever the rest of the chip does,
 // so a launch of few groups leaves most of the FP64 units idle. A group is
-// therefore worked on by a team of 1 to 16 warps (a block), every warp holding
-// the same 32 cells: the generated work is cut into tasks (a row, a block of
+// therefore worked on by a team of 1 to 16 warps (a block), or a cluster of
+// such blocks on several SMs, every warp holding the same 32 cells: the generated work is cut into tasks (a row, a block of
 // rows by columns, a range of reactions), the tasks are scheduled into steps
 // of kSegments segments that depend on earlier steps only, and warp w of W
 // runs segments w, w + W, ... of a step before the team's barrier. One module
@@ -381,39 +381,92 @@ void emit_tile(Ptx& x, const Matrix& A, const GenLayout& gl, int i0, int i1, int
     for (int j = j0; j < j1; ++j) x.store(gl.dense_item(i, j), acc[(size_t)(i - i0) * b + j - j0]);
 }
 
-// The factorization up to the dense square's own elimination.
+// The square's columns [j0, j1) of a leading row: assembly and every pivot's
+// updates, with the multipliers the row's own task has made.
+void emit_row_columns(Ptx& x, const Matrix& A, int i, int j0, int j1) {
+  std::vector<int> acc(j1 - j0, -1);
+  for (int j = j0; j < j1; ++j) {
+    if (A.at(i, j) < 0) continue;
+    const int64_t from = A.start[(size_t)i * A.n + j];
+    acc[j - j0] = from >= 0 ? x.load(from) : x.constant(0.0);
+  }
+  for (int k = 0; k < i; ++k) {
+    if (A.at(i, k) < 0) continue;
+    int nl = -1;
+    for (int j = j0; j < j1; ++j) {
+      if (A.at(k, j) < 0) continue;
+      if (acc[j - j0] < 0) throw std::logic_error("fill pattern not closed");
+      if (nl < 0) nl = x.neg(x.load(A.at(i, k)));
+      acc[j - j0] = x.fma(nl, x.load(A.at(k, j)), acc[j - j0]);
+      ++x.fmas;
+    }
+  }
+  for (int j = j0; j < j1; ++j)
+    if (acc[j - j0] >= 0) x.store(A.at(i, j), acc[j - j0]);
+}
+
+// The factorization up to the dense square's own elimination. A leading row's
+// columns before the square are one task, which alone makes its multipliers
+// and pivot; its columns in the square are tasks of about kRowWidth columns
+// each, which only the same columns of later rows wait for. With a row as one
+// task, the chain of the last leading rows (7,500 multiply-adds of the 210/500
+// mechanism) was a quarter of the factorization on a team of sixteen.
 std::vector<Task> factor_tasks(const Matrix& A, const GenLayout& gl, int tile) {
   constexpr int kRowWidth = 24;   // columns of a single row at a time
+  const int chunk = tile * std::max(1, kRowWidth / tile);
+  const int chunks = (A.n - A.d0 + chunk - 1) / chunk;
   std::vector<Task> tasks;
   std::vector<int> row_task(A.n, -1);
+  std::vector<int> column_task((size_t)A.n * std::max(1, chunks), -1);
   auto pivots = [&](const std::vector<int>& rows) {
-    std::vector<int> after;
+    std::vector<int> ks;
     for (int k = 0; k < std::min(A.d0, rows[0]); ++k)
       for (int i : rows)
         if (A.at(i, k) >= 0) {
-          if (row_task[k] >= 0) after.push_back(row_task[k]);
+          ks.push_back(k);
           break;
         }
+    return ks;
+  };
+  // the tasks that finish the pivots' rows before the square, or in a chunk
+  auto before = [&](const std::vector<int>& ks, int c) {
+    std::vector<int> after;
+    for (int k : ks) {
+      const int id = c < 0 ? row_task[k] : column_task[(size_t)k * chunks + c];
+      if (id >= 0) after.push_back(id);
+    }
     return after;
   };
   for (int i = 0; i < A.d0; ++i) {
     if (A.unit[i]) continue;
-    const std::vector<int> rows{i};
+    const std::vector<int> rows{i}, ks = pivots(rows);
     row_task[i] = (int)tasks.size();
-    tasks.push_back({pivots(rows), [&A, rows](Ptx& x) { emit_rows(x, A, rows, A.n, kRowWidth); }});
+    tasks.push_back({before(ks, -1), [&A, rows](Ptx& x) { emit_rows(x, A, rows, A.d0, kRowWidth); }});
+    for (int c = 0; c < chunks; ++c) {
+      const int j0 = A.d0 + c * chunk, j1 = std::min(A.n, j0 + chunk);
+      bool any = false;
+      for (int j = j0; j < j1 && !any; ++j) any = A.at(i, j) >= 0;
+      if (!any) continue;
+      std::vector<int> after = before(ks, c);
+      if (!ks.empty()) after.push_back(row_task[i]);
+      column_task[(size_t)i * chunks + c] = (int)tasks.size();
+      tasks.push_back({after, [&A, i, j0, j1](Ptx& x) { emit_row_columns(x, A, i, j0, j1); }});
+    }
   }
   for (int i0 = A.d0; i0 < A.n; i0 += tile) {
     const int i1 = std::min(A.n, i0 + tile);
     std::vector<int> rows;
     for (int i = i0; i < i1; ++i) rows.push_back(i);
-    std::vector<int> after = pivots(rows);
-    if (!after.empty()) {
-      const int mine = (int)tasks.size();
-      tasks.push_back({after, [&A, rows, tile](Ptx& x) { emit_rows(x, A, rows, A.d0, tile); }});
-      after = {mine};
+    const std::vector<int> ks = pivots(rows);
+    int mine = -1;
+    if (!ks.empty()) {
+      mine = (int)tasks.size();
+      tasks.push_back({before(ks, -1), [&A, rows, tile](Ptx& x) { emit_rows(x, A, rows, A.d0, tile); }});
     }
     for (int j0 = A.d0; j0 < A.n; j0 += tile) {
       const int j1 = std::min(A.n, j0 + tile);
+      std::vector<int> after = before(ks, (j0 - A.d0) / chunk);
+      if (mine >= 0) after.push_back(mine);
       tasks.push_back({after, [&A, &gl, i0, i1, j0, j1](Ptx& x) { emit_tile(x, A, gl, i0, i1, j0, j1); }});
     }
   }
@@ -790,6 +843,10 @@ std::string phase_function(const std::string& name, bool alpha, const std::vecto
   int labels = 0;
   auto label = [&](const char* what, int id) { return "$" + name + "_" + what + std::to_string(id); };
   const std::string regs = ";\n\t.reg .b64 %p;\n\t.reg .b64 %b;\n\t.reg .b64 %a;\n";
+  // the block's barrier, or the cluster's for a team of several blocks
+  const std::string barrier =
+      "\t@%team bar.sync 0;\n\t@%clus barrier.cluster.arrive.release.aligned;\n"
+      "\t@%clus barrier.cluster.wait.acquire.aligned;\n";
   for (size_t m = 0; m < mechs.size(); ++m) {
     if (m + 1 < mechs.size())
       body += "\tsetp.ne.s32 %q, %m, " + std::to_string(m) + ";\n\t@%q bra " + label("m", (int)m + 1) + ";\n";
@@ -831,7 +888,7 @@ std::string phase_function(const std::string& name, bool alpha, const std::vecto
         body += "\tbra " + label("n", id) + ";\n";
       }
       body += label("n", id) + ":\n\tadd.u32 %s, %s, %nw;\n\tbra " + label("l", id) + ";\n" + label("e", id) +
-              ":\n\t@%team bar.sync 0;\n";
+              ":\n" + barrier;
     }
     body += "\tret;\n";
     if (m + 1 < mechs.size()) body += label("m", (int)m + 1) + ":\n";
@@ -842,11 +899,12 @@ std::string phase_function(const std::string& name, bool alpha, const std::vecto
                   ", .param .b32 " + param("warps") + ", .param .b32 " + param("mech") + ")\n{\n\t.reg .f64 %d<" +
                   std::to_string(x.next + 1) + ">" + regs +
                   "\t.reg .b32 %m;\n\t.reg .b32 %w;\n\t.reg .b32 %nw;\n\t.reg .b32 %s;\n"
-                  "\t.reg .pred %q;\n\t.reg .pred %team;\n\tld.param.b64 %p, [" + param("base") + "];\n" +
+                  "\t.reg .pred %q;\n\t.reg .pred %team;\n\t.reg .pred %clus;\n\tld.param.b64 %p, [" + param("base") + "];\n" +
                   (alpha ? "\tld.param.b64 %a, [" + param("alpha") + "];\n" : "\tmov.b64 %a, 0x3FF0000000000000;\n") +
                   "\tmov.b64 %d0, %a;\n\tld.param.b32 %w, [" + param("warp") + "];\n\tld.param.b32 %nw, [" +
                   param("warps") + "];\n\tld.param.b32 %m, [" + param("mech") +
-                  "];\n\tcvta.to.global.u64 %b, %p;\n\tsetp.gt.u32 %team, %nw, 1;\n\t@%team bar.sync 0;\n";
+                  "];\n\tcvta.to.global.u64 %b, %p;\n\tsetp.gt.u32 %clus, %nw, " + std::to_string(kBlockWarps) +
+                  ";\n\tsetp.gt.u32 %team, %nw, 1;\n\t@%clus setp.ne.u32 %team, %nw, %nw;\n" + barrier;
   return s + body + "}\n\n";
 }
 

@@ -13,14 +13,18 @@
 
 namespace fo {
 
-// Segments of a step of generated work: the most warps a team can use.
-constexpr int kSegments = 16;
+// Segments of a step of generated work: the most warps of a team that a step
+// can use.
+constexpr int kSegments = 64;
+
+// Warps of a block; a larger team is a cluster of blocks of this many.
+constexpr int kBlockWarps = 16;
 
 struct GenOptions {
   // rows and columns of the register tiles of the factorization
   int tile = 6;
   // rows of a block of the triangular solves
-  int solve_block = 8;
+  int solve_block = 6;
   // instructions of consecutive tasks compiled as a function of their own
   int piece_lines = 400;
 };
@@ -30,7 +34,8 @@ struct GenOptions {
 //   .visible .func name(.param .b64 base, .param .b32 warp, .param .b32 warps, .param .b32 mech)
 // base points at this lane's item 0 of its scratch slot, laid out item-major
 // with 32 lanes (item q at byte offset 256 q) by GenLayout (layout.h). Every
-// phase begins and ends with the team's barrier (none for a team of one).
+// phase begins and ends with the team's barrier (none for a team of one, the
+// cluster's for a team of more than kBlockWarps).
 //   fo_gen_rhs       forcing at the point in item yr, into item ft
 //   fo_gen_jac       negated Jacobian values at yr, into item negj
 //   fo_gen_factor    (base, alpha, ...) assembles alpha*M - J and factors it up

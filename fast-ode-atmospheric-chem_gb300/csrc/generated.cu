@@ -12,7 +12,9 @@
 // warp holding the group's cells in its 32 lanes (the generated code's operand
 // stride). At most 128 registers per thread, so that sixteen warps are
 // resident per SM whatever the team's size; jit.cpp chooses it by the number
-// of blocks.
+// of blocks. Where the groups are too few even for one SM each, a cluster of
+// sixteen-warp blocks on several SMs works on a group (the integrator kernel
+// without the queue, unconstrained Rosenbrock loops).
 #define FO_LINK_GENERATED 1
 
 #include <cuda_runtime.h>
@@ -23,10 +25,11 @@
 extern "C" __global__ void __launch_bounds__(32 * 16, 1) fo_generated_solve_kernel(fo::SolveParams p) {
   extern __shared__ double smem[];
   double* red = smem;       // 32 doubles
-  double* w = smem + 32;    // the projection's work row (constrained mechanisms only)
-  double* scr = p.scratch + (int64_t)blockIdx.x * p.slot_doubles;
+  double* w = smem + 32;    // a cluster's partial sums
+  const int slot = blockIdx.x / cluster_blocks();
+  double* scr = p.scratch + (int64_t)slot * p.slot_doubles;
   if (p.queue == nullptr) {
-    fo::solve_group(p, blockIdx.x, scr, w, red);
+    fo::solve_group(p, slot, scr, w, red);
   } else {
     __shared__ int next;
     for (;;) {

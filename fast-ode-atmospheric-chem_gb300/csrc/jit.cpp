@@ -191,6 +191,8 @@ struct GenModule {
   cudaKernel_t adjoint_kernel = nullptr;  // fo_generated_adjoint_kernel
   std::mutex mutex;
   int configured_smem[3][64] = {};
+  int64_t attempt_work = 0;               // FP64 operations of an attempt (one mechanism)
+  int clusters[64][4] = {};               // resident clusters of 2^i blocks, plus one (0: not asked yet)
 };
 
 int gen_create(const std::vector<const HostTables*>& ts, const std::vector<GenOptions>& opts, const char* cache_dir,
@@ -248,6 +250,9 @@ int gen_create(const std::vector<const HostTables*>& ts, const std::vector<GenOp
     info->cubin_bytes = (int64_t)cubin.size();
     info->seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   }
+  if (ts.size() == 1)
+    m->attempt_work = ts[0]->lu_fma + 3 * ts[0]->solve_fma + (int64_t)ts[0]->jt_idx.size() +
+                      2 * (int64_t)ts[0]->s_rxn.size();
   *out = m;
   return FO_OK;
 }
@@ -299,7 +304,7 @@ cudaError_t ensure_smem(GenModule* m, int which, const void* fn, size_t smem) {
 }
 
 // Warps per group for a launch of `grid` blocks on the current device: the
-// largest power of two, up to kSegments, that still leaves every block
+// largest power of two, up to kBlockWarps, that still leaves every block
 // resident at sixteen warps per SM (the kernels' 128 registers per thread):
 // beyond that a larger team only makes groups wait for one another. One warp
 // per group and a team, measured on a GB300: eight intervals of TS1 on 64
@@ -314,7 +319,7 @@ int team_of(int grid) {
     return 1;
   }
   int team = 1;
-  while (2 * team <= kSegments && (int64_t)grid * 2 * team <= (int64_t)sms * 16) team *= 2;
+  while (2 * team <= kBlockWarps && (int64_t)grid * 2 * team <= (int64_t)sms * 16) team *= 2;
   return team;
 }
 
@@ -339,6 +344,52 @@ bool all_resident(const void* fn, int grid, int team, size_t smem) {
     return false;
   }
   return (int64_t)per_sm * sms >= grid;
+}
+
+// Blocks per cluster for a launch of `grid` groups on teams of kBlockWarps
+// warps: the largest of 8, 4 and 2 with which all clusters are resident at
+// once, or one. A cluster's barrier and the operands' way through L2 cost
+// about 2,200 cycles a step (a block's barrier 45, its operands come from L1),
+// so a mechanism with little work per attempt stays on one SM: 20/40 (1,600
+// operations) does, TS1 (21,000) does not. One SM and a cluster, measured: a
+// cold interval of one 210/500 group 66.5 and 32.0 ms, eight intervals of TS1
+// on two groups 34.4 and 25.8 ms (both with the leading rows' tasks split).
+constexpr int64_t kClusterWork = 10000;
+constexpr size_t kClusterSmem = sizeof(double) * (32 + 32 * kBlockWarps);
+
+cudaLaunchConfig_t cluster_config(int grid, int blocks, cudaStream_t stream, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid * blocks);
+  c.blockDim = dim3(32, kBlockWarps);
+  c.dynamicSmemBytes = kClusterSmem;
+  c.stream = stream;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = blocks;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  c.attrs = attr;
+  c.numAttrs = 1;
+  return c;
+}
+
+int cluster_of(GenModule* m, const void* fn, int grid) {
+  int dev = 0;
+  if (m->attempt_work < kClusterWork || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+  std::lock_guard<std::mutex> lock(m->mutex);
+  for (int i = 3; i > 0; --i) {
+    int& known = m->clusters[dev][i];
+    if (known == 0) {
+      int n = 0;
+      cudaLaunchAttribute attr;
+      const cudaLaunchConfig_t c = cluster_config(1, 1 << i, nullptr, &attr);
+      if (cudaOccupancyMaxActiveClusters(&n, fn, &c) != cudaSuccess) {
+        (void)cudaGetLastError();
+        n = 0;
+      }
+      known = n + 1;
+    }
+    if (grid <= known - 1) return 1 << i;
+  }
+  return 1;
 }
 
 }  // namespace
@@ -366,6 +417,14 @@ cudaError_t gen_launch(GenModule* m, const SolveParams& p, int grid, size_t smem
   if (q.rounds != nullptr && all_resident(fn, grid, team, smem))
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
   q.rounds = nullptr;
+  if (team == kBlockWarps && q.queue == nullptr && !q.t.has_constraints && q.o.loop != FO_LOOP_BACKWARD_EULER) {
+    const int blocks = cluster_of(m, fn, grid);
+    if (blocks > 1) {
+      cudaLaunchAttribute attr;
+      const cudaLaunchConfig_t c = cluster_config(grid, blocks, stream, &attr);
+      return cudaLaunchKernelExC(&c, fn, args);
+    }
+  }
   return cudaLaunchKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
 }
 

@@ -33,14 +33,30 @@ __device__ void fo_gen_solve_tp(double* base, int warp, int warps, int mech);
 __device__ void fo_gen_vjp(double* base, int warp, int warps, int mech);
 __device__ void fo_gen_hvp(double* base, int warp, int warps, int mech);
 }
-// The team: the warps of the block (blockDim = 32 x warps), all holding the
-// group's cells. Loops over species give warp w the species i = w mod warps
-// (a power of two), so that elementwise loops hand no value to another warp.
-#define TEAM_W ((int)threadIdx.y)
-#define TEAM_N ((int)blockDim.y)
+// The team: the warps of the block (blockDim = 32 x warps), or of a cluster of
+// such blocks, all holding the group's cells. Loops over species give warp w
+// the species i = w mod warps (a power of two), so that elementwise loops hand
+// no value to another warp.
+__device__ __forceinline__ int cluster_rank() {
+  int r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ int cluster_blocks() {
+  int r;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+#define TEAM_W ((int)threadIdx.y + cluster_rank() * (int)blockDim.y)
+#define TEAM_N ((int)blockDim.y * cluster_blocks())
+// the block's own warps (what each block of a cluster computes for itself)
+#define BLOCK_W ((int)threadIdx.y)
+#define BLOCK_N ((int)blockDim.y)
 #else
 #define TEAM_W 0
 #define TEAM_N 1
+#define BLOCK_W 0
+#define BLOCK_N 1
 #endif
 
 namespace fo {
@@ -73,7 +89,23 @@ __device__ __forceinline__ double quantize_step(double h, double interval) {
 
 // The team's barrier, and its one thread that writes a group's results.
 __device__ __forceinline__ void team_sync() {
+#ifdef FO_LINK_GENERATED
+  if (cluster_blocks() > 1) {
+    asm volatile(
+        "barrier.cluster.arrive.release.aligned;\n\t"
+        "barrier.cluster.wait.acquire.aligned;" ::
+            : "memory");
+    return;
+  }
+#endif
   if (TEAM_N > 1) __syncthreads();
+}
+__device__ __forceinline__ bool cluster_team() {
+#ifdef FO_LINK_GENERATED
+  return cluster_blocks() > 1;
+#else
+  return false;
+#endif
 }
 __device__ __forceinline__ bool team_leader() { return threadIdx.x == 0 && TEAM_W == 0; }
 
@@ -771,6 +803,58 @@ __device__ __forceinline__ void block_finish(double (&c)[kDB][kDB], const double
   }
 }
 
+// The same for a team of several blocks, right-looking: every step's pivots
+// update all remaining blocks at once, one warp each (a left-looking step has
+// only 2 (nb - s) - 1 blocks, whose updates grow with s), and the warp that
+// updates the next diagonal block factors it. Each entry receives the same
+// updates in the same order.
+__device__ __forceinline__ void block_factor(double (&c)[kDB][kDB]) {
+#pragma unroll
+  for (int k = 0; k < kDB; ++k) {
+    const double rk = 1.0 / c[k][k];
+    c[k][k] = rk;
+#pragma unroll
+    for (int i = k + 1; i < kDB; ++i) {
+      c[i][k] *= rk;
+#pragma unroll
+      for (int j = k + 1; j < kDB; ++j) c[i][j] = fma(-c[i][k], c[k][j], c[i][j]);
+    }
+  }
+}
+
+__device__ __noinline__ void dense_lu_spread(double* a, int nb) {
+  const int w = TEAM_W, wn = TEAM_N;
+#pragma unroll 1
+  for (int s = -1; s < nb - 1; ++s) {
+    // the updates of step s (none before the first), and block (s+1, s+1)
+    const int m = nb - 1 - s, count = s < 0 ? 1 : m * m;
+#pragma unroll 1
+    for (int q = w; q < count; q += wn) {
+      const int bi = s + 1 + (s < 0 ? 0 : q / m), bj = s + 1 + (s < 0 ? 0 : q % m);
+      double* t = dense_block(a, nb, bi, bj);
+      double c[kDB][kDB];
+      block_load(t, c);
+      if (s >= 0) block_update(c, dense_block(a, nb, bi, s), dense_block(a, nb, s, bj), 1, 0);
+      if (q == 0) block_factor(c);
+      block_store(t, c);
+    }
+    team_sync();
+    const int rest = 2 * (nb - 2 - s);
+    const double* d = dense_block(a, nb, s + 1, s + 1);
+#pragma unroll 1
+    for (int q = w; q < rest; q += wn) {
+      const int k = s + 2 + q / 2;
+      const bool left = (q & 1) != 0;
+      double* t = dense_block(a, nb, left ? k : s + 1, left ? s + 1 : k);
+      double c[kDB][kDB];
+      block_load(t, c);
+      block_finish(c, d, left);
+      block_store(t, c);
+    }
+    if (rest > 0) team_sync();
+  }
+}
+
 __device__ __noinline__ void dense_lu(double* a, int nb) {
   const int64_t ustep = (int64_t)nb * kDB * kDB * 32;
   const int w = TEAM_W, wn = TEAM_N;
@@ -790,17 +874,7 @@ __device__ __noinline__ void dense_lu(double* a, int nb) {
       block_load(t, c);
       block_update(c, dense_block(a, nb, bi, 0), dense_block(a, nb, 0, bj), s, ustep);
       if (q == 0) {
-#pragma unroll
-        for (int k = 0; k < kDB; ++k) {
-          const double rk = 1.0 / c[k][k];
-          c[k][k] = rk;
-#pragma unroll
-          for (int i = k + 1; i < kDB; ++i) {
-            c[i][k] *= rk;
-#pragma unroll
-            for (int j = k + 1; j < kDB; ++j) c[i][j] = fma(-c[i][k], c[k][j], c[i][j]);
-          }
-        }
+        block_factor(c);
       } else if (wn == 1) {
         block_finish(c, d, left);
       }
@@ -833,7 +907,10 @@ __device__ void factor_any(const SolveParams& p, const Lane& ln, double alpha, c
     fo_gen_factor_p(base, TEAM_W, TEAM_N, p.o.gen_index);
   } else {
     fo_gen_factor(base, alpha, TEAM_W, TEAM_N, p.o.gen_index);
-    if (p.sl.nb > 0) dense_lu(base + p.sl.dn * ln.L, p.sl.nb);
+    if (p.sl.nb > 0) {
+      if (cluster_team()) dense_lu_spread(base + p.sl.dn * ln.L, p.sl.nb);
+      else dense_lu(base + p.sl.dn * ln.L, p.sl.nb);
+    }
   }
 #else
   if (p.o.variant == FO_VARIANT_PLAIN) factor(p, ln, alpha, negj, lu, w, alg_only);
@@ -892,15 +969,15 @@ __device__ double block_sum(double v, double* red) {
   return s;
 }
 
-// A scalar that one warp of the team computes for all: f() by warp 0, handed
-// on in shared memory (`slot`, one per use). Every warp takes the same
+// A scalar that one warp of the team computes for all: f() by warp 0 of each
+// block, handed on in shared memory (`slot`, one per use). Every warp takes the same
 // decisions from it, and the FP64 units do its work once: with the
 // controller's powers and divisions evaluated by all sixteen warps, an attempt
 // of a 20-species mechanism took 142 us, with them done once 103 us.
 template <class F>
 __device__ __forceinline__ double team_once(double* slot, F f) {
-  if (TEAM_N == 1) return f();
-  if (TEAM_W == 0) {
+  if (BLOCK_N == 1) return f();
+  if (BLOCK_W == 0) {
     const double v = f();
     if (threadIdx.x == 0) *slot = v;
   }
@@ -919,7 +996,7 @@ __device__ __forceinline__ double error_root(double err) { return cbrt(err); }
 // pow takes 12,000, with roundings of the same size.
 __device__ __forceinline__ void team_powers(const DevOptions& o, double* red, bool filter, double err, double err_prev,
                                             double H, double h_prev, double (&v)[3]) {
-  for (int q = TEAM_W; q < 3; q += TEAM_N) {
+  for (int q = BLOCK_W; q < 3; q += BLOCK_N) {
     if (filter != (q > 0)) continue;
     double r;
     if (q == 0) {
@@ -929,10 +1006,10 @@ __device__ __forceinline__ void team_powers(const DevOptions& o, double* red, bo
       if (o.b == 4.0) r = __ddiv_rn(1.0, sqrt(sqrt(q == 1 ? cbrt(base) : base)));
       else r = pow(base, q == 1 ? -1.0 / __dmul_rn(o.b, o.k_exp) : -1.0 / o.b);
     }
-    if (TEAM_N == 1) v[q] = r;
+    if (BLOCK_N == 1) v[q] = r;
     else if (threadIdx.x == 0) red[kSlotPower + q] = r;
   }
-  if (TEAM_N == 1) return;
+  if (BLOCK_N == 1) return;
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < 3; ++q) v[q] = red[kSlotPower + q];
@@ -941,8 +1018,8 @@ __device__ __forceinline__ void team_powers(const DevOptions& o, double* red, bo
 // The scalars of an attempt of step H: returns alpha = 1 / (H gamma); a team
 // divides it and the stages' c(r, s) / H side by side, one warp each.
 __device__ __forceinline__ double attempt_scalars(const DevTableau& tb, double* red, double H) {
-  if (TEAM_N == 1) return 1.0 / __dmul_rn(H, tb.gamma);
-  for (int q = TEAM_W; q < 7; q += TEAM_N) {
+  if (BLOCK_N == 1) return 1.0 / __dmul_rn(H, tb.gamma);
+  for (int q = BLOCK_W; q < 7; q += BLOCK_N) {
     const int r = q < 1 ? 1 : q < 3 ? 2 : 3;
     double v = 0.0;
     if (q == 6) v = 1.0 / __dmul_rn(H, tb.gamma);
@@ -1041,7 +1118,7 @@ __device__ __noinline__ double attempt_generated(const SolveParams& p, const Lan
 #pragma unroll
     for (int s = 0; s < r; ++s)
       coef[s] = tb.c[r][s] == 0.0 ? 0.0
-                : warps > 1       ? red[kSlotCoef + r * (r - 1) / 2 + s]
+                : BLOCK_N > 1     ? red[kSlotCoef + r * (r - 1) / 2 + s]
                                   : __ddiv_rn(tb.c[r][s], H);
     const double* const f = anew || (r == 0 && fresh) ? Ft : F0;
     const bool keep = r == 0 && fresh;                    // F of the step's start into f0
@@ -1076,7 +1153,15 @@ __device__ __noinline__ double attempt_generated(const SolveParams& p, const Lan
         xs[i * 32] = v[b];
       }
     }
-    fo_gen_solve(base, warp, warps, mech);
+    if (cluster_team()) {
+      // a solve is a chain of small steps: one block with its own barriers
+      // and L1 is faster than the cluster (210/500: 0.32 M cycles and 0.38 M)
+      team_sync();   // the right-hand side, from every block
+      if (cluster_rank() == 0) fo_gen_solve(base, BLOCK_W, BLOCK_N, mech);
+      team_sync();
+    } else {
+      fo_gen_solve(base, warp, warps, mech);
+    }
   }
   // Y_new, E and the weighted sum of squares: min(n, 16) interleaved partial
   // sums (species s, s + 16, ...), added in order, whatever the team's size
@@ -1085,13 +1170,18 @@ __device__ __noinline__ double attempt_generated(const SolveParams& p, const Lan
   const double* const atol = p.atol;
   const int32_t* const perm = p.t.perm;
   const double rtol = p.rtol;
-  for (int s0 = warp; s0 < np; s0 += warps) {
+  // A team of several blocks leaves every species' square in ft first, each
+  // by its own warp, for the partial sums to pick up: its DP work would
+  // otherwise fall to the sixteen warps of one SM.
+  const bool spread = warps > kPartials;
+  const int stride = spread ? warps : np;
+  for (int s0 = warp; s0 < (spread ? n : np); s0 += spread ? n : warps) {
     double acc = 0.0;
-    for (int i0 = s0; i0 < n; i0 += kBatch * np) {
+    for (int i0 = s0; i0 < n; i0 += kBatch * stride) {
       double y[kBatch], k[S][kBatch], tol[kBatch];
 #pragma unroll
       for (int b = 0; b < kBatch; ++b) {
-        const int i = i0 + b * np;
+        const int i = i0 + b * stride;
         if (i >= n) continue;
         tol[b] = __ldg(atol + __ldg(perm + i));
         y[b] = Y[i * 32];
@@ -1101,7 +1191,7 @@ __device__ __noinline__ double attempt_generated(const SolveParams& p, const Lan
       }
 #pragma unroll
       for (int b = 0; b < kBatch; ++b) {
-        const int i = i0 + b * np;
+        const int i = i0 + b * stride;
         if (i >= n) continue;
         double yn = y[b], e = 0.0;
         bool first = true;
@@ -1121,12 +1211,29 @@ __device__ __noinline__ double attempt_generated(const SolveParams& p, const Lan
         // the step change (fastode/solvers.py:238-239)
         if (change && __ldg(mass + i) == 0.0) e = __dsub_rn(yn, y[b]);
         const double q = __ddiv_rn(e, __dadd_rn(tol[b], __dmul_rn(rtol, max_magnitude(y[b], yn))));
-        acc = __dadd_rn(acc, __dmul_rn(q, q));
+        if (spread) Ft[i * 32] = __dmul_rn(q, q);
+        else acc = __dadd_rn(acc, __dmul_rn(q, q));
       }
     }
-    Ft[s0 * 32] = acc;
+    if (!spread) Ft[s0 * 32] = acc;
   }
   team_sync();
+  if (spread) {
+    // every block adds the partial sums up for itself, one per warp, in place
+    // of the reduction buffer's other uses (32 lanes each)
+    double* const sums = red + 32 + lane;
+    const int w = BLOCK_W;
+    if (w < np) {
+      double acc = 0.0;
+      for (int i = w; i < n; i += np) acc = __dadd_rn(acc, Ft[i * 32]);
+      sums[w * 32] = acc;
+    }
+    __syncthreads();
+    if (w != 0) return 0.0;
+    double total = 0.0;
+    for (int s0 = 0; s0 < np; ++s0) total = __dadd_rn(total, sums[s0 * 32]);
+    return ln.active ? total : 0.0;
+  }
   if (warp != 0) return 0.0;
   double part[kPartials], total = 0.0;
 #pragma unroll
@@ -1137,7 +1244,7 @@ __device__ __noinline__ double attempt_generated(const SolveParams& p, const Lan
   return ln.active ? total : 0.0;
 }
 
-// A team returns the norm's sum in warp 0.
+// A team returns the norm's sum in warp 0 of each block.
 __device__ __forceinline__ double attempt(const SolveParams& p, const Lane& ln, double H, const double* Y, double* Ynew,
                                           double* scr, double*, double* red, long long& c_rhs, long long& c_solves,
                                           bool fresh, double* U = nullptr) {
@@ -1823,6 +1930,7 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
 
   double* mem = p.memory + (int64_t)g * 3;
   double h_next = mem[0], err_prev = mem[1], h_prev = mem[2];
+  if (cluster_team()) team_sync();   // no block writes the memory before all have read it
   if (!(o.carry && o.carry_memory)) err_prev = h_prev = 0.0;
   const double h_min = __dmul_rn(1.0e-15, dt);
   const double h_max = dt;

@@ -127,7 +127,7 @@ class _Staging:
     other threads and streams get others; a call that raises drops them. At
     most KEEP idle sets stay with a plan. With an allocation and a copy per
     array, a settled interval of one 20-species group took 696 us, of which
-    the kernel is about 100; now 391."""
+    the kernel is about 100; now 172."""
 
     KEEP = 4
 

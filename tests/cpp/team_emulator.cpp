@@ -1,5 +1,5 @@
 // Host emulation of the generated phases (codegen.h) for one cell: runs the
-// text generate_ptx writes on teams of 1, 4 and 16 warps, the last warp
+// text generate_ptx writes on teams of 1 to 128 warps, the last warp
 // first, and checks that
 //   - no warp reads or writes an item that another warp writes between the
 //     same two barriers, and every access lies in the plan's scratch;
@@ -65,8 +65,8 @@ std::map<std::string, Func> parse(const std::string& text) {
     while (!l.empty() && (l[0] == '\t' || l[0] == ' ')) l.erase(0, 1);
     if (l.empty() || l[0] == '{' || l[0] == '}' || l.rfind("ld.param", 0) == 0 || l.rfind("st.param", 0) == 0 ||
         l.rfind(".param", 0) == 0 || l.rfind("cvta", 0) == 0 || l.rfind("mov.b64", 0) == 0 ||
-        l.rfind("setp.gt", 0) == 0 || l.rfind("setp.ne", 0) == 0)
-      continue;
+        l.rfind("setp.gt", 0) == 0 || l.rfind("setp.ne", 0) == 0 || l.rfind("@%clus", 0) == 0)
+      continue;   // a cluster's barrier stands where the block's does
     if (l.rfind(".reg", 0) == 0) {
       if (l.find("%d<") != std::string::npos) f->regs = std::atoi(l.c_str() + l.find("%d<") + 3);
       continue;
@@ -320,7 +320,7 @@ int main(int argc, char** argv) {
       }
     }
   }
-  for (int warps : {1, 8, 16}) {
+  for (int warps : {1, 8, 32}) {
     Machine M(fs, al.items);
     for (int j = 0; j < R; ++j) M.mem[gl.s.kc + j] = k[j];
     for (int i = 0; i < n; ++i) {
@@ -380,7 +380,7 @@ int main(int argc, char** argv) {
     for (int i = n - 1; i >= 0; --i)
       for (int q = n - 1; q > i; --q)
         if (in[(size_t)q * n + i]) z[i] = std::fma(-A[(size_t)q * n + i], z[q], z[i]);
-    for (int warps : {1, 4, 16}) {
+    for (int warps : {1, 4, 16, 128}) {
       Machine M(fs, gl.s.items);
       for (int j = 0; j < R; ++j) M.mem[gl.s.kc + j] = k[j];
       for (int i = 0; i < n; ++i) M.mem[gl.s.yr + i] = x[i];

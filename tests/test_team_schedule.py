@@ -2,7 +2,7 @@
 (tests/cpp/team_emulator.cpp): no two warps of a team touch the same item
 between two barriers when one of them writes it, no access leaves the scratch,
 and evaluations, factors and solutions are those of plain loops bit for bit
-for teams of 1, 4 and 16 warps."""
+for teams of 1 to 128 warps."""
 import shutil
 import subprocess
 import sys
