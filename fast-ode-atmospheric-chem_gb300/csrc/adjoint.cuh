@@ -273,7 +273,7 @@ __device__ __noinline__ void reverse_step(const AdjParams& a, const Lane& ln, do
     // the generated transposed solve works on the slot's solve vector
     double* muv = scr + p.sl.xs * L;
     for (int i = TEAM_W; i < n; i += TEAM_N) SCR(muv, i) = SCR(Kbar + (int64_t)r * n * L, i);
-    fo_gen_solve_t(scr + lane, TEAM_W, TEAM_N, p.o.gen_index);           // mu_r
+    generated_solve<true, false>(p, scr + lane, BLOCK_W, BLOCK_N);       // mu_r
 #else
     double* muv = w;
     for (int i = TEAM_W; i < n; i += TEAM_N) WROW(i) = SCR(Kbar + (int64_t)r * n * L, i);
@@ -322,7 +322,7 @@ __device__ void solve_transposed_into(const SolveParams& p, const Lane& ln, cons
 #ifdef FO_LINK_GENERATED
   double* v = scr + p.sl.xs * L;
   for (int i = TEAM_W; i < n; i += TEAM_N) SCR(v, i) = SCR(b, i);
-  fo_gen_solve_tp(scr + lane, TEAM_W, TEAM_N, p.o.gen_index);
+  generated_solve<true, true>(p, scr + lane, BLOCK_W, BLOCK_N);
   for (int i = TEAM_W; i < n; i += TEAM_N) SCR(x, i) = SCR(v, i);
 #else
   for (int i = TEAM_W; i < n; i += TEAM_N) WROW(i) = SCR(b, i);

@@ -33,11 +33,12 @@
 // (fma(-l, u, a); l = a * (1 / pivot); 1 / pivot by an IEEE division), so the
 // factors are those of every other variant bit for bit.
 //
-// The solves: leading rows are single-row tasks; rows of the square are blocks
-// of `solve_block` rows, each updated by one finished block at a time. Every
-// row sums its terms in the order in which their values finish (ascending
-// columns forward, descending columns backward), as the plain variant's loops
-// do, so results match that variant bit for bit.
+// The solves: leading rows are single-row tasks, the square's rows lose their
+// terms in the leading columns `solve_block` rows at a time, and the square's
+// own triangle is a loop (square_solve in rosenbrock.cuh). Every row sums its
+// terms in the order in which their values finish (ascending columns forward,
+// descending columns backward), as the plain variant's loops do, so results
+// match that variant bit for bit.
 #include "codegen.h"
 
 #include <algorithm>
@@ -473,23 +474,21 @@ std::vector<Task> factor_tasks(const Matrix& A, const GenLayout& gl, int tile) {
   return tasks;
 }
 
-// One triangular solve in place on the solve vector (item xs): row r's value
-// is x_r minus the sum of entry(r, k) x_k over the rows k finished before it,
-// in that order, times the item scale(r) where that is not -1. Rows finish
-// in ascending order (`up`) or descending order.
+// The leading rows' part of a triangular solve in place on the solve vector
+// (item xs): row r's value is x_r minus the sum of entry(r, k) x_k over the
+// rows k finished before it, in that order, times the item scale(r) where that
+// is not -1. Rows finish in ascending order (`up`; the square's rows then lose
+// their terms in the leading columns, `block` rows a task) or in descending
+// order after the square's rows.
 std::vector<Task> triangle_tasks(const Matrix& A, const ScratchLayout& sl, int block, bool up,
                                  std::function<int64_t(int, int)> entry, std::function<int64_t(int)> scale) {
   const int n = A.n, d0 = A.d0;
   std::vector<Task> tasks;
-  std::vector<int> maker(n, -1);       // the task that finishes each row (none: it is never changed)
+  std::vector<int> maker(n, -1);       // the task that finishes each row (none: before the phase, or never changed)
   // rows [i0, i1) of the vector minus their terms in columns [k0, k1), then,
-  // when `finish`, the rows themselves in order
+  // when `finish`, times their scale
   auto emit = [&sl, up, entry, scale](Ptx& x, int i0, int i1, int k0, int k1, bool finish) {
     std::vector<int> acc(i1 - i0, -1);
-    auto sum = [&](int i, int64_t q, int xk) {
-      if (acc[i - i0] < 0) acc[i - i0] = x.load(sl.xs + i);
-      acc[i - i0] = x.fma(x.neg(x.load(q)), xk, acc[i - i0]);
-    };
     for (int m = 0; m < k1 - k0; ++m) {
       const int k = up ? k0 + m : k1 - 1 - m;
       int xk = -1;
@@ -497,19 +496,17 @@ std::vector<Task> triangle_tasks(const Matrix& A, const ScratchLayout& sl, int b
         const int64_t q = entry(i, k);
         if (q < 0) continue;
         if (xk < 0) xk = x.load(sl.xs + k);
-        sum(i, q, xk);
+        if (acc[i - i0] < 0) acc[i - i0] = x.load(sl.xs + i);
+        acc[i - i0] = x.fma(x.neg(x.load(q)), xk, acc[i - i0]);
       }
     }
-    if (finish)
-      for (int m = 0; m < i1 - i0; ++m) {
-        const int k = up ? i0 + m : i1 - 1 - m;
-        if (acc[k - i0] < 0) acc[k - i0] = x.load(sl.xs + k);
-        if (scale(k) >= 0) acc[k - i0] = x.mul(acc[k - i0], x.load(scale(k)));
-        for (int i = up ? k + 1 : i0; i < (up ? i1 : k); ++i)
-          if (entry(i, k) >= 0) sum(i, entry(i, k), acc[k - i0]);
+    for (int i = i0; i < i1; ++i) {
+      if (finish && scale(i) >= 0) {
+        if (acc[i - i0] < 0) acc[i - i0] = x.load(sl.xs + i);
+        acc[i - i0] = x.mul(acc[i - i0], x.load(scale(i)));
       }
-    for (int i = i0; i < i1; ++i)
       if (acc[i - i0] >= 0) x.store(sl.xs + i, acc[i - i0]);
+    }
   };
   auto terms = [&](int i0, int i1, int k0, int k1) {
     std::vector<int> after;
@@ -521,78 +518,41 @@ std::vector<Task> triangle_tasks(const Matrix& A, const ScratchLayout& sl, int b
           if (maker[k] >= 0) after.push_back(maker[k]);
           break;
         }
-    std::sort(after.begin(), after.end());
-    after.erase(std::unique(after.begin(), after.end()), after.end());
     return std::make_pair(any, after);
   };
-  auto leading = [&]() {
-    for (int m = 0; m < d0; ++m) {
-      const int i = up ? m : d0 - 1 - m;
-      const int k0 = up ? 0 : i + 1, k1 = up ? i : n;
-      auto [any, after] = terms(i, i + 1, k0, k1);
-      if (!any && scale(i) < 0) continue;
-      maker[i] = (int)tasks.size();
-      tasks.push_back({after, [=](Ptx& x) { emit(x, i, i + 1, k0, k1, true); }});
+  for (int m = 0; m < d0; ++m) {
+    const int i = up ? m : d0 - 1 - m;
+    // descending, the terms of the square's rows come first and need no
+    // other leading row: a task of their own, all of them in the first step
+    int square = -1;
+    if (!up && terms(i, i + 1, d0, n).first && terms(i, i + 1, i + 1, d0).first) {
+      square = (int)tasks.size();
+      tasks.push_back({{}, [=](Ptx& x) { emit(x, i, i + 1, d0, n, false); }});
     }
-  };
-  auto square = [&]() {
-    const int nb = (n - d0 + block - 1) / block;
-    auto lo = [=](int b) { return d0 + b * block; };
-    auto hi = [=](int b) { return std::min(n, d0 + (b + 1) * block); };
-    std::vector<int> last(nb, -1);       // the latest task on each block's rows
-    for (int b = 0; b < nb && up; ++b) {  // the columns before the square
-      auto [any, after] = terms(lo(b), hi(b), 0, d0);
-      if (!any) continue;
-      last[b] = (int)tasks.size();
-      const int i0 = lo(b), i1 = hi(b);
-      tasks.push_back({after, [=](Ptx& x) { emit(x, i0, i1, 0, d0, false); }});
-    }
-    for (int m = 0; m < nb; ++m) {
-      const int b = up ? m : nb - 1 - m;
-      const int i0 = lo(b), i1 = hi(b);
-      std::vector<int> after;
-      if (last[b] >= 0) after.push_back(last[b]);
-      const int mine = (int)tasks.size();
-      tasks.push_back({after, [=](Ptx& x) { emit(x, i0, i1, i0, i0, true); }});
-      for (int i = i0; i < i1; ++i) maker[i] = mine;
-      for (int c = up ? b + 1 : 0; c < (up ? nb : b); ++c) {
-        auto [any, from] = terms(lo(c), hi(c), i0, i1);
-        if (!any) continue;
-        if (last[c] >= 0) from.push_back(last[c]);
-        last[c] = (int)tasks.size();
-        const int r0 = lo(c), r1 = hi(c);
-        tasks.push_back({from, [=](Ptx& x) { emit(x, r0, r1, i0, i1, false); }});
-      }
-    }
-  };
-  if (up) leading();
-  square();
-  if (!up) leading();
+    const int k0 = up ? 0 : i + 1, k1 = up ? i : square >= 0 ? d0 : n;
+    auto [any, after] = terms(i, i + 1, k0, k1);
+    if (!any && scale(i) < 0) continue;
+    if (square >= 0) after.push_back(square);
+    maker[i] = (int)tasks.size();
+    tasks.push_back({after, [=](Ptx& x) { emit(x, i, i + 1, k0, k1, true); }});
+  }
+  for (int i0 = d0; i0 < n && up; i0 += block) {
+    const int i1 = std::min(n, i0 + block);
+    auto [any, after] = terms(i0, i1, 0, d0);
+    if (any) tasks.push_back({after, [=](Ptx& x) { emit(x, i0, i1, 0, d0, false); }});
+  }
   return tasks;
 }
 
-// (LU)^-1: L by ascending rows, then U by descending rows and 1 / pivot.
-Phase solve_phase(const Matrix& A, const ScratchLayout& sl, int block) {
-  auto below = [&A](int i, int k) { return k < i ? A.at(i, k) : (int64_t)-1; };
-  auto above = [&A](int i, int k) { return k > i ? A.at(i, k) : (int64_t)-1; };
-  auto none = [](int) { return (int64_t)-1; };
-  auto pivot = [&A](int i) { return A.unit[i] ? (int64_t)-1 : A.at(i, i); };
-  Phase p = schedule(triangle_tasks(A, sl, block, true, below, none));
-  Phase q = schedule(triangle_tasks(A, sl, block, false, above, pivot));
-  p.insert(p.end(), q.begin(), q.end());
-  return p;
-}
-
-// (LU)^-T: U^T by ascending rows and 1 / pivot, then L^T by descending rows.
-Phase solve_t_phase(const Matrix& A, const ScratchLayout& sl, int block) {
-  auto below = [&A](int i, int k) { return k < i ? A.at(k, i) : (int64_t)-1; };
-  auto above = [&A](int i, int k) { return k > i ? A.at(k, i) : (int64_t)-1; };
-  auto none = [](int) { return (int64_t)-1; };
-  auto pivot = [&A](int i) { return A.unit[i] ? (int64_t)-1 : A.at(i, i); };
-  Phase p = schedule(triangle_tasks(A, sl, block, true, below, pivot));
-  Phase q = schedule(triangle_tasks(A, sl, block, false, above, none));
-  p.insert(p.end(), q.begin(), q.end());
-  return p;
+// The leading parts of (LU)^-1 (L by ascending rows; U by descending rows and
+// 1 / pivot) and of (LU)^-T (U^T by ascending rows and 1 / pivot; L^T by
+// descending rows), the square's between them being the kernels' loop.
+Phase lead_phase(const Matrix& A, const ScratchLayout& sl, int block, bool up, bool transposed) {
+  auto entry = [&A, up, transposed](int i, int k) {
+    return (up ? k < i : k > i) ? (transposed ? A.at(k, i) : A.at(i, k)) : (int64_t)-1;
+  };
+  auto scale = [&A, up, transposed](int i) { return up != transposed || A.unit[i] ? (int64_t)-1 : A.at(i, i); };
+  return schedule(triangle_tasks(A, sl, block, up, entry, scale));
 }
 
 // Items [0, count) in kSegments contiguous ranges, `per` items of a range at
@@ -928,7 +888,9 @@ std::string generate_ptx(const std::vector<const HostTables*>& ts, const std::ve
     full.push_back(full_matrix(*ts[m], layouts[m]));
     proj.push_back(projection_matrix(*ts[m], layouts[m]));
   }
-  std::vector<Phase> rhs, jac, factor, solve, solve_t, pfactor, psolve, psolve_t, vjp, hvp;
+  std::vector<Phase> rhs, jac, factor, pfactor, vjp, hvp;
+  // leading parts of the solves: [full or projection][transposed][up or down]
+  std::vector<Phase> lead[2][2][2];
   int64_t expected = 0;
   for (size_t m = 0; m < count; ++m) {
     const HostTables& t = *ts[m];
@@ -939,13 +901,14 @@ std::string generate_ptx(const std::vector<const HostTables*>& ts, const std::ve
     vjp.push_back(vjp_phase(t, gl, adjoints[m]));
     hvp.push_back(hvp_phase(t, gl, adjoints[m]));
     factor.push_back(schedule(factor_tasks(full[m], gl, o.tile)));
-    solve.push_back(solve_phase(full[m], gl.s, o.solve_block));
-    solve_t.push_back(solve_t_phase(full[m], gl.s, o.solve_block));
     bool constrained = false;
     for (double v : t.mass) constrained = constrained || v == 0.0;
     pfactor.push_back(constrained ? schedule(factor_tasks(proj[m], gl, o.tile)) : Phase());
-    psolve.push_back(constrained ? solve_phase(proj[m], gl.s, o.solve_block) : Phase());
-    psolve_t.push_back(constrained ? solve_t_phase(proj[m], gl.s, o.solve_block) : Phase());
+    for (int p = 0; p < 2; ++p)
+      for (int tr = 0; tr < 2; ++tr)
+        for (int down = 0; down < 2; ++down)
+          lead[p][tr][down].push_back(p && !constrained ? Phase()
+                                                        : lead_phase(p ? proj[m] : full[m], gl.s, o.solve_block, !down, tr != 0));
     // the multiply-adds of the pivots before the dense square
     for (int i = 0; i < t.n; ++i)
       for (int q = t.lu_row_ptr[i]; q < t.lu_diag[i]; ++q)
@@ -961,15 +924,16 @@ std::string generate_ptx(const std::vector<const HostTables*>& ts, const std::ve
     *fma_count = 0;
     for (const HostTables* t : ts) *fma_count += t->lu_fma;
   }
-  out += phase_function("fo_gen_solve", false, solve, lines, &ignored);
-  out += phase_function("fo_gen_solve_t", false, solve_t, lines, &ignored);
+  for (int p = 0; p < 2; ++p)
+    for (int tr = 0; tr < 2; ++tr)
+      for (int down = 0; down < 2; ++down)
+        out += phase_function(std::string("fo_gen_solve") + (tr ? "_t" : "") + (p ? "_p" : "") + (down ? "_down" : "_up"),
+                              false, lead[p][tr][down], lines, &ignored);
   out += phase_function("fo_gen_rhs", false, rhs, lines, &ignored);
   out += phase_function("fo_gen_jac", false, jac, lines, &ignored);
   out += phase_function("fo_gen_vjp", false, vjp, lines, &ignored);
   out += phase_function("fo_gen_hvp", false, hvp, lines, &ignored);
   out += phase_function("fo_gen_factor_p", false, pfactor, lines, &ignored);
-  out += phase_function("fo_gen_solve_p", false, psolve, lines, &ignored);
-  out += phase_function("fo_gen_solve_tp", false, psolve_t, lines, &ignored);
   return out;
 }
 

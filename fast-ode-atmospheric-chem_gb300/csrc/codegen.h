@@ -24,7 +24,7 @@ struct GenOptions {
   // rows and columns of the register tiles of the factorization
   int tile = 6;
   // rows of a block of the triangular solves
-  int solve_block = 6;
+  int solve_block = 4;
   // instructions of consecutive tasks compiled as a function of their own
   int piece_lines = 400;
 };
@@ -41,13 +41,16 @@ struct GenOptions {
 //   fo_gen_factor    (base, alpha, ...) assembles alpha*M - J and factors it up
 //                    to the dense square, which it leaves assembled and updated
 //                    (dense_lu finishes it)
-//   fo_gen_solve     overwrites the solve vector (item xs) with (LU)^-1 of it
-//   fo_gen_solve_t   ... with (LU)^-T of it, for the adjoint
+//   fo_gen_solve_up, fo_gen_solve_down
+//                    the leading rows' part of (LU)^-1 on the solve vector (item
+//                    xs): before and after the square's (square_solve)
+//   fo_gen_solve_t_up, fo_gen_solve_t_down
+//                    the same of (LU)^-T, for the adjoint
 //   fo_gen_vjp       the adjoint's J(yr)^T v, weights and rates
 //   fo_gen_hvp       the adjoint's second derivatives of the Jacobian at yr
-//   fo_gen_factor_p, fo_gen_solve_p, fo_gen_solve_tp
-//                    the same for the projection's algebraic-rows-only matrix
-//                    (empty for unconstrained mechanisms)
+//   fo_gen_factor_p, fo_gen_solve_p_up, ..., fo_gen_solve_t_p_down
+//                    the same for the projection's algebraic-rows-only matrix,
+//                    which has no square (empty for unconstrained mechanisms)
 // `mech` is ignored (one mechanism).
 std::string generate_ptx(const HostTables& t, const GenOptions& o, int64_t* fma_count = nullptr);
 

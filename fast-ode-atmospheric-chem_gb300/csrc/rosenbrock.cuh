@@ -25,11 +25,15 @@ extern "C" {
 __device__ void fo_gen_rhs(double* base, int warp, int warps, int mech);
 __device__ void fo_gen_jac(double* base, int warp, int warps, int mech);
 __device__ void fo_gen_factor(double* base, double alpha, int warp, int warps, int mech);
-__device__ void fo_gen_solve(double* base, int warp, int warps, int mech);
-__device__ void fo_gen_solve_t(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_up(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_down(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_t_up(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_t_down(double* base, int warp, int warps, int mech);
 __device__ void fo_gen_factor_p(double* base, int warp, int warps, int mech);
-__device__ void fo_gen_solve_p(double* base, int warp, int warps, int mech);
-__device__ void fo_gen_solve_tp(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_p_up(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_p_down(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_t_p_up(double* base, int warp, int warps, int mech);
+__device__ void fo_gen_solve_t_p_down(double* base, int warp, int warps, int mech);
 __device__ void fo_gen_vjp(double* base, int warp, int warps, int mech);
 __device__ void fo_gen_hvp(double* base, int warp, int warps, int mech);
 }
@@ -899,6 +903,116 @@ __device__ __noinline__ void dense_lu(double* a, int nb) {
 }
 #endif
 
+#ifdef FO_LINK_GENERATED
+// One triangle of the square's solves in place on its part of the solve vector
+// (x, this lane's first item): blocks of kDB rows finish in ascending order
+// (kUp) or descending order, each row subtracting entry(i, k) x_k as its
+// values finish and then, kScale, taking the diagonal item (1 / pivot);
+// kTransposed: entry(i, k) is the stored (k, i). Warp w of wn (one block's
+// warps: a triangle is a chain of small steps) updates every wn-th block that
+// remains with the block just finished; the warp of the next block finishes it
+// too, so a step has one barrier. One warp alone sums a block's terms in
+// registers instead. As straight-line code a triangle of 72 rows was 0.6 MB,
+// fetched anew by every solve.
+template <bool kUp, bool kScale, bool kTransposed>
+__device__ __noinline__ void square_triangle(const double* a, double* x, int nb, int w, int wn) {
+  // c_i -= sum of entry(i, k) v_k over a whole block (block b's rows, block k's columns)
+  auto update = [&](double (&c)[kDB], int b, int k) {
+    const double* t = a + (int64_t)(kTransposed ? k * nb + b : b * nb + k) * kDB * kDB * 32;
+    const double* xk = x + (int64_t)k * kDB * 32;
+    double v[kDB], e[kDB][kDB];
+#pragma unroll
+    for (int q = 0; q < kDB; ++q) v[q] = xk[q * 32];
+#pragma unroll
+    for (int i = 0; i < kDB; ++i)
+#pragma unroll
+      for (int q = 0; q < kDB; ++q) e[i][q] = t[(kTransposed ? q * kDB + i : i * kDB + q) * 32];
+#pragma unroll
+    for (int m = 0; m < kDB; ++m) {
+      const int q = kUp ? m : kDB - 1 - m;
+#pragma unroll
+      for (int i = 0; i < kDB; ++i) c[i] = fma(-e[i][q], v[q], c[i]);
+    }
+  };
+  auto finish = [&](double (&c)[kDB], int b) {
+    const double* t = a + (int64_t)(b * nb + b) * kDB * kDB * 32;
+#pragma unroll
+    for (int m = 0; m < kDB; ++m) {
+      const int q = kUp ? m : kDB - 1 - m;
+      if (kScale) c[q] *= t[(q * kDB + q) * 32];
+#pragma unroll
+      for (int i = 0; i < kDB; ++i)
+        if (kUp ? i > q : i < q) c[i] = fma(-t[(kTransposed ? q * kDB + i : i * kDB + q) * 32], c[q], c[i]);
+    }
+  };
+  auto load = [&](double (&c)[kDB], int b) {
+#pragma unroll
+    for (int i = 0; i < kDB; ++i) c[i] = x[(int64_t)(b * kDB + i) * 32];
+  };
+  auto store = [&](const double (&c)[kDB], int b) {
+#pragma unroll
+    for (int i = 0; i < kDB; ++i) x[(int64_t)(b * kDB + i) * 32] = c[i];
+  };
+  if (wn == 1) {
+#pragma unroll 1
+    for (int m = 0; m < nb; ++m) {
+      const int b = kUp ? m : nb - 1 - m;
+      double c[kDB];
+      load(c, b);
+#pragma unroll 1
+      for (int q = 0; q < m; ++q) update(c, b, kUp ? q : nb - 1 - q);
+      finish(c, b);
+      store(c, b);
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int m = -1; m < nb - 1; ++m) {
+    // block m (in finishing order) is done; those after it take its terms
+    const int k = kUp ? m : nb - 1 - m;
+#pragma unroll 1
+    for (int r = m + 1 + w; r < (m < 0 ? 1 : nb); r += wn) {
+      const int b = kUp ? r : nb - 1 - r;
+      double c[kDB];
+      load(c, b);
+      if (m >= 0) update(c, b, k);
+      if (r == m + 1) finish(c, b);
+      store(c, b);
+    }
+    __syncthreads();
+  }
+}
+
+// x = A^-1 b or A^-T b in place on the solve vector, by the warps of a block;
+// the factors are the stage matrix's or, kProjection, the projection's. Every
+// warp's right-hand side is in place on entry (the phases begin and end with
+// the barrier of `wn` warps).
+template <bool kTransposed, bool kProjection>
+__device__ __forceinline__ void generated_solve(const SolveParams& p, double* base, int w, int wn) {
+  const int mech = p.o.gen_index, nb = kProjection ? 0 : p.sl.nb;
+  if (kProjection) {
+    if (kTransposed) fo_gen_solve_t_p_up(base, w, wn, mech);
+    else fo_gen_solve_p_up(base, w, wn, mech);
+  } else {
+    if (kTransposed) fo_gen_solve_t_up(base, w, wn, mech);
+    else fo_gen_solve_up(base, w, wn, mech);
+  }
+  if (nb > 0) {
+    const double* a = base + p.sl.dn * 32;
+    double* x = base + (p.sl.xs + p.t.n - (int64_t)nb * kDB) * 32;
+    square_triangle<true, kTransposed, kTransposed>(a, x, nb, w, wn);
+    square_triangle<false, !kTransposed, kTransposed>(a, x, nb, w, wn);
+  }
+  if (kProjection) {
+    if (kTransposed) fo_gen_solve_t_p_down(base, w, wn, mech);
+    else fo_gen_solve_p_down(base, w, wn, mech);
+  } else {
+    if (kTransposed) fo_gen_solve_t_down(base, w, wn, mech);
+    else fo_gen_solve_down(base, w, wn, mech);
+  }
+}
+#endif
+
 __device__ void factor_any(const SolveParams& p, const Lane& ln, double alpha, const double* negj, double* lu,
                            double* w, bool alg_only) {
 #ifdef FO_LINK_GENERATED
@@ -940,8 +1054,8 @@ __device__ void solve_into(const SolveParams& p, const Lane& ln, const double* l
   double* base = const_cast<double*>(lu) - p.sl.lu * ln.L;
   double* xs = base + p.sl.xs * ln.L;
   if (b != xs) copy_items(ln, p.t.n, b, xs);
-  if (alg_only) fo_gen_solve_p(base + ln.lane, TEAM_W, TEAM_N, p.o.gen_index);
-  else fo_gen_solve(base + ln.lane, TEAM_W, TEAM_N, p.o.gen_index);
+  if (alg_only) generated_solve<false, true>(p, base + ln.lane, BLOCK_W, BLOCK_N);
+  else generated_solve<false, false>(p, base + ln.lane, BLOCK_W, BLOCK_N);
   if (x != xs) copy_items(ln, p.t.n, xs, x);
 #else
   if (p.o.variant == FO_VARIANT_COMPACT) {
@@ -1157,10 +1271,10 @@ __device__ __noinline__ double attempt_generated(const SolveParams& p, const Lan
       // a solve is a chain of small steps: one block with its own barriers
       // and L1 is faster than the cluster (210/500: 0.32 M cycles and 0.38 M)
       team_sync();   // the right-hand side, from every block
-      if (cluster_rank() == 0) fo_gen_solve(base, BLOCK_W, BLOCK_N, mech);
+      if (cluster_rank() == 0) generated_solve<false, false>(p, base, BLOCK_W, BLOCK_N);
       team_sync();
     } else {
-      fo_gen_solve(base, warp, warps, mech);
+      generated_solve<false, false>(p, base, BLOCK_W, BLOCK_N);
     }
   }
   // Y_new, E and the weighted sum of squares: min(n, 16) interleaved partial

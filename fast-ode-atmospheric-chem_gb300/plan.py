@@ -75,7 +75,7 @@ class Plan:
         self.handle = handle
         self._finalizer = weakref.finalize(self, _abi.lib().fo_plan_destroy, handle)
         self.tile = int(tile)
-        _abi.check(_abi.lib().fo_plan_set_generation(handle, self.tile, 6), "fo_plan_set_generation")
+        _abi.check(_abi.lib().fo_plan_set_generation(handle, self.tile, 4), "fo_plan_set_generation")
         info = _abi.PlanInfo()
         _abi.check(_abi.lib().fo_plan_info_get(handle, C.byref(info)), "fo_plan_info_get")
         self.info = info.as_dict()

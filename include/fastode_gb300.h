@@ -232,7 +232,7 @@ int fo_plan_generate(fo_plan* plan, const char* cache_dir, fo_gen_info* info);
 /* The generated code's shape for this plan, before fo_plan_generate (and
  * before the plan joins a generated several-mechanism launch): the rows and
  * columns of the factorization's register tiles (1..16, default 6) and the
- * rows of a block of the solves (1..64, default 6). A tuning choice that
+ * rows of a block of the solves (1..64, default 4). A tuning choice that
  * changes no result: every tile gives the same factors bit for bit. Refused
  * once the plan's module exists with other options. */
 int fo_plan_set_generation(fo_plan* plan, int32_t tile, int32_t solve_block);

@@ -405,12 +405,30 @@ int main(int argc, char** argv) {
             if (!same(M.mem[gl.lu_item[q]], A[(size_t)i * n + t.lu_col[q]]))
               return printf("factor (%d, %d), %d warps\n", i, t.lu_col[q], warps), 12;
       }
+      // the square's triangles by plain loops (up: ascending rows)
+      auto square = [&](bool up, bool transposed) {
+        for (int m = 0; m < n - gl.d0 && !proj; ++m) {
+          const int i = up ? gl.d0 + m : n - 1 - m;
+          double& xi = M.mem[gl.s.xs + i];
+          for (int q = 0; q < m; ++q) {
+            const int kk = up ? gl.d0 + q : n - 1 - q;
+            xi = std::fma(-M.mem[transposed ? gl.dense_item(kk, i) : gl.dense_item(i, kk)], M.mem[gl.s.xs + kk], xi);
+          }
+          if (up == transposed) xi *= M.mem[gl.dense_item(i, i)];
+        }
+      };
       for (int i = 0; i < n; ++i) M.mem[gl.s.xs + i] = b[i];
-      M.call(proj ? "fo_gen_solve_p" : "fo_gen_solve", warps);
+      M.call(proj ? "fo_gen_solve_p_up" : "fo_gen_solve_up", warps);
+      square(true, false);
+      square(false, false);
+      M.call(proj ? "fo_gen_solve_p_down" : "fo_gen_solve_down", warps);
       for (int i = 0; i < n; ++i)
         if (!same(M.mem[gl.s.xs + i], y[i])) return printf("solve %d, projection %d, %d warps\n", i, proj, warps), 13;
       for (int i = 0; i < n; ++i) M.mem[gl.s.xs + i] = b[i];
-      M.call(proj ? "fo_gen_solve_tp" : "fo_gen_solve_t", warps);
+      M.call(proj ? "fo_gen_solve_t_p_up" : "fo_gen_solve_t_up", warps);
+      square(true, true);
+      square(false, true);
+      M.call(proj ? "fo_gen_solve_t_p_down" : "fo_gen_solve_t_down", warps);
       for (int i = 0; i < n; ++i)
         if (!same(M.mem[gl.s.xs + i], z[i])) return printf("transposed solve %d, projection %d\n", i, proj), 14;
     }
