@@ -23,6 +23,7 @@ namespace fo {
 cudaError_t launch_solve(const SolveParams& p, int grid, size_t smem, cudaStream_t stream);
 cudaError_t launch_eval(const SolveParams& p, int C, int want_jac, double* out, cudaStream_t stream);
 cudaError_t launch_adjoint(const AdjParams& a, int grid, int lanes, size_t smem, cudaStream_t stream);
+cudaError_t launch_round_policy(const SolveParams* batches, int nb, unsigned int* words, cudaStream_t stream);
 int set_last_error(int code, const char* what);
 cudaError_t launch_solve_multi(const SolveParams* batches, int nb, const int32_t* starts, int32_t* queue,
                                double* scratch, int64_t slot_doubles, int grid, int lanes, size_t smem,
@@ -426,6 +427,7 @@ struct fo_multi {
   double* d_scratch = nullptr;
   int64_t slot_doubles = 0;
   unsigned int* d_rounds = nullptr;      // lockstep rounds' barrier words, or null
+  bool one_wave = false;                 // every group has a block of its own
 };
 
 namespace {
@@ -583,6 +585,7 @@ int fo_multi_prepare(int32_t nb, const fo_batch_desc* b, void* workspace, size_t
   }
   m->nb = nb;
   m->grid = L.grid;
+  m->one_wave = L.grid >= L.total;
   m->lanes = L.lanes;
   m->smem = smem;
   m->d_batches = reinterpret_cast<fo::SolveParams*>(ws + L.params_off);
@@ -630,11 +633,13 @@ int fo_multi_launch(const fo_multi* m, void* stream) {
   if (m->d_rounds) {
     cudaError_t z = cudaMemsetAsync(m->d_rounds, 0, kRoundsWords * sizeof(unsigned int),
                                     static_cast<cudaStream_t>(stream));
-    if (z != cudaSuccess) return cuda_fail(z, "cudaMemsetAsync(rounds)");
+    if (z == cudaSuccess) z = fo::launch_round_policy(m->d_batches, m->nb, m->d_rounds, static_cast<cudaStream_t>(stream));
+    if (z != cudaSuccess) return cuda_fail(z, "lockstep rounds");
   }
   cudaError_t e = m->gen ? fo::gen_launch_multi(m->gen, m->d_batches, m->nb, m->d_starts, m->d_queue,
                                                 m->d_scratch, m->slot_doubles, m->grid, m->smem,
-                                                m->d_rounds != nullptr, static_cast<cudaStream_t>(stream))
+                                                m->d_rounds != nullptr, m->one_wave,
+                                                static_cast<cudaStream_t>(stream))
                          : fo::launch_solve_multi(m->d_batches, m->nb, m->d_starts, m->d_queue, m->d_scratch,
                                                   m->slot_doubles, m->grid, m->lanes, m->smem,
                                                   static_cast<cudaStream_t>(stream));

@@ -16,12 +16,14 @@
 #include <sys/stat.h>
 #include <unistd.h>
 
+#include <algorithm>
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
 #include <mutex>
+#include <numeric>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -437,16 +439,31 @@ cudaError_t gen_launch_adjoint(GenModule* m, const AdjParams& a, int grid, size_
   return cudaLaunchKernel(fn, dim3(grid), dim3(32, team_of(grid)), args, smem, stream);
 }
 
+// A multiplier that deals the items 0 .. grid - 1 out evenly over any run and
+// any arithmetic progression of blocks: the one nearest the golden section of
+// the grid with no common factor. A cooperative launch places its blocks SM
+// by SM where a plain one goes round all SMs; with the items in order, one
+// cold interval of 65,536 cells of three mechanisms (one wave) took 559 ms,
+// dealt out 517. With more groups than blocks the order stays: SMs full of the
+// largest mechanism balance their four sub-partitions and the others work off
+// the queue (196,608 cells, settled: 134 ms in order, 146 dealt out).
+int spread_of(int grid) {
+  for (int m = std::max(1, (int)(0.6180339887 * grid)); m > 1; --m)
+    if (std::gcd(m, grid) == 1) return m;
+  return 1;
+}
+
 cudaError_t gen_launch_multi(GenModule* m, const SolveParams* batches, int nb, const int32_t* starts,
                              int32_t* queue, double* scratch, int64_t slot_doubles, int grid, size_t smem,
-                             bool cooperative, cudaStream_t stream) {
+                             bool cooperative, bool one_wave, cudaStream_t stream) {
   const void* fn = reinterpret_cast<const void*>(m->multi_kernel);
   cudaError_t e = ensure_smem(m, 1, fn, smem);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(queue, 0, sizeof(int32_t), stream);
   if (e != cudaSuccess) return e;
-  void* args[] = {&batches, &nb, &starts, &queue, &scratch, &slot_doubles};
   const int team = team_of(grid);
+  int spread = cooperative && one_wave ? spread_of(grid) : 1;
+  void* args[] = {&batches, &nb, &starts, &queue, &scratch, &slot_doubles, &spread};
   if (cooperative) return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
   return cudaLaunchKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
 }

@@ -1945,7 +1945,8 @@ constexpr long long kRoundSpinLimit = 7500000;
 // Arrive with this block's activity in the round (1: it attempted); returns
 // the number of blocks that attempted in the round, or -1 once rounds are
 // given up. Barrier words: [0] arrivals, [1] activity sum, [2] generation,
-// [3] the last round's sum, [4] give-up. Every thread of the block calls it.
+// [3] the last round's sum, [4] give-up, [5] a several-mechanism launch's
+// choice (round_policy_kernel). Every thread of the block calls it.
 __device__ int round_barrier(unsigned int* w, int active) {
   __shared__ int result;
   __syncthreads();
