@@ -93,13 +93,25 @@ def forward_record(mech, Y0, k_of, dt, atol, rtol, intervals, group_size=32, alg
     return Trajectory(b, cps, ks, ptrs, steps, max_steps, pptrs, psteps, float(dt), at, sts)
 
 
-def _workspace(traj: Trajectory):
+def _workspace(traj: Trajectory, keep: bool = False):
+    """The adjoint's workspace; with `keep`, one that holds every replayed step
+    for the reverse sweep when that takes at most an eighth of the memory the
+    device has free (the gradients are the same either way)."""
     import torch
     b = traj.batch
-    need = C.c_size_t()
-    _abi.check(_abi.lib().fo_adjoint_workspace_bytes(b.plan.handle, b.ngroups, b.max_cells, traj.max_steps,
-                                                     C.byref(need)), "fo_adjoint_workspace_bytes")
-    return torch.empty(int(need.value), dtype=torch.uint8, device=b.Y.device)
+    dev = b.Y.device
+
+    def size(name):
+        need = C.c_size_t()
+        _abi.check(getattr(_abi.lib(), name)(b.plan.handle, b.ngroups, b.max_cells, traj.max_steps, C.byref(need)), name)
+        return int(need.value)
+
+    if keep:
+        kept = size("fo_adjoint_kept_bytes")
+        free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+        if kept <= free // 8:
+            return torch.empty(kept, dtype=torch.uint8, device=dev)
+    return torch.empty(size("fo_adjoint_workspace_bytes"), dtype=torch.uint8, device=dev)
 
 
 def _call(traj, i, mode, ws, Yin, lam=None, thbar=None, Yout=None, k=None):
@@ -144,7 +156,7 @@ def adjoint(traj: Trajectory, lam_final):
     from dL/dY at the end ((n, C) device)."""
     import torch
     b = traj.batch
-    ws = _workspace(traj)
+    ws = _workspace(traj, keep=True)
     lam = lam_final.clone()
     thbar = torch.zeros((b.plan.R, b.C), dtype=torch.float64, device=b.Y.device)
     for i in reversed(range(len(traj.checkpoints))):

@@ -666,6 +666,16 @@ int fo_adjoint_workspace_bytes(const fo_plan* plan, int32_t ngroups, int32_t max
   return FO_OK;
 }
 
+int fo_adjoint_kept_bytes(const fo_plan* plan, int32_t ngroups, int32_t max_group_cells, int32_t max_steps,
+                          size_t* bytes) {
+  if (!plan || !bytes || ngroups <= 0 || max_group_cells <= 0 || max_steps < 0)
+    return fail(FO_E_INVALID, "bad argument");
+  const fo::AdjLayout al = adjoint_layout(plan->host, max_steps);
+  const int64_t kept = (int64_t)max_steps * al.yp + (al.ys - al.yp);
+  *bytes = kHeader + sizeof(double) * (size_t)ngroups * (size_t)std::max(kept, al.items) * lanes_for(max_group_cells);
+  return FO_OK;
+}
+
 int fo_adjoint_interval(const fo_plan* plan, const fo_options* opt, int32_t ngroups, const int32_t* group_offsets,
                         int32_t max_group_cells, const double* Y, int64_t ycs, int64_t yss, const double* k,
                         int64_t kcs, int64_t krs, const double* atol, double dt, const int32_t* step_ptr,
@@ -702,6 +712,15 @@ int fo_adjoint_interval(const fo_plan* plan, const fo_options* opt, int32_t ngro
     smem = smem_bytes(plan->host, a.p.lanes, a.p.o.variant);
   }
   a.p.slot_doubles = a.al.items * a.p.lanes;
+  a.yp_doubles = a.al.yp * a.p.lanes;
+  a.step_doubles = 0;
+  size_t kept = 0;
+  fo_adjoint_kept_bytes(plan, ngroups, max_group_cells, max_steps, &kept);
+  if (generated && mode == 1 && max_steps > 0 && workspace_bytes >= kept) {
+    a.step_doubles = a.al.yp * a.p.lanes;
+    a.yp_doubles = max_steps * a.step_doubles;
+    a.p.slot_doubles = a.yp_doubles + (a.al.ys - a.al.yp) * a.p.lanes;
+  }
   a.p.scratch = reinterpret_cast<double*>(static_cast<char*>(workspace) + kHeader);
   a.Ycp = Y;
   a.ycs = ycs;

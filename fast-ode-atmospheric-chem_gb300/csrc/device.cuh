@@ -160,6 +160,8 @@ struct AdjParams {
   const int32_t* proj_ptr;  // ngroups+1, or null: the projection updates of each group
   const double* proj_steps; // their accepted line-search steps
   int mode;             // 0 replay, 1 adjoint
+  int64_t step_doubles; // generated: every replayed step keeps a slot of this size (0: one slot, steps recomputed)
+  int64_t yp_doubles;   // the states before the projection's updates, from the group's slot
   int32_t* status;
 };
 

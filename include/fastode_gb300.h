@@ -362,6 +362,12 @@ int fo_advance_clock(double* t_dev, double dt, void* stream);
  */
 int fo_adjoint_workspace_bytes(const fo_plan* plan, int32_t ngroups, int32_t max_group_cells, int32_t max_steps,
                                size_t* bytes);
+/* The workspace with which the generated adjoint (mode 1) keeps every replayed
+ * step (factors, stage solutions) for the reverse sweep instead of computing it
+ * again there: max_steps slots per group. A smaller workspace, from
+ * fo_adjoint_workspace_bytes up, gives the same gradients. */
+int fo_adjoint_kept_bytes(const fo_plan* plan, int32_t ngroups, int32_t max_group_cells, int32_t max_steps,
+                          size_t* bytes);
 int fo_adjoint_interval(const fo_plan* plan, const fo_options* opt, int32_t ngroups, const int32_t* group_offsets,
                         int32_t max_group_cells,
                         const double* Y, int64_t y_cell_stride, int64_t y_species_stride,

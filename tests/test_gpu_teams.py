@@ -46,6 +46,35 @@ def test_results_do_not_depend_on_the_team(cuda, case, groups, lockstep):
         assert torch.equal(got[2], want[2][None].expand_as(got[2])), g
 
 
+@pytest.mark.parametrize("case,intervals", [("ros3_20x40", 3), ("rodas3_dae_160x340", 2)])
+def test_adjoint_with_and_without_kept_steps(cuda, case, intervals, monkeypatch):
+    """The reverse sweep on the replay's kept steps gives the bits of the one
+    that computes every step again."""
+    from fastode_gb300 import RODAS3, ROS3, Algorithm, adjoint as A
+    torch = cuda
+    f = load(case)
+    dae = "mass" in f
+    mech = mechanism_of(f)
+    ks = [torch.from_numpy(np.ascontiguousarray(f["k"][i].T)).cuda() for i in range(intervals)]
+    traj = A.forward_record(mech, f["Y0"], lambda i: ks[i], float(f["dt"]), f["atol"], float(f["rtol"]), intervals,
+                            algorithm=Algorithm(RODAS3 if dae else ROS3), mass=f["mass"] if dae else None)
+    lam = torch.from_numpy(np.random.default_rng(3).standard_normal(traj.batch.Y.shape)).cuda() / traj.batch.Y.clamp_min(1e-14)
+    sizes, plain = [], A._workspace
+
+    def spy(t, keep=False):
+        ws = plain(t, keep)
+        sizes.append(ws.numel())
+        return ws
+
+    monkeypatch.setattr(A, "_workspace", spy)
+    kept = A.adjoint(traj, lam)
+    monkeypatch.setattr(A, "_workspace", lambda t, keep=False: spy(t, False))
+    again = A.adjoint(traj, lam)
+    assert sizes[0] > sizes[1]
+    for x, y in zip(kept, again):
+        assert torch.equal(x, y)
+
+
 def test_dropin_calls_share_no_buffers(cuda):
     """Drop-in calls of several shapes in turn, and from four threads on their
     own streams, against the same calls one at a time."""
