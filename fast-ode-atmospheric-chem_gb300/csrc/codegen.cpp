@@ -159,8 +159,30 @@ int64_t cost_of(const Task& t) {
   return c / 4 + 1;
 }
 
+// Splits tasks (longest first) between the segments that agree with `seg` in
+// their low `bit` bits: two halves of like cost, halved again down to single
+// segments. A team of 2^m warps gives a warp the segments that agree in m low
+// bits, so every team size finds its warps' loads balanced (one long task
+// leaves its warp alone with it).
+void halve(const std::vector<int>& tasks, const std::vector<int64_t>& cost, int bit, int seg,
+           const std::function<void(int, int)>& place) {
+  if (tasks.empty()) return;
+  if ((1 << bit) >= kSegments || (tasks.size() == 1)) {
+    for (int i : tasks) place(i, seg);
+    return;
+  }
+  std::vector<int> half[2];
+  int64_t load[2] = {0, 0};
+  for (int i : tasks) {
+    const int h = load[1] < load[0] ? 1 : 0;
+    half[h].push_back(i);
+    load[h] += cost[i];
+  }
+  for (int h = 0; h < 2; ++h) halve(half[h], cost, bit + 1, seg | (h << bit), place);
+}
+
 // Tasks into steps of kSegments segments. A step takes every task whose
-// inputs are ready, longest first onto the least loaded segment; a task whose
+// inputs are ready, spread over the segments (halve); a task whose
 // last inputs are made in one segment of the step follows them there when
 // that does not lengthen the step (a short step is lengthened: a barrier and
 // the first loads of a step cost about kStepCost), or when it is the only
@@ -194,7 +216,7 @@ Phase schedule(const std::vector<Task>& tasks) {
       placed.push_back(i);
       ++done;
     };
-    for (int i : ready) place(i, (int)(std::min_element(load.begin(), load.end()) - load.begin()));
+    halve(ready, cost, 0, 0, place);
     const bool serial = placed.size() < 3;
     const int64_t limit = std::max(*std::max_element(load.begin(), load.end()), kStepCost);
     for (size_t q = 0; q < placed.size(); ++q) {
