@@ -496,6 +496,7 @@ int fo_solve(const fo_plan* plan, const fo_options* opt, int32_t ngroups, const 
   // header, zeroed for every launch
   p.rounds = nullptr;
   p.round_attempts = 1;
+  p.round_halves = 1;
   if (opt->lockstep && p.o.variant == FO_VARIANT_GENERATED && p.o.loop == FO_LOOP_ALGORITHM &&
       fo::gen_rounds_pay(grid)) {
     p.rounds = reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + kRoundsOffset);

@@ -116,6 +116,8 @@ struct SolveParams {
   int32_t* trace_len;
   unsigned int* rounds;          // lockstep rounds (five barrier words), or null
   int round_attempts;            // attempts per round
+  int round_halves;              // a round's attempts also meet between the factorization and the solves
+                                 // (one attempt per round only)
 };
 
 // Extra per-lane scratch of the adjoint (items after the forward layout). The

@@ -2101,6 +2101,13 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
       const double alpha = attempt_scalars(o.tab, red, H);
       factor_any(p, ln, alpha, negj, lu, w, false);
       ++c_lu;
+      // Meet once more before the solves. The scheduler favours an SM's oldest
+      // warps, so groups leave the factorization, which fills the FP64 units,
+      // one after another; without this the youngest made its solves, which
+      // wait on memory and on one another, with the SM to itself. One settled
+      // interval of 65,536 cells of the 210/500 mechanism 120 and 110 ms,
+      // constrained 160/340 with 16,384 cells 31.4 and 28.1 ms.
+      if (p.rounds != nullptr && p.round_halves) round_barrier(p.rounds, 1);
       const double part = attempt(p, ln, H, Y, Ynew, scr, w, red, c_rhs, c_solves, fresh);
       fresh = false;
       const double err = team_once(red + kSlotError, [&] {
