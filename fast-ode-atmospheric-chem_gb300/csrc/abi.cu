@@ -495,8 +495,7 @@ int fo_solve(const fo_plan* plan, const fo_options* opt, int32_t ngroups, const 
   // lockstep rounds (fo_options.lockstep): barrier words in the workspace
   // header, zeroed for every launch
   p.rounds = nullptr;
-  p.round_attempts = 1;
-  p.round_halves = 1;
+  p.round_cost = fo::kRoundUnits;
   if (opt->lockstep && p.o.variant == FO_VARIANT_GENERATED && p.o.loop == FO_LOOP_ALGORITHM &&
       fo::gen_rounds_pay(grid)) {
     p.rounds = reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + kRoundsOffset);
@@ -615,7 +614,7 @@ int fo_multi_prepare(int32_t nb, const fo_batch_desc* b, void* workspace, size_t
     p.queue = m->d_queue;
     p.rounds = m->d_rounds;
     const int64_t cost = std::max<int64_t>(1, b[order[j]].plan->host.lu_fma + 3 * b[order[j]].plan->host.solve_fma);
-    p.round_attempts = (int)std::max<int64_t>(1, (cost_max + cost / 2) / cost);
+    p.round_cost = (int)std::max<int64_t>(1, cost * fo::kRoundUnits / cost_max);
   }
   e = cudaMemcpy(m->d_batches, params.data(), sizeof(fo::SolveParams) * nb, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)

@@ -92,6 +92,9 @@ struct ScratchLayout {
   int64_t items;                                   // total items per lane
 };
 
+// A round of lockstep, and the part of it before the solves.
+constexpr int kRoundUnits = 1024, kRoundSolves = 820;
+
 struct SolveParams {
   DevTables t;
   DevOptions o;
@@ -115,9 +118,7 @@ struct SolveParams {
   int trace_cap;
   int32_t* trace_len;
   unsigned int* rounds;          // lockstep rounds (five barrier words), or null
-  int round_attempts;            // attempts per round
-  int round_halves;              // a round's attempts also meet between the factorization and the solves
-                                 // (one attempt per round only)
+  int round_cost;                // an attempt's share of a round, in kRoundUnits
 };
 
 // Extra per-lane scratch of the adjoint (items after the forward layout). The

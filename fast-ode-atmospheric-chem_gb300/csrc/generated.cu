@@ -25,11 +25,12 @@
 extern "C" __global__ void __launch_bounds__(32 * 16, 1) fo_generated_solve_kernel(fo::SolveParams p) {
   extern __shared__ double smem[];
   double* red = smem;       // 32 doubles
+  fo::RoundPace pace;
   double* w = smem + 32;    // a cluster's partial sums
   const int slot = blockIdx.x / cluster_blocks();
   double* scr = p.scratch + (int64_t)slot * p.slot_doubles;
   if (p.queue == nullptr) {
-    fo::solve_group(p, slot, scr, w, red);
+    fo::solve_group(p, slot, scr, w, red, pace);
   } else {
     __shared__ int next;
     for (;;) {
@@ -38,7 +39,7 @@ extern "C" __global__ void __launch_bounds__(32 * 16, 1) fo_generated_solve_kern
       __syncthreads();
       const int g = next;
       if (g >= p.ngroups) break;
-      fo::solve_group(p, g, scr, w, red);
+      fo::solve_group(p, g, scr, w, red, pace);
     }
   }
   fo::rounds_drain(p.rounds);
@@ -53,6 +54,7 @@ extern "C" __global__ void __launch_bounds__(32 * 16, 1)
                               int32_t* queue, double* scratch, int64_t slot_doubles, int spread) {
   extern __shared__ double smem[];
   double* red = smem;
+  fo::RoundPace pace;
   double* w = smem + 32;
   double* scr = scratch + (int64_t)blockIdx.x * slot_doubles;
   __shared__ int next;
@@ -78,7 +80,7 @@ extern "C" __global__ void __launch_bounds__(32 * 16, 1)
       if (fo::team_leader()) params.rounds = nullptr;
       __syncthreads();
     }
-    fo::solve_group(params, item - starts[b], scr, w, red);
+    fo::solve_group(params, item - starts[b], scr, w, red, pace);
   }
   fo::rounds_drain(rounds);
 }

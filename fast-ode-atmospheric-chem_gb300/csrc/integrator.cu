@@ -36,10 +36,11 @@ namespace fo {
 __global__ void __maxnreg__(255) solve_kernel(SolveParams p) {
   extern __shared__ double smem[];
   double* red = smem;       // 32 doubles
+  RoundPace pace;
   double* w = smem + 32;    // n * lanes
   double* scr = p.scratch + (int64_t)blockIdx.x * p.slot_doubles;
   if (p.queue == nullptr) {
-    solve_group(p, blockIdx.x, scr, w, red);
+    solve_group(p, blockIdx.x, scr, w, red, pace);
     return;
   }
   __shared__ int next;
@@ -49,7 +50,7 @@ __global__ void __maxnreg__(255) solve_kernel(SolveParams p) {
     __syncthreads();
     const int g = next;
     if (g >= p.ngroups) break;
-    solve_group(p, g, scr, w, red);
+    solve_group(p, g, scr, w, red, pace);
   }
 }
 
@@ -101,6 +102,7 @@ __global__ void __maxnreg__(255) solve_multi_kernel(const SolveParams* __restric
                                                           double* scratch, int64_t slot_doubles) {
   extern __shared__ double smem[];
   double* red = smem;
+  RoundPace pace;
   double* w = smem + 32;
   double* scr = scratch + (int64_t)blockIdx.x * slot_doubles;
   __shared__ int next;
@@ -116,7 +118,7 @@ __global__ void __maxnreg__(255) solve_multi_kernel(const SolveParams* __restric
     int b = 0;
     while (b + 1 < nb && item >= starts[b + 1]) ++b;
     load_batch_params(batches, b, current, params);
-    solve_group(params, item - starts[b], scr, w, red);
+    solve_group(params, item - starts[b], scr, w, red, pace);
   }
 }
 

@@ -1927,11 +1927,10 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
 
 // Lockstep rounds. With every block of the launch resident at once (a
 // cooperative launch), the groups make their attempts in rounds: each block
-// makes one attempt (or p.round_attempts attempts, so that a round of a small
-// mechanism costs about as much as one of the largest in a several-mechanism
-// launch), then waits at a grid-wide barrier for the others; a block with no
-// group left keeps arriving with nothing to do until a round in which no
-// block attempted. The straight-line factorization is megabytes of code, so
+// makes one attempt (of a small mechanism in a several-mechanism launch as many
+// as cost about one of the largest, of one group after another), then waits
+// at a grid-wide barrier for the others; a block with no group left keeps
+// arriving with nothing to do until a round in which no block attempted. The straight-line factorization is megabytes of code, so
 // warps that drift apart each stream their own instructions and thrash the
 // SM's instruction cache; rounds keep the warps of an SM at the same place
 // (the cold first interval of the 210/500, 65,536-cell job: 1.47 s without
@@ -1940,6 +1939,13 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
 // bit. Each wait is bounded (kRoundSpinLimit polls about 4 us apart, some
 // 30 s); a wait that gives up raises the give-up word, after which every
 // block runs on without rounds.
+//
+// The blocks of a round also meet before the solves. The scheduler favours an
+// SM's oldest warps, so groups leave the factorization, which fills the FP64
+// units, one after another; without that the youngest made its solves, which
+// wait on memory and on one another, with the SM to itself. One settled
+// interval of 65,536 cells of the 210/500 mechanism 120 and 110 ms,
+// constrained 160/340 with 16,384 cells 31.4 and 28.1 ms.
 constexpr long long kRoundSpinLimit = 7500000;
 
 // Arrive with this block's activity in the round (1: it attempted); returns
@@ -2003,6 +2009,27 @@ __device__ __forceinline__ void load_batch_params(const SolveParams* __restrict_
   current = b;
 }
 
+// Where a block is in its round: the units done, and whether it has met the
+// others before the solves. It carries over from group to group.
+struct RoundPace {
+  int done = 0;
+  bool met = false;
+};
+
+// The block has done `units` more of its round.
+__device__ __forceinline__ void round_advance(const SolveParams& p, RoundPace& pace, int units) {
+  pace.done += units;
+  if (!pace.met && pace.done >= kRoundSolves) {
+    round_barrier(p.rounds, 1);
+    pace.met = true;
+  }
+  if (pace.met && pace.done >= kRoundUnits) {
+    round_barrier(p.rounds, 1);
+    pace.met = false;
+    pace.done -= kRoundUnits;
+  }
+}
+
 // A block with no group left: arrive idle until a round without attempts.
 __device__ __forceinline__ void rounds_drain(unsigned int* w) {
   if (w != nullptr)
@@ -2010,15 +2037,17 @@ __device__ __forceinline__ void rounds_drain(unsigned int* w) {
     }
 }
 
-__device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, double* w, double* red);
+__device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, double* w, double* red,
+                                      RoundPace& pace);
 
-__device__ void solve_group(const SolveParams& p, int g, double* scr, double* w, double* red) {
+__device__ void solve_group(const SolveParams& p, int g, double* scr, double* w, double* red, RoundPace& pace) {
   if (p.o.loop == FO_LOOP_RESTARTING) solve_group_restarting(p, g, scr, w, red);
   else if (p.o.loop == FO_LOOP_BACKWARD_EULER) solve_group_backward_euler(p, g, scr, w, red);
-  else solve_group_algorithm(p, g, scr, w, red);
+  else solve_group_algorithm(p, g, scr, w, red, pace);
 }
 
-__device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, double* w, double* red) {
+__device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, double* w, double* red,
+                                      RoundPace& pace) {
   const int L = blockDim.x, lane = threadIdx.x;
   const int n = p.t.n;
   const int64_t c0 = p.group_offsets[g], c1 = p.group_offsets[g + 1];
@@ -2033,7 +2062,6 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
 
   long long c_steps = 0, c_acc = 0, c_rej = 0, c_rhs = 0, c_jac = 0, c_lu = 0, c_solves = 0;
   int nrec = 0;
-  int since_round = 0;
 
   double* Y = scr + p.sl.y * L;
   double* Ynew = scr + p.sl.ynew * L;
@@ -2101,13 +2129,8 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
       const double alpha = attempt_scalars(o.tab, red, H);
       factor_any(p, ln, alpha, negj, lu, w, false);
       ++c_lu;
-      // Meet once more before the solves. The scheduler favours an SM's oldest
-      // warps, so groups leave the factorization, which fills the FP64 units,
-      // one after another; without this the youngest made its solves, which
-      // wait on memory and on one another, with the SM to itself. One settled
-      // interval of 65,536 cells of the 210/500 mechanism 120 and 110 ms,
-      // constrained 160/340 with 16,384 cells 31.4 and 28.1 ms.
-      if (p.rounds != nullptr && p.round_halves) round_barrier(p.rounds, 1);
+      const int to_solves = p.round_cost * kRoundSolves / kRoundUnits;
+      if (p.rounds != nullptr) round_advance(p, pace, to_solves);
       const double part = attempt(p, ln, H, Y, Ynew, scr, w, red, c_rhs, c_solves, fresh);
       fresh = false;
       const double err = team_once(red + kSlotError, [&] {
@@ -2167,10 +2190,7 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
         if (last) H = __dsub_rn(dt, t);
         ++c_rej;
       }
-      if (p.rounds != nullptr && ++since_round >= p.round_attempts) {
-        since_round = 0;
-        round_barrier(p.rounds, 1);
-      }
+      if (p.rounds != nullptr) round_advance(p, pace, p.round_cost - to_solves);
     }
   }
   if (status < 0) status = FO_STATUS_CONVERGED;
