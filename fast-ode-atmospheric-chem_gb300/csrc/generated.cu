@@ -14,7 +14,7 @@
 // resident per SM whatever the team's size; jit.cpp chooses it by the number
 // of blocks. Where the groups are too few even for one SM each, a cluster of
 // sixteen-warp blocks on several SMs works on a group (the integrator kernel
-// without the queue, unconstrained Rosenbrock loops).
+// without the queue).
 #define FO_LINK_GENERATED 1
 
 #include <cuda_runtime.h>

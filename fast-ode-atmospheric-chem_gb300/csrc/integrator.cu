@@ -127,8 +127,8 @@ __global__ void __maxnreg__(255) solve_multi_kernel(const SolveParams* __restric
 // a sixteenth of the interval. Such groups make many attempts, and rounds keep
 // the warps of an SM together; groups on settled steps make one to three, and
 // rounds only make the slots wait for one another between groups. Measured
-// with and without rounds on 196,608 cells of three mechanisms: cold 1103 and
-// 1248 ms, settled 149 and 137 ms.
+// with and without rounds on three mechanisms: 65,536 cells, settled, 66 and
+// 61 ms; 196,608 cells, cold, 976 and 1235 ms.
 __global__ void __launch_bounds__(1024) round_policy_kernel(const SolveParams* __restrict__ batches, int nb,
                                                             unsigned int* words) {
   int cold = 0, total = 0;

@@ -355,7 +355,9 @@ bool all_resident(const void* fn, int grid, int team, size_t smem) {
 // so a mechanism with little work per attempt stays on one SM: 20/40 (1,600
 // operations) does, TS1 (21,000) does not. One SM and a cluster, measured: a
 // cold interval of one 210/500 group 66.5 and 32.0 ms, eight intervals of TS1
-// on two groups 34.4 and 25.8 ms (both with the leading rows' tasks split).
+// on two groups 34.4 and 25.8 ms (both with the leading rows' tasks split);
+// two Newton iterations of backward Euler on 42 groups of 120/260 (clusters of
+// 2) 1.42 and 1.23 ms.
 constexpr int64_t kClusterWork = 10000;
 constexpr size_t kClusterSmem = sizeof(double) * (32 + 32 * kBlockWarps);
 
@@ -419,7 +421,7 @@ cudaError_t gen_launch(GenModule* m, const SolveParams& p, int grid, size_t smem
   if (q.rounds != nullptr && all_resident(fn, grid, team, smem))
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
   q.rounds = nullptr;
-  if (team == kBlockWarps && q.queue == nullptr && !q.t.has_constraints && q.o.loop != FO_LOOP_BACKWARD_EULER) {
+  if (team == kBlockWarps && q.queue == nullptr) {
     const int blocks = cluster_of(m, fn, grid);
     if (blocks > 1) {
       cudaLaunchAttribute attr;

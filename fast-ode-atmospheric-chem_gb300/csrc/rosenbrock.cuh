@@ -1011,6 +1011,20 @@ __device__ __forceinline__ void generated_solve(const SolveParams& p, double* ba
     else fo_gen_solve_down(base, w, wn, mech);
   }
 }
+
+// x = A^-1 b in place on the solve vector by the whole team. A solve is a chain
+// of small steps: one block of a cluster with its own barriers and L1 is
+// faster than all of them (210/500: 0.32 M cycles and 0.38 M).
+template <bool kProjection>
+__device__ __forceinline__ void team_solve(const SolveParams& p, double* base) {
+  if (cluster_team()) {
+    team_sync();   // the right-hand side, from every block
+    if (cluster_rank() == 0) generated_solve<false, kProjection>(p, base, BLOCK_W, BLOCK_N);
+    team_sync();
+  } else {
+    generated_solve<false, kProjection>(p, base, BLOCK_W, BLOCK_N);
+  }
+}
 #endif
 
 __device__ void factor_any(const SolveParams& p, const Lane& ln, double alpha, const double* negj, double* lu,
@@ -1054,8 +1068,8 @@ __device__ void solve_into(const SolveParams& p, const Lane& ln, const double* l
   double* base = const_cast<double*>(lu) - p.sl.lu * ln.L;
   double* xs = base + p.sl.xs * ln.L;
   if (b != xs) copy_items(ln, p.t.n, b, xs);
-  if (alg_only) generated_solve<false, true>(p, base + ln.lane, BLOCK_W, BLOCK_N);
-  else generated_solve<false, false>(p, base + ln.lane, BLOCK_W, BLOCK_N);
+  if (alg_only) team_solve<true>(p, base + ln.lane);
+  else team_solve<false>(p, base + ln.lane);
   if (x != xs) copy_items(ln, p.t.n, xs, x);
 #else
   if (p.o.variant == FO_VARIANT_COMPACT) {
@@ -1267,15 +1281,7 @@ __device__ __noinline__ double attempt_generated(const SolveParams& p, const Lan
         xs[i * 32] = v[b];
       }
     }
-    if (cluster_team()) {
-      // a solve is a chain of small steps: one block with its own barriers
-      // and L1 is faster than the cluster (210/500: 0.32 M cycles and 0.38 M)
-      team_sync();   // the right-hand side, from every block
-      if (cluster_rank() == 0) generated_solve<false, false>(p, base, BLOCK_W, BLOCK_N);
-      team_sync();
-    } else {
-      generated_solve<false, false>(p, base, BLOCK_W, BLOCK_N);
-    }
+    team_solve<false>(p, base);
   }
   // Y_new, E and the weighted sum of squares: min(n, 16) interleaved partial
   // sums (species s, s + 16, ...), added in order, whatever the team's size
@@ -1523,21 +1529,48 @@ __device__ void trace_record(const SolveParams& p, int g, int& nrec, double t, d
   ++nrec;
 }
 
-// Block-wide max with NaN propagation (numpy max) and block-wide AND.
-__device__ double block_max(double v, double* red) {
+// One double per block of a cluster, of each block's v, for every block: in
+// the slot's partial derivatives, which no evaluation uses here.
+__device__ __forceinline__ void cluster_gather(const SolveParams& p, double v, double (&all)[8]) {
+#ifdef FO_LINK_GENERATED
+  const int blocks = cluster_blocks();
+  double* const at = p.scratch + (int64_t)(blockIdx.x / blocks) * p.slot_doubles + p.sl.d * 32;
+  if (threadIdx.x == 0 && BLOCK_W == 0) at[cluster_rank() * 32] = v;
+  team_sync();
+#pragma unroll
+  for (int b = 0; b < 8; ++b) all[b] = b < blocks ? at[b * 32] : v;
+  team_sync();
+#endif
+}
+
+// Team-wide max with NaN propagation (numpy max) and team-wide AND.
+__device__ double block_max(const SolveParams& p, double v, double* red) {
   for (int off = 16; off > 0; off >>= 1) v = npmax(v, __shfl_xor_sync(0xffffffffu, v, off));
-  const int nw = (blockDim.x >> 5) * TEAM_N;
+  const int nw = (blockDim.x >> 5) * BLOCK_N;
   if (nw == 1) return v;
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[(threadIdx.x >> 5) + TEAM_W] = v;
+  if ((threadIdx.x & 31) == 0) red[(threadIdx.x >> 5) + BLOCK_W] = v;
   __syncthreads();
   double s = red[0];
   for (int i = 1; i < nw; ++i) s = npmax(s, red[i]);
+  if (cluster_team()) {
+    double all[8];
+    cluster_gather(p, s, all);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) s = npmax(s, all[b]);
+  }
   return s;
 }
 
-__device__ bool block_all(bool v) {
-  return __syncthreads_and(v ? 1 : 0) != 0;
+__device__ bool block_all(const SolveParams& p, bool v) {
+  bool all_true = __syncthreads_and(v ? 1 : 0) != 0;
+  if (cluster_team()) {
+    double all[8];
+    cluster_gather(p, all_true ? 1.0 : 0.0, all);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) all_true = all_true && all[b] != 0.0;
+  }
+  return all_true;
 }
 
 struct ProjectionCounts {
@@ -1551,7 +1584,7 @@ __device__ bool alg_finite(const SolveParams& p, const Lane& ln, const double* A
   if (ln.active)
     for (int i = TEAM_W; i < p.t.n; i += TEAM_N)
       if (__ldg(p.t.mass + i) == 0.0 && !isfinite(SCR(A, i))) ok = false;
-  return block_all(ok);
+  return block_all(p, ok);
 }
 
 // max over the group's algebraic entries of |A|
@@ -1561,7 +1594,7 @@ __device__ double alg_absmax(const SolveParams& p, const Lane& ln, const double*
   if (ln.active)
     for (int i = TEAM_W; i < p.t.n; i += TEAM_N)
       if (__ldg(p.t.mass + i) == 0.0) m = npmax(m, fabs(SCR(A, i)));
-  return block_max(m, red);
+  return block_max(p, m, red);
 }
 
 // The weighted Newton correction of fastode/solvers.py:119-124:
@@ -1582,7 +1615,7 @@ __device__ double weighted(const SolveParams& p, const Lane& ln, const double* Z
       else q = (d == 0.0) ? 0.0 : CUDART_INF;
       m = npmax(m, q);
     }
-  return block_max(m, red);
+  return block_max(p, m, red);
 }
 
 // G = F(Z) with the differential rows zeroed (fastode/solvers.py:110-114).
@@ -1869,7 +1902,7 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
           conv = conv && isfinite(d) && fabs(d) <= bound;
         }
       }
-      if (iterations > 1) ok = block_all(!ln.active || conv);
+      if (iterations > 1) ok = block_all(p, !ln.active || conv);
       if (ok || iterations >= o.max_iterations) break;
     }
     ++c_steps;
@@ -1883,7 +1916,7 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
         status = FO_STATUS_ACCEPTED_UNCONVERGED;
         bool finite = true;
         for (int i = TEAM_W; i < n; i += TEAM_N) finite = finite && isfinite(SCR(Yn1, i));
-        if (!block_all(!ln.active || finite)) status = FO_STATUS_NAN_OR_INF;
+        if (!block_all(p, !ln.active || finite)) status = FO_STATUS_NAN_OR_INF;
         break;
       }
       for (int i = TEAM_W; i < n; i += TEAM_N) SCR(Yn1, i) = SCR(Yn, i);
