@@ -305,6 +305,17 @@ cudaError_t ensure_smem(GenModule* m, int which, const void* fn, size_t smem) {
   return cudaSuccess;
 }
 
+// Multiprocessors of the current device, or 0.
+int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  return sms;
+}
+
 // Warps per group for a launch of `grid` blocks on the current device: the
 // largest power of two, up to kBlockWarps, that still leaves every block
 // resident at sixteen warps per SM (the kernels' 128 registers per thread):
@@ -314,25 +325,27 @@ cudaError_t ensure_smem(GenModule* m, int which, const void* fn, size_t smem) {
 // (257 groups, teams of 8) 27.0 and 9.2 ms; the cold interval of 16,384 cells
 // of the 210/500 mechanism (512 groups, teams of 4) 452 and 270 ms.
 int team_of(int grid) {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return 1;
-  }
+  const int sms = device_sms();
   int team = 1;
   while (2 * team <= kBlockWarps && (int64_t)grid * 2 * team <= (int64_t)sms * 16) team *= 2;
   return team;
 }
 
-// Whether lockstep rounds pay for launches of such teams: they keep the
-// groups of an SM in the same part of the generated code, which pays where
-// three or more share an SM (teams of up to four), and make every group wait
-// for the slowest each attempt. With and without rounds, ms: 210/500 cold,
-// 16,384 cells (teams of 4) 268 and 300; 9,600 cells (8) 198 and 168; 4,800
-// cells (16) 115 and 95; TS1, 65,536 cells (1) 44.8 and 53.0, 2,048 cells (16)
-// 4.9 and 4.8; 20/40, 64 cells x 20 (16) 2.7 and 2.4.
-bool rounds_pay(int team) { return team <= 4; }
+// Whether lockstep rounds pay for a launch of `grid` groups: they keep the
+// groups of an SM in the same part of the generated code and let them solve
+// together, and make every group wait for the slowest each attempt. That pays
+// with two or more groups per SM where the SMs are evenly loaded (85% of the
+// fullest; with four or more per SM, always). With and without rounds, ms:
+// 210/500 cold, 16,384 cells (3.4 groups per SM) 229 and 302; 13,000 (2.7) 188
+// and 216; 10,000 (2.06) 178 and 160; 9,600 (1.97) 143 and 158; 8,192 (1.7) 125
+// and 125; 4,800 (0.99) 95 and 76; TS1, 65,536 cells (13.5) 41 and 56, 2,048
+// cells (0.4) 5.0 and 4.5.
+bool rounds_pay(int grid) {
+  const int sms = device_sms();
+  if (sms <= 0) return false;
+  const int64_t per_sm = ((int64_t)grid + sms - 1) / sms;
+  return per_sm >= 4 || (per_sm >= 2 && 100 * (int64_t)grid >= 85 * per_sm * sms);
+}
 
 // Whether `grid` blocks of `team` warps of kernel `fn` with `smem` bytes of
 // dynamic shared memory are all resident at once on the current device (what
@@ -398,7 +411,7 @@ int cluster_of(GenModule* m, const void* fn, int grid) {
 
 }  // namespace
 
-bool gen_rounds_pay(int grid) { return rounds_pay(team_of(grid)); }
+bool gen_rounds_pay(int grid) { return rounds_pay(grid); }
 
 bool gen_resident(GenModule* m, bool multi, int grid, size_t smem) {
   const void* fn = reinterpret_cast<const void*>(multi ? m->multi_kernel : m->kernel);
