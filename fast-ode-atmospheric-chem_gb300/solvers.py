@@ -100,16 +100,18 @@ def _device_solve(solver, system, Y, dt, atol, rtol, counts: Counts, mem):
     st.h_k[:] = k
     stream = torch.cuda.current_stream(st.dev.device)
     with torch.cuda.stream(stream):
-        st.dev.copy_(st.host, non_blocking=True)
-        rc = _abi.lib().fo_solve(
-            plan.handle, C.byref(opts), 1, st.offsets.data_ptr(), C_cells,
-            st.p_Y, n, 1, st.p_k, 0 if k.shape[0] == 1 else plan.R, 1,
-            st.p_atol, float(rtol), float(dt),
-            st.p_memory, st.p_counts, st.p_status, st.ws.data_ptr(), st.ws.numel(), 0,
-            None, 0, None, C.c_void_p(stream.cuda_stream))
-        _abi.check(rc, "fo_solve")
-        st.host_out.copy_(st.dev_out, non_blocking=True)
-    stream.synchronize()
+        try:
+            st.dev.copy_(st.host, non_blocking=True)
+            rc = _abi.lib().fo_solve(
+                plan.handle, C.byref(opts), 1, st.offsets.data_ptr(), C_cells,
+                st.p_Y, n, 1, st.p_k, 0 if k.shape[0] == 1 else plan.R, 1,
+                st.p_atol, float(rtol), float(dt),
+                st.p_memory, st.p_counts, st.p_status, st.ws.data_ptr(), st.ws.numel(), 0,
+                None, 0, None, C.c_void_p(stream.cuda_stream))
+            _abi.check(rc, "fo_solve")
+            st.host_out.copy_(st.dev_out, non_blocking=True)
+        finally:
+            stream.synchronize()   # a refused call's buffers go back with their copy done, too
     if mem is not None:
         mem.h_next, mem.err_prev, mem.h_prev = (float(v) for v in st.h_memory)
     counts.add_row(st.h_counts)
