@@ -82,6 +82,9 @@ struct DevOptions {
 // block and two columns of operands fit the 128 registers of a thread.
 constexpr int kDenseBlock = 6;
 
+// The most blocks of a cluster that work on one group.
+constexpr int kMaxCluster = 8;
+
 // Per-lane scratch layout, in items (each item is `lanes` doubles).
 struct ScratchLayout {
   int64_t lu, negj, d, r, y, ynew, f0, ft, yr, k;  // offsets
@@ -117,7 +120,7 @@ struct SolveParams {
   double* trace;
   int trace_cap;
   int32_t* trace_len;
-  unsigned int* rounds;          // lockstep rounds (five barrier words), or null
+  unsigned int* rounds;          // lockstep rounds (barrier words), or null
   int round_cost;                // an attempt's share of a round, in kRoundUnits
 };
 

@@ -193,7 +193,7 @@ struct GenModule {
   cudaKernel_t adjoint_kernel = nullptr;  // fo_generated_adjoint_kernel
   std::mutex mutex;
   int configured_smem[3][64] = {};
-  int64_t attempt_work = 0;               // FP64 operations of an attempt (one mechanism)
+  int64_t attempt_work = 0;               // FP64 operations of an attempt (one mechanism; 0: no clusters)
   int clusters[64][4] = {};               // resident clusters of 2^i blocks, plus one (0: not asked yet)
 };
 
@@ -252,7 +252,9 @@ int gen_create(const std::vector<const HostTables*>& ts, const std::vector<GenOp
     info->cubin_bytes = (int64_t)cubin.size();
     info->seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   }
-  if (ts.size() == 1)
+  // a cluster's blocks exchange a value each through the items of the slot's
+  // partial derivatives and rates, of which there are at least R
+  if (ts.size() == 1 && ts[0]->R >= kMaxCluster)
     m->attempt_work = ts[0]->lu_fma + 3 * ts[0]->solve_fma + (int64_t)ts[0]->jt_idx.size() +
                       2 * (int64_t)ts[0]->s_rxn.size();
   *out = m;

@@ -1530,15 +1530,16 @@ __device__ void trace_record(const SolveParams& p, int g, int& nrec, double t, d
 }
 
 // One double per block of a cluster, of each block's v, for every block: in
-// the slot's partial derivatives, which no evaluation uses here.
-__device__ __forceinline__ void cluster_gather(const SolveParams& p, double v, double (&all)[8]) {
+// the slot's partial derivatives and rates (R items or more, so R is at least
+// kMaxCluster wherever clusters run), which no evaluation uses here.
+__device__ __forceinline__ void cluster_gather(const SolveParams& p, double v, double (&all)[kMaxCluster]) {
 #ifdef FO_LINK_GENERATED
   const int blocks = cluster_blocks();
   double* const at = p.scratch + (int64_t)(blockIdx.x / blocks) * p.slot_doubles + p.sl.d * 32;
   if (threadIdx.x == 0 && BLOCK_W == 0) at[cluster_rank() * 32] = v;
   team_sync();
 #pragma unroll
-  for (int b = 0; b < 8; ++b) all[b] = b < blocks ? at[b * 32] : v;
+  for (int b = 0; b < kMaxCluster; ++b) all[b] = b < blocks ? at[b * 32] : v;
   team_sync();
 #endif
 }
@@ -1554,10 +1555,10 @@ __device__ double block_max(const SolveParams& p, double v, double* red) {
   double s = red[0];
   for (int i = 1; i < nw; ++i) s = npmax(s, red[i]);
   if (cluster_team()) {
-    double all[8];
+    double all[kMaxCluster];
     cluster_gather(p, s, all);
 #pragma unroll
-    for (int b = 0; b < 8; ++b) s = npmax(s, all[b]);
+    for (int b = 0; b < kMaxCluster; ++b) s = npmax(s, all[b]);
   }
   return s;
 }
@@ -1565,10 +1566,10 @@ __device__ double block_max(const SolveParams& p, double v, double* red) {
 __device__ bool block_all(const SolveParams& p, bool v) {
   bool all_true = __syncthreads_and(v ? 1 : 0) != 0;
   if (cluster_team()) {
-    double all[8];
+    double all[kMaxCluster];
     cluster_gather(p, all_true ? 1.0 : 0.0, all);
 #pragma unroll
-    for (int b = 0; b < 8; ++b) all_true = all_true && all[b] != 0.0;
+    for (int b = 0; b < kMaxCluster; ++b) all_true = all_true && all[b] != 0.0;
   }
   return all_true;
 }

@@ -110,3 +110,30 @@ def test_dropin_calls_share_no_buffers(cuda):
         for w, g in zip(want, got[t]):
             np.testing.assert_array_equal(w[0], g[0])
             assert w[1:] == g[1:]
+
+
+def test_few_reactions_and_many_species(cuda):
+    """Four reactions with hundreds of products: enough work for a cluster, but
+    fewer rates than a cluster's blocks exchange values. Two groups and 400
+    (one-block teams) of the same cells give the same bits."""
+    from fastode_gb300 import BackwardEuler, Mechanism
+    from fastode_gb300.batch import Batch
+    from fastode_gb300.plan import analyze
+    torch = cuda
+    n, rng = 600, np.random.default_rng(11)
+    names = [f"S{i}" for i in range(n)]
+    mech = Mechanism(names, [([names[2 * j], names[2 * j + 1]], [(s, 0.01 * (1 + i % 7)) for i, s in enumerate(names[8:])])
+                             for j in range(4)])
+    a = analyze(mech)
+    assert a["lu_fma"] + 3 * a["solve_fma"] + a["jac_terms"] + 2 * a["stoich_nnz"] > 10000
+    Y0, k0 = 10.0 ** rng.uniform(-9, -3, (64, n)), 10.0 ** rng.uniform(0, 3, (64, 4))
+    got = []
+    for copies in (1, 200):
+        b = Batch(mech, np.tile(Y0, (copies, 1)), group_size=32, algorithm=BackwardEuler())
+        atol = torch.full((n,), 1e-17, dtype=torch.float64, device="cuda")
+        k = torch.from_numpy(np.ascontiguousarray(np.tile(k0, (copies, 1)).T)).cuda()
+        for _ in range(2):
+            b.step(k, 30.0, atol, 1e-3)
+        got.append((b.Y.view(n, copies, 64).clone(), b.counts.view(copies, 2, 13).clone()))
+    assert torch.equal(got[1][0], got[0][0].expand_as(got[1][0]))
+    assert torch.equal(got[1][1], got[0][1].expand_as(got[1][1]))
