@@ -717,17 +717,14 @@ __device__ __forceinline__ bool solves_in_place(const SolveParams& p) {
 
 #ifdef FO_LINK_GENERATED
 // The dense square's elimination (GenLayout): nb x nb blocks of kDenseBlock
-// rows and columns in tile-major order, `a` this lane's first item. Step s
-// finishes block (s, s) and the blocks below and right of it, left-looking:
-// every block of the step first takes the updates of the pivots before the
-// step (one warp per block: the block in registers, two columns of operands
-// in flight, 36 DFMAs per 12 loads), the diagonal block is factored, and after
-// a barrier the others take the step's own pivots. A team of one does both
-// without the barriers and the round trip. Each entry receives its updates in
-// ascending pivot order, as in the row-by-row elimination. The loop is a few
-// kilobytes of code, so the warps of an SM share it in the instruction cache
-// wherever each of them is.
+// rows and columns in tile-major order, `a` this lane's first item. A warp
+// holds a block in registers while it takes the updates of earlier pivots, two
+// columns of operands in flight (36 DFMAs per 12 loads). Each entry receives
+// its updates in ascending pivot order, as in the row-by-row elimination. The
+// loops are a few kilobytes of code, so the warps of an SM share them in the
+// instruction cache wherever each of them is.
 constexpr int kDB = kDenseBlock;
+constexpr int kDensePanel = 2;   // of a block's team (dense_lu_team)
 
 __device__ __forceinline__ double* dense_block(double* a, int nb, int bi, int bj) {
   return a + (int64_t)(bi * nb + bj) * kDB * kDB * 32;
@@ -807,11 +804,7 @@ __device__ __forceinline__ void block_finish(double (&c)[kDB][kDB], const double
   }
 }
 
-// The same for a team of several blocks, right-looking: every step's pivots
-// update all remaining blocks at once, one warp each (a left-looking step has
-// only 2 (nb - s) - 1 blocks, whose updates grow with s), and the warp that
-// updates the next diagonal block factors it. Each entry receives the same
-// updates in the same order.
+// The diagonal block's own pivots.
 __device__ __forceinline__ void block_factor(double (&c)[kDB][kDB]) {
 #pragma unroll
   for (int k = 0; k < kDB; ++k) {
@@ -826,30 +819,47 @@ __device__ __forceinline__ void block_factor(double (&c)[kDB][kDB]) {
   }
 }
 
-__device__ __noinline__ void dense_lu_spread(double* a, int nb) {
+// A team, `panel` pivot blocks at a time. Step s updates its row and column of
+// blocks with the pivots of its panel before it, one warp per block, and the
+// warp of the diagonal block factors that; after a barrier the others take the
+// step's own pivots. The step that begins a panel updates all remaining blocks
+// with the last panel's. A sub-partition issues one DFMA in 64 cycles or more
+// whichever of its warps it comes from, so what counts is how evenly a step's
+// blocks fill four sub-partitions: left-looking (one panel of all) the last
+// steps have 1, 3, 5, ... blocks, with the most updates each, and the 506
+// updates of 12 x 12 blocks take the time of 644; in panels of two, of 524.
+// 4,096 cells of 210/500, recorded and reversed (one team of 16 per SM): 180.6
+// ms left-looking, 172.2 in panels of two (one: 172.4, three: 168.8 in runs
+// where two took 168.7); 8,192 cells of 120/260, three host intervals: 9.97 and
+// 9.58 ms (9.40, 9.64). A cluster's barrier is dear and its sub-partitions
+// are many, so it takes panels of one.
+__device__ __noinline__ void dense_lu_team(double* a, int nb, int panel) {
+  const int64_t ustep = (int64_t)nb * kDB * kDB * 32;
   const int w = TEAM_W, wn = TEAM_N;
 #pragma unroll 1
-  for (int s = -1; s < nb - 1; ++s) {
-    // the updates of step s (none before the first), and block (s+1, s+1)
-    const int m = nb - 1 - s, count = s < 0 ? 1 : m * m;
+  for (int s = 0; s < nb; ++s) {
+    // a step that begins a panel updates every remaining block with the last
+    // panel's pivots; the others only their own row and column of blocks
+    const int in = s % panel, from = in ? s - in : s > 0 ? s - panel : 0;
+    const int m = nb - s, count = s == 0 ? 1 : in ? 2 * m - 1 : m * m;
 #pragma unroll 1
     for (int q = w; q < count; q += wn) {
-      const int bi = s + 1 + (s < 0 ? 0 : q / m), bj = s + 1 + (s < 0 ? 0 : q % m);
+      const int bi = s + (!in ? q / m : q & 1 ? (q + 1) / 2 : 0), bj = s + (!in ? q % m : q & 1 ? 0 : q / 2);
       double* t = dense_block(a, nb, bi, bj);
       double c[kDB][kDB];
       block_load(t, c);
-      if (s >= 0) block_update(c, dense_block(a, nb, bi, s), dense_block(a, nb, s, bj), 1, 0);
+      block_update(c, dense_block(a, nb, bi, from), dense_block(a, nb, from, bj), s - from, ustep);
       if (q == 0) block_factor(c);
       block_store(t, c);
     }
     team_sync();
-    const int rest = 2 * (nb - 2 - s);
-    const double* d = dense_block(a, nb, s + 1, s + 1);
+    const int rest = 2 * (m - 1);
+    const double* d = dense_block(a, nb, s, s);
 #pragma unroll 1
     for (int q = w; q < rest; q += wn) {
-      const int k = s + 2 + q / 2;
+      const int k = s + 1 + q / 2;
       const bool left = (q & 1) != 0;
-      double* t = dense_block(a, nb, left ? k : s + 1, left ? s + 1 : k);
+      double* t = dense_block(a, nb, left ? k : s, left ? s : k);
       double c[kDB][kDB];
       block_load(t, c);
       block_finish(c, d, left);
@@ -859,17 +869,17 @@ __device__ __noinline__ void dense_lu_spread(double* a, int nb) {
   }
 }
 
-__device__ __noinline__ void dense_lu(double* a, int nb) {
+// One warp alone, left-looking: a block takes all its updates and its own
+// step's pivots in registers, in one pass over the square.
+__device__ __noinline__ void dense_lu_warp(double* a, int nb) {
   const int64_t ustep = (int64_t)nb * kDB * kDB * 32;
-  const int w = TEAM_W, wn = TEAM_N;
 #pragma unroll 1
   for (int s = 0; s < nb; ++s) {
     // block 0 of the step is the diagonal one, 2m - 1 and 2m those m below
     // and m right of it
-    const int count = 2 * (nb - s) - 1;
-    double* d = dense_block(a, nb, s, s);
+    const double* d = dense_block(a, nb, s, s);
 #pragma unroll 1
-    for (int q = w; q < count; q += wn) {
+    for (int q = 0; q < 2 * (nb - s) - 1; ++q) {
       const int m = s + (q + 1) / 2;
       const bool left = (q & 1) != 0;
       const int bi = left ? m : s, bj = left ? s : m;
@@ -877,29 +887,16 @@ __device__ __noinline__ void dense_lu(double* a, int nb) {
       double c[kDB][kDB];
       block_load(t, c);
       block_update(c, dense_block(a, nb, bi, 0), dense_block(a, nb, 0, bj), s, ustep);
-      if (q == 0) {
-        block_factor(c);
-      } else if (wn == 1) {
-        block_finish(c, d, left);
-      }
+      if (q == 0) block_factor(c);
+      else block_finish(c, d, left);
       block_store(t, c);
     }
-    team_sync();
-    if (wn > 1 && count > 1) {
-#pragma unroll 1
-      for (int q = w; q < count; q += wn) {
-        if (q == 0) continue;
-        const int m = s + (q + 1) / 2;
-        const bool left = (q & 1) != 0;
-        double* t = dense_block(a, nb, left ? m : s, left ? s : m);
-        double c[kDB][kDB];
-        block_load(t, c);
-        block_finish(c, d, left);
-        block_store(t, c);
-      }
-      team_sync();
-    }
   }
+}
+
+__device__ __forceinline__ void dense_lu(double* a, int nb) {
+  if (TEAM_N == 1) dense_lu_warp(a, nb);
+  else dense_lu_team(a, nb, cluster_team() ? 1 : kDensePanel);
 }
 #endif
 
@@ -1036,8 +1033,7 @@ __device__ void factor_any(const SolveParams& p, const Lane& ln, double alpha, c
   } else {
     fo_gen_factor(base, alpha, TEAM_W, TEAM_N, p.o.gen_index);
     if (p.sl.nb > 0) {
-      if (cluster_team()) dense_lu_spread(base + p.sl.dn * ln.L, p.sl.nb);
-      else dense_lu(base + p.sl.dn * ln.L, p.sl.nb);
+      dense_lu(base + p.sl.dn * ln.L, p.sl.nb);
     }
   }
 #else
