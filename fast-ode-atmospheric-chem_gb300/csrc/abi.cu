@@ -23,7 +23,6 @@ namespace fo {
 cudaError_t launch_solve(const SolveParams& p, int grid, size_t smem, cudaStream_t stream);
 cudaError_t launch_eval(const SolveParams& p, int C, int want_jac, double* out, cudaStream_t stream);
 cudaError_t launch_adjoint(const AdjParams& a, int grid, int lanes, size_t smem, cudaStream_t stream);
-cudaError_t launch_round_policy(const SolveParams* batches, int nb, unsigned int* words, cudaStream_t stream);
 int set_last_error(int code, const char* what);
 cudaError_t launch_solve_multi(const SolveParams* batches, int nb, const int32_t* starts, int32_t* queue,
                                double* scratch, int64_t slot_doubles, int grid, int lanes, size_t smem,
@@ -90,9 +89,9 @@ size_t smem_bytes(const fo::HostTables& t, int lanes, int variant = FO_VARIANT_P
   return sizeof(double) * (32 + (size_t)items * lanes);
 }
 
-constexpr size_t kHeader = 256;  // queue counter at the start of the workspace
-constexpr size_t kRoundsOffset = 64;  // the lockstep barrier words, inside the header
-constexpr int kRoundsWords = 8;
+constexpr size_t kRoundsOffset = 256;  // the lockstep rounds' words, after the queue counter
+constexpr size_t kRoundsBytes = sizeof(unsigned int) * fo::kRoundStates * fo::kRoundStride;
+constexpr size_t kHeader = kRoundsOffset + kRoundsBytes;  // the workspace before its slots
 constexpr int kMaxLanes = 256;
 
 template <typename T>
@@ -426,8 +425,7 @@ struct fo_multi {
   int32_t* d_queue = nullptr;
   double* d_scratch = nullptr;
   int64_t slot_doubles = 0;
-  unsigned int* d_rounds = nullptr;      // lockstep rounds' barrier words, or null
-  bool one_wave = false;                 // every group has a block of its own
+  unsigned int* d_rounds = nullptr;      // the lockstep rounds' words, or null
 };
 
 namespace {
@@ -492,14 +490,14 @@ int fo_solve(const fo_plan* plan, const fo_options* opt, int32_t ngroups, const 
   } else {
     p.queue = nullptr;
   }
-  // lockstep rounds (fo_options.lockstep): barrier words in the workspace
+  // lockstep rounds (fo_options.lockstep): their words in the workspace
   // header, zeroed for every launch
   p.rounds = nullptr;
   p.round_cost = fo::kRoundUnits;
   if (opt->lockstep && p.o.variant == FO_VARIANT_GENERATED && p.o.loop == FO_LOOP_ALGORITHM &&
       fo::gen_rounds_pay(grid)) {
     p.rounds = reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + kRoundsOffset);
-    e = cudaMemsetAsync(p.rounds, 0, kRoundsWords * sizeof(unsigned int), s);
+    e = cudaMemsetAsync(p.rounds, 0, kRoundsBytes, s);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(rounds)");
   }
   if (p.o.variant == FO_VARIANT_GENERATED) e = fo::gen_launch(plan->gen, p, grid, smem, s);
@@ -585,7 +583,6 @@ int fo_multi_prepare(int32_t nb, const fo_batch_desc* b, void* workspace, size_t
   }
   m->nb = nb;
   m->grid = L.grid;
-  m->one_wave = L.grid >= L.total;
   m->lanes = L.lanes;
   m->smem = smem;
   m->d_batches = reinterpret_cast<fo::SolveParams*>(ws + L.params_off);
@@ -594,7 +591,7 @@ int fo_multi_prepare(int32_t nb, const fo_batch_desc* b, void* workspace, size_t
   m->d_scratch = reinterpret_cast<double*>(ws + L.scratch_off);
   m->slot_doubles = L.items * L.lanes;
   // lockstep rounds when every batch asks for them and runs the generated
-  // Algorithm loop, and every slot is resident;
+  // Algorithm loop;
   // each batch makes as many attempts per round as the largest mechanism's
   // attempt costs over its own (LU and three solves), at least one
   bool lockstep = ngen == nb;
@@ -604,7 +601,7 @@ int fo_multi_prepare(int32_t nb, const fo_batch_desc* b, void* workspace, size_t
     lockstep = lockstep && d.opt.lockstep && params[j].o.loop == FO_LOOP_ALGORITHM;
     cost_max = std::max<int64_t>(cost_max, d.plan->host.lu_fma + 3 * d.plan->host.solve_fma);
   }
-  if (lockstep) lockstep = fo::gen_rounds_pay(m->grid) && fo::gen_resident(m->gen, true, m->grid, smem);
+  lockstep = lockstep && fo::gen_rounds_pay(m->grid);
   m->d_rounds = lockstep ? reinterpret_cast<unsigned int*>(ws + kRoundsOffset) : nullptr;
   for (int j = 0; j < nb; ++j) {
     fo::SolveParams& p = params[j];
@@ -631,14 +628,11 @@ int fo_multi_prepare(int32_t nb, const fo_batch_desc* b, void* workspace, size_t
 int fo_multi_launch(const fo_multi* m, void* stream) {
   if (!m) return fail(FO_E_INVALID, "null argument");
   if (m->d_rounds) {
-    cudaError_t z = cudaMemsetAsync(m->d_rounds, 0, kRoundsWords * sizeof(unsigned int),
-                                    static_cast<cudaStream_t>(stream));
-    if (z == cudaSuccess) z = fo::launch_round_policy(m->d_batches, m->nb, m->d_rounds, static_cast<cudaStream_t>(stream));
-    if (z != cudaSuccess) return cuda_fail(z, "lockstep rounds");
+    cudaError_t z = cudaMemsetAsync(m->d_rounds, 0, kRoundsBytes, static_cast<cudaStream_t>(stream));
+    if (z != cudaSuccess) return cuda_fail(z, "cudaMemsetAsync(rounds)");
   }
   cudaError_t e = m->gen ? fo::gen_launch_multi(m->gen, m->d_batches, m->nb, m->d_starts, m->d_queue,
                                                 m->d_scratch, m->slot_doubles, m->grid, m->smem,
-                                                m->d_rounds != nullptr, m->one_wave,
                                                 static_cast<cudaStream_t>(stream))
                          : fo::launch_solve_multi(m->d_batches, m->nb, m->d_starts, m->d_queue, m->d_scratch,
                                                   m->slot_doubles, m->grid, m->lanes, m->smem,

@@ -97,6 +97,8 @@ struct ScratchLayout {
 
 // A round of lockstep, and the part of it before the solves.
 constexpr int kRoundUnits = 1024, kRoundSolves = 820;
+// The words of lockstep rounds: a state per SM, by its number, 32 bytes apart.
+constexpr int kRoundStates = 256, kRoundStride = 8;
 
 struct SolveParams {
   DevTables t;
@@ -120,7 +122,7 @@ struct SolveParams {
   double* trace;
   int trace_cap;
   int32_t* trace_len;
-  unsigned int* rounds;          // lockstep rounds (barrier words), or null
+  unsigned int* rounds;          // lockstep rounds (kRoundStates states), or null
   int round_cost;                // an attempt's share of a round, in kRoundUnits
 };
 

@@ -29,6 +29,7 @@ extern "C" __global__ void __launch_bounds__(32 * 16, 1) fo_generated_solve_kern
   double* w = smem + 32;    // a cluster's partial sums
   const int slot = blockIdx.x / cluster_blocks();
   double* scr = p.scratch + (int64_t)slot * p.slot_doubles;
+  fo::rounds_join(p.rounds, pace);
   if (p.queue == nullptr) {
     fo::solve_group(p, slot, scr, w, red, pace);
   } else {
@@ -42,7 +43,7 @@ extern "C" __global__ void __launch_bounds__(32 * 16, 1) fo_generated_solve_kern
       fo::solve_group(p, g, scr, w, red, pace);
     }
   }
-  fo::rounds_drain(p.rounds);
+  fo::rounds_leave(pace);
 }
 
 // Several mechanisms in one persistent launch (the generated form of
@@ -51,7 +52,7 @@ extern "C" __global__ void __launch_bounds__(32 * 16, 1) fo_generated_solve_kern
 // module; each block integrates whatever group it pulls next.
 extern "C" __global__ void __launch_bounds__(32 * 16, 1)
     fo_generated_multi_kernel(const fo::SolveParams* __restrict__ batches, int nb, const int32_t* __restrict__ starts,
-                              int32_t* queue, double* scratch, int64_t slot_doubles, int spread) {
+                              int32_t* queue, double* scratch, int64_t slot_doubles) {
   extern __shared__ double smem[];
   double* red = smem;
   fo::RoundPace pace;
@@ -60,29 +61,20 @@ extern "C" __global__ void __launch_bounds__(32 * 16, 1)
   __shared__ int next;
   __shared__ fo::SolveParams params;
   int current = -1;
-  // the same words in every batch; word 5: whether this launch uses them
-  unsigned int* rounds = batches[0].rounds;
-  if (rounds != nullptr && rounds[5] == 0u) rounds = nullptr;
+  fo::rounds_join(batches[0].rounds, pace);   // the same words in every batch
   const int total = starts[nb];
   for (;;) {
     __syncthreads();
     if (fo::team_leader()) next = atomicAdd(queue, 1);
     __syncthreads();
-    int item = next;
+    const int item = next;
     if (item >= total) break;
-    // a cooperative launch fills one cluster of SMs after another, so the
-    // first items, the largest mechanism's, are dealt out across the blocks
-    if (item < (int)gridDim.x) item = (int)((int64_t)item * spread % (int)gridDim.x);
     int b = 0;
     while (b + 1 < nb && item >= starts[b + 1]) ++b;
     fo::load_batch_params(batches, b, current, params);
-    if (rounds == nullptr) {
-      if (fo::team_leader()) params.rounds = nullptr;
-      __syncthreads();
-    }
     fo::solve_group(params, item - starts[b], scr, w, red, pace);
   }
-  fo::rounds_drain(rounds);
+  fo::rounds_leave(pace);
 }
 
 // The discrete adjoint of one interval (adjoint.cuh) on the mechanism's

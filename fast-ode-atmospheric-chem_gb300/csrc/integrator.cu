@@ -122,32 +122,6 @@ __global__ void __maxnreg__(255) solve_multi_kernel(const SolveParams* __restric
   }
 }
 
-// Whether a several-mechanism launch makes its attempts in rounds (word 5 of
-// the barrier words): when at least half of its groups start with steps below
-// a sixteenth of the interval. Such groups make many attempts, and rounds keep
-// the warps of an SM together; groups on settled steps make one to three, and
-// rounds only make the slots wait for one another between groups. Measured
-// with and without rounds on three mechanisms: 65,536 cells, settled, 66 and
-// 61 ms; 196,608 cells, cold, 976 and 1235 ms.
-__global__ void __launch_bounds__(1024) round_policy_kernel(const SolveParams* __restrict__ batches, int nb,
-                                                            unsigned int* words) {
-  int cold = 0, total = 0;
-  for (int b = 0; b < nb; ++b) {
-    const SolveParams& p = batches[b];
-    for (int g0 = 0; g0 < p.ngroups; g0 += blockDim.x) {
-      const int g = g0 + threadIdx.x;
-      cold += __syncthreads_count(g < p.ngroups && !(p.o.carry && p.memory[3 * (int64_t)g] > p.dt * 0.0625));
-    }
-    total += p.ngroups;
-  }
-  if (threadIdx.x == 0) words[5] = 2 * cold >= total ? 1u : 0u;
-}
-
-cudaError_t launch_round_policy(const SolveParams* batches, int nb, unsigned int* words, cudaStream_t stream) {
-  round_policy_kernel<<<1, 1024, 0, stream>>>(batches, nb, words);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_solve_multi(const SolveParams* batches, int nb, const int32_t* starts, int32_t* queue,
                                double* scratch, int64_t slot_doubles, int grid, int lanes, size_t smem,
                                cudaStream_t stream) {

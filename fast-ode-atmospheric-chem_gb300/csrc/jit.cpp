@@ -333,34 +333,17 @@ int team_of(int grid) {
   return team;
 }
 
-// Whether lockstep rounds pay for a launch of `grid` groups: they keep the
+// Whether lockstep rounds pay for a launch of `grid` blocks: they keep the
 // groups of an SM in the same part of the generated code and let them solve
-// together, and make every group wait for the slowest each attempt. That pays
-// with two or more groups per SM where the SMs are evenly loaded (85% of the
-// fullest; with four or more per SM, always). With and without rounds, ms:
-// 210/500 cold, 16,384 cells (3.4 groups per SM) 229 and 302; 13,000 (2.7) 188
-// and 216; 10,000 (2.06) 178 and 160; 9,600 (1.97) 143 and 158; 8,192 (1.7) 125
-// and 125; 4,800 (0.99) 95 and 76; TS1, 65,536 cells (13.5) 41 and 56, 2,048
-// cells (0.4) 5.0 and 4.5.
+// together, which takes two groups on the fullest SMs and on half of them. With
+// and without rounds, ms: one cold interval of 210/500, 6,400 cells (1.3 groups
+// per SM) 110.4 and 108.4; 8,192 (1.7) 114 and 122; 9,600 119 and 160; 13,000
+// 163 and 218; 16,384 206 and 305; 65,536 716 and 1135; settled, 65,536 cells
+// 107 and 137, 100,000 (more groups than slots) 208 and 218; TS1 settled, 8,200
+// cells 4.37 and 4.69, 65,536 23.1 and 33.3.
 bool rounds_pay(int grid) {
   const int sms = device_sms();
-  if (sms <= 0) return false;
-  const int64_t per_sm = ((int64_t)grid + sms - 1) / sms;
-  return per_sm >= 4 || (per_sm >= 2 && 100 * (int64_t)grid >= 85 * per_sm * sms);
-}
-
-// Whether `grid` blocks of `team` warps of kernel `fn` with `smem` bytes of
-// dynamic shared memory are all resident at once on the current device (what
-// a cooperative launch needs).
-bool all_resident(const void* fn, int grid, int team, size_t smem) {
-  int dev = 0, sms = 0, per_sm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return false;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * team, smem) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return false;
-  }
-  return (int64_t)per_sm * sms >= grid;
+  return sms > 0 && 2 * (int64_t)grid > 3 * (int64_t)sms;
 }
 
 // Blocks per cluster for a launch of `grid` groups on teams of kBlockWarps
@@ -415,28 +398,14 @@ int cluster_of(GenModule* m, const void* fn, int grid) {
 
 bool gen_rounds_pay(int grid) { return rounds_pay(grid); }
 
-bool gen_resident(GenModule* m, bool multi, int grid, size_t smem) {
-  const void* fn = reinterpret_cast<const void*>(multi ? m->multi_kernel : m->kernel);
-  if (ensure_smem(m, multi ? 1 : 0, fn, smem) != cudaSuccess) {
-    (void)cudaGetLastError();
-    return false;
-  }
-  return all_resident(fn, grid, team_of(grid), smem);
-}
-
 cudaError_t gen_launch(GenModule* m, const SolveParams& p, int grid, size_t smem, cudaStream_t stream) {
   const void* fn = reinterpret_cast<const void*>(m->kernel);
   cudaError_t e = ensure_smem(m, 0, fn, smem);
   if (e != cudaSuccess) return e;
   SolveParams q = p;
   void* args[] = {&q};
-  // lockstep rounds need every block resident: a cooperative launch; a grid
-  // that does not fit runs without rounds
   const int team = team_of(grid);
-  if (q.rounds != nullptr && all_resident(fn, grid, team, smem))
-    return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
-  q.rounds = nullptr;
-  if (team == kBlockWarps && q.queue == nullptr) {
+  if (team == kBlockWarps && q.queue == nullptr && q.rounds == nullptr) {
     const int blocks = cluster_of(m, fn, grid);
     if (blocks > 1) {
       cudaLaunchAttribute attr;
@@ -456,33 +425,16 @@ cudaError_t gen_launch_adjoint(GenModule* m, const AdjParams& a, int grid, size_
   return cudaLaunchKernel(fn, dim3(grid), dim3(32, team_of(grid)), args, smem, stream);
 }
 
-// A multiplier that deals the items 0 .. grid - 1 out evenly over any run and
-// any arithmetic progression of blocks: the one nearest the golden section of
-// the grid with no common factor. A cooperative launch places its blocks SM
-// by SM where a plain one goes round all SMs; with the items in order, one
-// cold interval of 65,536 cells of three mechanisms (one wave) took 559 ms,
-// dealt out 517. With more groups than blocks the order stays: SMs full of the
-// largest mechanism balance their four sub-partitions and the others work off
-// the queue (196,608 cells, settled: 134 ms in order, 146 dealt out).
-int spread_of(int grid) {
-  for (int m = std::max(1, (int)(0.6180339887 * grid)); m > 1; --m)
-    if (std::gcd(m, grid) == 1) return m;
-  return 1;
-}
-
 cudaError_t gen_launch_multi(GenModule* m, const SolveParams* batches, int nb, const int32_t* starts,
                              int32_t* queue, double* scratch, int64_t slot_doubles, int grid, size_t smem,
-                             bool cooperative, bool one_wave, cudaStream_t stream) {
+                             cudaStream_t stream) {
   const void* fn = reinterpret_cast<const void*>(m->multi_kernel);
   cudaError_t e = ensure_smem(m, 1, fn, smem);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(queue, 0, sizeof(int32_t), stream);
   if (e != cudaSuccess) return e;
-  const int team = team_of(grid);
-  int spread = cooperative && one_wave ? spread_of(grid) : 1;
-  void* args[] = {&batches, &nb, &starts, &queue, &scratch, &slot_doubles, &spread};
-  if (cooperative) return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
-  return cudaLaunchKernel(fn, dim3(grid), dim3(32, team), args, smem, stream);
+  void* args[] = {&batches, &nb, &starts, &queue, &scratch, &slot_doubles};
+  return cudaLaunchKernel(fn, dim3(grid), dim3(32, team_of(grid)), args, smem, stream);
 }
 
 }  // namespace fo

@@ -1955,71 +1955,111 @@ __device__ __noinline__ void solve_group_backward_euler(const SolveParams& p, in
   }
 }
 
-// Lockstep rounds. With every block of the launch resident at once (a
-// cooperative launch), the groups make their attempts in rounds: each block
-// makes one attempt (of a small mechanism in a several-mechanism launch as many
-// as cost about one of the largest, of one group after another), then waits
-// at a grid-wide barrier for the others; a block with no group left keeps
-// arriving with nothing to do until a round in which no block attempted. The straight-line factorization is megabytes of code, so
-// warps that drift apart each stream their own instructions and thrash the
-// SM's instruction cache; rounds keep the warps of an SM at the same place
-// (the cold first interval of the 210/500, 65,536-cell job: 1.47 s without
-// rounds, 0.96 s with). The barrier only orders time: no group reads
-// another's data, so results are those of the unsynchronized launch bit for
-// bit. Each wait is bounded (kRoundSpinLimit polls about 4 us apart, some
-// 30 s); a wait that gives up raises the give-up word, after which every
-// block runs on without rounds.
+// Lockstep rounds. The blocks of an SM make their attempts in rounds: each
+// block makes one attempt (of a small mechanism in a several-mechanism launch as
+// many as cost about one of the largest, of one group after another), then
+// waits for the SM's others. The straight-line code is megabytes, so warps that
+// drift apart each stream their own instructions and thrash the SM's
+// instruction cache; rounds keep them at the same place. The blocks of a round
+// also meet before the solves: the scheduler favours an SM's oldest warps, so
+// groups leave the factorization, which fills the FP64 units, one after
+// another, and the youngest would make its solves, which wait on memory and on
+// one another, with the SM to itself (one settled interval of 65,536 cells of
+// the 210/500 mechanism 120 ms without the second meeting and 110 with it).
 //
-// The blocks of a round also meet before the solves. The scheduler favours an
-// SM's oldest warps, so groups leave the factorization, which fills the FP64
-// units, one after another; without that the youngest made its solves, which
-// wait on memory and on one another, with the SM to itself. One settled
-// interval of 65,536 cells of the 210/500 mechanism 120 and 110 ms,
-// constrained 160/340 with 16,384 cells 31.4 and 28.1 ms.
-constexpr long long kRoundSpinLimit = 7500000;
+// An SM's state is one word: the blocks that take part (bits 0-7), those that
+// have arrived at the meeting (8-15) and the meetings so far (16-31), even
+// before a round's solves. A block joins when it starts and leaves when it has
+// no group left, so nothing has to be resident but the blocks that wait, and a
+// launch of any size can run in rounds on the plain launch's even placement.
+// With one barrier over the whole grid every SM waited for the fullest, and the
+// cooperative launch that it needs filled one SM after another (65,536 cells
+// of 210/500 on 128 of 152 SMs). Grid-wide rounds and an SM's, ms: one cold
+// interval of 210/500, 9,600 cells 139 and 119, 13,000 185 and 163, 16,384 226
+// and 206, 65,536 756 and 716; three mechanisms, 196,608 cells, settled (where
+// grid-wide rounds lost to none) 136 and 112, cold 1019 and 856.
+//
+// The rounds only order time: no group reads another's data, so results are
+// those of the unsynchronized launch bit for bit. A wait is bounded
+// (kRoundSpinLimit polls about 1 us apart, some 30 s); a block that gives up
+// leaves the rounds and runs on without them.
+constexpr int kRoundSpinLimit = 30000000;
+constexpr unsigned int kRoundMember = 1u, kRoundArrival = 1u << 8, kRoundMeeting = 1u << 16;
 
-// Arrive with this block's activity in the round (1: it attempted); returns
-// the number of blocks that attempted in the round, or -1 once rounds are
-// given up. Barrier words: [0] arrivals, [1] activity sum, [2] generation,
-// [3] the last round's sum, [4] give-up, [5] a several-mechanism launch's
-// choice (round_policy_kernel). Every thread of the block calls it.
-__device__ int round_barrier(unsigned int* w, int active) {
-  __shared__ int result;
+// Adds `change` to an SM's state and holds the meeting if that completes it;
+// returns the state before.
+__device__ __forceinline__ unsigned int round_update(unsigned int* w, unsigned int change) {
+  unsigned int old = *reinterpret_cast<volatile unsigned int*>(w);
+  for (;;) {
+    unsigned int s = old + change;
+    if ((s & 0xffu) != 0u && (s >> 8 & 0xffu) == (s & 0xffu)) s = (s & 0xffff00ffu) + kRoundMeeting;
+    const unsigned int seen = atomicCAS(w, old, s);
+    if (seen == old) return old;
+    old = seen;
+  }
+}
+
+// Where a block is in its round: its SM's state (null: no rounds), the units
+// done, and whether it has met the others before the solves. It carries over
+// from group to group.
+struct RoundPace {
+  unsigned int* state = nullptr;
+  int done = 0;
+  bool met = false;
+};
+
+// Waits for the SM's other blocks. Every thread of the block calls it.
+__device__ void round_meet(RoundPace& pace) {
+  __shared__ int held;
   __syncthreads();
   if (team_leader()) {
-    volatile unsigned int* vw = w;
-    if (vw[4] != 0u) {
-      result = -1;
-    } else {
-      const unsigned int gen = vw[2];
-      __threadfence();
-      atomicAdd(w + 1, (unsigned int)active);
-      __threadfence();
-      if (atomicAdd(w, 1u) + 1u == gridDim.x) {
-        const unsigned int total = atomicExch(w + 1, 0u);
-        atomicExch(w + 3, total);
-        atomicExch(w, 0u);
-        __threadfence();
-        atomicAdd(w + 2, 1u);
-        result = (int)total;
-      } else {
-        long long spins = 0;
-        while (vw[2] == gen && vw[4] == 0u && spins < kRoundSpinLimit) {
-          __nanosleep(4000);
-          ++spins;
-        }
-        __threadfence();
-        if (vw[2] != gen) {
-          result = (int)vw[3];
-        } else {
-          atomicExch(w + 4, 1u);
-          result = -1;
-        }
-      }
+    const volatile unsigned int* state = pace.state;
+    const unsigned int meeting = round_update(pace.state, kRoundArrival) >> 16;
+    for (int spins = 0; *state >> 16 == meeting && spins < kRoundSpinLimit; ++spins) __nanosleep(1000);
+    held = 1;
+    unsigned int s = *state;
+    while (s >> 16 == meeting) {   // given up: neither a member nor arrived any more
+      unsigned int left = s - kRoundMember - kRoundArrival;
+      if ((left & 0xffu) != 0u && (left >> 8 & 0xffu) == (left & 0xffu)) left = (left & 0xffff00ffu) + kRoundMeeting;
+      const unsigned int seen = atomicCAS(pace.state, s, left);
+      held = seen == s ? 0 : 1;
+      if (seen == s) break;
+      s = seen;
     }
   }
   __syncthreads();
-  return result;
+  if (!held) pace.state = nullptr;
+}
+
+// The block joins its SM's rounds (`words` null: none), between two rounds:
+// where the others are at their solves it waits for them to finish.
+__device__ void rounds_join(unsigned int* words, RoundPace& pace) {
+  __shared__ int at, wait;
+  if (words == nullptr) return;
+  if (team_leader()) {
+    unsigned int sm;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+    at = (int)(sm % kRoundStates) * kRoundStride;
+    unsigned int* w = words + at;
+    unsigned int old = *reinterpret_cast<volatile unsigned int*>(w);
+    for (;;) {
+      const bool first = (old & 0xffu) == 0u, solves = (old >> 16 & 1u) != 0u;
+      const unsigned int s = old + kRoundMember + (first && solves ? kRoundMeeting : 0u);
+      const unsigned int seen = atomicCAS(w, old, s);
+      if (seen == old) {
+        wait = !first && solves;
+        break;
+      }
+      old = seen;
+    }
+  }
+  __syncthreads();
+  pace.state = words + at;
+  if (wait) round_meet(pace);
+}
+
+__device__ __forceinline__ void rounds_leave(RoundPace& pace) {
+  if (pace.state != nullptr && team_leader()) round_update(pace.state, 0u - kRoundMember);
 }
 
 // The parameters of batch b of a several-mechanism launch, copied from the
@@ -2039,32 +2079,19 @@ __device__ __forceinline__ void load_batch_params(const SolveParams* __restrict_
   current = b;
 }
 
-// Where a block is in its round: the units done, and whether it has met the
-// others before the solves. It carries over from group to group.
-struct RoundPace {
-  int done = 0;
-  bool met = false;
-};
-
 // The block has done `units` more of its round.
-__device__ __forceinline__ void round_advance(const SolveParams& p, RoundPace& pace, int units) {
+__device__ __forceinline__ void round_advance(RoundPace& pace, int units) {
   pace.done += units;
   if (!pace.met && pace.done >= kRoundSolves) {
-    round_barrier(p.rounds, 1);
     pace.met = true;
+    round_meet(pace);
+    if (pace.state == nullptr) return;
   }
   if (pace.met && pace.done >= kRoundUnits) {
-    round_barrier(p.rounds, 1);
     pace.met = false;
     pace.done -= kRoundUnits;
+    round_meet(pace);
   }
-}
-
-// A block with no group left: arrive idle until a round without attempts.
-__device__ __forceinline__ void rounds_drain(unsigned int* w) {
-  if (w != nullptr)
-    while (round_barrier(w, 0) > 0) {
-    }
 }
 
 __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, double* w, double* red,
@@ -2160,7 +2187,7 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
       factor_any(p, ln, alpha, negj, lu, w, false);
       ++c_lu;
       const int to_solves = p.round_cost * kRoundSolves / kRoundUnits;
-      if (p.rounds != nullptr) round_advance(p, pace, to_solves);
+      if (pace.state != nullptr) round_advance(pace, to_solves);
       const double part = attempt(p, ln, H, Y, Ynew, scr, w, red, c_rhs, c_solves, fresh);
       fresh = false;
       const double err = team_once(red + kSlotError, [&] {
@@ -2220,7 +2247,7 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
         if (last) H = __dsub_rn(dt, t);
         ++c_rej;
       }
-      if (p.rounds != nullptr) round_advance(p, pace, p.round_cost - to_solves);
+      if (pace.state != nullptr) round_advance(pace, p.round_cost - to_solves);
     }
   }
   if (status < 0) status = FO_STATUS_CONVERGED;

@@ -29,7 +29,9 @@
 #include "fastode_gb300.h"
 
 // The scratch: the queue counter at offset 0, then as many group slots as fit.
-static __device__ __align__(256) unsigned char g_static_scratch[FO_STATIC_SCRATCH_BYTES];
+// FO_STATIC_SCRATCH_BYTES, and the words of the lockstep rounds beside it
+constexpr size_t kCapacity = FO_STATIC_SCRATCH_BYTES + 8192;
+static __device__ __align__(256) unsigned char g_static_scratch[kCapacity];
 
 namespace fo {
 int set_last_error(int code, const char* what);  // abi.cu
@@ -76,16 +78,16 @@ extern "C" int fo_solve_static(const fo_plan* plan, const fo_options* opt, int32
   rc = fo_workspace_bytes(plan, 2, max_group_cells, &two);
   if (rc != FO_OK) return rc;
   const size_t slot = two - one, header = one - slot;
-  if (one > (size_t)FO_STATIC_SCRATCH_BYTES)
+  if (one > kCapacity)
     return fo::set_last_error(FO_E_UNSUPPORTED,
                               "one group of this mechanism needs more scratch than the static "
                               "FO_STATIC_SCRATCH_BYTES array holds: use fo_solve with a workspace");
-  size_t fit = ((size_t)FO_STATIC_SCRATCH_BYTES - header) / slot;
+  size_t fit = (kCapacity - header) / slot;
   const int32_t slots = (int32_t)(fit < (size_t)ngroups ? fit : (size_t)ngroups);
   void* scratch = nullptr;
   rc = static_scratch_address(&scratch);
   if (rc != FO_OK) return rc;
   return fo_solve(plan, opt, ngroups, group_offsets, max_group_cells, Y, y_cell_stride, y_species_stride, k,
                   k_cell_stride, k_reaction_stride, atol, rtol, dt, memory, counts, status, scratch,
-                  (size_t)FO_STATIC_SCRATCH_BYTES, slots, nullptr, 0, nullptr, stream);
+                  kCapacity, slots, nullptr, 0, nullptr, stream);
 }

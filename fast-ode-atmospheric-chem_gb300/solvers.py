@@ -190,7 +190,7 @@ class Algorithm:
         solves' summation order. ``tile``: the generated factorization's
         register tiles (rows and columns), a speed choice only. ``lockstep``:
         with the generated kernel and one block per group, the groups make
-        their attempts in rounds in a cooperative launch (fo_options.lockstep),
+        their attempts in rounds where SMs hold several (fo_options.lockstep),
         also a speed choice only."""
         self.tableau = tableau
         self.controller = controller

@@ -132,12 +132,12 @@ typedef struct fo_options {
   int32_t nreductions;        /* entries of reductions used, 0..8 (5) */
   double reductions[8];       /* step factor after the i-th failed step (0.5, 0.5, 0.5, 0.5, 0.1); each > 0 */
   double small;               /* floor of the convergence bound (1e-40) */
-  /* Nonzero: with FO_VARIANT_GENERATED and FO_LOOP_ALGORITHM, when every
-   * block of the launch is resident at once, fo_solve and fo_multi_launch
-   * make the groups' attempts in rounds (one attempt per block, then a
-   * grid-wide barrier) in a cooperative launch, which keeps the warps of an
-   * SM in the same part of the generated code. Results are the same bit for
-   * bit; otherwise the groups run unsynchronized. */
+  /* Nonzero: with FO_VARIANT_GENERATED and FO_LOOP_ALGORITHM, where SMs hold
+   * several groups, fo_solve and fo_multi_launch make an SM's attempts in
+   * rounds (its blocks wait for one another after the factorization and after
+   * the attempt), which keeps the warps of an SM in the same part of the
+   * generated code. Results are the same bit for bit; otherwise the groups run
+   * unsynchronized. */
   int32_t lockstep;
 } fo_options;
 
@@ -180,11 +180,13 @@ typedef struct fo_options {
  * (its transposed solves need the whole vector on chip) and the generated
  * adjoint for GENERATED. */
 #define FO_VARIANT_COMPACT 2
-/* GENERATED runs the mechanism's own factorization and solves, generated as
- * straight-line code from its fill pattern and compiled when the plan is
- * prepared with fo_plan_generate (register tiles of the factorization, every
- * operand at an immediate offset, no schedule tables). Groups of at most 32
- * cells. Factors and solutions are those of PLAIN bit for bit. */
+/* GENERATED runs the mechanism's own evaluations, factorization and solves,
+ * generated as straight-line code from its patterns and compiled when the plan
+ * is prepared with fo_plan_generate (every operand at an immediate offset, no
+ * schedule tables). Groups of at most 32 cells, each worked on by a team of 1
+ * to 16 warps, or by a cluster of such blocks, chosen by the number of groups
+ * in the launch. Factors and solutions are those of PLAIN bit for bit,
+ * whatever the team. */
 #define FO_VARIANT_GENERATED 3
 
 /* What fo_plan_generate did. */
@@ -216,15 +218,15 @@ int fo_plan_destroy(fo_plan* plan);
 int fo_plan_permutation(const fo_plan* plan, int32_t* perm);
 
 /* Prepare a plan for FO_VARIANT_GENERATED: generate the mechanism's
- * factorization of alpha*M - J and its triangular solves as straight-line PTX
- * from the plan's fill pattern (the per-mechanism form of
+ * evaluations, factorization of alpha*M - J and triangular solves as
+ * straight-line PTX from the plan's patterns (the per-mechanism form of
  * fastode/linalg.py:70-81 and of the Jacobian assembly of
  * fastode/linalg.py:60-67), link it with the library's integrator kernel
  * (nvJitLink, opened at run time) and load the module on the current device.
  * The linked module is cached in cache_dir under a hash of its inputs (NULL:
  * $FASTODE_GB300_CACHE, else $XDG_CACHE_HOME/fastode_gb300, else
  * ~/.cache/fastode_gb300; "": no cache). Linking compiles the generated code:
- * about a minute for 200,000 multiply-adds; a cached module loads in
+ * some seconds for 200,000 multiply-adds; a cached module loads in
  * milliseconds. info may be NULL. Idempotent. Returns FO_E_UNSUPPORTED when
  * nvJitLink is missing or linking fails (fo_last_error has the log). */
 int fo_plan_generate(fo_plan* plan, const char* cache_dir, fo_gen_info* info);
