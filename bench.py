@@ -44,10 +44,10 @@ METRIC = "cell-intervals/s at rtol=1e-3 on 1 GB300 vs plain GPU + CPU ref; adjoi
 # --plain-steps 0` (3.590 TB over 0.799 PFLOP; the traffic is dominated by the
 # elimination's U operands, 8 bytes per 2-FLOP update, so it scales with the
 # FLOPs). generated: the two timed launches of `bench.py --cells 8192 --steps 2
-# --warmup 3 --no-cpu --e2e-steps 0 --plain-steps 0 --no-extras` (167.3 GB over
+# --warmup 3 --no-cpu --e2e-steps 0 --plain-steps 0 --no-extras` (197.0 GB over
 # 99.9 GFLOP), a case small enough for the capture, scaled by the FLOPs. A
 # variant without a calibration reports no traffic.
-DRAM_BYTES_PER_FLOP = {"compact": 4.491, "generated": 1.675}
+DRAM_BYTES_PER_FLOP = {"compact": 4.491, "generated": 1.972}
 # the integrator kernel of each variant, as ncu names it
 KERNEL_NAME = {"generated": "fo_generated_solve_kernel"}
 

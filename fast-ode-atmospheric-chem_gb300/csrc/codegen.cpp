@@ -12,12 +12,13 @@
 // every 64 cycles on its SM sub-partition whatever the rest of the chip does,
 // so a launch of few groups leaves most of the FP64 units idle. A group is
 // therefore worked on by a team of 1 to 16 warps (a block), or a cluster of
-// such blocks on several SMs, every warp holding the same 32 cells: the generated work is cut into tasks (a row, a block of
-// rows by columns, a range of reactions), the tasks are scheduled into steps
-// of kSegments segments that depend on earlier steps only, and warp w of W
-// runs segments w, w + W, ... of a step before the team's barrier. One module
-// serves every team size, and since a task is run by one warp with one order
-// of operations, results do not depend on the team size.
+// such blocks on several SMs, every warp holding the same 32 cells: the
+// generated work is cut into tasks (a row, a block of rows by columns, a range
+// of reactions), the tasks are scheduled into steps of kSegments segments that
+// depend on earlier steps only, and warp w of W runs segments w, w + W, ... of
+// a step before the team's barrier. One module serves every team size, and
+// since a task is run by one warp with one order of operations, results do not
+// depend on the team size.
 //
 // The factorization: the leading rows are single-row tasks (their elimination
 // DAG gives the parallelism); the rows of the trailing dense square are
@@ -35,7 +36,7 @@
 //
 // The solves: leading rows are single-row tasks, the square's rows lose their
 // terms in the leading columns `solve_block` rows at a time, and the square's
-// own triangle is a loop (square_solve in rosenbrock.cuh). Every row sums its
+// own triangle is a loop (square_triangle in rosenbrock.cuh). Every row sums its
 // terms in the order in which their values finish (ascending columns forward,
 // descending columns backward), as the plain variant's loops do, so results
 // match that variant bit for bit.

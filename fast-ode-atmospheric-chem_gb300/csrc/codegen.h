@@ -43,7 +43,7 @@ struct GenOptions {
 //                    (dense_lu finishes it)
 //   fo_gen_solve_up, fo_gen_solve_down
 //                    the leading rows' part of (LU)^-1 on the solve vector (item
-//                    xs): before and after the square's (square_solve)
+//                    xs): before and after the square's (square_triangle)
 //   fo_gen_solve_t_up, fo_gen_solve_t_down
 //                    the same of (LU)^-T, for the adjoint
 //   fo_gen_vjp       the adjoint's J(yr)^T v, weights and rates

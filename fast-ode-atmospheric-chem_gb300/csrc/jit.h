@@ -27,7 +27,7 @@ int gen_check(const HostTables& t, const GenOptions& opt, bool do_link, fo_gen_i
 // team of warps of 32 lanes each.
 cudaError_t gen_launch(GenModule* m, const SolveParams& p, int grid, size_t smem, cudaStream_t stream);
 // One launch of the generated adjoint kernel (fo_adjoint_interval): grid
-// blocks of 32 lanes.
+// blocks of a team of warps of 32 lanes.
 cudaError_t gen_launch_adjoint(GenModule* m, const AdjParams& a, int grid, size_t smem, cudaStream_t stream);
 // One persistent launch of the generated several-mechanism kernel (the
 // module made from every batch's tables, each batch's gen_index set).
