@@ -137,3 +137,30 @@ def test_few_reactions_and_many_species(cuda):
         got.append((b.Y.view(n, copies, 64).clone(), b.counts.view(copies, 2, 13).clone()))
     assert torch.equal(got[1][0], got[0][0].expand_as(got[1][0]))
     assert torch.equal(got[1][1], got[0][1].expand_as(got[1][1]))
+
+
+@pytest.mark.parametrize("slots", [0, 700])
+def test_rounds_with_groups_that_end_early(cuda, slots):
+    """Groups that fail in the middle of a round (a NaN rate constant), cold
+    and settled ones, one block per group and a queue that blocks join with
+    one group after another: the bits of a run without rounds."""
+    from fastode_gb300 import Algorithm, synthetic as syn
+    from fastode_gb300.batch import Batch
+    torch = cuda
+    groups = 1500
+    wl = syn.plain_small(n_cells=32 * groups, intervals=2)
+    at = torch.from_numpy(wl.atol).cuda()
+    k = [torch.from_numpy(np.ascontiguousarray(wl.k_at(i).T)).cuda() for i in range(2)]
+    k[1] = k[1].clone()
+    k[1][:, ::32 * 7] = float("nan")      # every seventh group fails at its first attempt
+    out = []
+    for lockstep in (True, False):
+        b = Batch(wl.sm.mech, wl.cells.Y0, group_size=32, slots=slots, algorithm=Algorithm(lockstep=lockstep))
+        b.step(k[0], wl.dt, at, wl.rtol)
+        b.memory[::3] = 0.0               # every third group starts cold again
+        b.step(k[1], wl.dt, at, wl.rtol)
+        torch.cuda.synchronize()
+        out.append((b.state(), b.counts.cpu().numpy(), b.memory.cpu().numpy(), b.status.cpu().numpy()))
+    assert len(set(out[0][3])) == 2
+    for x, y in zip(*out):
+        np.testing.assert_array_equal(x, y)
