@@ -495,7 +495,7 @@ int fo_solve(const fo_plan* plan, const fo_options* opt, int32_t ngroups, const 
   p.rounds = nullptr;
   p.round_cost = fo::kRoundUnits;
   if (opt->lockstep && p.o.variant == FO_VARIANT_GENERATED && p.o.loop == FO_LOOP_ALGORITHM &&
-      fo::gen_rounds_pay(grid)) {
+      plan->gen != nullptr && fo::gen_rounds_pay(plan->gen, grid)) {
     p.rounds = reinterpret_cast<unsigned int*>(static_cast<char*>(workspace) + kRoundsOffset);
     e = cudaMemsetAsync(p.rounds, 0, kRoundsBytes, s);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(rounds)");
@@ -601,7 +601,7 @@ int fo_multi_prepare(int32_t nb, const fo_batch_desc* b, void* workspace, size_t
     lockstep = lockstep && d.opt.lockstep && params[j].o.loop == FO_LOOP_ALGORITHM;
     cost_max = std::max<int64_t>(cost_max, d.plan->host.lu_fma + 3 * d.plan->host.solve_fma);
   }
-  lockstep = lockstep && fo::gen_rounds_pay(m->grid);
+  lockstep = lockstep && fo::gen_rounds_pay(m->gen, m->grid);
   m->d_rounds = lockstep ? reinterpret_cast<unsigned int*>(ws + kRoundsOffset) : nullptr;
   for (int j = 0; j < nb; ++j) {
     fo::SolveParams& p = params[j];

@@ -193,7 +193,8 @@ struct GenModule {
   cudaKernel_t adjoint_kernel = nullptr;  // fo_generated_adjoint_kernel
   std::mutex mutex;
   int configured_smem[3][64] = {};
-  int64_t attempt_work = 0;               // FP64 operations of an attempt (one mechanism; 0: no clusters)
+  int64_t attempt_work = 0;               // FP64 operations of an attempt (the largest mechanism's)
+  bool may_cluster = false;
   int clusters[64][4] = {};               // resident clusters of 2^i blocks, plus one (0: not asked yet)
 };
 
@@ -252,11 +253,12 @@ int gen_create(const std::vector<const HostTables*>& ts, const std::vector<GenOp
     info->cubin_bytes = (int64_t)cubin.size();
     info->seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
   }
+  for (const HostTables* t : ts)
+    m->attempt_work = std::max(m->attempt_work, t->lu_fma + 3 * t->solve_fma + (int64_t)t->jt_idx.size() +
+                                                    2 * (int64_t)t->s_rxn.size());
   // a cluster's blocks exchange a value each through the items of the slot's
   // partial derivatives and rates, of which there are at least R
-  if (ts.size() == 1 && ts[0]->R >= kMaxCluster)
-    m->attempt_work = ts[0]->lu_fma + 3 * ts[0]->solve_fma + (int64_t)ts[0]->jt_idx.size() +
-                      2 * (int64_t)ts[0]->s_rxn.size();
+  m->may_cluster = ts.size() == 1 && ts[0]->R >= kMaxCluster;
   *out = m;
   return FO_OK;
 }
@@ -340,11 +342,11 @@ int team_of(int grid) {
 // per SM) 110.4 and 108.4; 8,192 (1.7) 114 and 122; 9,600 119 and 160; 13,000
 // 163 and 218; 16,384 206 and 305; 65,536 716 and 1135; settled, 65,536 cells
 // 107 and 137, 100,000 (more groups than slots) 208 and 218; TS1 settled, 8,200
-// cells 4.37 and 4.69, 65,536 23.1 and 33.3.
-bool rounds_pay(int grid) {
-  const int sms = device_sms();
-  return sms > 0 && 2 * (int64_t)grid > 3 * (int64_t)sms;
-}
+// cells 4.37 and 4.69, 65,536 23.1 and 33.3. The code of a small mechanism
+// stays in the instruction cache by itself (9,000 cells cold, ms: 20/40, 1,435
+// operations, 1.52 and 1.44; 36/75, 4,130, 2.13 and 2.03; 48/100, 7,330, 5.00
+// and 5.61).
+constexpr int64_t kRoundsWork = 5000;
 
 // Blocks per cluster for a launch of `grid` groups on teams of kBlockWarps
 // warps: the largest of 8, 4 and 2 with which all clusters are resident at
@@ -375,7 +377,7 @@ cudaLaunchConfig_t cluster_config(int grid, int blocks, cudaStream_t stream, cud
 
 int cluster_of(GenModule* m, const void* fn, int grid) {
   int dev = 0;
-  if (m->attempt_work < kClusterWork || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+  if (!m->may_cluster || m->attempt_work < kClusterWork || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
   std::lock_guard<std::mutex> lock(m->mutex);
   for (int i = 3; i > 0; --i) {
     int& known = m->clusters[dev][i];
@@ -396,7 +398,10 @@ int cluster_of(GenModule* m, const void* fn, int grid) {
 
 }  // namespace
 
-bool gen_rounds_pay(int grid) { return rounds_pay(grid); }
+bool gen_rounds_pay(const GenModule* m, int grid) {
+  const int sms = device_sms();
+  return m->attempt_work >= kRoundsWork && sms > 0 && 2 * (int64_t)grid > 3 * (int64_t)sms;
+}
 
 cudaError_t gen_launch(GenModule* m, const SolveParams& p, int grid, size_t smem, cudaStream_t stream) {
   const void* fn = reinterpret_cast<const void*>(m->kernel);

@@ -35,6 +35,6 @@ cudaError_t gen_launch_multi(GenModule* m, const SolveParams* batches, int nb, c
                              int32_t* queue, double* scratch, int64_t slot_doubles, int grid, size_t smem,
                              cudaStream_t stream);
 // Whether lockstep rounds pay for a launch of `grid` blocks.
-bool gen_rounds_pay(int grid);
+bool gen_rounds_pay(const GenModule* m, int grid);
 
 }  // namespace fo

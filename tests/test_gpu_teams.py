@@ -142,13 +142,15 @@ def test_few_reactions_and_many_species(cuda):
 @pytest.mark.parametrize("slots", [0, 700])
 def test_rounds_with_groups_that_end_early(cuda, slots):
     """Groups that fail in the middle of a round (a NaN rate constant), cold
-    and settled ones, one block per group and a queue that blocks join with
-    one group after another: the bits of a run without rounds."""
+    and settled ones, one block per group (more than are resident, so that
+    blocks join rounds under way) and a queue: the bits of a run without
+    rounds."""
     from fastode_gb300 import Algorithm, synthetic as syn
     from fastode_gb300.batch import Batch
     torch = cuda
-    groups = 1500
-    wl = syn.plain_small(n_cells=32 * groups, intervals=2)
+    groups = 2600
+    sm = syn.synthetic_mechanism(48, 100, 3)
+    wl = syn.Workload("ros3-48x100", sm, syn.synthetic_cells(sm, 32 * groups, 5), 30.0, 2, 1.0e-3, 32, False)
     at = torch.from_numpy(wl.atol).cuda()
     k = [torch.from_numpy(np.ascontiguousarray(wl.k_at(i).T)).cuda() for i in range(2)]
     k[1] = k[1].clone()
