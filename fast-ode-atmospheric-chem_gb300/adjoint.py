@@ -96,7 +96,8 @@ def forward_record(mech, Y0, k_of, dt, atol, rtol, intervals, group_size=32, alg
 def _workspace(traj: Trajectory, keep: bool = False):
     """The adjoint's workspace; with `keep`, one that holds every replayed step
     for the reverse sweep when that takes at most an eighth of the memory the
-    device has free (the gradients are the same either way)."""
+    device has free and torch can allocate it (the gradients are the same
+    either way)."""
     import torch
     b = traj.batch
     dev = b.Y.device
@@ -110,7 +111,12 @@ def _workspace(traj: Trajectory, keep: bool = False):
         kept = size("fo_adjoint_kept_bytes")
         free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
         if kept <= free // 8:
-            return torch.empty(kept, dtype=torch.uint8, device=dev)
+            # free memory says nothing of a cap on the process or of a cache in
+            # fragments: where torch refuses, the small workspace serves
+            try:
+                return torch.empty(kept, dtype=torch.uint8, device=dev)
+            except torch.cuda.OutOfMemoryError:
+                pass
     return torch.empty(size("fo_adjoint_workspace_bytes"), dtype=torch.uint8, device=dev)
 
 
