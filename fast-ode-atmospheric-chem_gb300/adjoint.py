@@ -94,8 +94,9 @@ def forward_record(mech, Y0, k_of, dt, atol, rtol, intervals, group_size=32, alg
 
 
 def _workspace(traj: Trajectory, keep: bool = False):
-    """The adjoint's workspace; with `keep`, one that holds every replayed step
-    for the reverse sweep when that takes at most an eighth of the memory the
+    """The adjoint's workspace; with `keep` and the generated kernel (the others
+    compute every step again), one that holds every replayed step for the
+    reverse sweep when that takes at most an eighth of the memory the
     device has free and torch can allocate it (the gradients are the same
     either way)."""
     import torch
@@ -107,7 +108,7 @@ def _workspace(traj: Trajectory, keep: bool = False):
         _abi.check(getattr(_abi.lib(), name)(b.plan.handle, b.ngroups, b.max_cells, traj.max_steps, C.byref(need)), name)
         return int(need.value)
 
-    if keep:
+    if keep and b.opts.variant == _abi.VARIANTS["generated"]:
         kept = size("fo_adjoint_kept_bytes")
         free = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
         if kept <= free // 8:

@@ -57,3 +57,10 @@ def test_small_workspace_when_the_large_one_is_refused(ask):
     fragments: a refused allocation must not fail a call that the small
     workspace serves."""
     assert ask(8 * KEPT, KEPT - 1) == PLAIN
+
+
+@pytest.mark.parametrize("variant", ["compact", "pipelined", "plain"])
+def test_only_the_generated_adjoint_keeps_steps(ask, variant):
+    """The table-driven kernels compute every step again whatever the
+    workspace, so they get the small one."""
+    assert ask(8 * KEPT, KEPT, variant) == PLAIN
