@@ -127,11 +127,14 @@ class _Staging:
     its leading part) and the group's workspace. A call owns its buffers from
     ``take`` to ``give``, after its stream has finished with them, so calls on
     other threads and streams get others; a call that raises drops them. At
-    most KEEP idle sets stay with a plan. With an allocation and a copy per
-    array, a settled interval of one 20-species group took 696 us, of which
-    the kernel is about 100; now 172."""
+    most KEEP idle sets stay with a plan, and of those with a workspace above
+    LARGE bytes (a group of 32 cells of 210 species and 500 reactions takes
+    4.2 MB, one of 256 cells 33 MB) only the last. With an allocation and a
+    copy per array, a settled interval of one 20-species group took 696 us, of
+    which the kernel is about 100; now 172."""
 
     KEEP = 4
+    LARGE = 8 << 20
 
     def __init__(self, plan, C_cells, rows):
         import torch
@@ -164,6 +167,8 @@ class _Staging:
 
     def give(self, plan):
         with plan.staging_lock:
+            if self.ws.numel() > self.LARGE:
+                plan.staging[:] = [st for st in plan.staging if st.ws.numel() <= self.LARGE]
             plan.staging.append(self)
             del plan.staging[:-self.KEEP]
 
