@@ -2199,6 +2199,9 @@ __device__ void solve_group_algorithm(const SolveParams& p, int g, double* scr, 
       if (isnan(err) || isinf(err)) {
         trace_record(p, g, nrec, t, H, err, -1.0);
         status = FO_STATUS_NAN_OR_INF;
+        // the round ends here too: half of one carried to the block's next
+        // group would put that one's solves among the others' factorizations
+        if (pace.state != nullptr) round_advance(pace, p.round_cost - to_solves);
         break;
       }
       if (err < 1.0 && shortened) {
