@@ -724,7 +724,6 @@ __device__ __forceinline__ bool solves_in_place(const SolveParams& p) {
 // loops are a few kilobytes of code, so the warps of an SM share them in the
 // instruction cache wherever each of them is.
 constexpr int kDB = kDenseBlock;
-constexpr int kDensePanel = 2;   // of a block's team (dense_lu_team)
 
 __device__ __forceinline__ double* dense_block(double* a, int nb, int bi, int bj) {
   return a + (int64_t)(bi * nb + bj) * kDB * kDB * 32;
@@ -819,36 +818,33 @@ __device__ __forceinline__ void block_factor(double (&c)[kDB][kDB]) {
   }
 }
 
-// A team, `panel` pivot blocks at a time. Step s updates its row and column of
-// blocks with the pivots of its panel before it, one warp per block, and the
-// warp of the diagonal block factors that; after a barrier the others take the
-// step's own pivots. The step that begins a panel updates all remaining blocks
-// with the last panel's. A sub-partition issues one DFMA in 64 cycles or more
-// whichever of its warps it comes from, so what counts is how evenly a step's
-// blocks fill four sub-partitions: left-looking (one panel of all) the last
-// steps have 1, 3, 5, ... blocks, with the most updates each, and the 506
-// updates of 12 x 12 blocks take the time of 644; in panels of two, of 524.
-// 4,096 cells of 210/500, recorded and reversed (one team of 16 per SM): 180.6
-// ms left-looking, 172.2 in panels of two (one: 172.4, three: 168.8 in runs
-// where two took 168.7); 8,192 cells of 120/260, three host intervals: 9.97 and
-// 9.58 ms (9.40, 9.64). A cluster's barrier is dear and its sub-partitions
-// are many, so it takes panels of one.
-__device__ __noinline__ void dense_lu_team(double* a, int nb, int panel) {
+// A team, right-looking. Step s updates every block that remains with the
+// pivots of the block before it, one warp per block, and the warp of the
+// diagonal block factors that; after a barrier the others of its row and column
+// take the step's own pivots. A sub-partition issues one DFMA in 64 cycles or
+// more whichever of its warps it comes from, so what counts is how evenly a
+// step's blocks fill four sub-partitions: left-looking the last steps have 1,
+// 3, 5, ... blocks, with the most updates each, and the 506 updates of 12 x 12
+// blocks take the time of 644. 4,096 cells of 210/500, recorded and reversed
+// (one team of 16 per SM): 180.6 ms left-looking, 172.4 right-looking. Panels of
+// two pivot blocks, which load and store a block half as often, gain nothing
+// beyond the runs' spread. With and without them, ms: the same adjoint 168.2 and
+// 169.5 (runs of one side differ by 0.9%), three host intervals of 8,192 cells of
+// 120/260 9.02 and 8.94, two intervals of TS1 on 8,200 cells 7.75 and 7.68, one
+// 210/500 group on a cluster 27.3 and 25.5.
+__device__ __noinline__ void dense_lu_team(double* a, int nb) {
   const int64_t ustep = (int64_t)nb * kDB * kDB * 32;
   const int w = TEAM_W, wn = TEAM_N;
 #pragma unroll 1
   for (int s = 0; s < nb; ++s) {
-    // a step that begins a panel updates every remaining block with the last
-    // panel's pivots; the others only their own row and column of blocks
-    const int in = s % panel, from = in ? s - in : s > 0 ? s - panel : 0;
-    const int m = nb - s, count = s == 0 ? 1 : in ? 2 * m - 1 : m * m;
+    const int m = nb - s, count = s > 0 ? m * m : 1, before = s > 0 ? s - 1 : 0;
 #pragma unroll 1
     for (int q = w; q < count; q += wn) {
-      const int bi = s + (!in ? q / m : q & 1 ? (q + 1) / 2 : 0), bj = s + (!in ? q % m : q & 1 ? 0 : q / 2);
+      const int bi = s + q / m, bj = s + q % m;
       double* t = dense_block(a, nb, bi, bj);
       double c[kDB][kDB];
       block_load(t, c);
-      block_update(c, dense_block(a, nb, bi, from), dense_block(a, nb, from, bj), s - from, ustep);
+      block_update(c, dense_block(a, nb, bi, before), dense_block(a, nb, before, bj), s - before, ustep);
       if (q == 0) block_factor(c);
       block_store(t, c);
     }
@@ -896,7 +892,7 @@ __device__ __noinline__ void dense_lu_warp(double* a, int nb) {
 
 __device__ __forceinline__ void dense_lu(double* a, int nb) {
   if (TEAM_N == 1) dense_lu_warp(a, nb);
-  else dense_lu_team(a, nb, cluster_team() ? 1 : kDensePanel);
+  else dense_lu_team(a, nb);
 }
 #endif
 
