@@ -192,7 +192,6 @@ struct GenModule {
   cudaKernel_t multi_kernel = nullptr;  // fo_generated_multi_kernel
   cudaKernel_t adjoint_kernel = nullptr;  // fo_generated_adjoint_kernel
   std::mutex mutex;
-  int configured_smem[3][64] = {};
   int64_t attempt_work = 0;               // FP64 operations of an attempt (the largest mechanism's)
   bool may_cluster = false;
   int clusters[64][4] = {};               // resident clusters of 2^i blocks, plus one (0: not asked yet)
@@ -292,23 +291,6 @@ void gen_destroy(GenModule* m) {
 
 namespace {
 
-// The dynamic shared-memory limit above 48 KB, set once per kernel, device
-// and size under the module's lock.
-cudaError_t ensure_smem(GenModule* m, int which, const void* fn, size_t smem) {
-  if (smem <= 48 * 1024) return cudaSuccess;
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  std::lock_guard<std::mutex> lock(m->mutex);
-  if ((int)smem > m->configured_smem[which][dev]) {
-    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    m->configured_smem[which][dev] = (int)smem;
-  }
-  return cudaSuccess;
-}
-
 // Multiprocessors of the current device, or 0.
 int device_sms() {
   int dev = 0, sms = 0;
@@ -405,8 +387,6 @@ bool gen_rounds_pay(const GenModule* m, int grid) {
 
 cudaError_t gen_launch(GenModule* m, const SolveParams& p, int grid, size_t smem, cudaStream_t stream) {
   const void* fn = reinterpret_cast<const void*>(m->kernel);
-  cudaError_t e = ensure_smem(m, 0, fn, smem);
-  if (e != cudaSuccess) return e;
   SolveParams q = p;
   void* args[] = {&q};
   const int team = team_of(grid);
@@ -423,8 +403,6 @@ cudaError_t gen_launch(GenModule* m, const SolveParams& p, int grid, size_t smem
 
 cudaError_t gen_launch_adjoint(GenModule* m, const AdjParams& a, int grid, size_t smem, cudaStream_t stream) {
   const void* fn = reinterpret_cast<const void*>(m->adjoint_kernel);
-  cudaError_t e = ensure_smem(m, 2, fn, smem);
-  if (e != cudaSuccess) return e;
   AdjParams q = a;
   void* args[] = {&q};
   return cudaLaunchKernel(fn, dim3(grid), dim3(32, team_of(grid)), args, smem, stream);
@@ -434,9 +412,7 @@ cudaError_t gen_launch_multi(GenModule* m, const SolveParams* batches, int nb, c
                              int32_t* queue, double* scratch, int64_t slot_doubles, int grid, size_t smem,
                              cudaStream_t stream) {
   const void* fn = reinterpret_cast<const void*>(m->multi_kernel);
-  cudaError_t e = ensure_smem(m, 1, fn, smem);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(queue, 0, sizeof(int32_t), stream);
+  cudaError_t e = cudaMemsetAsync(queue, 0, sizeof(int32_t), stream);
   if (e != cudaSuccess) return e;
   void* args[] = {&batches, &nb, &starts, &queue, &scratch, &slot_doubles};
   return cudaLaunchKernel(fn, dim3(grid), dim3(32, team_of(grid)), args, smem, stream);
