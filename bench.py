@@ -746,13 +746,15 @@ def run_extras(args):
 
 def run_reference(args, rank, world):
     """The reference's CPU path on every host core: the reference's own
-    Algorithm(ROS3).solve from its installation in baseline/_ref (the oracle's
-    restatement when it is not installed); each step advances one group per
-    worker by one interval."""
+    Algorithm(ROS3).solve from its installation in baseline/_ref; each step
+    advances one group per worker by one interval. Without the installation
+    there is no code of the reference to time, and the line says so."""
     import multiprocessing as mp
     workers = args.cpu_workers or os.cpu_count()
     ctx = mp.get_context("spawn")
-    from oracle.pool import GroupPool
+    from oracle.pool import GroupPool, reference_installed
+    if not reference_installed():
+        return {"impl": "reference", "unavailable": "the reference is not installed in baseline/_ref"}
     with GroupPool(ctx, workers, args.cells) as pool:
         kind = pool.kind
         for i in range(args.warmup):
@@ -771,9 +773,8 @@ def run_reference(args, rank, world):
         "impl": "reference",
         "cpu_baseline": {"value": value, "unit": "cell-intervals/s", "cores": workers, "kind": kind,
                          "sample": f"{workers} groups of 32 cells (one per process), each step one interval "
-                                   f"of each, from the initial state; "
-                                   + ("the unmodified reference installed in baseline/_ref" if kind == "reference"
-                                      else "the oracle's restatement of the reference")},
+                                   f"of each, from the initial state; the unmodified reference installed in "
+                                   f"baseline/_ref"},
         "e2e": {"value": value, "unit": "cell-intervals/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
 

@@ -73,7 +73,7 @@ def _worker(conn, group, n_cells):
             Y, mem, counts, interval = fresh()
             conn.send("ok")
         else:
-            conn.send(tuple(counts.as_dict().values()))
+            conn.send("ok")
             return
 
 
