@@ -590,10 +590,9 @@ int fo_multi_prepare(int32_t nb, const fo_batch_desc* b, void* workspace, size_t
   m->d_queue = reinterpret_cast<int32_t*>(ws);
   m->d_scratch = reinterpret_cast<double*>(ws + L.scratch_off);
   m->slot_doubles = L.items * L.lanes;
-  // lockstep rounds when every batch asks for them and runs the generated
-  // Algorithm loop;
-  // each batch makes as many attempts per round as the largest mechanism's
-  // attempt costs over its own (LU and three solves), at least one
+  // lockstep rounds when every batch asks for them, runs the generated
+  // Algorithm loop and they pay; an attempt counts as the share of a round
+  // that it costs of the largest mechanism's (LU and three solves)
   bool lockstep = ngen == nb;
   int64_t cost_max = 1;
   for (int j = 0; j < nb; ++j) {

@@ -7,7 +7,8 @@
 // fastode/solvers.py:89-97. For each group, one block replays that map from the
 // interval's checkpoint, keeping the state at the start of every step, then
 // walks the steps backwards: it recomputes the step (Jacobian, factorization,
-// stages) and runs the reverse stage sweep
+// stages; the generated kernel keeps those of the replay where the workspace has
+// room) and runs the reverse stage sweep
 //
 //   mu_r   = A^-T Kbar_r                      (transposed solves with the same LU)
 //   Fbar  += mu_r, Kbar_s += (c_rs/h) M mu_r  (s < r)

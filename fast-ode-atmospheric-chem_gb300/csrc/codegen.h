@@ -14,7 +14,7 @@
 namespace fo {
 
 // Segments of a step of generated work: the most warps of a team that a step
-// can use.
+// can use (half of those of a cluster of eight blocks).
 constexpr int kSegments = 64;
 
 // Warps of a block; a larger team is a cluster of blocks of this many.

@@ -82,7 +82,9 @@ struct DevOptions {
 // block and two columns of operands fit the 128 registers of a thread.
 constexpr int kDenseBlock = 6;
 
-// The most blocks of a cluster that work on one group.
+// The most blocks of a cluster that work on one group. A cluster of eight has
+// 128 warps, twice the segments of a generated step (kSegments in codegen.h):
+// blocks 4 to 7 work in the loops over species and blocks alone.
 constexpr int kMaxCluster = 8;
 
 // Per-lane scratch layout, in items (each item is `lanes` doubles).

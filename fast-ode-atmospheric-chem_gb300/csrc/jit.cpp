@@ -5,9 +5,9 @@
 //
 // nvJitLink is opened at run time (dlopen), so the library loads on hosts
 // without it; fo_plan_generate then fails with a clear message. Linking runs
-// ptxas on the generated code, which takes about a minute for a
-// 210-species / 500-reaction mechanism (200,000 multiply-adds of straight-line
-// code); the cache makes that a one-time cost per mechanism and host.
+// ptxas on the generated code, some seconds on 16 cores for a 210-species /
+// 500-reaction mechanism (200,000 multiply-adds); the cache makes that a
+// one-time cost per mechanism and host.
 #include "jit.h"
 
 #include <cuda_runtime.h>
@@ -325,17 +325,18 @@ int team_of(int grid) {
 // 163 and 218; 16,384 206 and 305; 65,536 716 and 1135; settled, 65,536 cells
 // 107 and 137, 100,000 (more groups than slots) 208 and 218; TS1 settled, 8,200
 // cells 4.37 and 4.69, 65,536 23.1 and 33.3. The code of a small mechanism
-// stays in the instruction cache by itself (9,000 cells cold, ms: 20/40, 1,435
-// operations, 1.52 and 1.44; 36/75, 4,130, 2.13 and 2.03; 48/100, 7,330, 5.00
-// and 5.61).
+// stays in the instruction cache by itself (9,000 cells cold, ms, synthetic
+// mechanisms of seed 3, the larger two with third bodies: 20/40, 1,435
+// operations (attempt_work), 1.52 and 1.44; 36/75, 4,130, 2.13 and 2.03; 48/100,
+// 7,330, 5.00 and 5.61).
 constexpr int64_t kRoundsWork = 5000;
 
 // Blocks per cluster for a launch of `grid` groups on teams of kBlockWarps
 // warps: the largest of 8, 4 and 2 with which all clusters are resident at
 // once, or one. A cluster's barrier and the operands' way through L2 cost
 // about 2,200 cycles a step (a block's barrier 45, its operands come from L1),
-// so a mechanism with little work per attempt stays on one SM: 20/40 (1,600
-// operations) does, TS1 (21,000) does not. One SM and a cluster, measured: a
+// so a mechanism with little work per attempt (attempt_work) stays on one SM:
+// 20/40 (1,064 to 1,623 operations by its seed) does, TS1 (20,867) does not. One SM and a cluster, measured: a
 // cold interval of one 210/500 group 66.5 and 32.0 ms, eight intervals of TS1
 // on two groups 34.4 and 25.8 ms (both with the leading rows' tasks split);
 // two Newton iterations of backward Euler on 42 groups of 120/260 (clusters of
