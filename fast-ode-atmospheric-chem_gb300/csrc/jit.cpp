@@ -336,11 +336,11 @@ constexpr int64_t kRoundsWork = 5000;
 // once, or one. A cluster's barrier and the operands' way through L2 cost
 // about 2,200 cycles a step (a block's barrier 45, its operands come from L1),
 // so a mechanism with little work per attempt (attempt_work) stays on one SM:
-// 20/40 (1,064 to 1,623 operations by its seed) does, TS1 (20,867) does not. One SM and a cluster, measured: a
-// cold interval of one 210/500 group 66.5 and 32.0 ms, eight intervals of TS1
-// on two groups 34.4 and 25.8 ms (both with the leading rows' tasks split);
-// two Newton iterations of backward Euler on 42 groups of 120/260 (clusters of
-// 2) 1.42 and 1.23 ms.
+// 20/40 (1,064 to 1,623 operations by its seed) does, TS1 (20,867) does not.
+// One SM and a cluster, measured: a cold interval of one 210/500 group 66.5 and
+// 32.0 ms, eight intervals of TS1 on two groups 34.4 and 25.8 ms (both with the
+// leading rows' tasks split); two Newton iterations of backward Euler on 42
+// groups of 120/260 (clusters of 2) 1.42 and 1.23 ms.
 constexpr int64_t kClusterWork = 10000;
 constexpr size_t kClusterSmem = sizeof(double) * (32 + 32 * kBlockWarps);
 
