@@ -37,17 +37,30 @@ sys.path.insert(0, str(ROOT))
 METRIC = "cell-intervals/s at rtol=1e-3 on 1 GB300 vs plain GPU + CPU ref; adjoint/forward cost"
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per algorithmic
-# FLOP of the integrator kernel on this workload, by kernel variant, from ncu
-# captures (profiles/): the bench reports this ratio times its own FLOPs per
-# launch as `roofline.traffic`. compact: the first two timed launches of
-# `bench.py --kernel compact --steps 2 --warmup 3 --no-cpu --e2e-steps 0
-# --plain-steps 0` (3.590 TB over 0.799 PFLOP; the traffic is dominated by the
-# elimination's U operands, 8 bytes per 2-FLOP update, so it scales with the
-# FLOPs). generated: the two timed launches of `bench.py --cells 8192 --steps 2
-# --warmup 3 --no-cpu --e2e-steps 0 --plain-steps 0 --no-extras` (197.0 GB over
-# 99.9 GFLOP), a case small enough for the capture, scaled by the FLOPs. A
-# variant without a calibration reports no traffic.
-DRAM_BYTES_PER_FLOP = {"compact": 4.491, "generated": 1.972}
+# FLOP of the integrator kernel, by kernel variant, from one-pass ncu captures of
+# full-size launches (profiles/): the bench reports this ratio times its own
+# FLOPs per launch as `roofline.traffic`. Plain workload: the first two timed
+# launches of `bench.py --steps 2 --warmup 3 --no-cpu --e2e-steps 0
+# --plain-steps 0`, with --kernel compact 3.590 TB over 0.799 PFLOP, generated
+# 2.307 TB over 0.799 PFLOP. Batched workload: the two timed launches of
+# `bench.py --workload batched --cells 1048576 --steps 2 --warmup 3`, generated
+# 13.722 TB over 4.716 PFLOP. The traffic is dominated by the elimination's
+# operands, so it scales with the FLOPs of launches of that shape. The
+# generated kernel's hold for one warp per group, which launches of more than
+# eight groups per SM take (8,192 cells of the plain workload, teams of eight:
+# 2.20). Without a calibration no traffic is reported.
+DRAM_BYTES_PER_FLOP = {"plain": {"compact": 4.491, "generated": 2.886}, "batched": {"generated": 2.909}}
+
+
+def dram_traffic(workload, kernel, groups, flops):
+    """Estimated DRAM bytes of a launch over `groups` groups with `flops`
+    algorithmic FLOPs, or None where no calibration applies."""
+    import torch
+    ratio = DRAM_BYTES_PER_FLOP[workload].get(kernel)
+    one_warp = groups > 8 * torch.cuda.get_device_properties(0).multi_processor_count
+    return ratio * flops if ratio and (one_warp or kernel != "generated") else None
+
+
 # the integrator kernel of each variant, as ncu names it
 KERNEL_NAME = {"generated": "fo_generated_solve_kernel"}
 
@@ -335,6 +348,7 @@ def run_ours(args, rank, world):
     flops = algorithmic_flops(batch.plan, counts, batch.offsets_host)
     kernel_s = sum(solve_ms) / 1e3
     achieved = flops / kernel_s / 1e12
+    traffic = dram_traffic("plain", args.kernel, batch.ngroups, flops / args.steps)
     peak = 2.0 * fma_rate.value / 1e12
     value = job_value(Cc * args.steps, world, elapsed)
 
@@ -403,13 +417,12 @@ def run_ours(args, rank, world):
             "rejected": float(counts[:, 2].sum() / len(counts) / args.steps)},
         "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                      "frac": achieved / peak,
-                     "traffic": (DRAM_BYTES_PER_FLOP[args.kernel] * flops / args.steps
-                                 if args.kernel in DRAM_BYTES_PER_FLOP else None),
+                     "traffic": traffic,
                      "traffic_unit": "bytes per launch",
-                     "traffic_source": (f"ncu DRAM bytes per algorithmic FLOP of this kernel on this workload "
-                                        f"({DRAM_BYTES_PER_FLOP[args.kernel]} B/FLOP, measured on an 8,192-cell case) "
-                                        "times this run's FLOPs per launch" if args.kernel in DRAM_BYTES_PER_FLOP else
-                                        "not calibrated for this kernel variant"),
+                     "traffic_source": ("not calibrated for this launch" if traffic is None else
+                                        f"ncu DRAM bytes per algorithmic FLOP of this kernel on this workload "
+                                        f"({DRAM_BYTES_PER_FLOP['plain'][args.kernel]} B/FLOP over its first two "
+                                        f"intervals) times this run's FLOPs per launch"),
                      "kernel": KERNEL_NAME.get(args.kernel, "solve_kernel"),
                      "kernel_ms_per_launch": sum(solve_ms) / len(solve_ms),
                      "peak_source": "fo_fp64_fma_rate: full-warp DFMA kernel, same GPU, same run (the driver's "
@@ -546,9 +559,8 @@ def run_batched(args):
             "autotune": tuning,
             "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                          "frac": achieved / peak,
-                         "traffic": (DRAM_BYTES_PER_FLOP[kernel] * flops / args.steps
-                                     if kernel in DRAM_BYTES_PER_FLOP else None),
-                         "traffic_unit": "bytes per interval (the 210/500 ratio; smaller mechanisms stream less)",
+                         "traffic": dram_traffic("batched", kernel, sum(p.ngroups for p in parts), flops / args.steps),
+                         "traffic_unit": "bytes per interval",
                          "time": "CUDA events around the graph replays of the timed intervals",
                          "peak_source": "fo_fp64_fma_rate, same GPU, same run"}}
 
