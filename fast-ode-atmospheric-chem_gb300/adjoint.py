@@ -160,7 +160,9 @@ def replay(traj: Trajectory, Y0=None, ks=None):
 
 def adjoint(traj: Trajectory, lam_final):
     """dL/dY0 ((n, C)) and dL/dlog k per cell ((R, C), summed over intervals)
-    from dL/dY at the end ((n, C) device)."""
+    from dL/dY at the end ((n, C) device). The workspace (``_workspace``, up to
+    an eighth of the free memory) goes back to torch's cache, from where
+    ``torch.cuda.empty_cache()`` returns it to the device."""
     import torch
     b = traj.batch
     ws = _workspace(traj, keep=True)

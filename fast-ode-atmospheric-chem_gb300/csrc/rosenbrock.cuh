@@ -1007,7 +1007,7 @@ __device__ __forceinline__ void generated_solve(const SolveParams& p, double* ba
 
 // x = A^-1 b in place on the solve vector by the whole team. A solve is a chain
 // of small steps: one block of a cluster with its own barriers and L1 is
-// faster than all of them (210/500: 0.32 M cycles and 0.38 M).
+// faster than all of them (a solve of 210/500: 0.32 M cycles and 0.38 M).
 template <bool kProjection>
 __device__ __forceinline__ void team_solve(const SolveParams& p, double* base) {
   if (cluster_team()) {
